@@ -239,3 +239,30 @@ def test_slot_downlink_from_information_bits():
     assert mb.ops.device_error() == 0
     assert a.abs().max().item() > 0
     assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("Z,stride_pad", [(2, 0), (7, 1), (24, 2), (31, 0), (36, 3), (64, 0), (104, 5), (352, 1)])
+def test_encoder_odd_lifting_sizes_and_strides(Z, stride_pad):
+    """Columns that share words, columns shorter than a word and rows that
+    start on any byte, against the restated encoder."""
+    mb = _mb()
+    entries = _big_graph(Z, seed=3)
+    kb = ldpc.KB[1]
+    g = ldpc.Graph(entries, kb, Z, 17)
+    rng = np.random.default_rng(Z)
+    info = rng.integers(0, 2, (3, kb * Z), dtype=np.uint8)
+    packed = np.packbits(info, axis=-1)
+    # the unused bits of the last byte and the row padding are set: not read
+    rows = np.full((3, packed.shape[1] + stride_pad), 0xFF, np.uint8)
+    rows[:, :packed.shape[1]] = packed
+    if kb * Z % 8:
+        rows[:, packed.shape[1] - 1] |= 0xFF >> (kb * Z % 8)
+    code = mb.Ldpc(entries, kb, Z, 17)
+    n = (code.cw_bits + 7) // 8
+    out = torch.full((3, n + stride_pad), 0xA5, dtype=torch.uint8, device="cuda")
+    code.encode(torch.from_numpy(rows).cuda(), out=out)
+    torch.cuda.synchronize()
+    got = out.cpu().numpy()
+    assert (got[:, n:] == 0xA5).all()
+    want = np.stack([np.packbits(ldpc.encode(g, info[k])[2 * Z:]) for k in range(3)])
+    np.testing.assert_array_equal(got[:, :n], want)
