@@ -45,8 +45,7 @@ typedef enum {
   MB_TIMEOUT = 5,      /* a bounded device-side wait gave up */
   MB_NO_MEMORY = 6,    /* create-time allocation failed */
   MB_UNSUPPORTED = 7,  /* valid request this build does not implement */
-  MB_TOO_LARGE = 8     /* request needs more than mb_equalize_tc_noalloc's
-                          fixed scratch */
+  MB_TOO_LARGE = 8     /* request beyond mb_equalize_tc_noalloc's limit */
 } mb_status;
 
 typedef enum {
@@ -278,7 +277,9 @@ mb_status mb_equalize(const mb_c32 *W, const mb_c32 *y, uint32_t K,
  * same contract and outputs as mb_equalize): BF16 W and y, FP32
  * accumulation (tcgen05.mma), the same FP16 demapper and layouts.  The
  * caller provides two device scratch buffers whose sizes
- * mb_equalize_tc_scratch returns.  Requires sg % 8 == 0 and K <= 64. */
+ * mb_equalize_tc_scratch returns (neither may be NULL; this build rounds W
+ * and y to BF16 on their way into shared memory and leaves the buffers as
+ * they are).  Requires sg % 8 == 0 and K <= 64. */
 mb_status mb_equalize_tc_scratch(uint32_t K, uint32_t M, uint32_t S,
                                  uint32_t sg, uint32_t n_sym,
                                  uint64_t *img_bytes, uint64_t *ylp_bytes);
@@ -293,25 +294,20 @@ mb_status mb_equalize_tc(const mb_c32 *W, const mb_c32 *y, uint32_t K,
  * memory (no counterpart in the reference): hosts whose real-time threads
  * may not enter the driver's allocator, or whose device memory is fixed at
  * start-up by a framework that owns every allocation.  Inputs, outputs and
- * results are those of mb_equalize_tc, but the scratch lives in one 32 MiB
- * array compiled into the library (held by every device that loads it until
- * the process exits), so the caller passes no scratch and nothing is
- * allocated or freed.  Limit: the BF16 detector images of all groups plus
- * the BF16 rows of one symbol, 4*M*ceil8(S) bytes, must fit in 32 MiB;
- * larger requests return MB_TOO_LARGE (e.g. 256 antennas x 32 users with
- * 3276 subcarriers fits; symbols beyond what fits are processed in turn).
- * The first call on each device looks the array's device address up with
- * cudaGetSymbolAddress (device current); make that first call before any
- * stream capture.  All calls on a device share the array and it keeps the
- * previous call's contents: calls that can overlap on the GPU (different
- * streams, other host threads) race and must be serialised by the caller.
- * Nothing in the scratch needs to start at zero: every byte a call reads was
- * written earlier in the same call.  A bounded device wait that gives up
- * sets bit 1 of an error word that is also fixed in the library (the
- * library's own word is allocated on first use); mb_device_error reports
- * and clears it together with that word.  The device addresses looked up
- * at the first call belong to the device's context: after cudaDeviceReset
- * this entry point must not be called again in the process. */
+ * results are those of mb_equalize_tc; the caller passes no scratch and
+ * nothing is allocated or freed.  Limit: the BF16 detector images of all
+ * groups plus the BF16 rows of one symbol, 4*M*ceil8(S) bytes, must fit in
+ * 32 MiB; larger requests return MB_TOO_LARGE (e.g. 256 antennas x 32 users
+ * with 3276 subcarriers fits).  The first call on each device looks the
+ * address of the entry point's error word up with cudaGetSymbolAddress
+ * (device current); make that first call before any stream capture.  Calls
+ * share nothing else, so they may overlap on the GPU.  A bounded device wait
+ * that gives up sets bit 1 of that error word, which is fixed in the library
+ * (the library's own word is allocated on first use); mb_device_error
+ * reports and clears it together with that word.  The device address looked
+ * up at the first call belongs to the device's context: after
+ * cudaDeviceReset this entry point must not be called again in the
+ * process. */
 mb_status mb_equalize_tc_noalloc(const mb_c32 *W, const mb_c32 *y, uint32_t K,
                                  uint32_t M, uint32_t S, uint32_t sg,
                                  uint32_t n_sym, uint32_t Qm, uint64_t cb_size,

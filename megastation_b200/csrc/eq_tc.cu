@@ -154,28 +154,6 @@ __global__ void __launch_bounds__(kEqThreads, 1)
   if (warp == 0) tc::tmem_dealloc(tmem, q.tmem_cols);
 }
 
-// W [G][M][K] (fp32 complex) -> the per-group A image (see top of file)
-__global__ void w_image_kernel(const float2 *W, __nv_bfloat16 *img, uint32_t M, uint32_t K,
-                               uint32_t Mp, uint32_t MM, uint32_t nkt) {
-  const uint32_t g = blockIdx.x;
-  const uint64_t per_group = (uint64_t)nkt * MM * kKT;  // elements
-  const float2 *wg = W + (uint64_t)g * M * K;
-  __nv_bfloat16 *ig = img + (uint64_t)g * per_group;
-  for (uint64_t e = threadIdx.x; e < per_group; e += blockDim.x) {
-    // e enumerates the image in memory order: kt, row group, k chunk, row, k
-    const uint32_t kin_e = e % 8, rr = (e / 8) % 8, kchunk = (e / 64) % 8;
-    const uint32_t rg = (uint32_t)((e / 512) % (MM / 8)), kt = (uint32_t)(e / (512 * (MM / 8)));
-    const uint32_t r = rg * 8 + rr, kk = kt * kKT + kchunk * 8 + kin_e;
-    const uint32_t plane = kk / Mp, b = kk % Mp, u = r / 2, ri = r & 1;
-    float v = 0.f;
-    if (u < K && b < M) {
-      const float2 w = wg[(uint64_t)b * K + u];
-      v = ri == 0 ? (plane == 0 ? w.x : -w.y) : (plane == 0 ? w.y : w.x);
-    }
-    ig[e] = __float2bfloat16_rn(v);
-  }
-}
-
 TcShape tc_shape(uint32_t M, uint32_t K) {
   TcShape s;
   s.MM = 2 * K <= 64 ? 64 : 128;
@@ -183,16 +161,6 @@ TcShape tc_shape(uint32_t M, uint32_t K) {
   s.nkt = 2 * s.Mp / kKT;
   s.img_group_bytes = (uint64_t)s.nkt * s.MM * kKT * 2;
   return s;
-}
-
-mb_status w_image(const float2 *W, void *img, uint32_t G, uint32_t M, uint32_t K,
-                  cudaStream_t st) {
-  TcShape s = tc_shape(M, K);
-  if (G == 0) return MB_OK;
-  w_image_kernel<<<G, 256, 0, st>>>(W, reinterpret_cast<__nv_bfloat16 *>(img), M, K, s.Mp,
-                                    s.MM, s.nkt);
-  MB_LAUNCH_CHECK();
-  return MB_OK;
 }
 
 using EqTcKernel = void (*)(const EqTcParams, const CUtensorMap);
@@ -280,26 +248,206 @@ mb_status equalize_tc(const EqParams &p, const void *a_img, const void *y_lp, ui
 
 namespace mb {
 
-__global__ void y_to_lp_kernel(const float2 *y, __nv_bfloat16 *ylp, uint32_t M, uint32_t S,
-                               uint32_t S_pad, uint64_t rows) {
-  for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < rows * S;
-       e += (uint64_t)gridDim.x * blockDim.x) {
-    const uint64_t row = e / S, s = e % S;  // row = sym * M + b
-    const uint64_t sym = row / M, b = row % M;
-    const float2 v = y[e];
-    ylp[((sym * 2 + 0) * M + b) * S_pad + s] = __float2bfloat16_rn(v.x);
-    ylp[((sym * 2 + 1) * M + b) * S_pad + s] = __float2bfloat16_rn(v.y);
+// ---- the same GEMM from FP32 operands (mb_equalize_tc) -------------------
+// W [G][M][K] and y [sym][M][S] are read once, as they are, and rounded to
+// BF16 on their way into shared memory: the images and planar rows that the
+// slot's FFT and ZF kernels prepare do not exist here, and writing them first
+// moved 107 MB more at the 256 x 32 cell (12 symbols, 3276 subcarriers) in two
+// more launches.  DRAM bound: 94 MB of operands and 16 MB of results there.
+// The 256 threads hold the next 32 antennas of both operands in registers
+// (about 32 KB of loads in flight per CTA, three CTAs per SM) while the tensor
+// core multiplies the previous two tiles.  One call there: 130 us with
+// the three launches, 32 us with this one (kernel 30 us, 3.6 TB/s).
+// Layouts per tile (32 antennas, planes re and im one after the other):
+//   Y: MN-major, core matrices of 8 antennas x 8 columns, antenna groups 128 B
+//      apart, column chunks kTSbo apart;
+//   A: K-major, rows 2u / 2u + 1 the real and imaginary part of user u, k
+//      core matrices 128 B apart, 8-row groups kTSbo apart.
+// kTSbo is 512 + 16 bytes so that lanes that store neighbouring chunks or row
+// groups meet different banks.  Rows past 2K of A and columns past ncols of Y
+// hold leftovers: they only reach accumulators that nothing reads.
+constexpr int kTA = 32;           // antennas per tile
+constexpr uint32_t kTSbo = 528;
+constexpr int kYUnits = 8;        // column pairs per thread and tile, at most
+constexpr uint32_t kTY = 16 * kTSbo;  // one plane of Y
+
+template <int MM, int QM>
+__global__ void __launch_bounds__(kEqThreads, MM == 64 ? 3 : 2)
+    equalize_tc_c32_kernel(const EqParams p, uint32_t l0, uint32_t nb, uint32_t spc, uint32_t N,
+                           uint32_t tmem_cols, uint32_t vw_log2, uint32_t vec, int *err) {
+  extern __shared__ __align__(128) uint8_t ec_smem[];
+  __shared__ __align__(8) uint64_t bar[2];
+  __shared__ uint32_t tmem_base_slot;
+  constexpr uint32_t a_plane = MM / 8 * kTSbo, stage_bytes = 2 * kTY + 2 * a_plane;
+  constexpr uint32_t KP = MM / 2;  // users a tile has room for
+  const uint32_t g = blockIdx.x, tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
+  const uint32_t l_off = blockIdx.y * spc, nbc = min(spc, nb - l_off), ncols = nbc * p.sg;
+  const uint32_t s_base = g * p.sg;
+  if (tid == 0) {
+    tc::mbar_init(&bar[0], 1);
+    tc::mbar_init(&bar[1], 1);
+    tc::fence_mbar_init();
   }
+  if (warp == 0) tc::tmem_alloc(&tmem_base_slot, tmem_cols);
+  tc::fence_before_sync();
+  __syncthreads();
+  tc::fence_after_sync();
+  const uint32_t tmem = tmem_base_slot;
+
+  // y: this thread's column pair v of the tile's antennas yb, yb + ystep, ...
+  const uint32_t v = tid & ((1u << vw_log2) - 1), yb = tid >> vw_log2, ystep = kEqThreads >> vw_log2;
+  const uint32_t c = 2 * v, l = c / p.sg, s = s_base + c - l * p.sg;
+  const bool y0_on = c < ncols && s < p.S, y1_on = c < ncols && s + 1 < p.S;
+  const float2 *yp = p.y + ((uint64_t)(l0 + l_off + l) * p.M + yb) * p.S + s;
+  const uint32_t y_dst = (v / 4) * kTSbo + (v % 4) * 4;
+  // W: user u, the tile's antennas 8 kc .. 8 kc + 7
+  const uint32_t u = tid % KP, kc = tid / KP;
+  const bool w_on = kc < kTA / 8 && u < p.K;
+  const float2 *wp = p.W + ((uint64_t)g * p.M + 8 * kc) * p.K + u;
+  const uint32_t a_dst = 2 * kTY + (u / 4) * kTSbo + (2 * u % 8) * 16 + kc * 128;
+
+  float4 yr[kYUnits];
+  float2 wr[8];
+  auto load = [&](uint32_t b0) {
+#pragma unroll
+    for (int j = 0; j < kYUnits; j++) {
+      yr[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+      const uint32_t b = yb + j * ystep;
+      if (b >= kTA || b0 + b >= p.M) continue;
+      const float2 *q = yp + (uint64_t)(b0 + j * ystep) * p.S;
+      if (vec && y1_on) {
+        yr[j] = __ldg(reinterpret_cast<const float4 *>(q));
+      } else {
+        if (y0_on) *reinterpret_cast<float2 *>(&yr[j].x) = __ldg(q);
+        if (y1_on) *reinterpret_cast<float2 *>(&yr[j].z) = __ldg(q + 1);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+      wr[j] = make_float2(0.f, 0.f);
+      if (w_on && b0 + 8 * kc + j < p.M) wr[j] = __ldg(wp + (uint64_t)(b0 + j) * p.K);
+    }
+  };
+  auto pack = [](float lo, float hi) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t *>(&h);
+  };
+  auto store = [&](uint8_t *st) {
+    if (c < ncols) {
+#pragma unroll
+      for (int j = 0; j < kYUnits; j++) {
+        const uint32_t b = yb + j * ystep;
+        if (b >= kTA) break;
+        uint8_t *d = st + y_dst + (b / 8) * 128 + (b % 8) * 16;
+        *reinterpret_cast<uint32_t *>(d) = pack(yr[j].x, yr[j].z);
+        *reinterpret_cast<uint32_t *>(d + kTY) = pack(yr[j].y, yr[j].w);
+      }
+    }
+    if (w_on) {
+      uint4 re, im, ng;
+      re = make_uint4(pack(wr[0].x, wr[1].x), pack(wr[2].x, wr[3].x), pack(wr[4].x, wr[5].x), pack(wr[6].x, wr[7].x));
+      im = make_uint4(pack(wr[0].y, wr[1].y), pack(wr[2].y, wr[3].y), pack(wr[4].y, wr[5].y), pack(wr[6].y, wr[7].y));
+      ng = make_uint4(im.x ^ 0x80008000u, im.y ^ 0x80008000u, im.z ^ 0x80008000u, im.w ^ 0x80008000u);
+      uint8_t *d = st + a_dst;
+      *reinterpret_cast<uint4 *>(d) = re;                  // x.re = W.re y.re - W.im y.im
+      *reinterpret_cast<uint4 *>(d + 16) = im;             // x.im = W.im y.re + W.re y.im
+      *reinterpret_cast<uint4 *>(d + a_plane) = ng;
+      *reinterpret_cast<uint4 *>(d + a_plane + 16) = re;
+    }
+  };
+
+  const uint32_t idesc = tc::idesc_bf16(kCols, N, true, false);
+  const uint32_t nt = (p.M + kTA - 1) / kTA;
+  bool ok = true;
+  load(0);
+  for (uint32_t t = 0; t < nt; t++) {
+    const uint32_t sidx = t & 1;
+    // the stage's previous tile (t - 2) must have been multiplied
+    if (t >= 2 && !tc::mbar_wait(&bar[sidx], ((t - 2) >> 1) & 1)) ok = false;
+    uint8_t *st = ec_smem + sidx * stage_bytes;
+    store(st);
+    if (t + 1 < nt) load((t + 1) * kTA);
+    tc::fence_proxy_async_smem();
+    if (__syncthreads_or(!ok)) {
+      ok = false;
+      break;
+    }
+    if (tid == 0) {
+      tc::fence_after_sync();
+      const uint32_t y0 = tc::smem_u32(st), a0 = y0 + 2 * kTY;
+#pragma unroll
+      for (int k = 0; k < 2 * (kTA / 16); k++) {
+        const uint32_t pl = k / (kTA / 16), ks = k % (kTA / 16);
+        tc::mma_f16(tmem, tc::smem_desc(y0 + pl * kTY + ks * 256, 128, kTSbo),
+                    tc::smem_desc(a0 + pl * a_plane + ks * 256, 128, kTSbo), idesc, (t | k) != 0);
+      }
+      tc::mma_commit(&bar[sidx]);
+    }
+  }
+  // the epilogue's per-thread setup overlaps the last MMAs
+  EqTcEpilogue<MM, QM> epi;
+  epi.prepare(p, s_base, l_off, ncols, l0, N, warp, lane);
+  // the last tile's commit covers every MMA issued before it
+  if (ok && !tc::mbar_wait(&bar[(nt - 1) & 1], ((nt - 1) >> 1) & 1)) ok = false;
+  if (__syncthreads_or(!ok)) {
+    if (tid == 0 && err) atomicOr(err, tc::kErrTimeout);
+  } else {
+    tc::fence_after_sync();
+    epi.run(p, tmem, warp, lane);
+  }
+  tc::fence_before_sync();
+  __syncthreads();
+  if (warp == 0) tc::tmem_dealloc(tmem, tmem_cols);
 }
 
-mb_status y_to_lp(const float2 *y, void *y_lp, uint32_t nb, uint32_t M, uint32_t S,
-                  uint32_t S_pad, cudaStream_t st) {
-  const uint64_t rows = (uint64_t)nb * M;
-  if (rows == 0) return MB_OK;
-  const unsigned blocks = (unsigned)std::min<uint64_t>((rows * S + 255) / 256, 148 * 32);
-  y_to_lp_kernel<<<blocks, 256, 0, st>>>(y, reinterpret_cast<__nv_bfloat16 *>(y_lp), M, S,
-                                         S_pad, rows);
-  MB_LAUNCH_CHECK();
+template <int MM>
+static void eq_tc_c32_launch(const EqParams &p, uint32_t l0, uint32_t nb, int *err, cudaStream_t st, bool configure,
+                             cudaError_t *e) {
+  constexpr size_t smem = 2 * (2 * (size_t)kTY + 2 * MM / 8 * (size_t)kTSbo);
+  auto k = p.Qm == 2   ? equalize_tc_c32_kernel<MM, 2>
+           : p.Qm == 4 ? equalize_tc_c32_kernel<MM, 4>
+           : p.Qm == 6 ? equalize_tc_c32_kernel<MM, 6>
+                       : equalize_tc_c32_kernel<MM, 8>;
+  if (configure) {
+    *e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    return;
+  }
+  const uint32_t N = (2 * p.K + 15) / 16 * 16;
+  uint32_t tmem_cols = 32;
+  while (tmem_cols < N) tmem_cols *= 2;
+  // symbols per CTA: as many as fill the 128 columns, spread evenly over the
+  // CTAs a group needs
+  const uint32_t spc_max = std::max<uint32_t>(1, kCols / p.sg), ny = (nb + spc_max - 1) / spc_max;
+  const uint32_t spc = (nb + ny - 1) / ny;
+  // column pairs side by side in the 256 threads: a power of two, at least
+  // the 8 with which the threads cover a tile's 32 antennas in one pass
+  uint32_t vw = 3;
+  while ((2u << vw) < spc * p.sg) vw++;
+  const uint32_t vec = p.S % 2 == 0 && (reinterpret_cast<uintptr_t>(p.y) & 15) == 0;
+  const dim3 grid((p.S + p.sg - 1) / p.sg, ny);
+  k<<<grid, kEqThreads, smem, st>>>(p, l0, nb, spc, N, tmem_cols, vw, vec, err);
+  *e = cudaGetLastError();
+}
+
+mb_status equalize_tc_c32(const EqParams &p, int *err, cudaStream_t st) {
+  if (!equalize_tc_supported(p.K, p.sg, 1)) return MB_UNSUPPORTED;
+  auto launch = p.K <= 32 ? eq_tc_c32_launch<64> : eq_tc_c32_launch<128>;
+  static std::atomic<uint64_t> configured[8] = {};
+  const int which = (p.K <= 32 ? 0 : 4) + (int)p.Qm / 2 - 1;
+  int dev = 0;
+  cudaError_t e = cudaSuccess;
+  MB_CUDA_TRY(cudaGetDevice(&dev));
+  const uint64_t bit = 1ull << (dev & 63);
+  if (!(configured[which].load() & bit)) {
+    launch(p, 0, 0, err, st, true, &e);
+    MB_CUDA_TRY(e);
+    configured[which].fetch_or(bit);
+  }
+  constexpr uint32_t kMaxSyms = 32768;  // grid.y's range
+  for (uint32_t l0 = 0; l0 < p.n_sym; l0 += kMaxSyms) {
+    launch(p, l0, std::min(kMaxSyms, p.n_sym - l0), err, st, false, &e);
+    MB_CUDA_TRY(e);
+  }
   return MB_OK;
 }
 
@@ -334,28 +482,8 @@ extern "C" mb_status mb_equalize_tc(const mb_c32 *W, const mb_c32 *y, uint32_t K
   if (!scratch_img || !scratch_ylp) return MB_BAD_ARG;
   p.x = reinterpret_cast<float2 *>(x);
   if (n_sym == 0) return MB_OK;
-  uint32_t nb_max = std::max<uint32_t>(1, 256 / sg);
-  while (nb_max > 1 && !equalize_tc_supported(K, sg, nb_max)) nb_max--;
-  if (!equalize_tc_supported(K, sg, 1) && !equalize_tc_supported(K, sg, nb_max))
-    return MB_UNSUPPORTED;
+  if (!equalize_tc_supported(K, sg, 1)) return MB_UNSUPPORTED;
   const DeviceTables *tab = device_tables();
   if (!tab) return MB_CUDA_ERROR;
-  cudaStream_t st = as_stream(stream);
-  const uint32_t G = (S + sg - 1) / sg;
-  const uint32_t S_pad = s_pad_of(S);
-  s = w_image(reinterpret_cast<const float2 *>(W), scratch_img, G, M, K, st);
-  if (s != MB_OK) return s;
-  s = y_to_lp(reinterpret_cast<const float2 *>(y), scratch_ylp, n_sym, M, S, S_pad, st);
-  if (s != MB_OK) return s;
-  for (uint32_t l0 = 0; l0 < n_sym;) {
-    uint32_t nb = std::min(nb_max, n_sym - l0);
-    while (nb > 1 && !equalize_tc_supported(K, sg, nb)) nb--;
-    if (!equalize_tc_supported(K, sg, nb)) return MB_UNSUPPORTED;
-    const uint8_t *ylp = reinterpret_cast<const uint8_t *>(scratch_ylp) +
-                         (uint64_t)l0 * 2 * M * S_pad * 2;
-    s = equalize_tc(p, scratch_img, ylp, S_pad, l0, nb, tab->err, st);
-    if (s != MB_OK) return s;
-    l0 += nb;
-  }
-  return MB_OK;
+  return equalize_tc_c32(p, tab->err, as_stream(stream));
 }

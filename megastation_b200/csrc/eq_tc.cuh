@@ -25,9 +25,6 @@ struct TcShape {
 
 TcShape tc_shape(uint32_t M, uint32_t K);
 bool equalize_tc_supported(uint32_t K, uint32_t sg, uint32_t nb);
-// W [G][M][K] c32 -> detector images
-mb_status w_image(const float2 *W, void *img, uint32_t G, uint32_t M, uint32_t K,
-                  cudaStream_t st);
 // equalize nb symbols (outputs at symbol offset l0 of p's outputs); a CTA
 // takes the symbols of one group that fit in max_cols (<= 128, 0: 128)
 // (symbol, subcarrier) columns
@@ -36,8 +33,7 @@ mb_status equalize_tc(const EqParams &p, const void *a_img, const void *y_lp, ui
 // error word of mb_equalize_tc_noalloc's kernels on the current device
 // (0 when it has not run there), cleared when clear is set
 mb_status noalloc_error_word(int *bits, bool clear);
-// y [nb][M][S] c32 -> y_lp [nb][re|im][M][S_pad] BF16
-mb_status y_to_lp(const float2 *y, void *y_lp, uint32_t nb, uint32_t M, uint32_t S,
-                  uint32_t S_pad, cudaStream_t st);
+// equalize p's n_sym symbols straight from the FP32 W and y of p
+mb_status equalize_tc_c32(const EqParams &p, int *err, cudaStream_t st);
 
 }  // namespace mb

@@ -5,11 +5,9 @@
 // real-time fronthaul thread that may not block on the driver's allocator,
 // a process whose device memory is carved up and fixed at start-up, or an
 // embedding framework that owns every allocation itself.  mb_equalize_tc
-// asks such callers for two scratch buffers; this variant instead keeps its
-// scratch (the BF16 detector images and the BF16 copy of the FFT output) in
-// one fixed array compiled into the library, so a call needs nothing but
-// its inputs and outputs.
-#include <algorithm>
+// asks such callers for two scratch buffers; this variant takes none, and its
+// error word is fixed in the library, so a call needs nothing but its inputs
+// and outputs.
 #include <mutex>
 
 #include "common.cuh"
@@ -17,24 +15,22 @@
 
 namespace {
 
-// Fixed scratch shared by every call on a device.  Each device that loads
-// the library holds these bytes until the process exits.
+// The entry point's limit: the BF16 operands of one symbol (detector images
+// of all groups and one symbol's rows) fit in 32 MiB.
 constexpr uint64_t kNoAllocScratchBytes = 32ull << 20;
-static __device__ __align__(256) uint8_t g_noalloc_scratch[kNoAllocScratchBytes];
 // The error word of this entry point's kernels (bit 1: a bounded mbarrier
-// wait gave up), kept beside the scratch because the library's own error
-// word is allocated on first use.  mb_device_error reports and clears it
+// wait gave up), fixed because the library's own error word is allocated on
+// first use.  mb_device_error reports and clears it
 // together with that word.
 static __device__ int g_noalloc_err;
 
-// Device addresses of g_noalloc_scratch and g_noalloc_err per device, looked
-// up once per device with that device current.  In host code the arrays'
-// names are only handles for the runtime, not device addresses.  The cached
-// addresses belong to the device's current context: after cudaDeviceReset
-// they are stale, and this entry point must not be called again in that
-// process (as with every other per-device table of the library).
+// Device address of g_noalloc_err per device, looked up once per device with
+// that device current.  In host code the word's name is only a handle for the
+// runtime, not a device address.  The cached address belongs to the device's
+// current context: after cudaDeviceReset it is stale, and this entry point
+// must not be called again in that process (as with every other per-device
+// table of the library).
 std::mutex g_noalloc_mu;
-void *g_noalloc_addr[64];
 int *g_noalloc_err_addr[64];
 
 }  // namespace
@@ -73,56 +69,27 @@ extern "C" mb_status mb_equalize_tc_noalloc(const mb_c32 *W, const mb_c32 *y, ui
   if (n_sym == 0) return MB_OK;
   if (!equalize_tc_supported(K, sg, 1)) return MB_UNSUPPORTED;
 
-  // scratch layout: detector images, then as many symbols of BF16 rows as fit
-  const TcShape sh = tc_shape(M, K);
-  const uint32_t G = (S + sg - 1) / sg;
-  const uint32_t S_pad = (S + 7) / 8 * 8;
-  const uint64_t img_bytes = ((uint64_t)G * sh.img_group_bytes + 255) / 256 * 256;
-  const uint64_t sym_bytes = (uint64_t)2 * M * S_pad * 2;
+  const uint64_t G = (S + sg - 1) / sg;
+  const uint64_t img_bytes = (G * tc_shape(M, K).img_group_bytes + 255) / 256 * 256;
+  const uint64_t sym_bytes = (uint64_t)2 * M * ((S + 7) / 8 * 8) * 2;
   if (img_bytes + sym_bytes > kNoAllocScratchBytes) return MB_TOO_LARGE;
-  const uint32_t sym_fit = (uint32_t)std::min<uint64_t>((kNoAllocScratchBytes - img_bytes) / sym_bytes, 1u << 20);
 
   int dev = 0;
   MB_CUDA_TRY(cudaGetDevice(&dev));
   if (dev < 0 || dev >= 64) return MB_UNSUPPORTED;
-  uint8_t *base = nullptr;
   int *err = nullptr;
   {
     std::lock_guard<std::mutex> lk(g_noalloc_mu);
-    if (!g_noalloc_addr[dev]) {
-      void *addr = nullptr, *eaddr = nullptr;
-      cudaError_t e = cudaGetSymbolAddress(&addr, g_noalloc_scratch);
-      if (e == cudaSuccess) e = cudaGetSymbolAddress(&eaddr, g_noalloc_err);
+    if (!g_noalloc_err_addr[dev]) {
+      void *eaddr = nullptr;
+      const cudaError_t e = cudaGetSymbolAddress(&eaddr, g_noalloc_err);
       if (e != cudaSuccess) {
         (void)cudaGetLastError();
         return record_error(e);
       }
       g_noalloc_err_addr[dev] = reinterpret_cast<int *>(eaddr);
-      g_noalloc_addr[dev] = addr;
     }
-    base = reinterpret_cast<uint8_t *>(g_noalloc_addr[dev]);
     err = g_noalloc_err_addr[dev];
   }
-  uint8_t *img = base;
-  uint8_t *ylp = base + img_bytes;
-
-  cudaStream_t st = as_stream(stream);
-  s = w_image(reinterpret_cast<const float2 *>(W), img, G, M, K, st);
-  if (s != MB_OK) return s;
-  uint32_t nb_max = std::max<uint32_t>(1, 256 / sg);
-  while (nb_max > 1 && !equalize_tc_supported(K, sg, nb_max)) nb_max--;
-  for (uint32_t c0 = 0; c0 < n_sym; c0 += sym_fit) {
-    const uint32_t nc = std::min(sym_fit, n_sym - c0);
-    s = y_to_lp(reinterpret_cast<const float2 *>(y) + (uint64_t)c0 * M * S, ylp, nc, M, S, S_pad,
-                st);
-    if (s != MB_OK) return s;
-    for (uint32_t j = 0; j < nc;) {
-      uint32_t nb = std::min(nb_max, nc - j);
-      while (nb > 1 && !equalize_tc_supported(K, sg, nb)) nb--;
-      s = equalize_tc(p, img, ylp + (uint64_t)j * sym_bytes, S_pad, c0 + j, nb, err, st);
-      if (s != MB_OK) return s;
-      j += nb;
-    }
-  }
-  return MB_OK;
+  return equalize_tc_c32(p, err, as_stream(stream));
 }

@@ -339,3 +339,43 @@ def test_mixed_hard_bits_match_plain_path(mb, iq_dtype):
     sent = d["bits"][..., :n_valid]
     ber_p, ber_m = np.mean(bp != sent), np.mean(bm != sent)
     assert ber_m <= ber_p + np.mean(~sure)
+
+
+@pytest.mark.parametrize("K,M,S,sg,n_sym,Qm", [
+    (1, 1, 8, 8, 1, 2), (5, 33, 101, 8, 3, 4), (7, 64, 95, 24, 5, 6), (16, 40, 200, 16, 9, 6), (31, 65, 129, 32, 2, 8),
+    (32, 96, 250, 128, 1, 4), (33, 70, 120, 40, 4, 2), (64, 256, 77, 16, 17, 6), (50, 31, 128, 64, 3, 8)])
+def test_equalize_tc_tile_edges(K, M, S, sg, n_sym, Qm):
+    """mb_equalize_tc over partial antenna tiles, column tiles and groups, odd
+    rows (no 16-byte loads) and both image heights: x against the FP64 product
+    of the BF16-rounded operands.  FP32 accumulation of 2M products is off by
+    at most 2M 2^-23 of the sum of their magnitudes."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from megastation_b200 import ops
+    g = torch.Generator().manual_seed(K * 1000 + M)
+    G = (S + sg - 1) // sg
+
+    def cn(*shape):
+        return torch.complex(torch.randn(*shape, generator=g), torch.randn(*shape, generator=g))
+
+    W, y = cn(G, M, K), cn(n_sym, M, S)
+    llr = torch.full((n_sym, K, S * Qm), 7.0, dtype=torch.float16, device="cuda")
+    x = torch.zeros(n_sym, K, S, dtype=torch.complex64, device="cuda")
+    ops.Equalize.equalize_tc(W.cuda(), y.cuda(), llr, sg, Qm, S * Qm, 0, x=x)
+    torch.cuda.synchronize()
+    assert ops.device_error() == 0
+
+    def low(t):
+        return torch.view_as_complex(torch.view_as_real(t).bfloat16().double())
+
+    grp = torch.arange(S) // sg
+    Wl, yl = low(W)[grp], low(y)  # [S][M][K], [L][M][S]
+    ref = torch.einsum("smk,lms->lks", Wl, yl)
+    mag = torch.einsum("smk,lms->lks", Wl.abs(), yl.abs())
+    err = (x.cpu().to(torch.complex128) - ref).abs()
+    assert (err <= 2 * M * 2.0 ** -23 * mag + 1e-30).all()
+    # the LLRs are the demapper's output for x: its first pair is linear in x
+    scale = -20 * 2 ** 0.5 if Qm == 2 else 100.0
+    first = llr.cpu().float().reshape(n_sym, K, S, Qm)[..., :2]
+    want = torch.view_as_real(x.cpu()) * scale
+    assert ((first - want).abs() <= want.abs() * 2.0 ** -10 + 1e-6).all()
