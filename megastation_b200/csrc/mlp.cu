@@ -3,7 +3,9 @@
 // FP32 master weights; every product takes BF16 weights and BF16
 // activations (or upstream gradients) with FP32 accumulation, the training
 // products on the tensor cores (tcgen05.mma), trained by the project's own
-// forward, backward and Adam kernels.  No counterpart in the reference.
+// forward, backward and Adam kernels: one fused kernel per step for the
+// networks that fit (mlp_step.cu), the products below one by one for wider
+// ones.  No counterpart in the reference.
 //
 // The training loss is the quadratic form the initialiser needs: each sample
 // carries a symmetric O x O matrix A, a vector b and a scalar c, and for the
@@ -19,6 +21,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "mlp_step.cuh"
 #include "tc.cuh"
 
 namespace mb {
@@ -225,12 +228,20 @@ cudaError_t gemm(int M, int N, int K, const TA *A, int lda, const TB *B, int ldb
   return cudaGetLastError();
 }
 
-// out[n] = sum_m X[m][n] (bias gradients), X row-major [M][N]
-__global__ void colsum_kernel(const float *X, int M, int N, float *out) {
-  const int n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= N) return;
+// out[n] = sum_m X[m][n] (bias gradients), X row-major [M][N]: a CTA of 32
+// columns by 8 interleaved row runs (a thread per column alone walked all M
+// rows: 109 us for 4096 x 256)
+__global__ void __launch_bounds__(256) colsum_kernel(const float *X, int M, int N, float *out) {
+  __shared__ float sums[8][32];
+  const int n = blockIdx.x * 32 + threadIdx.x % 32, r = threadIdx.x / 32;
   float s = 0.f;
-  for (int m = 0; m < M; m++) s += X[(size_t)m * N + n];
+  if (n < N)
+#pragma unroll 8
+    for (int m = r; m < M; m += 8) s += X[(size_t)m * N + n];
+  sums[r][threadIdx.x % 32] = s;
+  __syncthreads();
+  if (r || n >= N) return;
+  for (int k = 1; k < 8; k++) s += sums[k][threadIdx.x];
   out[n] = s;
 }
 
@@ -258,8 +269,20 @@ __global__ void quad_loss_kernel(const float *Y, const float *A, const float *b,
   if ((threadIdx.x & 31) == 0 && loss) atomicAdd(loss, li);
 }
 
+// the BF16 copies of parameter i: flat, and (img not null) in the image the
+// fused training step copies into shared memory
+__device__ __forceinline__ void put_bf16(float v, uint64_t i, __nv_bfloat16 *wb, __nv_bfloat16 *img,
+                                         const MlpStepShape &s) {
+  const __nv_bfloat16 h = __float2bfloat16_rn(v);
+  wb[i] = h;
+  if (!img) return;
+  const int e = mlp_step_img(s, i);
+  if (e >= 0) img[e] = h;
+}
+
 __global__ void adam_kernel(float *p, const float *g, float *m, float *v, uint64_t n, float lr,
-                            float b1, float b2, float eps, float c1, float c2) {
+                            float b1, float b2, float eps, float c1, float c2, __nv_bfloat16 *wb,
+                            __nv_bfloat16 *img, const MlpStepShape s) {
   const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float gi = g[i];
@@ -267,7 +290,9 @@ __global__ void adam_kernel(float *p, const float *g, float *m, float *v, uint64
   const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
   m[i] = mi;
   v[i] = vi;
-  p[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+  const float pi = p[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+  p[i] = pi;
+  put_bf16(pi, i, wb, img, s);
 }
 
 // Inference: all three layers in one kernel, ROWS samples per CTA with the
@@ -437,9 +462,10 @@ __global__ void __launch_bounds__(256) mlp_infer_smem_kernel(const float *x, int
   }
 }
 
-__global__ void to_bf16_kernel(const float *x, __nv_bfloat16 *y, uint64_t n) {
+__global__ void to_bf16_kernel(const float *x, __nv_bfloat16 *y, uint64_t n, __nv_bfloat16 *img,
+                               const MlpStepShape s) {
   const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (i < n) y[i] = __float2bfloat16_rn(x[i]);
+  if (i < n) put_bf16(x[i], i, y, img, s);
 }
 
 }  // namespace
@@ -455,13 +481,15 @@ struct mb_mlp {
   float *p, *g, *m, *v;        // params, grads, Adam moments
   __nv_bfloat16 *wb;           // BF16 copies of p (all entries; only W* are read)
   float *z1, *h1, *z2, *h2, *y, *dy, *d2, *d1;  // activations and their gradients
-  float *part;                 // split-K partial sums of the weight gradients
+  float *part;                 // partial sums of the gradients (split-K, or the fused step's slots)
+  __nv_bfloat16 *img;          // weight images of the fused step (mlp_step.cu); null: a product per launch
+  MlpStepShape ss;             // its shape, when img is not null
   uint32_t step;
 };
 
 static cudaError_t mlp_refresh_bf16(mb_mlp *n, cudaStream_t st) {
   const unsigned blocks = (unsigned)((n->n_params + 255) / 256);
-  to_bf16_kernel<<<blocks, 256, 0, st>>>(n->p, n->wb, n->n_params);
+  to_bf16_kernel<<<blocks, 256, 0, st>>>(n->p, n->wb, n->n_params, n->img, n->ss);
   return cudaGetLastError();
 }
 
@@ -469,7 +497,7 @@ extern "C" mb_status mb_mlp_destroy(mb_mlp *n) {
   if (!n) return MB_BAD_ARG;
   for (void *q : {(void *)n->p, (void *)n->g, (void *)n->m, (void *)n->v, (void *)n->wb,
                   (void *)n->z1, (void *)n->h1, (void *)n->z2, (void *)n->h2, (void *)n->y,
-                  (void *)n->dy, (void *)n->d2, (void *)n->d1, (void *)n->part})
+                  (void *)n->dy, (void *)n->d2, (void *)n->d1, (void *)n->part, (void *)n->img})
     cudaFree(q);
   delete n;
   return MB_OK;
@@ -507,16 +535,29 @@ extern "C" mb_status mb_mlp_create(uint32_t n_in, uint32_t width, uint32_t n_out
   alloc((void **)&n->m, P);
   alloc((void **)&n->v, P);
   alloc((void **)&n->wb, sizeof(__nv_bfloat16) * o);
-  const size_t BW = sizeof(float) * (size_t)max_batch * width;
-  alloc((void **)&n->z1, BW);
-  alloc((void **)&n->h1, BW);
-  alloc((void **)&n->z2, BW);
-  alloc((void **)&n->h2, BW);
-  alloc((void **)&n->d2, BW);
-  alloc((void **)&n->d1, BW);
-  alloc((void **)&n->y, sizeof(float) * (size_t)max_batch * n_out);
-  alloc((void **)&n->dy, sizeof(float) * (size_t)max_batch * n_out);
-  alloc((void **)&n->part, sizeof(float) * kMaxSplits * (size_t)std::max(n_in, width) * std::max(width, n_out));
+  if (mlp_step_shape(n_in, width, n_out, n->off, o, &n->ss)) {
+    const size_t slots = std::min<uint64_t>((max_batch + (uint64_t)kStepTile - 1) / kStepTile, kStepSlots);
+    alloc((void **)&n->img, sizeof(__nv_bfloat16) * n->ss.img_elems());
+    alloc((void **)&n->part, sizeof(float) * slots * n->ss.slot);
+    // the images' padding stays zero; of a slot's, only the last few floats
+    // (read, never used) are not written by every step
+    if (st == MB_OK) {
+      cudaError_t e = cudaMemset(n->img, 0, sizeof(__nv_bfloat16) * n->ss.img_elems());
+      if (e != cudaSuccess) st = record_error(e);
+    }
+  } else {
+    const size_t BW = sizeof(float) * (size_t)max_batch * width;
+    alloc((void **)&n->z1, BW);
+    alloc((void **)&n->h1, BW);
+    alloc((void **)&n->z2, BW);
+    alloc((void **)&n->h2, BW);
+    alloc((void **)&n->d2, BW);
+    alloc((void **)&n->d1, BW);
+    alloc((void **)&n->y, sizeof(float) * (size_t)max_batch * n_out);
+    alloc((void **)&n->dy, sizeof(float) * (size_t)max_batch * n_out);
+    alloc((void **)&n->part,
+          sizeof(float) * kMaxSplits * (size_t)std::max(n_in, width) * std::max(width, n_out));
+  }
   if (st == MB_OK) {
     // He-normal hidden layers; the output layer starts at zero weights so the
     // untrained network returns its bias (set by the caller)
@@ -592,6 +633,11 @@ extern "C" mb_status mb_mlp_forward(mb_mlp *n, const float *x, uint32_t batch, f
                                     void *stream) {
   if (!n || !x || !y) return MB_BAD_ARG;
   if (batch == 0) return MB_OK;
+  if (n->img) {
+    MB_CUDA_TRY(mlp_fwd_tc(n->ss, n->img, n->p, x, nullptr, 0, batch, y,
+                           device_tables() ? device_tables()->err : nullptr, as_stream(stream)));
+    return MB_OK;
+  }
   constexpr int kRows = 8;
   const __nv_bfloat16 *wb = n->wb;
   {
@@ -634,6 +680,13 @@ extern "C" mb_status mb_mlp_forward(mb_mlp *n, const float *x, uint32_t batch, f
   return MB_OK;
 }
 
+mb_status mb::mlp_forward_stats(mb_mlp *n, const float *stats, uint32_t sg, uint32_t B, float *y, cudaStream_t st) {
+  if (!n || !n->img || n->n_in != sg + 6) return MB_UNSUPPORTED;
+  MB_CUDA_TRY(mlp_fwd_tc(n->ss, n->img, n->p, nullptr, stats, sg, B, y,
+                         device_tables() ? device_tables()->err : nullptr, st));
+  return MB_OK;
+}
+
 extern "C" mb_status mb_mlp_loss_grad(mb_mlp *n, const float *x, const float *A, const float *b,
                                       const float *c, uint32_t batch, float *loss, void *stream) {
   if (!n || !x || !A || !b) return MB_BAD_ARG;
@@ -642,6 +695,11 @@ extern "C" mb_status mb_mlp_loss_grad(mb_mlp *n, const float *x, const float *A,
   const int I = n->n_in, W = n->width, O = n->n_out, B = (int)batch;
   const __nv_bfloat16 *wb = n->wb;
   float *g = n->g;
+  if (n->img) {
+    MB_CUDA_TRY(mlp_step(n->ss, n->img, n->p, x, A, b, c, batch, n->part, g, loss,
+                         device_tables() ? device_tables()->err : nullptr, st));
+    return MB_OK;
+  }
   MB_CUDA_TRY(mlp_fwd(n, x, batch, n->y, st));
   if (loss) MB_CUDA_TRY(cudaMemsetAsync(loss, 0, sizeof(float), st));
   quad_loss_kernel<<<(B + 255) / 256, 256, 0, st>>>(n->y, A, b, c, B, O, n->dy, loss);
@@ -650,19 +708,19 @@ extern "C" mb_status mb_mlp_loss_grad(mb_mlp *n, const float *x, const float *A,
   // layer 3: dW3 = H2^T dY, db3 = colsum dY, dH2 = (dY W3^T) * relu'(Z2)
   MB_CUDA_TRY((gemm<float, float, true, false>(W, O, B, n->h2, W, n->dy, O, g + n->off[4], O, nullptr,
                                                nullptr, nullptr, 0, 0, st, n->part, err)));
-  colsum_kernel<<<(O + 255) / 256, 256, 0, st>>>(n->dy, B, O, g + n->off[5]);
+  colsum_kernel<<<(O + 31) / 32, 256, 0, st>>>(n->dy, B, O, g + n->off[5]);
   MB_CUDA_TRY((gemm<float, __nv_bfloat16, false, true>(B, W, O, n->dy, O, wb + n->off[4], O, n->d2, W,
                                                        nullptr, n->z2, nullptr, 0, 0, st, nullptr, err)));
   // layer 2
   MB_CUDA_TRY((gemm<float, float, true, false>(W, W, B, n->h1, W, n->d2, W, g + n->off[2], W, nullptr,
                                                nullptr, nullptr, 0, 0, st, n->part, err)));
-  colsum_kernel<<<(W + 255) / 256, 256, 0, st>>>(n->d2, B, W, g + n->off[3]);
+  colsum_kernel<<<(W + 31) / 32, 256, 0, st>>>(n->d2, B, W, g + n->off[3]);
   MB_CUDA_TRY((gemm<float, __nv_bfloat16, false, true>(B, W, W, n->d2, W, wb + n->off[2], W, n->d1, W,
                                                        nullptr, n->z1, nullptr, 0, 0, st, nullptr, err)));
   // layer 1
   MB_CUDA_TRY((gemm<float, float, true, false>(I, W, B, x, I, n->d1, W, g + n->off[0], W, nullptr,
                                                nullptr, nullptr, 0, 0, st, n->part, err)));
-  colsum_kernel<<<(W + 255) / 256, 256, 0, st>>>(n->d1, B, W, g + n->off[1]);
+  colsum_kernel<<<(W + 31) / 32, 256, 0, st>>>(n->d1, B, W, g + n->off[1]);
   MB_CUDA_TRY(cudaGetLastError());
   return MB_OK;
 }
@@ -674,9 +732,9 @@ extern "C" mb_status mb_mlp_adam_step(mb_mlp *n, float lr, void *stream) {
   const float b1 = 0.9f, b2 = 0.999f;
   const float c1 = 1.f - std::pow(b1, (float)n->step), c2 = 1.f - std::pow(b2, (float)n->step);
   const unsigned blocks = (unsigned)((n->n_params + 255) / 256);
-  adam_kernel<<<blocks, 256, 0, st>>>(n->p, n->g, n->m, n->v, n->n_params, lr, b1, b2, 1e-8f, c1, c2);
+  adam_kernel<<<blocks, 256, 0, st>>>(n->p, n->g, n->m, n->v, n->n_params, lr, b1, b2, 1e-8f, c1, c2,
+                                      n->wb, n->img, n->ss);
   MB_CUDA_TRY(cudaGetLastError());
-  MB_CUDA_TRY(mlp_refresh_bf16(n, st));
   return MB_OK;
 }
 

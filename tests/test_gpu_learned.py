@@ -236,3 +236,40 @@ def test_lzf_far_start_takes_exact_inverse(mb):
     far = np.nonzero(fl == 2)[0]
     Wn, We = W.cpu().numpy(), W_ex.cpu().numpy()
     assert np.abs(Wn[far] - We[far]).max() <= 1e-5 * np.abs(We).max()
+
+
+@pytest.mark.parametrize("n_in,width,n_out,B", [
+    (1, 1, 1, 1), (16, 100, 4, 63), (17, 128, 5, 64), (64, 129, 16, 65), (22, 200, 4, 130), (6, 64, 4, 9500),
+    (30, 254, 3, 9473), (22, 320, 4, 300), (65, 64, 4, 130)])
+def test_mlp_step_shape_edges(mb, n_in, width, n_out, B):
+    """The fused step at the edges of its sample tiles, neuron tiles and
+    padding, past one tile per CTA (148 x 64 samples) and, last two, just
+    outside its shapes; per block as in test_mlp_gradients_match_oracle."""
+    from megastation_b200 import learned
+    net = learned.MLP(n_in, width, n_out, max_batch=B, seed=1)
+    rng = np.random.default_rng(n_in + width + B)
+    p = (rng.standard_normal(net.num_params()) * 0.3 / np.sqrt(width / 64 + 1)).astype(np.float32)
+    net.set_params(p)
+    x = rng.standard_normal((B, n_in)).astype(np.float32)
+    Mx = rng.standard_normal((B, n_out, n_out))
+    A = (np.einsum("bij,bkj->bik", Mx, Mx) / n_out).astype(np.float32)
+    b = rng.standard_normal((B, n_out)).astype(np.float32)
+    c = rng.standard_normal(B).astype(np.float32)
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    for cc in (c, None):
+        loss = net.loss_grad(dev(x), dev(A), dev(b), None if cc is None else dev(cc))
+        g = net.grads()
+        lr, gr = om.mlp_loss_grad(p, x, A, b, cc, n_in, width, n_out)
+        assert mb.ops.device_error() == 0
+        assert abs(float(loss.item()) - lr) <= 1e-4 * max(1.0, abs(lr))
+        o = 0
+        for s in (n_in * width, width, width * width, width, width * n_out, n_out):
+            blk, ref = g[o:o + s], gr[o:o + s]
+            assert np.abs(blk - ref).max() <= 1e-3 * np.abs(ref).max() + 1e-7, (o, s)
+            o += s
+    # the step reads the weights Adam wrote: its loss is the forward pass's
+    net.adam_step(1e-3)
+    q = net.params()
+    loss = float(net.loss_grad(dev(x), dev(A), dev(b), dev(c)).item())
+    lr, _ = om.mlp_loss_grad(q, x, A, b, c, n_in, width, n_out)
+    assert abs(loss - lr) <= 1e-4 * max(1.0, abs(lr))
