@@ -12,6 +12,8 @@
 // runs the same schedule in double.  Unlike the reference, which ignores
 // cuSOLVER's info array, a non positive definite Gram is reported per group
 // (status 1) and its W is zeroed.
+#include <cooperative_groups.h>
+
 #include <algorithm>
 #include <atomic>
 
@@ -187,9 +189,61 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// beam_utils.cuh:40-80 as a standalone kernel: one CTA per group.
+// beam_utils.cuh:40-80 as a standalone kernel: a cluster of CTAs per group,
+// each with mb antennas of it in shared memory.  W is read once (a CTA per
+// group that read it for the maximum and again, tile by tile between
+// barriers, for the transposition took 38 us for 205 groups of 256 x 64;
+// 16 us here); the group's maximum crosses the cluster through
+// distributed shared memory.  HBM bound: W in, P out.
 __global__ void __launch_bounds__(256)
-    precoder_kernel(const float2 *W, float2 *P, uint32_t M, uint32_t K) {
+    precoder_kernel(const float2 *W, float2 *P, uint32_t M, uint32_t K, uint32_t mb) {
+  namespace cg = cooperative_groups;
+  extern __shared__ float2 pc_tile[];  // [mb][ldt]
+  __shared__ float red[8], cmax;
+  const cg::cluster_group cl = cg::this_cluster();
+  const uint32_t cn = cl.num_blocks(), rank = cl.block_rank(), g = blockIdx.x / cn;
+  const uint32_t b0 = rank * mb, nb = b0 < M ? min(mb, M - b0) : 0, ldt = K | 1;
+  const uint32_t lane = threadIdx.x % 32, warp = threadIdx.x / 32;
+  const float2 *wg = W + ((uint64_t)g * M + b0) * K;
+  float mx = 0.f;
+  uint32_t b = threadIdx.x / K, u = threadIdx.x % K;  // element threadIdx.x, then 256 further each time
+  const uint32_t db = 256 / K, du = 256 % K;
+#pragma unroll 8
+  for (uint32_t e = threadIdx.x; e < nb * K; e += 256) {
+    const float2 v = __ldg(wg + e);
+    mx = fmaxf(mx, sqrtf(v.x * v.x + v.y * v.y));
+    pc_tile[b * ldt + u] = v;
+    b += db;
+    u += du;
+    if (u >= K) {
+      u -= K;
+      b++;
+    }
+  }
+  for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  if (lane == 0) red[warp] = mx;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 8; w++) mx = fmaxf(mx, red[w]);
+    cmax = mx;
+  }
+  cl.sync();
+  mx = 0.f;
+  for (uint32_t r = 0; r < cn; r++) mx = fmaxf(mx, *cl.map_shared_rank(&cmax, r));
+  cl.sync();  // no CTA exits while another reads its maximum
+  const float inv = 1.0f / mx;
+  float2 *pg = P + (uint64_t)g * M * K + b0;
+  for (uint32_t r = warp; r < K; r += 8)
+    for (uint32_t c = lane; c < nb; c += 32) {
+      const float2 v = pc_tile[c * ldt + r];
+      pg[(uint64_t)r * M + c] = make_float2(v.x * inv, v.y * inv);
+    }
+}
+
+// The same for matrices whose eighth exceeds one SM's shared memory (more than
+// about 28,000 entries): one CTA per group, W read twice.
+__global__ void __launch_bounds__(256)
+    precoder_wide_kernel(const float2 *W, float2 *P, uint32_t M, uint32_t K) {
   __shared__ float red[256];
   const uint32_t g = blockIdx.x;
   const float2 *wg = W + (uint64_t)g * M * K;
@@ -326,7 +380,38 @@ mb_status precoder_scale(const float2 *W, float2 *P, const float *wmax, uint32_t
 mb_status precoder_launch(const float2 *W, float2 *P, uint32_t M, uint32_t K,
                           uint32_t groups, cudaStream_t st) {
   if (groups == 0) return MB_OK;
-  precoder_kernel<<<groups, 256, 0, st>>>(W, P, M, K);
+  // 32 antennas a CTA while the portable cluster of eight lasts, more beyond
+  uint32_t cn = 1;
+  while (cn < 8 && cn * 32 < M) cn *= 2;
+  const uint32_t mb = std::max<uint32_t>(32, (M + cn - 1) / cn);
+  const size_t smem = sizeof(float2) * (size_t)std::min(mb, M) * (K | 1);
+  int dev = 0, maxs = 0;
+  MB_CUDA_TRY(cudaGetDevice(&dev));
+  MB_CUDA_TRY(cudaDeviceGetAttribute(&maxs, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+  if (smem + 1024 > (size_t)maxs || (uint64_t)groups * cn > 0x7FFFFFFFull) {
+    // an eighth of W does not fit one SM: two passes over it
+    precoder_wide_kernel<<<groups, 256, 0, st>>>(W, P, M, K);
+    MB_LAUNCH_CHECK();
+    return MB_OK;
+  }
+  static std::atomic<uint64_t> configured{0};
+  const uint64_t bit = 1ull << (dev & 63);
+  if (!(configured.load() & bit)) {
+    MB_CUDA_TRY(cudaFuncSetAttribute(precoder_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, maxs - 1024));
+    configured.fetch_or(bit);
+  }
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = cn;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cudaLaunchConfig_t lc{};
+  lc.gridDim = dim3(groups * cn);
+  lc.blockDim = dim3(256);
+  lc.dynamicSmemBytes = smem;
+  lc.stream = st;
+  lc.attrs = &at;
+  lc.numAttrs = 1;
+  MB_CUDA_TRY(cudaLaunchKernelEx(&lc, precoder_kernel, W, P, M, K, mb));
   MB_LAUNCH_CHECK();
   return MB_OK;
 }
