@@ -50,116 +50,286 @@ __global__ void zf_fill_tail_kernel(float2 *csi, uint32_t G, uint32_t M,
   }
 }
 
-// One CTA per group.  Shared memory: C as [K][M+1] complex of T, the Gram /
-// Cholesky factor as [K][K+1], and a reduction buffer.
-template <typename T>
+// Rows i > k of the K x K Hermitian A minus a_ik / a_kk times row k, pivot by
+// pivot, the multipliers' negatives left in the eliminated entries and taken
+// along like the rest of their row: A = L D L^H ends as D on the diagonal and
+// L^{-1} strictly below it (what lies above is scratch).  The row of thread t is t / TPR, its
+// columns t % TPR + TPR m in registers, rotated by one slot every TPR pivots
+// so that the pivot column always sits in slot 0; the pivot row goes through
+// shared memory, two buffers of KP at the head of A (free while the rows are
+// in registers; a small A's buffers run on into the 1 KB behind it): one
+// barrier a pivot.
+template <typename T, int KP>
+__device__ __forceinline__ void ldl_eliminate(Cplx<T> *A, uint32_t lda, uint32_t K, int *not_pd) {
+  constexpr int TPR = 256 / KP, NC = KP / TPR > 0 ? KP / TPR : 1;
+  const uint32_t i = threadIdx.x / TPR, sub = threadIdx.x % TPR;
+  Cplx<T> v[NC];
+#pragma unroll
+  for (int m = 0; m < NC; m++) {
+    const uint32_t c = sub + TPR * m;
+    v[m] = i < K && c < K ? A[i * lda + c] : mk<T>(i == c ? (T)1 : (T)0, (T)0);
+  }
+  __syncthreads();
+#pragma unroll 1
+  for (uint32_t r = 0; r < (uint32_t)NC && r * TPR < K; r++) {
+#pragma unroll
+    for (int s = 0; s < TPR; s++) {
+      const uint32_t k = r * TPR + s;
+      if (k < K) {  // uniform
+        Cplx<T> f;  // this row's entry in column k
+        f.x = __shfl_sync(0xffffffffu, v[0].x, s, TPR);
+        f.y = __shfl_sync(0xffffffffu, v[0].y, s, TPR);
+        Cplx<T> *pr = A + (k & 1) * KP;
+        if (i == k) {
+          T d = f.x;
+          if (!(d > (T)0)) {
+            *not_pd = 1;
+            d = (T)1;
+          }
+          // in the buffer the pivot's own slot carries 1 / d
+          if (sub == (uint32_t)s) v[0] = mk<T>(d, (T)0);
+#pragma unroll
+          for (int m = 0; m < NC; m++) pr[sub + TPR * m] = v[m];
+          if (sub == (uint32_t)s) pr[s] = mk<T>((T)1 / d, (T)0);
+        }
+        __syncthreads();
+        if (i > k) {
+          const T inv = pr[s].x;
+          const Cplx<T> q = mk<T>(f.x * inv, f.y * inv);
+#pragma unroll
+          for (int m = 0; m < NC; m++) {
+            const Cplx<T> w = pr[sub + TPR * m];
+            v[m].x -= q.x * w.x - q.y * w.y;
+            v[m].y -= q.x * w.y + q.y * w.x;
+          }
+          if (sub == (uint32_t)s) v[0] = mk<T>(-q.x, -q.y);
+        }
+      }
+    }
+    const Cplx<T> t = v[0];
+#pragma unroll
+    for (int m = 0; m < NC - 1; m++) v[m] = v[m + 1];
+    v[NC - 1] = t;
+  }
+  __syncthreads();
+  // slot m holds column sub + TPR ((m + rotations) % NC)
+  const uint32_t rot = min((uint32_t)NC, (K + TPR - 1) / TPR);
+  if (i < K) {
+#pragma unroll
+    for (int m = 0; m < NC; m++) {
+      uint32_t c = m + rot;
+      if (c >= (uint32_t)NC) c -= NC;
+      c = sub + TPR * c;
+      if (c <= i) A[i * lda + c] = v[m];
+    }
+  }
+  __syncthreads();
+}
+
+// One CTA per group.  Shared memory: C as [K][M+1] complex of T, A as
+// [K][K+1].  W = A^{-1} C as L^{-H} D^{-1} (L^{-1} C): with L^{-1} at hand both
+// products run over all rows and antennas at once, where the triangular
+// solves of a Cholesky factor left one thread per antenna a chain of K^2
+// dependent steps and the factor itself three barriers a column.  Latency
+// bound for small cells (75 groups of 64 x 16: 20.4 us
+// before, 9.0 us).
+template <typename T, int KP>
 __global__ void __launch_bounds__(256)
     zf_chol_kernel(float2 *csi, float2 *precoder, uint32_t M, uint32_t K,
                    int32_t *status, float *cond_out) {
   extern __shared__ __align__(16) unsigned char zf_smem_raw[];
   using C = Cplx<T>;
+  constexpr int GT = KP / 16;  // Gram: GT x GT outputs per thread
   const uint32_t g = blockIdx.x;
   const uint32_t ldc = M + 1, lda = K + 1;
   C *Cs = reinterpret_cast<C *>(zf_smem_raw);
   C *A = Cs + (size_t)K * ldc;
   float *red = reinterpret_cast<float *>(A + (size_t)K * lda);
   __shared__ int not_pd;
-  const int tid = threadIdx.x, nt = blockDim.x;
+  const uint32_t tid = threadIdx.x;
+  constexpr uint32_t nt = 256;
   float2 *cg = csi + (uint64_t)g * M * K;
 
   if (tid == 0) not_pd = 0;
   // load C[u][b] = csi[g][b][u] (coalesced in b*K + u)
-  for (uint32_t e = tid; e < M * K; e += nt) {
-    float2 v = cg[e];
-    uint32_t b = e / K, u = e % K;
-    Cs[u * ldc + b] = mk<T>((T)v.x, (T)v.y);
-  }
-  __syncthreads();
-
-  // Gram A = C C^H, lower triangle
-  const uint32_t ntri = K * (K + 1) / 2;
-  for (uint32_t q = tid; q < ntri; q += nt) {
-    // q -> (i, j), j <= i
-    uint32_t i = (uint32_t)((sqrtf(8.f * q + 1.f) - 1.f) * 0.5f);
-    while (i * (i + 1) / 2 > q) i--;
-    while ((i + 1) * (i + 2) / 2 <= q) i++;
-    uint32_t j = q - i * (i + 1) / 2;
-    const C *ci = Cs + i * ldc, *cj = Cs + j * ldc;
-    T sr = 0, si = 0;
-    for (uint32_t b = 0; b < M; b++) {
-      C a = ci[b], c = cj[b];
-      sr += a.x * c.x + a.y * c.y;
-      si += a.y * c.x - a.x * c.y;
-    }
-    A[i * lda + j] = mk<T>(sr, si);
-  }
-  __syncthreads();
-
-  // right-looking Cholesky A = L L^H in place (lower)
-  for (uint32_t j = 0; j < K; j++) {
-    if (tid == 0) {
-      T d = A[j * lda + j].x;
-      if (!(d > (T)0)) {
-        not_pd = 1;
-        d = (T)1;
+  const uint32_t db = nt / K, du = nt % K;
+  {
+    uint32_t b = tid / K, u = tid % K;
+#pragma unroll 4
+    for (uint32_t e = tid; e < M * K; e += nt) {
+      const float2 v = cg[e];
+      Cs[u * ldc + b] = mk<T>((T)v.x, (T)v.y);
+      b += db;
+      u += du;
+      if (u >= K) {
+        u -= K;
+        b++;
       }
-      A[j * lda + j] = mk<T>(sqrt(d), (T)0);
-    }
-    __syncthreads();
-    const T inv = (T)1 / A[j * lda + j].x;
-    for (uint32_t i = j + 1 + tid; i < K; i += nt) {
-      C v = A[i * lda + j];
-      A[i * lda + j] = mk<T>(v.x * inv, v.y * inv);
-    }
-    __syncthreads();
-    const uint32_t rem = K - j - 1;
-    for (uint32_t q = tid; q < rem * rem; q += nt) {
-      uint32_t i = j + 1 + q / rem, k = j + 1 + q % rem;
-      if (k > i) continue;
-      C a = A[i * lda + j], b = A[k * lda + j];
-      // A[i][k] -= L[i][j] * conj(L[k][j])
-      C c = A[i * lda + k];
-      c.x -= a.x * b.x + a.y * b.y;
-      c.y -= a.y * b.x - a.x * b.y;
-      A[i * lda + k] = c;
-    }
-    __syncthreads();
-  }
-
-  // W = A^{-1} C: thread per column b, solve in place in Cs[:, b]
-  for (uint32_t b = tid; b < M; b += nt) {
-    for (uint32_t i = 0; i < K; i++) {
-      C s = Cs[i * ldc + b];
-      for (uint32_t k = 0; k < i; k++) {
-        C l = A[i * lda + k], z = Cs[k * ldc + b];
-        s.x -= l.x * z.x - l.y * z.y;
-        s.y -= l.x * z.y + l.y * z.x;
-      }
-      T d = A[i * lda + i].x;
-      Cs[i * ldc + b] = mk<T>(s.x / d, s.y / d);
-    }
-    for (int i = (int)K - 1; i >= 0; i--) {
-      C s = Cs[i * ldc + b];
-      for (uint32_t k = i + 1; k < K; k++) {
-        C l = A[k * lda + i], z = Cs[k * ldc + b];  // conj(L[k][i]) * z
-        s.x -= l.x * z.x + l.y * z.y;
-        s.y -= l.x * z.y - l.y * z.x;
-      }
-      T d = A[i * lda + i].x;
-      Cs[i * ldc + b] = mk<T>(s.x / d, s.y / d);
     }
   }
   __syncthreads();
 
+  // Gram A = C C^H: rows ti + 16 a, columns tj + 16 b of the thread, the
+  // lower triangle's 16 x 16 blocks
+  {
+    const uint32_t ti = tid / 16, tj = tid % 16;
+    C acc[GT][GT];
+#pragma unroll
+    for (int a = 0; a < GT; a++)
+#pragma unroll
+      for (int b = 0; b < GT; b++) acc[a][b] = mk<T>((T)0, (T)0);
+    const C *ca[GT], *cb[GT];
+#pragma unroll
+    for (int a = 0; a < GT; a++) {
+      // rows past K repeat row K - 1: their outputs are not stored
+      ca[a] = Cs + min(ti + 16 * a, K - 1) * ldc;
+      cb[a] = Cs + min(tj + 16 * a, K - 1) * ldc;
+    }
+#pragma unroll 4
+    for (uint32_t m = 0; m < M; m++) {
+      C av[GT], bv[GT];
+#pragma unroll
+      for (int a = 0; a < GT; a++) {
+        av[a] = ca[a][m];
+        bv[a] = cb[a][m];
+      }
+#pragma unroll
+      for (int a = 0; a < GT; a++)
+#pragma unroll
+        for (int b = 0; b <= a; b++) {
+          acc[a][b].x += av[a].x * bv[b].x + av[a].y * bv[b].y;
+          acc[a][b].y += av[a].y * bv[b].x - av[a].x * bv[b].y;
+        }
+    }
+#pragma unroll
+    for (int a = 0; a < GT; a++)
+#pragma unroll
+      for (int b = 0; b <= a; b++) {
+        const uint32_t i = ti + 16 * a, j = tj + 16 * b;
+        if (i >= K || j > i) continue;
+        const C v = acc[a][b];
+        A[i * lda + j] = v;
+        if (j < i) A[j * lda + i] = mk<T>(v.x, -v.y);
+      }
+  }
+  __syncthreads();
+  ldl_eliminate<T, KP>(A, lda, K, &not_pd);
   const bool bad = not_pd != 0;
+
+  // Products over blocks of four rows: thread (part, column b), `cols` columns
+  // and `parts` blocks side by side.  Z = L^{-1} C in place from the last
+  // rows up (a row reads the rows above it), then W = L^{-H} D^{-1} Z from the
+  // first rows down; the barriers keep the blocks of one round, whose rows
+  // read one another's old values, apart.
+  uint32_t cols = 32;
+  while (cols < M && cols < nt) cols *= 2;
+  const uint32_t parts = nt / cols, part = tid / cols, nb = (K + 3) / 4;
+  for (uint32_t b0 = 0; b0 < M; b0 += cols) {
+    const uint32_t b = b0 + tid % cols;
+    const bool on = b < M;
+    for (uint32_t r = 0; r < nb; r += parts) {
+      const uint32_t i0 = r + part < nb ? 4 * (nb - 1 - r - part) : 0;
+      const bool act = on && r + part < nb;
+      C z[4];
+      if (act) {
+#pragma unroll
+        for (int q = 0; q < 4; q++) z[q] = i0 + q < K ? Cs[(i0 + q) * ldc + b] : mk<T>((T)0, (T)0);
+        const C *l[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) l[q] = A + min(i0 + q, K - 1) * lda;
+#pragma unroll 4
+        for (uint32_t k = 0; k < i0; k++) {
+          const C c = Cs[k * ldc + b];
+#pragma unroll
+          for (int q = 0; q < 4; q++) {
+            const C w = l[q][k];
+            z[q].x += w.x * c.x - w.y * c.y;
+            z[q].y += w.x * c.y + w.y * c.x;
+          }
+        }
+        // within the block: rows i0 .. i0 + 2 of C
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+          if (i0 + k + 1 >= K) break;
+          const C c = Cs[(i0 + k) * ldc + b];
+#pragma unroll
+          for (int q = k + 1; q < 4; q++) {
+            const C w = l[q][i0 + k];
+            if (i0 + q < K) {
+              z[q].x += w.x * c.x - w.y * c.y;
+              z[q].y += w.x * c.y + w.y * c.x;
+            }
+          }
+        }
+      }
+      if (parts > 1) __syncthreads();
+      if (act) {
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+          if (i0 + q < K) {
+            const T d = (T)1 / A[(i0 + q) * lda + i0 + q].x;
+            Cs[(i0 + q) * ldc + b] = mk<T>(z[q].x * d, z[q].y * d);
+          }
+      }
+      if (parts > 1) __syncthreads();
+    }
+    for (uint32_t r = 0; r < nb; r += parts) {
+      const uint32_t i0 = 4 * (r + part);
+      const bool act = on && r + part < nb;
+      C z[4];
+      if (act) {
+#pragma unroll
+        for (int q = 0; q < 4; q++) z[q] = i0 + q < K ? Cs[(i0 + q) * ldc + b] : mk<T>((T)0, (T)0);
+#pragma unroll
+        for (int k = 1; k < 4; k++) {
+          if (i0 + k >= K) break;
+          const C c = Cs[(i0 + k) * ldc + b];
+#pragma unroll
+          for (int q = 0; q < k; q++) {
+            const C w = A[(i0 + k) * lda + i0 + q];  // conj
+            z[q].x += w.x * c.x + w.y * c.y;
+            z[q].y += w.x * c.y - w.y * c.x;
+          }
+        }
+#pragma unroll 4
+        for (uint32_t k = i0 + 4; k < K; k++) {
+          const C c = Cs[k * ldc + b];
+#pragma unroll
+          for (int q = 0; q < 4; q++) {
+            const C w = A[k * lda + i0 + q];
+            z[q].x += w.x * c.x + w.y * c.y;
+            z[q].y += w.x * c.y - w.y * c.x;
+          }
+        }
+      }
+      if (parts > 1) __syncthreads();
+      if (act) {
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+          if (i0 + q < K) Cs[(i0 + q) * ldc + b] = z[q];
+      }
+      if (parts > 1) __syncthreads();
+    }
+  }
+  __syncthreads();
+
   // write W back in the CSI layout; track max |W| for the precoder
   float mx = 0.f;
-  for (uint32_t e = tid; e < M * K; e += nt) {
-    uint32_t b = e / K, u = e % K;
-    C w = Cs[u * ldc + b];
-    float2 o = bad ? make_float2(0.f, 0.f) : make_float2((float)w.x, (float)w.y);
-    cg[e] = o;
-    mx = fmaxf(mx, sqrtf(o.x * o.x + o.y * o.y));
+  {
+    uint32_t b = tid / K, u = tid % K;
+#pragma unroll 4
+    for (uint32_t e = tid; e < M * K; e += nt) {
+      const C w = Cs[u * ldc + b];
+      const float2 o = bad ? make_float2(0.f, 0.f) : make_float2((float)w.x, (float)w.y);
+      cg[e] = o;
+      mx = fmaxf(mx, sqrtf(o.x * o.x + o.y * o.y));
+      b += db;
+      u += du;
+      if (u >= K) {
+        u -= K;
+        b++;
+      }
+    }
   }
   if (status && tid == 0) status[g] = bad ? 1 : 0;
   if (cond_out && tid == 0) {
@@ -170,23 +340,23 @@ __global__ void __launch_bounds__(256)
       lo = d < lo ? d : lo;
       hi = d > hi ? d : hi;
     }
-    cond_out[g] = bad ? INFINITY : (float)((hi / lo) * (hi / lo));
+    cond_out[g] = bad ? INFINITY : (float)(hi / lo);
   }
   if (!precoder) return;
   red[tid] = mx;
   __syncthreads();
-  for (int s = nt / 2; s > 0; s >>= 1) {
+  for (uint32_t s = nt / 2; s > 0; s >>= 1) {
     if (tid < s) red[tid] = fmaxf(red[tid], red[tid + s]);
     __syncthreads();
   }
   const float inv = 1.0f / red[0];
   float2 *pg = precoder + (uint64_t)g * M * K;
-  for (uint32_t e = tid; e < M * K; e += nt) {
-    uint32_t u = e / M, b = e % M;
-    C w = Cs[u * ldc + b];
-    float2 o = bad ? make_float2(0.f, 0.f) : make_float2((float)w.x, (float)w.y);
-    pg[e] = make_float2(o.x * inv, o.y * inv);
-  }
+  for (uint32_t u = tid / 32; u < K; u += nt / 32)
+    for (uint32_t b = tid % 32; b < M; b += 32) {
+      const C w = Cs[u * ldc + b];
+      const float2 o = bad ? make_float2(0.f, 0.f) : make_float2((float)w.x, (float)w.y);
+      pg[(uint64_t)u * M + b] = make_float2(o.x * inv, o.y * inv);
+    }
 }
 
 // beam_utils.cuh:40-80 as a standalone kernel: a cluster of CTAs per group,
@@ -326,46 +496,40 @@ mb_status zf_fill_tail(float2 *csi, uint32_t groups, uint32_t S, uint32_t sg,
   return MB_OK;
 }
 
-template <typename T>
-static mb_status set_smem_attr(size_t smem) {
+template <typename T, int KP>
+static mb_status zf_chol_launch(float2 *csi, float2 *precoder, uint32_t groups, uint32_t M, uint32_t K, size_t smem,
+                                int32_t *status, float *cond, cudaStream_t st) {
   static std::atomic<uint64_t> configured{0};
-  int dev = 0;
+  static std::atomic<int> static_smem{0};
+  int dev = 0, maxs = 0;
   MB_CUDA_TRY(cudaGetDevice(&dev));
+  MB_CUDA_TRY(cudaDeviceGetAttribute(&maxs, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
   const uint64_t bit = 1ull << (dev & 63);
   if (!(configured.load() & bit)) {
-    int maxs = 0;
     cudaFuncAttributes fa;
-    MB_CUDA_TRY(cudaDeviceGetAttribute(&maxs, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    MB_CUDA_TRY(cudaFuncGetAttributes(&fa, zf_chol_kernel<T>));
-    MB_CUDA_TRY(cudaFuncSetAttribute(zf_chol_kernel<T>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
+    MB_CUDA_TRY(cudaFuncGetAttributes(&fa, zf_chol_kernel<T, KP>));
+    MB_CUDA_TRY(cudaFuncSetAttribute(zf_chol_kernel<T, KP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      maxs - (int)fa.sharedSizeBytes));
+    static_smem = (int)fa.sharedSizeBytes;
     configured.fetch_or(bit);
   }
-  (void)smem;
+  if (smem + (size_t)static_smem.load() > (size_t)maxs) return MB_UNSUPPORTED;
+  if (groups == 0) return MB_OK;
+  zf_chol_kernel<T, KP><<<groups, 256, smem, st>>>(csi, precoder, M, K, status, cond);
+  MB_LAUNCH_CHECK();
   return MB_OK;
 }
 
 mb_status zf_chol(float2 *csi, float2 *precoder, uint32_t groups, uint32_t M,
                   uint32_t K, bool dbl, int32_t *status, float *cond,
                   cudaStream_t st) {
-  size_t smem = zf_chol_smem(M, K, dbl);
-  int dev = 0, maxs = 0;
-  MB_CUDA_TRY(cudaGetDevice(&dev));
-  MB_CUDA_TRY(cudaDeviceGetAttribute(&maxs, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-  if (smem + 64 > (size_t)maxs) return MB_UNSUPPORTED;
-  if (groups == 0) return MB_OK;
+  const size_t smem = zf_chol_smem(M, K, dbl);
   if (dbl) {
-    mb_status s = set_smem_attr<double>(smem);
-    if (s != MB_OK) return s;
-    zf_chol_kernel<double><<<groups, 256, smem, st>>>(csi, precoder, M, K, status, cond);
-  } else {
-    mb_status s = set_smem_attr<float>(smem);
-    if (s != MB_OK) return s;
-    zf_chol_kernel<float><<<groups, 256, smem, st>>>(csi, precoder, M, K, status, cond);
+    auto f = K <= 16 ? zf_chol_launch<double, 16> : K <= 32 ? zf_chol_launch<double, 32> : zf_chol_launch<double, 64>;
+    return f(csi, precoder, groups, M, K, smem, status, cond, st);
   }
-  MB_LAUNCH_CHECK();
-  return MB_OK;
+  auto f = K <= 16 ? zf_chol_launch<float, 16> : K <= 32 ? zf_chol_launch<float, 32> : zf_chol_launch<float, 64>;
+  return f(csi, precoder, groups, M, K, smem, status, cond, st);
 }
 
 mb_status precoder_scale(const float2 *W, float2 *P, const float *wmax, uint32_t M, uint32_t K,
