@@ -37,6 +37,7 @@
 #include "common.cuh"
 #include "eq_tc.cuh"
 #include "eq_tc_epi.cuh"
+#include "gj.cuh"
 #include "tc.cuh"
 #include "zf.cuh"
 
@@ -72,6 +73,15 @@ struct ZfmParams {
   EqParams ep;
   uint32_t eq_nb, eq_spc, eq_nct, eq_N;
 };
+
+// MM == 128: bytes of G's region and of X's, which the Gram's two hi slots share
+__host__ __device__ constexpr uint32_t zfm_gx_bytes(uint32_t K) {
+  return (K * (K + 1) * (uint32_t)sizeof(float2) + 1023) / 1024 * 1024;
+}
+__host__ __device__ constexpr uint32_t zfm_x_bytes(uint32_t K) {
+  const uint32_t two_tiles = 2 * 128 * kKT * 2;
+  return zfm_gx_bytes(K) > two_tiles ? zfm_gx_bytes(K) : two_tiles;
+}
 
 __device__ __forceinline__ uint32_t img_off(uint32_t r, uint32_t kk, uint32_t MM) {
   // canonical K-major, no swizzle: [k tile][row group][k chunk][row][8]
@@ -116,88 +126,14 @@ __device__ bool chol_smem(C *A, uint32_t K, uint32_t lda, int *flag) {
   return *flag == 0;
 }
 
-// Inverse of the K x K Hermitian positive definite matrix G (leading dim ld)
-// into X by in-place Gauss-Jordan without pivoting (every pivot of a
-// positive definite matrix is real and positive): at pivot k the pivot row
-// becomes a_kj / a_kk with a_kk <- 1 / a_kk, and every other row i becomes
-// a_ij - a_ik a_kj' with a_ik <- -a_ik / a_kk, so column k of G is replaced
-// by column k of the inverse and no identity half is carried.  The matrix is
-// padded to KP x KP with an identity block.  Thread t holds row t / TPR in
-// registers, columns t % TPR + TPR m; the pivot row goes through shared
-// memory (prow, two buffers of KP), so each pivot costs one barrier.  The
-// register row is rotated by one slot after every TPR pivots, so the pivot
-// column always sits in slot 0 and the loop body indexes registers
-// statically without being unrolled over the row (a short body: the
-// unrolled form stalled on instruction fetch at KP = 64).
-// Returns false when a pivot is not positive (the output is then garbage).
-template <int KP>
-__device__ __forceinline__ bool gj_inverse(const float2 *G, float2 *X, uint32_t K, uint32_t ld,
-                                           float2 *prow, int *bad) {
-  constexpr int TPR = kThreads / KP, NC = KP / TPR;
-  const uint32_t i = threadIdx.x / TPR, sub = threadIdx.x % TPR;
-  // v[m] holds column sub + TPR ((m + r) % NC) after r rotations
-  float2 v[NC];
-#pragma unroll
-  for (int m = 0; m < NC; m++) {
-    const uint32_t c = sub + TPR * m;
-    v[m] = (i < K && c < K) ? G[i * ld + c] : make_float2(i == c ? 1.f : 0.f, 0.f);
-  }
-#pragma unroll 1
-  for (uint32_t r = 0; r < (uint32_t)NC; r++) {
-#pragma unroll
-    for (int s = 0; s < TPR; s++) {
-      const uint32_t k = r * TPR + s;
-      float2 f;  // this row's entry in column k
-      f.x = __shfl_sync(0xffffffffu, v[0].x, s, TPR);
-      f.y = __shfl_sync(0xffffffffu, v[0].y, s, TPR);
-      float2 *pr = prow + (k & 1) * KP;
-      if (i == k) {
-        if (!(f.x > 0.f)) *bad = 1;
-        const float inv = __frcp_rn(f.x);
-        if (sub == (uint32_t)s) v[0] = make_float2(1.f, 0.f);
-#pragma unroll
-        for (int m = 0; m < NC; m++) {
-          v[m].x *= inv;
-          v[m].y *= inv;
-          pr[sub + TPR * m] = v[m];
-        }
-      }
-      __syncthreads();
-      if (i != k) {
-        if (sub == (uint32_t)s) v[0] = make_float2(0.f, 0.f);
-#pragma unroll
-        for (int m = 0; m < NC; m++) {
-          const float2 w = pr[sub + TPR * m];
-          v[m].x -= f.x * w.x - f.y * w.y;
-          v[m].y -= f.x * w.y + f.y * w.x;
-        }
-      }
-    }
-    const float2 t = v[0];
-#pragma unroll
-    for (int m = 0; m < NC - 1; m++) v[m] = v[m + 1];
-    v[NC - 1] = t;
-  }
-  __syncthreads();
-  const bool ok = *bad == 0;
-  if (i < K) {
-#pragma unroll
-    for (int m = 0; m < NC; m++) {
-      const uint32_t c = sub + TPR * m;
-      if (c < K) X[i * ld + c] = v[m];
-    }
-  }
-  __syncthreads();
-  return ok;
-}
-
 // C = A B for K x K complex matrices in shared memory (leading dims given);
 // out(i, j, c) receives each entry.  Thread t owns the outputs
 // (t / 16 + 16a, t % 16 + 16b), a, b < T: T*T independent accumulators that
 // share each A and B load.  Needs 256 threads and K <= 16 T.  HERM: C is
 // known to be Hermitian, so only the 16 x 16 blocks a <= b are computed and
 // the blocks below the diagonal are written as their conjugate transposes.
-template <int T, bool HERM, typename Out>
+// INPLACE: out may overwrite A or B (a barrier before the first output).
+template <int T, bool HERM, bool INPLACE, typename Out>
 __device__ __forceinline__ void cmatmul(const float2 *A, uint32_t lda, const float2 *B, uint32_t ldb,
                                         uint32_t K, Out out) {
   const uint32_t ti = threadIdx.x / 16, tj = threadIdx.x % 16;
@@ -228,6 +164,7 @@ __device__ __forceinline__ void cmatmul(const float2 *A, uint32_t lda, const flo
         acc[a][b].y = fmaf(av[a].x, bv[b].y, fmaf(av[a].y, bv[b].x, acc[a][b].y));
       }
   }
+  if (INPLACE) __syncthreads();
 #pragma unroll
   for (int a = 0; a < T; a++)
 #pragma unroll
@@ -242,19 +179,19 @@ __device__ __forceinline__ void cmatmul(const float2 *A, uint32_t lda, const flo
 }
 
 // K <= MM / 2: MM = 64 covers K <= 32, MM = 128 covers K <= 64
-template <int MM, bool HERM = false, typename Out>
+template <int MM, bool HERM = false, bool INPLACE = false, typename Out>
 __device__ __forceinline__ void cmatmul_any(const float2 *A, uint32_t lda, const float2 *B, uint32_t ldb,
                                             uint32_t K, Out out) {
   if (MM == 64) {
     if (K <= 16)
-      cmatmul<1, HERM>(A, lda, B, ldb, K, out);
+      cmatmul<1, HERM, INPLACE>(A, lda, B, ldb, K, out);
     else
-      cmatmul<2, HERM>(A, lda, B, ldb, K, out);
+      cmatmul<2, HERM, INPLACE>(A, lda, B, ldb, K, out);
   } else {
     if (K <= 48)
-      cmatmul<3, HERM>(A, lda, B, ldb, K, out);
+      cmatmul<3, HERM, INPLACE>(A, lda, B, ldb, K, out);
     else
-      cmatmul<4, HERM>(A, lda, B, ldb, K, out);
+      cmatmul<4, HERM, INPLACE>(A, lda, B, ldb, K, out);
   }
 }
 
@@ -440,13 +377,13 @@ __device__ __forceinline__ void sq_readout(uint32_t tmem, F f) {
 // of the detector image), otherwise the caller falls back to the exact
 // inverse.  The network: BF16 weights and activations into every product,
 // FP32 accumulation, ReLU hidden layers (the arithmetic of mb_mlp_forward).
-// Result in Xs.  This CUDA-core form serves 32 < K <= 64 (MM = 128); for
+// Result in Xs; P2 and Ts may be one buffer.  This CUDA-core form serves 32 < K <= 64 (MM = 128); for
 // K <= 32 the kernel takes the same steps with its products on the tensor
 // cores (the sq_* helpers above).
 template <int MM>
-__device__ bool poly_init(const float2 *Gs, uint32_t ld, float2 *Xs, float2 *P2, float2 *P3, float2 *Ts,
-                          float2 *Xn, uint32_t K, uint32_t M, const ZfNetView &net, uint32_t ns_iters,
-                          float *sred, float *act, float *coef) {
+__device__ bool poly_init(const float2 *Gs, uint32_t ld, float2 *Xs, float2 *P2, float2 *Ts, uint32_t K,
+                          uint32_t M, const ZfNetView &net, uint32_t ns_iters, float *sred, float *act,
+                          float *coef) {
   const int tid = threadIdx.x;
   // tau and the diagonal's range
   float d = 0.f, z1 = 0.f, z2 = 0.f, dmin = INFINITY, dmax = -INFINITY;
@@ -488,27 +425,21 @@ __device__ bool poly_init(const float2 *Gs, uint32_t ld, float2 *Xs, float2 *P2,
   __syncthreads();
   zf_net_eval(net, act, coef);
   const float c0 = coef[8], c1 = coef[9], c2 = coef[10], c3 = coef[11];
-  // Gn^3 = Gn Gn^2 (Hermitian)
-  cmatmul_any<MM, true>(Gs, ld, P2, K, K,
-                        [&](uint32_t i, uint32_t j, float2 s) { P3[i * K + j] = make_float2(s.x * it, s.y * it); });
-  __syncthreads();
-  for (uint32_t e = tid; e < K * K; e += kThreads) {
-    const uint32_t i = e / K, j = e % K;
-    const float2 g = Gs[i * ld + j], p2 = P2[e], p3 = P3[e];
-    const float re = (i == j ? c0 : 0.f) + c1 * g.x * it + c2 * p2.x + c3 * p3.x;
-    const float im = c1 * g.y * it + c2 * p2.y + c3 * p3.y;
+  // X0 from Gn^3 = Gn Gn^2 (Hermitian) as it comes out of the product
+  cmatmul_any<MM, true>(Gs, ld, P2, K, K, [&](uint32_t i, uint32_t j, float2 s) {
+    const float2 g = Gs[i * ld + j], p2 = P2[i * K + j];
+    const float re = (i == j ? c0 : 0.f) + c1 * g.x * it + c2 * p2.x + c3 * (s.x * it);
+    const float im = c1 * g.y * it + c2 * p2.y + c3 * (s.y * it);
     Xs[i * ld + j] = make_float2(re * it, im * it);
-  }
+  });
   __syncthreads();
-  float2 *xc = Xs, *xn = Xn;
-  uint32_t ldc = ld, ldn = K;
   float e_last = INFINITY;
   // ns_iters steps, then up to two more only to rescue a near miss
   // (0.04 < ||E|| < 0.3); a start further off goes to the exact inverse
   for (uint32_t s = 0; s < ns_iters + 2; s++) {
     if (s >= ns_iters && (e_last <= kPolyAccept || e_last >= 0.3f)) break;  // uniform
     float en = 0.f;
-    cmatmul_any<MM, true>(Gs, ld, xc, ldc, K, [&](uint32_t i, uint32_t j, float2 v) {
+    cmatmul_any<MM, true>(Gs, ld, Xs, ld, K, [&](uint32_t i, uint32_t j, float2 v) {
       const float ex = (i == j ? 1.f : 0.f) - v.x, ey = -v.y;  // E = I - G X; T = I + E
       en += ex * ex + ey * ey;
       Ts[i * K + j] = make_float2((i == j ? 1.f : 0.f) + ex, ey);
@@ -517,17 +448,7 @@ __device__ bool poly_init(const float2 *Gs, uint32_t ld, float2 *Xs, float2 *P2,
     block_reduce5(en, u0, u1, m0, m1, sred);  // also orders the Ts writes before their reads
     e_last = sqrtf(en);
     if (!(e_last < 1.f)) return false;  // uniform: the iteration would not converge
-    cmatmul_any<MM, true>(xc, ldc, Ts, K, K, [&](uint32_t i, uint32_t j, float2 v) { xn[i * ldn + j] = v; });
-    __syncthreads();
-    float2 *t = xc;
-    xc = xn;
-    xn = t;
-    const uint32_t l = ldc;
-    ldc = ldn;
-    ldn = l;
-  }
-  if (xc != Xs) {
-    for (uint32_t e = tid; e < K * K; e += kThreads) Xs[(e / K) * ld + e % K] = xc[e];
+    cmatmul_any<MM, true, true>(Xs, ld, Ts, K, K, [&](uint32_t i, uint32_t j, float2 v) { Xs[i * ld + j] = v; });
     __syncthreads();
   }
   return e_last <= kPolyAccept;
@@ -538,8 +459,10 @@ __device__ bool poly_init(const float2 *Gs, uint32_t ld, float2 *Xs, float2 *P2,
 // shared memory and equalizes the group's symbols (modulation order QMF)
 // from the planar BF16 samples that ymap describes
 template <int MM, int QMF>
-__global__ void __launch_bounds__(kThreads, MM == 64 ? 2 : 1)
+__global__ void __launch_bounds__(kThreads, 2)
     zf_mixed_kernel(const ZfmParams q, const __grid_constant__ CUtensorMap ymap) {
+  // two CTAs per SM in every form: with one, 205 groups of 256 x 64 took two
+  // waves, the second with 57 of 148 SMs busy (184 us; 130 us with two)
   static_assert(QMF == 0 || MM == 64, "the fused equalize needs K <= 32");
   extern __shared__ __align__(1024) uint8_t zsm[];
   __shared__ __align__(8) uint64_t tile_bar[2];
@@ -564,9 +487,16 @@ __global__ void __launch_bounds__(kThreads, MM == 64 ? 2 : 1)
   const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
   const uint32_t ld = K + 1;
   const uint32_t HS = q.resident ? nh : 2;  // hi-tile slots
-  // shared memory carve-up
-  uint8_t *hi_base = zsm;
-  uint8_t *lo_t[2] = {zsm + HS * tile_bytes, zsm + (HS + 1) * tile_bytes};
+  // shared memory carve-up.  MM == 128 (K <= 64): G, then X, then a third
+  // region; the tiles of the Gram (two hi slots over X, two lo behind them)
+  // are done when G is written, T = 2I - G X (and Gn^2 of the learned start)
+  // takes the third region, products update X in place, R(X) then takes T's
+  // place and the rebuilt hi tiles of W = X C take X's: 98 KB at K = 64, two
+  // CTAs per SM.
+  const uint32_t gx_bytes = MM == 64 ? 0 : zfm_gx_bytes(K);
+  uint8_t *hi_base = zsm + (MM == 64 ? 0 : gx_bytes);
+  uint8_t *lo_base = MM == 64 ? zsm + HS * tile_bytes : zsm + gx_bytes + zfm_x_bytes(K);
+  uint8_t *lo_t[2] = {lo_base, lo_base + tile_bytes};
   // MM == 64 (K <= 32): behind the tiles the split images of Gn = G / tau
   // and of the iterate Y = tau X, then G (K x ld), then K x ld float2 more
   // (the FP64 fallback's Gram spans both) that hold the network's weights
@@ -574,21 +504,16 @@ __global__ void __launch_bounds__(kThreads, MM == 64 ? 2 : 1)
   // (16 < K <= 32) X of the exact start and the residual's image go in the
   // lo tiles and W = X C reads the iterate's hi image; with the CUDA-core
   // products (K <= 16: a 16 x 16 product is a fraction of one tensor-core
-  // round trip) X and the powers Gn^2, Gn^3 take the Gn images' place and
-  // R(X) the iterate's.
+  // round trip) X and the power Gn^2 take the Gn images' place and R(X) the
+  // iterate's.
   const bool tcns = MM == 64 && q.tcns;  // uniform
   uint8_t *gn_img = zsm + (HS + 2) * tile_bytes;
   uint8_t *y_img = gn_img + 2 * kSqImg;
-  // MM == 128: R(X) (MM x MM BF16), G, X, and the powers Gn^2, Gn^3 of the
-  // learned initial iterate (allotted only when the kernel runs learned);
-  // Newton-Schulz temporaries (leading dim K): T in the lo tiles, the other
-  // iterate in the R(X) image (both free between the Gram and W = X C)
-  uint8_t *ximg = MM == 64 ? y_img : zsm + (HS + 2) * tile_bytes;
-  float2 *Gs = reinterpret_cast<float2 *>(MM == 64 ? y_img + 2 * kSqImg : ximg + MM * MM * 2);
-  float2 *Xs = MM == 64 ? reinterpret_cast<float2 *>(tcns ? lo_t[0] : gn_img) : Gs + K * ld;
+  uint8_t *ximg = MM == 64 ? y_img : lo_base;
+  float2 *Gs = reinterpret_cast<float2 *>(MM == 64 ? y_img + 2 * kSqImg : zsm);
+  float2 *Xs = reinterpret_cast<float2 *>(MM == 64 ? (tcns ? lo_t[0] : gn_img) : hi_base);
   float2 *Ts = reinterpret_cast<float2 *>(lo_t[0]);
-  float2 *Xn = reinterpret_cast<float2 *>(ximg);
-  float2 *P2 = Xs + K * ld, *P3 = P2 + K * K;
+  float2 *P2 = MM == 64 ? Xs + K * ld : Ts;
   uint8_t *wsm = reinterpret_cast<uint8_t *>(Gs + K * ld);
 
   float2 *cg = q.csi + (uint64_t)g * M * K;
@@ -645,8 +570,10 @@ __global__ void __launch_bounds__(kThreads, MM == 64 ? 2 : 1)
     }
   }
   // rows 2K..MM-1 of the R(C) tiles are padding: zero them once
-  for (uint32_t c = tid; c < (HS + 2) * tile_bytes / 16; c += kThreads)
-    reinterpret_cast<uint4 *>(zsm)[c] = make_uint4(0, 0, 0, 0);
+  for (uint32_t c = tid; c < HS * tile_bytes / 16; c += kThreads)
+    reinterpret_cast<uint4 *>(hi_base)[c] = make_uint4(0, 0, 0, 0);
+  for (uint32_t c = tid; c < 2 * tile_bytes / 16; c += kThreads)
+    reinterpret_cast<uint4 *>(lo_base)[c] = make_uint4(0, 0, 0, 0);
   if (warp == 0) tc::tmem_alloc(&tmem_slot, TC);
   tc::fence_before_sync();
   __syncthreads();
@@ -1024,7 +951,7 @@ __global__ void __launch_bounds__(kThreads, MM == 64 ? 2 : 1)
     } else {
       bool pd = false;
       if (q.learned)
-        used_learned = poly_init<MM>(Gs, ld, Xs, P2, P3, Ts, Xn, K, M, netv, q.ns_iters, zi_red, zi_act, zi_coef);
+        used_learned = poly_init<MM>(Gs, ld, Xs, P2, Ts, K, M, netv, q.ns_iters, zi_red, zi_act, zi_coef);
       if (!used_learned) {
         if (MM == 64)
           pd = K <= 16 ? gj_inverse<16>(Gs, Xs, K, ld, prow, &piv_bad)
@@ -1033,27 +960,15 @@ __global__ void __launch_bounds__(kThreads, MM == 64 ? 2 : 1)
           pd = gj_inverse<64>(Gs, Xs, K, ld, prow, &piv_bad);
       }
       if (pd) {
-        // Newton-Schulz: T = 2I - G X; X <- X T, ping-ponging Xs and Xn
-        float2 *xc = Xs, *xn = Xn;
-        uint32_t ldc = ld, ldn = K;
+        // Newton-Schulz: T = 2I - G X; X <- X T in place
         for (uint32_t it = 0; it < q.ns_iters; it++) {
-          cmatmul_any<MM>(Gs, ld, xc, ldc, K, [&](uint32_t i, uint32_t j, float2 s) {
+          cmatmul_any<MM>(Gs, ld, Xs, ld, K, [&](uint32_t i, uint32_t j, float2 s) {
             Ts[i * K + j] = make_float2((i == j ? 2.f : 0.f) - s.x, -s.y);
           });
           __syncthreads();
           // X T = 2X - X G X is Hermitian for Hermitian X: upper blocks only
-          cmatmul_any<MM, true>(xc, ldc, Ts, K, K,
-                                [&](uint32_t i, uint32_t j, float2 s) { xn[i * ldn + j] = s; });
-          __syncthreads();
-          float2 *t = xc;
-          xc = xn;
-          xn = t;
-          const uint32_t l = ldc;
-          ldc = ldn;
-          ldn = l;
-        }
-        if (xc != Xs) {
-          for (uint32_t e = tid; e < K * K; e += kThreads) Xs[(e / K) * ld + e % K] = xc[e];
+          cmatmul_any<MM, true, true>(Xs, ld, Ts, K, K,
+                                      [&](uint32_t i, uint32_t j, float2 s) { Xs[i * ld + j] = s; });
           __syncthreads();
         }
       }
@@ -1122,7 +1037,17 @@ __global__ void __launch_bounds__(kThreads, MM == 64 ? 2 : 1)
       }
       tc::fence_proxy_async_smem();
       __syncthreads();
+      // the hi slots' padding rows 2K..MM-1 held X: zero again
+      if (MM == 128)
+        for (uint32_t e = tid; e < HS * (MM - 2 * K) * 8; e += kThreads) {
+          const uint32_t r = 2 * K + e / 8 % (MM - 2 * K), sl = e / 8 / (MM - 2 * K);
+          *reinterpret_cast<uint4 *>(hi_base + sl * tile_bytes + img_off(r, e % 8 * 8, MM)) = make_uint4(0, 0, 0, 0);
+        }
     }
+    // tiles that did not stay in shared memory are rebuilt from the CSI, the
+    // next one's loads in flight while the current one is multiplied
+    float2 pf[kIpt][8];
+    if (!q.resident) load_items(0, pf);
     const uint32_t idesc_w = tc::idesc_bf16(MM, kKT, false, true);
     for (uint32_t kt0 = 0; kt0 < nh && ok; kt0 += TCH) {
       const uint32_t nt = min(TCH, nh - kt0);
@@ -1132,17 +1057,17 @@ __global__ void __launch_bounds__(kThreads, MM == 64 ? 2 : 1)
         if (q.resident) {
           hi = hi_base + (kt0 + t) * tile_bytes;
         } else {
-          // rebuild the hi tile from the CSI (not yet overwritten: W rows
-          // of a tile are stored only after all of its pass is multiplied)
+          // rebuild the hi tile from the CSI (not yet overwritten: W rows of
+          // a tile are stored after all of its pass is multiplied, and the
+          // tile loaded ahead belongs to this pass or the next)
           s = tiles_used % 2;
           const uint32_t use = tiles_used / 2;
           tiles_used++;
           if (use >= 1 && !tc::mbar_wait(&tile_bar[s], (use - 1) & 1)) ok = false;
           if (__syncthreads_or(!ok)) break;
           hi = hi_base + s * tile_bytes;
-          float2 pf[kIpt][8];
-          load_items(kt0 + t, pf);
           store_items(pf, hi, nullptr);
+          if (kt0 + t + 1 < nh) load_items(kt0 + t + 1, pf);
           tc::fence_proxy_async_smem();
           __syncthreads();
         }
@@ -1394,7 +1319,7 @@ static size_t zfm_smem(uint32_t K, uint32_t MM, uint32_t hi_slots, bool learned,
     }
     return (hi_slots + 2) * tile + 4 * (size_t)kSqImg + gk + std::max(gk, net);
   }
-  return (hi_slots + 2) * tile + (size_t)MM * MM * 2 + 2 * gk + (learned ? 2 * (size_t)K * K * sizeof(float2) : 0);
+  return zfm_gx_bytes(K) + zfm_x_bytes(K) + 2 * tile;
 }
 
 uint64_t zf_mixed_scratch_bytes(uint32_t groups, uint32_t M, uint32_t K) {
@@ -1513,7 +1438,8 @@ static mb_status zf_mixed_launch(float2 *csi, void *img_w, uint32_t groups, uint
   const size_t avail = (size_t)maxs - (size_t)static_smem[which].load();
   // keep every hi tile in shared memory when it fits, else stream two
   const uint32_t width = learned ? net->width : 0;
-  q.resident = zfm_smem(K, s.MM, q.nh, learned, width) <= avail ? 1 : 0;
+  // (MM == 128: always streamed, so that two CTAs share an SM)
+  q.resident = s.MM == 64 && zfm_smem(K, s.MM, q.nh, learned, width) <= avail ? 1 : 0;
   q.write_w = write_w ? 1 : 0;
   size_t smem = zfm_smem(K, s.MM, q.resident ? q.nh : 2, learned, width);
   if (qmf) {
