@@ -31,7 +31,6 @@
 #include <atomic>
 
 #include "common.cuh"
-#include "eq_common.cuh"
 #include "eq_tc.cuh"
 #include "eq_tc_epi.cuh"
 #include "sgemv.cuh"

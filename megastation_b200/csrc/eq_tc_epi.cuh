@@ -108,7 +108,7 @@ struct EqTcEpilogue {
       for (int j = 0; j < 8; j++) {
         if (ch * 8 + j >= p.K) break;
         const float2 x = make_float2(v[2 * j], v[2 * j + 1]);
-        __half2 lv[QM / 2];  // (Re, Im) pairs, bit-identical to demod()
+        __half2 lv[QM / 2];  // (Re, Im) pairs
         demod2<QM>(x, lv);
         if (llr_on) {
           if (pair) {
