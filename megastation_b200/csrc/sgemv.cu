@@ -265,22 +265,24 @@ __global__ void __launch_bounds__(256) precode_kernel(const PcParams p) {
   const uint32_t nl = min(p.L, p.n_sym - l0);
   const uint32_t b_base = blockIdx.z * BT * TB;
   const int tid = threadIdx.x, tc = tid % CT, tb = tid / CT;
-  if (g == G) {
+  {
     // guard bins: subcarrier indices i in [S, N) map to the bins
-    // (i + start + N/2) % N, one run of N - S bins per row that may wrap
-    // around N: zero the runs of this CTA's rows, a warp per row
+    // (i + start + N/2) % N; every group's CTA zeroes its share of them in its
+    // own rows (one CTA per row block for all of them was the launch's tail:
+    // 5.2 of 12.6 MB from 8 CTAs at 6 symbols of 128 antennas, N = 2048)
     const uint32_t nb = min((uint32_t)(BT * TB), p.M - b_base);
-    const uint32_t ng = p.N - p.S;
-    const uint32_t k0 = (p.S + p.start + p.N / 2) % p.N;
-    const uint32_t n1 = min(ng, p.N - k0);  // bins k0 .. k0 + n1 - 1, then 0 .. ng - n1 - 1
-    const int warp = tid / 32, lane = tid % 32;
-    for (uint32_t r = warp; r < nl * nb; r += blockDim.x / 32) {
-      const uint32_t b = b_base + r % nb, l = l0 + r / nb;
-      float2 *row = p.out + ((uint64_t)l * p.M + b) * p.N;
-      for (uint32_t e = lane; e < n1; e += 32) row[k0 + e] = make_float2(0.f, 0.f);
-      for (uint32_t e = lane; e < ng - n1; e += 32) row[e] = make_float2(0.f, 0.f);
+    const uint64_t ng = p.N - p.S;
+    const uint32_t e0 = (uint32_t)(ng * g / G), n = (uint32_t)(ng * (g + 1) / G) - e0;
+    const uint32_t k0 = (p.S + e0 + p.start + p.N / 2) % p.N;
+    uint32_t w = 1;  // lanes per row: a power of two up to 32
+    while (w < n && w < 32) w *= 2;
+    for (uint32_t r = tid / w; r < nl * nb; r += blockDim.x / w) {
+      float2 *row = p.out + ((uint64_t)(l0 + r / nb) * p.M + b_base + r % nb) * p.N;
+      for (uint32_t e = tid % w; e < n; e += w) {
+        const uint32_t k = k0 + e;
+        row[k < p.N ? k : k - p.N] = make_float2(0.f, 0.f);
+      }
     }
-    return;
   }
   const uint32_t s_begin = g * p.sg;
   const uint32_t ns = min(p.sg, p.S - s_begin);
@@ -346,7 +348,7 @@ mb_status precode_fp32(const float2 *P, const float2 *s, float2 *out,
   const uint32_t ncols = L * sg;
   const uint32_t G = (S + sg - 1) / sg;
   constexpr int TB = 4;
-  dim3 grid(G + 1, (n_sym + L - 1) / L, (M + 8 * TB - 1) / (8 * TB));
+  dim3 grid(G, (n_sym + L - 1) / L, (M + 8 * TB - 1) / (8 * TB));
   if (ncols <= 32)
     precode_kernel<TB, 1><<<grid, 256, 0, st>>>(p);
   else if (ncols <= 64)
