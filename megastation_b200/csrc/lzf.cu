@@ -32,6 +32,8 @@
 #include <vector>
 
 #include "common.cuh"
+#include "gj.cuh"
+#include "mlp_step.cuh"
 
 namespace mb {
 namespace {
@@ -155,16 +157,6 @@ __global__ void inverse_kernel(const typename CT<T>::V *src, const uint32_t *idx
     X[(uint64_t)i * K * K + e] = A[(e / K) * W + K + e % K];
 }
 
-// Gc[g] = Gs[centre(g)]
-__global__ void gather_kernel(const float2 *Gs, const uint32_t *cidx, float2 *Gc, uint32_t K, uint32_t G) {
-  const uint64_t total = (uint64_t)G * K * K;
-  for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < total;
-       e += (uint64_t)gridDim.x * blockDim.x) {
-    const uint32_t g = (uint32_t)(e / (K * K)), r = (uint32_t)(e % (K * K));
-    Gc[e] = Gs[(uint64_t)cidx[g] * K * K + r];
-  }
-}
-
 // ||I - G_s X_s||_F per subcarrier
 __global__ void residual_kernel(const float2 *Gm, const float2 *X, float *res, uint32_t K, uint32_t S) {
   const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -217,18 +209,78 @@ __device__ __forceinline__ void interp_pos(uint32_t s, uint32_t u, uint32_t sg, 
   t = G > 1 ? fminf(fmaxf((float)(num - g0 * (int)sg) / (float)sg, 0.f), 1.f) : 0.f;
 }
 
-// c_s [M][K] of subcarrier s into shared memory; ig / iw: per (s, u) the
-// lower pilot group and the weight of the upper one (interp_pos, tabulated)
+// Rows of the CSI staged in shared memory are ldc(K) long: the next even
+// number (16-byte loads of two users) plus one 16-byte chunk, so that
+// neighbouring antennas sit in different banks; K < 8 keeps K.
+__host__ __device__ constexpr uint32_t ldc_of(uint32_t K) { return K < 8 ? K : (K + 1) / 2 * 2 + 2; }
+
+// elements i and i + 1 (vec: i is even and a 16-byte load will do)
+__device__ __forceinline__ float4 pair_at(const float2 *p, bool vec) {
+  if (vec) return *reinterpret_cast<const float4 *>(p);
+  return make_float4(p[0].x, p[0].y, p[1].x, p[1].y);
+}
+
+// c_s [M][ldc] of subcarrier s into shared memory; ig / iw: per (s, u) the
+// lower pilot group and the weight of the upper one (interp_pos, tabulated).
+// A thread keeps one user; the element past a row's users is 0 for K odd.
 __device__ __forceinline__ void interp_smem(const float2 *csi, const int *ig, const float *iw, float2 *c,
-                                            uint32_t s, uint32_t M, uint32_t K, uint32_t G) {
-  for (uint32_t e = threadIdx.x; e < M * K; e += blockDim.x) {
-    const uint32_t b = e / K, u = e % K;
-    const int g0 = ig[s * K + u];
-    const float t = iw[s * K + u];
-    const float2 a = csi[((uint64_t)g0 * M + b) * K + u];
-    const float2 d = G > 1 ? csi[((uint64_t)(g0 + 1) * M + b) * K + u] : a;
-    c[e] = make_float2((1.f - t) * a.x + t * d.x, (1.f - t) * a.y + t * d.y);
+                                            uint32_t s, uint32_t M, uint32_t K, uint32_t G, uint32_t ldc) {
+  uint32_t kp = 1;
+  while (kp < K) kp *= 2;
+  const uint32_t u = threadIdx.x % kp, step = blockDim.x / kp;
+  if (u >= K) {
+    if (u == K && ldc > K)
+      for (uint32_t b = threadIdx.x / kp; b < M; b += step) c[b * ldc + u] = make_float2(0.f, 0.f);
+    return;
   }
+  const int g0 = ig[s * K + u];
+  const float t = iw[s * K + u];
+  const float2 *lo = csi + (uint64_t)g0 * M * K + u, *hi = G > 1 ? lo + (uint64_t)M * K : lo;
+#pragma unroll 8
+  for (uint32_t b = threadIdx.x / kp; b < M; b += step) {
+    const float2 a = __ldg(lo + (uint64_t)b * K), d = __ldg(hi + (uint64_t)b * K);
+    c[b * ldc + u] = make_float2((1.f - t) * a.x + t * d.x, (1.f - t) * a.y + t * d.y);
+  }
+}
+
+// The Gram of the staged CSI into gm [K][K] (in shared memory): 2 x 2 outputs
+// a thread, the antennas split over up to four groups of threads whose sums
+// meet in gm, b1, b2, b3 ([K][K] scratch each).  All threads.
+__device__ __forceinline__ void gram_smem(const float2 *c, float2 *gm, float2 *b1, float2 *b2, float2 *b3, uint32_t M,
+                                          uint32_t K, uint32_t ldc) {
+  const uint32_t T2 = (K + 1) / 2, nt = T2 * T2, parts = min(4u, blockDim.x / nt), tid = threadIdx.x;
+  const uint32_t part = tid / nt, u = tid % nt / T2 * 2, v = tid % T2 * 2;
+  const bool vec = ldc % 2 == 0;
+  if (part < parts) {
+    float2 a[2][2] = {{cz<float2>(), cz<float2>()}, {cz<float2>(), cz<float2>()}};
+#pragma unroll 4
+    for (uint32_t b = part; b < M; b += parts) {
+      const float4 cu = pair_at(c + b * ldc + u, vec), cv = pair_at(c + b * ldc + v, vec);
+      const float2 u0 = make_float2(cu.x, cu.y), u1 = make_float2(cu.z, cu.w);
+      const float2 v0 = make_float2(cv.x, cv.y), v1 = make_float2(cv.z, cv.w);
+      a[0][0] = cjfma(v0, u0, a[0][0]);
+      a[0][1] = cjfma(v1, u0, a[0][1]);
+      a[1][0] = cjfma(v0, u1, a[1][0]);
+      a[1][1] = cjfma(v1, u1, a[1][1]);
+    }
+    float2 *d = part == 0 ? gm : part == 1 ? b1 : part == 2 ? b2 : b3;
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+#pragma unroll
+      for (int j = 0; j < 2; j++)
+        if (u + i < K && v + j < K) d[(u + i) * K + v + j] = a[i][j];
+  }
+  __syncthreads();
+  for (uint32_t e = tid; parts > 1 && e < K * K; e += blockDim.x) {
+    float2 s = gm[e];
+    for (uint32_t q = 1; q < parts; q++) {
+      const float2 w = (q == 1 ? b1 : q == 2 ? b2 : b3)[e];
+      s.x += w.x;
+      s.y += w.y;
+    }
+    gm[e] = s;
+  }
+  __syncthreads();
 }
 
 __global__ void interp_table_kernel(int *ig, float *iw, uint32_t K, uint32_t S, uint32_t sg, uint32_t G) {
@@ -241,62 +293,23 @@ __global__ void interp_table_kernel(int *ig, float *iw, uint32_t K, uint32_t S, 
   iw[e] = t;
 }
 
-// Gauss-Jordan inverse of the K x K matrix in the first K columns of A
-// (K x 2K, row-major, the right half set to I by the caller) by all
-// threads; returns false when a pivot is not positive
-template <typename V, typename T>
-__device__ bool gj_smem(V *A, uint32_t K, int *bad) {
-  const uint32_t W = 2 * K;
-  if (threadIdx.x == 0) *bad = 0;
-  __syncthreads();
-  for (uint32_t k = 0; k < K; k++) {
-    const T p = A[k * W + k].x;
-    if (!(p > (T)0)) {
-      if (threadIdx.x == 0) *bad = 1;
-      break;  // uniform: every thread read the same pivot
-    }
-    const T inv = (T)1 / p;
-    __syncthreads();
-    for (uint32_t c = threadIdx.x; c < W; c += blockDim.x) {
-      V v = A[k * W + c];
-      v.x *= inv;
-      v.y *= inv;
-      A[k * W + c] = v;
-    }
-    __syncthreads();
-    for (uint32_t e = threadIdx.x; e < K * W; e += blockDim.x) {
-      const uint32_t r = e / W, c = e % W;
-      if (r == k || c == k) continue;
-      const V f = A[r * W + k];
-      const V rk = A[k * W + c];
-      V v = A[r * W + c];
-      v.x -= f.x * rk.x - f.y * rk.y;
-      v.y -= f.x * rk.y + f.y * rk.x;
-      A[r * W + c] = v;
-    }
-    __syncthreads();
-    for (uint32_t r = threadIdx.x; r < K; r += blockDim.x)
-      if (r != k) A[r * W + k] = cz<V>();
-    __syncthreads();
-  }
-  __syncthreads();
-  return *bad == 0;
-}
-
-// per subcarrier: interpolated CSI in shared memory, then its Gram
-__global__ void sub_gram_kernel(const float2 *csi, const int *ig, const float *iw, float2 *Gm, uint32_t M,
-                                uint32_t K, uint32_t G) {
+// The Gram at each group's centre subcarrier and its inverse, a CTA per group
+__global__ void __launch_bounds__(256) centre_kernel(const float2 *csi, const int *ig, const float *iw,
+                                                     const uint32_t *cidx, float2 *Gc, float2 *Xc, uint32_t M,
+                                                     uint32_t K, uint32_t G, int *flag) {
   extern __shared__ __align__(16) unsigned char sgm[];
-  float2 *c = reinterpret_cast<float2 *>(sgm);
-  const uint32_t s = blockIdx.x;
-  interp_smem(csi, ig, iw, c, s, M, K, G);
+  __shared__ int bad;
+  const uint32_t g = blockIdx.x, KK = K * K, ldc = ldc_of(K);
+  float2 *gm = reinterpret_cast<float2 *>(sgm), *b1 = gm + KK, *b2 = b1 + KK, *b3 = b2 + KK, *c = b3 + KK;
+  if (threadIdx.x == 0) bad = 0;
+  interp_smem(csi, ig, iw, c, cidx[g], M, K, G, ldc);
   __syncthreads();
-  for (uint32_t e = threadIdx.x; e < K * K; e += blockDim.x) {
-    const uint32_t u = e / K, v = e % K;
-    float2 acc = make_float2(0.f, 0.f);
-    for (uint32_t b = 0; b < M; b++) acc = cjfma(c[b * K + v], c[b * K + u], acc);
-    Gm[(uint64_t)s * K * K + e] = acc;
-  }
+  gram_smem(c, gm, b1, b2, b3, M, K, ldc);
+  for (uint32_t e = threadIdx.x; e < KK; e += blockDim.x) Gc[(uint64_t)g * KK + e] = gm[e];
+  float2 *prow = c + M * ldc + 2;
+  const bool ok = K <= 16 ? gj_inverse<16>(gm, b1, K, K, prow, &bad) : gj_inverse<32>(gm, b1, K, K, prow, &bad);
+  if (threadIdx.x == 0 && flag) flag[g] = ok ? 0 : 1;
+  for (uint32_t e = threadIdx.x; e < KK; e += blockDim.x) Xc[(uint64_t)g * KK + e] = b1[e];
 }
 
 // per group g: ||Gc[g]||_F, and for j = -1, +1, +2 the relative distance
@@ -349,32 +362,41 @@ __global__ void features2_kernel(const float *st, float *F, uint32_t S, uint32_t
   }
 }
 
-// per subcarrier: initial iterate (coarse / learned blend / exact
+// per subcarrier: interpolated CSI, its Gram (kept for the residual
+// diagnostic), the initial iterate (coarse / learned blend / exact
 // Gauss-Jordan), Newton-Schulz steps, then the detector W_s = X C, all in
-// shared memory; X is also stored for the residual diagnostic
-__global__ void sub_detect_kernel(const float2 *csi, const int *ig, const float *iw, const float2 *Gm,
-                                  const float2 *Xc, const float *alpha, int mode, uint32_t iters,
-                                  float2 *Xout, float2 *W, uint32_t M, uint32_t K, uint32_t sg,
-                                  uint32_t G, int *flag) {
+// shared memory with the CSI staged once; X is also stored for the residual.
+// FP32 and shared-memory bound: the Gram and W take 2 x 2 and 2 x 4 outputs a
+// thread with 16-byte loads.  1200 subcarriers of 128 x 16, two steps: 24 us
+// for a Gram kernel and 43 us for the rest, an output a thread; 50 us for
+// both here.
+__global__ void __launch_bounds__(256) sub_detect_kernel(const float2 *csi, const int *ig, const float *iw,
+                                                         float2 *Gm, const float2 *Xc, const float *alpha, int mode,
+                                                         uint32_t iters, float2 *Xout, float2 *W, uint32_t M,
+                                                         uint32_t K, uint32_t sg, uint32_t G, int *flag) {
   extern __shared__ __align__(16) unsigned char dsm[];
   __shared__ int bad;
-  const uint32_t KK = K * K;
-  float2 *g = reinterpret_cast<float2 *>(dsm), *x = g + KK, *t = x + KK, *aug = t + KK;
-  float2 *c = aug;  // K x 2K for the exact inverse, then M x K of CSI
+  __shared__ float e0sq;  // ||I - G X0||_F^2 of the initial iterate
+  const uint32_t KK = K * K, ldc = ldc_of(K), tid = threadIdx.x;
+  float2 *g = reinterpret_cast<float2 *>(dsm), *x = g + KK, *t = x + KK, *r4 = t + KK;
+  float2 *c = r4 + KK, *prow = c + M * ldc + 2;
   const uint32_t s = blockIdx.x, grp = s / sg;
-  for (uint32_t e = threadIdx.x; e < KK; e += blockDim.x) g[e] = Gm[(uint64_t)s * KK + e];
+  if (tid == 0) {
+    bad = 0;
+    e0sq = 0.f;
+  }
+  interp_smem(csi, ig, iw, c, s, M, K, G, ldc);
+  __syncthreads();
+  gram_smem(c, g, x, t, r4, M, K, ldc);
+  for (uint32_t e = tid; e < KK; e += blockDim.x) Gm[(uint64_t)s * KK + e] = g[e];
+  auto exact = [&]() {
+    return K <= 16 ? gj_inverse<16>(g, x, K, K, prow, &bad) : gj_inverse<32>(g, x, K, K, prow, &bad);
+  };
   if (mode == 2) {
-    __syncthreads();
-    for (uint32_t e = threadIdx.x; e < 2 * KK; e += blockDim.x) {
-      const uint32_t r = e / (2 * K), q = e % (2 * K);
-      aug[e] = q < K ? g[r * K + q] : make_float2(q - K == r ? 1.f : 0.f, 0.f);
-    }
-    __syncthreads();
-    const bool ok = gj_smem<float2, float>(aug, K, &bad);
-    if (threadIdx.x == 0 && flag) flag[s] = ok ? 0 : 1;
-    for (uint32_t e = threadIdx.x; e < KK; e += blockDim.x) x[e] = aug[(e / K) * 2 * K + K + e % K];
+    const bool ok = exact();
+    if (tid == 0 && flag) flag[s] = ok ? 0 : 1;
   } else {
-    for (uint32_t e = threadIdx.x; e < KK; e += blockDim.x) {
+    for (uint32_t e = tid; e < KK; e += blockDim.x) {
       float2 acc = make_float2(0.f, 0.f);
       if (mode == 0) {
         acc = Xc[(uint64_t)grp * KK + e];
@@ -389,18 +411,15 @@ __global__ void sub_detect_kernel(const float2 *csi, const int *ig, const float 
       }
       x[e] = acc;
     }
-  }
-  __shared__ float e0sq;  // ||I - G X0||_F^2 of the initial iterate
-  if (threadIdx.x == 0) {
-    e0sq = 0.f;
-    if (mode != 2 && flag) flag[s] = 0;
+    if (tid == 0 && flag) flag[s] = 0;
   }
   __syncthreads();
   for (uint32_t it = 0; it < iters; it++) {
     float part = 0.f;
-    for (uint32_t e = threadIdx.x; e < KK; e += blockDim.x) {
+    for (uint32_t e = tid; e < KK; e += blockDim.x) {
       const uint32_t r = e / K, q = e % K;
       float2 acc = make_float2(0.f, 0.f);
+#pragma unroll 8
       for (uint32_t k = 0; k < K; k++) acc = cfma(g[r * K + k], x[k * K + q], acc);
       t[e] = make_float2((r == q ? 2.f : 0.f) - acc.x, -acc.y);
       const float ex = (r == q ? 1.f : 0.f) - acc.x;
@@ -408,7 +427,7 @@ __global__ void sub_detect_kernel(const float2 *csi, const int *ig, const float 
     }
     if (it == 0 && mode != 2) {
       for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-      if ((threadIdx.x & 31) == 0) atomicAdd(&e0sq, part);
+      if ((tid & 31) == 0) atomicAdd(&e0sq, part);
     }
     __syncthreads();
     if (it == 0 && mode != 2 && !(e0sq < 1.f)) {
@@ -416,43 +435,84 @@ __global__ void sub_detect_kernel(const float2 *csi, const int *ig, const float 
       // off (the blend of neighbouring groups' inverses under a channel that
       // changes too fast across the band) takes the exact inverse instead,
       // flagged 2 (uniform: every thread read the same sum)
-      for (uint32_t e = threadIdx.x; e < 2 * KK; e += blockDim.x) {
-        const uint32_t r = e / (2 * K), q = e % (2 * K);
-        aug[e] = q < K ? g[r * K + q] : make_float2(q - K == r ? 1.f : 0.f, 0.f);
-      }
-      __syncthreads();
-      const bool ok = gj_smem<float2, float>(aug, K, &bad);
-      if (threadIdx.x == 0 && flag) flag[s] = ok ? 2 : 1;
-      for (uint32_t e = threadIdx.x; e < KK; e += blockDim.x) x[e] = aug[(e / K) * 2 * K + K + e % K];
-      __syncthreads();
+      const bool ok = exact();
+      if (tid == 0 && flag) flag[s] = ok ? 2 : 1;
       break;
     }
     float2 nx[4];
     uint32_t n = 0;
-    for (uint32_t e = threadIdx.x; e < KK; e += blockDim.x, n++) {
+    for (uint32_t e = tid; e < KK; e += blockDim.x, n++) {
       const uint32_t r = e / K, q = e % K;
       float2 acc = make_float2(0.f, 0.f);
+#pragma unroll 8
       for (uint32_t k = 0; k < K; k++) acc = cfma(x[r * K + k], t[k * K + q], acc);
       nx[n] = acc;
     }
     __syncthreads();
     n = 0;
-    for (uint32_t e = threadIdx.x; e < KK; e += blockDim.x, n++) x[e] = nx[n];
+    for (uint32_t e = tid; e < KK; e += blockDim.x, n++) x[e] = nx[n];
     __syncthreads();
   }
-  // X transposed into t (xt[v][u]) so that the lanes of a warp, which hold
-  // consecutive users u, read consecutive words
-  for (uint32_t e = threadIdx.x; e < KK; e += blockDim.x) {
-    if (Xout) Xout[(uint64_t)s * KK + e] = x[e];
-    t[(e % K) * K + e / K] = x[e];
+  // X transposed into xt [v][u] (rows of an even length): a thread's two
+  // users are neighbours
+  const uint32_t ldx = (K + 1) / 2 * 2;
+  float2 *xt = t;  // with r4 behind it: room for K odd's rows of K + 1 (K = 1: two entries)
+  for (uint32_t e = tid; e < KK; e += blockDim.x) {
+    const float2 v = x[e];
+    Xout[(uint64_t)s * KK + e] = v;
+    xt[(e % K) * ldx + e / K] = v;
   }
-  interp_smem(csi, ig, iw, c, s, M, K, G);
   __syncthreads();
-  for (uint32_t e = threadIdx.x; e < M * K; e += blockDim.x) {
-    const uint32_t b = e / K, u = e % K;
-    float2 acc = make_float2(0.f, 0.f);
-    for (uint32_t v = 0; v < K; v++) acc = cfma(t[v * K + u], c[b * K + v], acc);
-    W[(uint64_t)s * M * K + e] = acc;
+  const uint32_t T2 = (K + 1) / 2, nq = blockDim.x / T2, u = tid % T2 * 2, bq = tid / T2;
+  const bool vc = ldc % 2 == 0, two = u + 1 < K, w16 = K % 2 == 0 && (reinterpret_cast<uintptr_t>(W) & 15) == 0;
+  if (bq >= nq) return;
+  for (uint32_t b0 = bq; b0 < M; b0 += 4 * nq) {
+    float2 a[4][2];
+#pragma unroll
+    for (int i = 0; i < 4; i++) a[i][0] = a[i][1] = make_float2(0.f, 0.f);
+    auto step = [&](uint32_t v, const float2 (&cv)[4]) {
+      const float4 xv = pair_at(xt + v * ldx + u, true);
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        a[i][0] = cfma(make_float2(xv.x, xv.y), cv[i], a[i][0]);
+        a[i][1] = cfma(make_float2(xv.z, xv.w), cv[i], a[i][1]);
+      }
+    };
+    const float2 *cr[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) cr[i] = c + min(b0 + i * nq, M - 1) * ldc;
+    uint32_t v = 0;
+    if (vc)
+#pragma unroll 4
+      for (; v + 1 < K; v += 2) {
+        float2 c0[4], c1[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+          const float4 q = *reinterpret_cast<const float4 *>(cr[i] + v);
+          c0[i] = make_float2(q.x, q.y);
+          c1[i] = make_float2(q.z, q.w);
+        }
+        step(v, c0);
+        step(v + 1, c1);
+      }
+    for (; v < K; v++) {
+      float2 c0[4];
+#pragma unroll
+      for (int i = 0; i < 4; i++) c0[i] = cr[i][v];
+      step(v, c0);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const uint32_t b = b0 + i * nq;
+      if (b >= M) break;
+      float2 *w = W + ((uint64_t)s * M + b) * K + u;
+      if (w16) {
+        *reinterpret_cast<float4 *>(w) = make_float4(a[i][0].x, a[i][0].y, a[i][1].x, a[i][1].y);
+      } else {
+        w[0] = a[i][0];
+        if (two) w[1] = a[i][1];
+      }
+    }
   }
 }
 
@@ -535,27 +595,24 @@ extern "C" mb_status mb_lzf_create(uint32_t M, uint32_t K, uint32_t S, uint32_t 
 
 extern "C" uint32_t mb_lzf_num_features(uint32_t sg) { return sg + 6; }
 
-// interpolated CSI and Grams per subcarrier, centre Grams and their
-// inverses, per-group feature statistics (FP32)
+// four K x K matrices, the staged CSI and the pivot rows of the inverse
+static size_t detect_smem(const mb_lzf *z) {
+  return sizeof(float2) * (4 * (size_t)z->K * z->K + (size_t)z->M * ldc_of(z->K) + 2 + 64);
+}
+
+// centre Grams and their inverses, per-group feature statistics (FP32)
 static mb_status lzf_front(mb_lzf *z, const mb_c32 *csi, cudaStream_t st) {
-  const uint32_t M = z->M, K = z->K, S = z->S;
-  sub_gram_kernel<<<S, 256, sizeof(float2) * M * K, st>>>(reinterpret_cast<const float2 *>(csi), z->ig, z->iw,
-                                                          z->Gs, M, K, z->G);
-  gather_kernel<<<grid_for((uint64_t)z->G * K * K), 256, 0, st>>>(z->Gs, z->cidx, z->Gc, K, z->G);
-  inverse_kernel<float><<<z->G, 256, sizeof(float2) * 2 * K * K, st>>>(z->Gc, nullptr, z->Xc, K, z->flag);
+  const uint32_t M = z->M, K = z->K;
+  centre_kernel<<<z->G, 256, detect_smem(z), st>>>(reinterpret_cast<const float2 *>(csi), z->ig, z->iw, z->cidx,
+                                                   z->Gc, z->Xc, M, K, z->G, z->flag);
   group_stats_kernel<<<z->G, 256, 0, st>>>(z->Gc, z->stats, K, z->G);
   MB_CUDA_TRY(cudaGetLastError());
   return MB_OK;
 }
 
-static size_t detect_smem(const mb_lzf *z) {
-  return sizeof(float2) * (3 * (size_t)z->K * z->K + std::max<size_t>(2 * (size_t)z->K * z->K,
-                                                                     (size_t)z->M * z->K));
-}
-
 // The kernels that stage one subcarrier's M x K CSI in shared memory take
 // up to the device's opt-in limit (raised once per device): 256 x 32 needs
-// 64 KB (FP32 Gram), 88 KB (detector) and 128 KB (FP64 Gram of the targets).
+// 101 KB (detector) and 128 KB (FP64 Gram of the targets).
 static mb_status lzf_configure(size_t *limit) {
   static std::atomic<uint64_t> configured{0};
   static std::atomic<int> lim[64] = {};
@@ -565,7 +622,7 @@ static mb_status lzf_configure(size_t *limit) {
   if (!(configured.load() & bit)) {
     MB_CUDA_TRY(cudaDeviceGetAttribute(&maxs, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     int l = maxs;
-    const void *ks[3] = {(const void *)sub_gram_kernel, (const void *)sub_detect_kernel,
+    const void *ks[3] = {(const void *)centre_kernel, (const void *)sub_detect_kernel,
                          (const void *)gram_kernel<double>};
     for (const void *k : ks) {
       cudaFuncAttributes fa;
@@ -609,9 +666,13 @@ extern "C" mb_status mb_lzf_run(mb_lzf *z, const mb_c32 *csi, mb_mlp *mlp, int i
   mb_status r = lzf_front(z, csi, st);
   if (r != MB_OK) return r;
   if (init == MB_LZF_LEARNED) {
-    features2_kernel<<<grid_for((uint64_t)S * (z->sg + 6)), 256, 0, st>>>(z->stats, z->feat, S, z->sg);
-    MB_CUDA_TRY(cudaGetLastError());
-    r = mb_mlp_forward(mlp, z->feat, S, z->alpha, st);
+    // the features go straight into the network's input tiles where its shape allows
+    r = mlp_forward_stats(mlp, z->stats, z->sg, S, z->alpha, st);
+    if (r == MB_UNSUPPORTED) {
+      features2_kernel<<<grid_for((uint64_t)S * (z->sg + 6)), 256, 0, st>>>(z->stats, z->feat, S, z->sg);
+      MB_CUDA_TRY(cudaGetLastError());
+      r = mb_mlp_forward(mlp, z->feat, S, z->alpha, st);
+    }
     if (r != MB_OK) return r;
   }
   const size_t smem = detect_smem(z);
