@@ -22,16 +22,16 @@
 // positive = bit 0) into a __half2 array in shared memory with the graph's
 // entries; the rows in order as layers; per check node and block:
 // q_e = app - r_e (r_e the node's previous message to entry e, rebuilt from
-// its compressed state), min1 (first index), min2 and the parity of the
-// sign bits of q, then app = q_e + r'_e, r'_e = +-min(0.75 min, 256).  Rows
+// its compressed state), min1, min2 and the parity of the sign bits of q,
+// then app = q_e + r'_e, r'_e = +-min(0.75 min, 256).  Rows
 // of up to 20 entries keep q in registers (ldpc_node, variants for 4, 6, 10
 // and 20 entries).  FP16 is the reference decoder's precision (cuPHY), and
 // the pairs halve the instructions per block; channel LLRs clamped to
 // +-1024 and messages to +-256 keep every value finite for up to 32 passes.
 // Within a layer the Z check nodes touch disjoint variables (a circulant is
-// a permutation), so a layer needs one barrier.  The compressed state (min1,
-// min2, index, sign bits) per (layer, check node) lives in global memory,
-// loaded two layers ahead.  Every step is one IEEE FP16 operation, so the
+// a permutation), so a layer needs one barrier.  The compressed state (the two
+// message magnitudes, who takes the second, sign bits) per (layer, check node)
+// lives in global memory, loaded two layers ahead.  Every step is one IEEE FP16 operation, so the
 // results equal the float16 restatement bit for bit.
 #include <algorithm>
 #include <cstring>
@@ -191,141 +191,154 @@ __device__ __forceinline__ __half2 llr_clamp(__half2 v) {
   return __hmax2(__hmin2(v, __float2half2_rn(kLlrMax)), __float2half2_rn(-kLlrMax));
 }
 
-// A check node's state for the pair (one uint4 per layer and node):
-//   x, y  min1, min2 (__half2: |q| of each block)
-//   z     signs of q for entries 0..15: bit e block 0, bit 16 + e block 1
-//   w     signs for entries 16..26 in bits 0..10 / 16..26, and the index of
-//         min1 of block 0 in bits 11..15, of block 1 in bits 27..31
-// The interleaving puts both blocks' bits for entry e at the same distance
-// from bits 15 and 31, so one shift lines them up with the FP16 sign bits.
-// The node's messages rebuilt from the state:
-struct PairMsg {
-  uint32_t m1, m2;    // min(0.75 min1, kMsgMax), min(0.75 min2, kMsgMax) (__half2 bits)
-  uint32_t sgl, sgh;  // z / w with each block's sign parity applied: the message signs
-  uint32_t ohl, ohh;  // min1's index one-hot in the same interleaved layout
-};
-__device__ __forceinline__ PairMsg pair_msg(const uint4 &st) {
-  PairMsg m;
-  const __half2 a = __float2half2_rn(kAlpha);  // 0.75, exact in FP16
-  const __half2 cap = __float2half2_rn(kMsgMax);
-  m.m1 = h2u(__hmin2(__hmul2(a, u2h(st.x)), cap));
-  m.m2 = h2u(__hmin2(__hmul2(a, u2h(st.y)), cap));
-  const uint32_t par0 = (__popc(st.z & 0xFFFFu) + __popc(st.w & 0x7FFu)) & 1u;
-  const uint32_t par1 = (__popc(st.z >> 16) + __popc(st.w & 0x07FF0000u)) & 1u;
-  const uint32_t flip = (par0 ? 0x0000FFFFu : 0u) | (par1 ? 0xFFFF0000u : 0u);
-  m.sgl = st.z ^ flip;
-  m.sgh = st.w ^ flip;  // only bits 0..10 and 16..26 are read
-  const uint32_t p0 = (st.w >> 11) & 31u, p1 = st.w >> 27;
-  m.ohl = (p0 < 16 ? 1u << p0 : 0u) | (p1 < 16 ? 1u << (16 + p1) : 0u);
-  m.ohh = (p0 >= 16 ? 1u << (p0 - 16) : 0u) | (p1 >= 16 ? 1u << p1 : 0u);
+// A check node's state for the pair (one uint4 per layer and node) holds its
+// messages: x, y the magnitudes min(0.75 min1, kMsgMax) and min(0.75 min2,
+// kMsgMax) (__half2), z the message signs of entries 0..15 (bit e block 0, bit
+// 16 + e block 1), and w
+//   rows of at most kShortDeg entries: which entries take y (the |q| = min1
+//     ones, in the layout of z);
+//   longer rows: the signs of entries 16..26 in bits 0..10 / 16..26, and the
+//     index of one |q| = min1 entry of block 0 in bits 11..15, of block 1 in
+//     bits 27..31.
+// Where several entries tie at min1, min2 = min1 and x = y, so neither form
+// has to tell them apart.  The interleaving puts both blocks' bits for entry e
+// at the same distance from bits 15 and 31, so one shift lines them up with
+// the FP16 sign bits.
+constexpr uint32_t kShortDeg = 10;
+// bits 15 / 31 spread over their halves (byte permute with the selector's
+// sign-replicate bit: bytes 1 and 3's top bits)
+__device__ __forceinline__ uint32_t half_mask(uint32_t v) {
+  uint32_t m;
+  asm("prmt.b32 %0, %1, %2, 0xBB99;" : "=r"(m) : "r"(v), "r"(0u));
   return m;
 }
-// the message to entry j: the (capped) 0.75 min2 at min1's index, 0.75
-// min1 elsewhere, with the sign of q_j times the parity of all signs
-__device__ __forceinline__ __half2 pair_r(const PairMsg &m, uint32_t j) {
-  const uint32_t sh = j < 16 ? 15 - j : 31 - j;
-  const uint32_t oh = (j < 16 ? m.ohl : m.ohh) << sh;
-  const uint32_t sg = (j < 16 ? m.sgl : m.sgh) << sh;
-  // bits 15 / 31 of oh spread over their halves (byte permute with the
-  // selector's sign-replicate bit: bytes 1 and 3's top bits)
-  uint32_t sel;
-  asm("prmt.b32 %0, %1, %2, 0xBB99;" : "=r"(sel) : "r"(oh), "r"(0u));
-  const uint32_t mag = (m.m1 & ~sel) | (m.m2 & sel);
-  return u2h(mag ^ (sg & 0x80008000u));
+// the message to entry j: z / w's bits for j in sg / y2 (w's for j >= 16)
+__device__ __forceinline__ __half2 old_msg(uint32_t m1, uint32_t m2, uint32_t sg, uint32_t y2, uint32_t j) {
+  const uint32_t sh = j < 16 ? 15 - j : 31 - j, sel = half_mask(y2 << sh);
+  const uint32_t mag = (m1 & ~sel) | (m2 & sel);
+  return u2h(mag ^ ((sg << sh) & 0x80008000u));
 }
-// min tracking of entry j's |q| (blocks apart): the first index of min1 and
-// the least of the others, as a sequential scan in entry order keeps them;
-// the signs of q go into nl / nh
-__device__ __forceinline__ void pair_track(__half2 q, uint32_t j, __half2 &min1, __half2 &min2, uint32_t &pos,
-                                           uint32_t &nl, uint32_t &nh) {
-  const uint32_t qb = h2u(q);
-  const __half2 mag = u2h(qb & 0x7FFF7FFFu);
-  const uint32_t lt = __hlt2_mask(mag, min1);
-  pos = (pos & ~lt) | ((j * 0x00010001u) & lt);
-  min2 = __hmin2(min2, __hmax2(min1, mag));
-  min1 = __hmin2(min1, mag);
-  if (j < 16)
-    nl |= (qb >> (15 - j)) & (0x00010001u << j);
-  else
-    nh |= (qb >> (31 - j)) & (0x00010001u << (j - 16));
+// a longer row's |q| = min1 indices as bits in the layout of z (entries 0..15)
+// and of w's signs (16..26)
+__device__ __forceinline__ void pos_bits(uint32_t w, uint32_t &lo, uint32_t &hi) {
+  const uint32_t p0 = (w >> 11) & 31u, p1 = w >> 27;
+  lo = (p0 < 16 ? 1u << p0 : 0u) | (p1 < 16 ? 1u << (16 + p1) : 0u);
+  hi = (p0 >= 16 ? 1u << (p0 - 16) : 0u) | (p1 >= 16 ? 1u << p1 : 0u);
 }
-__device__ __forceinline__ uint4 pair_state(__half2 min1, __half2 min2, uint32_t pos, uint32_t nl, uint32_t nh,
-                                            uint32_t deg) {
-  if (deg == 1) min2 = min1;
-  return make_uint4(h2u(min1), h2u(min2), nl, nh | ((pos & 31u) << 11) | ((pos >> 16) << 27));
+// the least and second least |q| so far and the signs' parity (bits 15, 31)
+struct PairMin {
+  __half2 min1, min2;
+  uint32_t par;
+  __device__ __forceinline__ void init() {
+    min1 = min2 = __float2half2_rn(INFINITY);
+    par = 0;
+  }
+  __device__ __forceinline__ void add(__half2 q) {
+    const __half2 mag = u2h(h2u(q) & 0x7FFF7FFFu);
+    min2 = __hmin2(min2, __hmax2(min1, mag));
+    min1 = __hmin2(min1, mag);
+    par ^= h2u(q);
+  }
+};
+// the new messages and state of a row
+struct PairNew {
+  uint32_t m1, m2, sg, w;
+  __device__ __forceinline__ void init(const PairMin &t, uint32_t deg) {
+    const __half2 a = __float2half2_rn(kAlpha);  // 0.75, exact in FP16
+    const __half2 cap = __float2half2_rn(kMsgMax);
+    m1 = h2u(__hmin2(__hmul2(a, t.min1), cap));
+    m2 = deg == 1 ? m1 : h2u(__hmin2(__hmul2(a, t.min2), cap));
+    sg = w = 0;
+  }
+  // app = q + the message to entry j; SHORT: the short rows' state
+  template <bool SHORT>
+  __device__ __forceinline__ __half2 add(__half2 q, const PairMin &t, uint32_t j) {
+    const uint32_t qb = h2u(q), sel = __heq2_mask(u2h(qb & 0x7FFF7FFFu), t.min1);
+    const uint32_t sign = (qb ^ t.par) & 0x80008000u;
+    if (SHORT || j < 16) sg |= sign >> (15 - j);
+    else w |= sign >> (31 - j);
+    if (SHORT) {
+      w |= sel & (0x00010001u << j);
+    } else {
+      const uint32_t idx = sel & 0xF800F800u;  // the index fields: bits 11..15, 27..31
+      w = (w & ~idx) | (j * 0x08000800u & idx);
+    }
+    return __hadd2(q, u2h(((m1 & ~sel) | (m2 & sel)) | sign));
+  }
+  __device__ __forceinline__ uint4 state() const { return make_uint4(m1, m2, sg, w); }
+};
+// entry en's slot of check node z (tid4 = 4 z): the variables wrap at Z
+__device__ __forceinline__ __half2 *app_slot(uint8_t *app, const uint2 &en, uint32_t tid, uint32_t Z4) {
+  return reinterpret_cast<__half2 *>(app + (en.x + 4 * tid - (tid >= en.y ? Z4 : 0u)));
 }
 
 // One check node's update for the pair over a row of at most D entries, all
 // in registers: every app load issued before any store (a row holds one
 // circulant per column block, so the node's D slots are distinct), then
-// q_e = app - r_e (r_e rebuilt from the node's previous state) with the min
-// tracking, then app = q_e + r'_e.  Returns the new state.
+// q_e = app - r_e (r_e from the node's previous state) with the min tracking,
+// then app = q_e + r'_e.  Returns the new state.
 template <int D>
-__device__ __forceinline__ uint4 ldpc_node(__half2 *app, const uint2 *ent, uint32_t deg, uint32_t tid, uint32_t Z,
+__device__ __forceinline__ uint4 ldpc_node(uint8_t *app, const uint2 *ent, uint32_t deg, uint32_t tid, uint32_t Z4,
                                            const uint4 &st) {
-  // rows of more than 10 entries recompute the slot indices for the stores
-  // rather than hold them (register pressure)
-  constexpr bool kKeepIdx = D <= 10;
-  auto slot = [&](int j) {
-    const uint2 en = ent[j];
-    return en.x + tid - (tid >= en.y ? Z : 0u);
-  };
-  const PairMsg mo = pair_msg(st);
-  uint32_t idx[kKeepIdx ? D : 1];
+  constexpr bool kShort = D <= (int)kShortDeg;
+  // longer rows recompute the slots for the stores rather than hold them
+  // (register pressure)
+  __half2 *slot[kShort ? D : 1];
   __half2 q[D];
 #pragma unroll
   for (int j = 0; j < D; j++) {
     if (j < (int)deg) {
-      const uint32_t ix = slot(j);
-      if constexpr (kKeepIdx) idx[j] = ix;
-      q[j] = app[ix];
+      __half2 *a = app_slot(app, ent[j], tid, Z4);
+      if constexpr (kShort) slot[j] = a;
+      q[j] = *a;
     }
   }
-  __half2 min1 = __float2half2_rn(INFINITY), min2 = min1;
-  uint32_t pos = 0, nl = 0, nh = 0;
+  uint32_t y_lo = st.w, y_hi = 0;
+  if constexpr (!kShort) pos_bits(st.w, y_lo, y_hi);
+  PairMin t;
+  t.init();
 #pragma unroll
   for (int j = 0; j < D; j++) {
     if (j < (int)deg) {
-      q[j] = __hsub2(q[j], pair_r(mo, j));
-      pair_track(q[j], j, min1, min2, pos, nl, nh);
+      q[j] = __hsub2(q[j], old_msg(st.x, st.y, j < 16 ? st.z : st.w, j < 16 ? y_lo : y_hi, j));
+      t.add(q[j]);
     }
   }
-  const uint4 ns = pair_state(min1, min2, pos, nl, nh, deg);
-  const PairMsg mn = pair_msg(ns);
+  PairNew n;
+  n.init(t, deg);
 #pragma unroll
   for (int j = 0; j < D; j++) {
     if (j < (int)deg) {
-      uint32_t ix;
-      if constexpr (kKeepIdx) ix = idx[j];
-      else ix = slot(j);
-      app[ix] = __hadd2(q[j], pair_r(mn, j));
+      __half2 *a;
+      if constexpr (kShort) a = slot[j];
+      else a = app_slot(app, ent[j], tid, Z4);
+      *a = n.template add<kShort>(q[j], t, j);
     }
   }
-  return ns;
+  return n.state();
 }
 
 // The same update for rows of any degree (up to kMaxDeg): q_e is stored in
 // place of app between the two passes.
-__device__ __forceinline__ uint4 ldpc_node_any(__half2 *app, const uint2 *ent, uint32_t deg, uint32_t tid,
-                                               uint32_t Z, const uint4 &st) {
-  const PairMsg mo = pair_msg(st);
-  __half2 min1 = __float2half2_rn(INFINITY), min2 = min1;
-  uint32_t pos = 0, nl = 0, nh = 0;
+__device__ __forceinline__ uint4 ldpc_node_any(uint8_t *app, const uint2 *ent, uint32_t deg, uint32_t tid,
+                                               uint32_t Z4, const uint4 &st) {
+  uint32_t y_lo, y_hi;
+  pos_bits(st.w, y_lo, y_hi);
+  PairMin t;
+  t.init();
   for (uint32_t e = 0; e < deg; e++) {
-    const uint2 en = ent[e];
-    __half2 *a = app + en.x + tid - (tid >= en.y ? Z : 0u);
-    const __half2 qe = __hsub2(*a, pair_r(mo, e));
+    __half2 *a = app_slot(app, ent[e], tid, Z4);
+    const __half2 qe = __hsub2(*a, old_msg(st.x, st.y, e < 16 ? st.z : st.w, e < 16 ? y_lo : y_hi, e));
     *a = qe;
-    pair_track(qe, e, min1, min2, pos, nl, nh);
+    t.add(qe);
   }
-  const uint4 ns = pair_state(min1, min2, pos, nl, nh, deg);
-  const PairMsg mn = pair_msg(ns);
+  PairNew n;
+  n.init(t, deg);
   for (uint32_t e = 0; e < deg; e++) {
-    const uint2 en = ent[e];
-    __half2 *a = app + en.x + tid - (tid >= en.y ? Z : 0u);
-    *a = __hadd2(*a, pair_r(mn, e));
+    __half2 *a = app_slot(app, ent[e], tid, Z4);
+    *a = n.add<false>(*a, t, e);
   }
-  return ns;
+  return n.state();
 }
 
 // CTA p decodes code blocks b0 + 2p and b0 + 2p + 1 (the second only when
@@ -345,9 +358,12 @@ __global__ void __launch_bounds__(kMaxZ, 2) ldpc_decode_kernel(mb_ldpc h, const 
   const __half *in0 = llr + (uint64_t)cb * llr_stride;
   const __half *in1 = two ? in0 + llr_stride : in0;
   for (uint32_t v = tid; v < N; v += nt) app[v] = llr_clamp(__halves2half2(in0[v], in1[v]));
-  // entry e as {col * Z + shift, Z - shift}: check node z meets variable
-  // col * Z + (z + shift) mod Z, i.e. x + z, less Z once z >= y
-  for (uint32_t e = tid; e < h.nnz; e += nt) ent[e] = make_uint2((uint32_t)h.col[e] * Z + h.sh[e], Z - h.sh[e]);
+  // entry e as {4 (col * Z + shift), Z - shift}: check node z meets variable
+  // col * Z + (z + shift) mod Z, at byte x + 4 z, less 4 Z once z >= y
+  for (uint32_t e = tid; e < h.nnz; e += nt)
+    ent[e] = make_uint2(4 * ((uint32_t)h.col[e] * Z + h.sh[e]), Z - h.sh[e]);
+  uint8_t *appb = reinterpret_cast<uint8_t *>(app);
+  const uint32_t Z4 = 4 * Z;
   for (uint32_t i = tid; i <= mb; i += nt) r_ptr[i] = h.row_ptr[i];
   __syncthreads();
   // Thread z only ever reads and writes check node z's state, so its loads
@@ -371,15 +387,15 @@ __global__ void __launch_bounds__(kMaxZ, 2) ldpc_decode_kernel(mb_ldpc h, const 
         // every thread of the layer takes the same branch
         uint4 ns;
         if (deg <= 4)
-          ns = ldpc_node<4>(app, ent + e0, deg, tid, Z, st);
+          ns = ldpc_node<4>(appb, ent + e0, deg, tid, Z4, st);
         else if (deg <= 6)
-          ns = ldpc_node<6>(app, ent + e0, deg, tid, Z, st);
+          ns = ldpc_node<6>(appb, ent + e0, deg, tid, Z4, st);
         else if (deg <= 10)
-          ns = ldpc_node<10>(app, ent + e0, deg, tid, Z, st);
+          ns = ldpc_node<10>(appb, ent + e0, deg, tid, Z4, st);
         else if (deg <= 20)
-          ns = ldpc_node<20>(app, ent + e0, deg, tid, Z, st);
+          ns = ldpc_node<20>(appb, ent + e0, deg, tid, Z4, st);
         else
-          ns = ldpc_node_any(app, ent + e0, deg, tid, Z, st);
+          ns = ldpc_node_any(appb, ent + e0, deg, tid, Z4, st);
         state[i * Z + tid] = ns;
       }
       __syncthreads();

@@ -9,5 +9,5 @@ struct mb_ldpc {
   uint16_t *col, *sh;  // [nnz] device, rows < mb, by (row, col)
   uint32_t *inv;       // device: B^-1's circulants, block row i's entries (block column << 16 | shift)
                        // at inv[i] .. inv[i + 1] - 1
-  uint4 *state;        // [(max_batch + 1) / 2][mb][Z] device, per pair of blocks: min1, min2, signs + index
+  uint4 *state;        // [(max_batch + 1) / 2][mb][Z] device, per pair of blocks: message magnitudes, signs, who takes the second
 };
