@@ -18,10 +18,11 @@
 // one (k across its rows), so each serves every product it enters without a
 // transposition.
 // Eight steps of 22 -> 256 -> 256 -> 4 on batches of 4096 (with the host copies
-// of gradients and weights at the end): 6,950 us with a product per launch, 497
-// us here (31 us this kernel, 4.4 us the reduction, 2.8 us Adam per step).
+// of gradients and weights at the end): 6,950 us with a product per launch, 455
+// us here (25 us this kernel, 4.2 us the reduction, 2.8 us Adam per step).
 #include <algorithm>
 #include <atomic>
+#include <type_traits>
 
 #include "mlp_step.cuh"
 #include "tc.cuh"
@@ -134,63 +135,56 @@ __global__ void __launch_bounds__(128 * MT, 1) mlp_step_kernel(const StepParams 
   };
   // gradient element e of this CTA's slot: written by the first tile, added to by the others
   auto acc1 = [&](uint64_t e, float v) { slot[e] = pass ? slot[e] + v : v; };
-  // ReLU layer: z columns at col + bias -> BF16 activations, sign mask
-  auto hidden = [&](uint32_t col, float bias, uint8_t *h, uint32_t nv, uint32_t (&mask)[2]) {
-    mask[0] = mask[1] = 0;
-#pragma unroll
+  // ReLU layer: z columns at col + bias -> BF16 activations, sign mask.  The
+  // loops over 16-column chunks stay loops: the kernel runs its code once, and
+  // fetching it costs as much as running it
+  auto hidden = [&](uint32_t col, float bias, uint8_t *h, uint32_t nv, uint64_t &mask) {
+    mask = 0;
+#pragma unroll 1
     for (uint32_t c = 0; c < 4; c++) {
       float v[16];
       tc::tmem_ld16(my + col + tl * kT + c * 16, v);
+      uint32_t bits = 0;
 #pragma unroll
       for (uint32_t j = 0; j < 16; j++) {
         const float z = v[j] + bias;
-        if (z > 0.f) mask[c / 2] |= 1u << (c % 2 * 16 + j);
+        if (z > 0.f) bits |= 1u << j;
         v[j] = 16 * c + j < nv ? fmaxf(z, 0.f) : 0.f;
       }
+      mask |= (uint64_t)bits << (16 * c);
       put16(h, n, c, v);
     }
   };
   // upstream gradient: columns at col where the mask is set -> BF16, and their FP32 sum
-  auto upstream = [&](uint32_t col, uint8_t *d, const uint32_t (&mask)[2]) {
+  auto upstream = [&](uint32_t col, uint8_t *d, uint64_t mask) {
     float sum = 0.f;
-#pragma unroll
+#pragma unroll 1
     for (uint32_t c = 0; c < 4; c++) {
       float v[16];
       tc::tmem_ld16(my + col + tl * kT + c * 16, v);
+      const uint32_t bits = (uint32_t)(mask >> (16 * c));
 #pragma unroll
       for (uint32_t j = 0; j < 16; j++) {
-        if (!(mask[c / 2] >> (c % 2 * 16 + j) & 1u)) v[j] = 0.f;
+        if (!(bits >> j & 1u)) v[j] = 0.f;
         sum += v[j];
       }
       put16(d, n, c, v);
     }
     return sum;
   };
-  // dW2 rows 128 t .. 128 t + 127 into the slot: a thread holds 128 columns of one row
+  // dW2 columns 128 t .. 128 t + 127 (dW2^T = dz2^T h1: a thread holds 128
+  // rows of one column) into the slot: a warp's lanes store neighbouring
+  // columns of one row
   auto drain_w2 = [&](uint32_t t) {
-    const uint32_t k1 = t * 128 + warp % 4 * 32 + lane, c0 = warp / 4 * 128;
+    const uint32_t n2 = t * 128 + warp % 4 * 32 + lane, r0 = warp / 4 * 128;
 #pragma unroll 1
-    for (uint32_t c = c0; c < c0 + 128; c += 16) {
+    for (uint32_t r = r0; r < r0 + 128; r += 16) {
       float v[16];
-      tc::tmem_ld16(my + c_w2 + c, v);
-      if (k1 >= W) continue;
-      float *d = slot + s.off[2] + (uint64_t)k1 * W + c;
-      if (W % 4 == 0) {
-#pragma unroll
-        for (uint32_t j = 0; j < 16; j += 4) {
-          if (c + j >= W) break;
-          float4 o = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-          if (pass) {
-            const float4 a = *reinterpret_cast<const float4 *>(d + j);
-            o = make_float4(a.x + o.x, a.y + o.y, a.z + o.z, a.w + o.w);
-          }
-          *reinterpret_cast<float4 *>(d + j) = o;
-        }
-      } else {
+      tc::tmem_ld16(my + c_w2 + r, v);
+      if (n2 < W)
 #pragma unroll
         for (uint32_t j = 0; j < 16; j++)
-          if (c + j < W) d[j] = pass ? d[j] + v[j] : v[j];
-      }
+          if (r + j < W) acc1(s.off[2] + (uint64_t)(r + j) * W + n2, v[j]);
     }
   };
 
@@ -224,14 +218,13 @@ __global__ void __launch_bounds__(128 * MT, 1) mlp_step_kernel(const StepParams 
       for (uint32_t e = tid; e < nv * O; e += nthr) abc[kT * 16 + e] = __ldg(q.b + (uint64_t)row0 * O + e);
       for (uint32_t e = tid; e < nv; e += nthr) abc[kT * 20 + e] = q.c ? __ldg(q.c + row0 + e) : 0.f;
     }
-    // all threads wait, so that a copy still landing holds no later step up alone
-    if (!tc::mbar_wait(&wbar1, pass & 1) || !tc::mbar_wait(&wbar2, pass & 1)) ok = false;
+    if (!tc::mbar_wait(&wbar1, pass & 1)) ok = false;
     publish();
     if (__syncthreads_or(!ok)) {
       ok = false;
       break;
     }
-    uint32_t m1[2], m2[2];
+    uint64_t m1, m2;
     if (tid == 0) {
       for (uint32_t t = 0; t < MT; t++)
         mma_steps(tmem + c_a + t * kT, mnmajor(a_h2 + t * 2048, rs2), kmajor(a_x, rsx), id_z1, Ip / 16);
@@ -239,7 +232,12 @@ __global__ void __launch_bounds__(128 * MT, 1) mlp_step_kernel(const StepParams 
     }
     if (!(ok = arrived(&bar, ph))) break;
     hidden(c_a, bias1, h1, nv, m1);
+    if (!tc::mbar_wait(&wbar2, pass & 1)) ok = false;  // W2 has had the first layer to land
     publish();
+    if (__syncthreads_or(!ok)) {
+      ok = false;
+      break;
+    }
     if (tid == 0) {
       for (uint32_t t = 0; t < MT; t++)
         mma_steps(tmem + c_b + t * kT, mnmajor(a_w2 + t * 2048, rs2), mnmajor(a_h1, kH), id_z2, Wp / 16);
@@ -276,21 +274,28 @@ __global__ void __launch_bounds__(128 * MT, 1) mlp_step_kernel(const StepParams 
       const float *Ai = stage_abc ? abc + tid * O * O : q.A + (uint64_t)(row0 + (in ? tid : 0)) * O * O;
       const float *bi = stage_abc ? abc + kT * 16 + tid * O : q.b + (uint64_t)(row0 + (in ? tid : 0)) * O;
 #pragma unroll
-      for (uint32_t r = 0; r < 16; r++) y[r] = r < O ? y[r] + __ldg(q.params + s.off[5] + r) : 0.f;
-      float quad_y = 0.f, lin = 0.f;
-#pragma unroll
       for (uint32_t r = 0; r < 16; r++) {
+        y[r] = r < O ? y[r] + __ldg(q.params + s.off[5] + r) : 0.f;
         g[r] = 0.f;
-        if (r < O && in) {
-          float ay = 0.f;
-#pragma unroll
-          for (uint32_t k = 0; k < 16; k++)
-            if (k < O) ay = fmaf(Ai[r * O + k], y[k], ay);
-          quad_y = fmaf(y[r], ay, quad_y);
-          lin = fmaf(bi[r], y[r], lin);
-          g[r] = 2.f * (ay - bi[r]) / (float)q.B;
-        }
       }
+      float quad_y = 0.f, lin = 0.f;
+      auto outputs = [&](auto om) {  // rows and columns up to om (>= O)
+        constexpr uint32_t OM = decltype(om)::value;
+#pragma unroll
+        for (uint32_t r = 0; r < OM; r++) {
+          if (r < O && in) {
+            float ay = 0.f;
+#pragma unroll
+            for (uint32_t k = 0; k < OM; k++)
+              if (k < O) ay = fmaf(Ai[r * O + k], y[k], ay);
+            quad_y = fmaf(y[r], ay, quad_y);
+            lin = fmaf(bi[r], y[r], lin);
+            g[r] = 2.f * (ay - bi[r]) / (float)q.B;
+          }
+        }
+      };
+      if (O <= 4) outputs(std::integral_constant<uint32_t, 4>{});
+      else outputs(std::integral_constant<uint32_t, 16>{});
       uint8_t *d = dy + tid / 8 * rsd + tid % 8 * 16;
       *reinterpret_cast<uint4 *>(d) = make_uint4(pack2(g[0], g[1]), pack2(g[2], g[3]), pack2(g[4], g[5]), pack2(g[6], g[7]));
       *reinterpret_cast<uint4 *>(d + 128) =
@@ -320,17 +325,21 @@ __global__ void __launch_bounds__(128 * MT, 1) mlp_step_kernel(const StepParams 
     {
       float v[16];
       tc::tmem_ld16(my + c_w3 + tl * 16, v);
-      if (n < W)
+      float *d = slot + s.off[4] + (uint64_t)n * O;
+      if (n < W && O == 4 && W % 4 == 0 && !pass) {
+        *reinterpret_cast<float4 *>(d) = make_float4(v[0], v[1], v[2], v[3]);
+      } else if (n < W) {
 #pragma unroll
         for (uint32_t o = 0; o < 16; o++)
-          if (o < O) acc1(s.off[4] + (uint64_t)n * O + o, v[o]);
+          if (o < O) d[o] = pass ? d[o] + v[o] : v[o];
+      }
     }
     publish();
     if (tid == 0) {
       for (uint32_t t = 0; t < MT; t++)
         mma_steps(tmem + c_b + t * kT, kmajor(a_w2 + t * 16 * rs2, rs2), mnmajor(a_h2, kH), id_d1, Wp / 16);
       tc::mma_commit(&bar);
-      mma_steps(tmem + c_w2, kmajor(a_h1, kH), kmajor(a_h2, kH), id_w2, kT / 16);
+      mma_steps(tmem + c_w2, kmajor(a_h2, kH), kmajor(a_h1, kH), id_w2, kT / 16);
       tc::mma_commit(&bar_g);
     }
     if (!(ok = arrived(&bar, ph))) break;
@@ -350,11 +359,12 @@ __global__ void __launch_bounds__(128 * MT, 1) mlp_step_kernel(const StepParams 
     if (MT == 2) {
       publish();
       if (tid == 0) {
-        mma_steps(tmem + c_w2, kmajor(a_h1 + 16 * kH, kH), kmajor(a_h2, kH), id_w2, kT / 16);
+        mma_steps(tmem + c_w2, kmajor(a_h2 + 16 * kH, kH), kmajor(a_h1, kH), id_w2, kT / 16);
         tc::mma_commit(&bar_g);
       }
     }
     if (!(ok = arrived(&bar, ph))) break;
+#pragma unroll 1
     for (uint32_t i0 = 0; i0 < Ip; i0 += 16) {
       float v[16];
       tc::tmem_ld16(my + c_w1 + tl * Ip + i0, v);
@@ -368,7 +378,12 @@ __global__ void __launch_bounds__(128 * MT, 1) mlp_step_kernel(const StepParams 
       drain_w2(1);
     }
   }
-  if (!ok && tid == 0 && q.err) atomicOr(q.err, tc::kErrTimeout);
+  if (!ok && tid == 0) {
+    if (q.err) atomicOr(q.err, tc::kErrTimeout);
+    // copies still in flight land before the CTA exits
+    tc::mbar_wait(&wbar1, pass & 1);
+    tc::mbar_wait(&wbar2, pass & 1);
+  }
   tc::fence_before_sync();
   __syncthreads();
   if (warp == 0) tc::tmem_dealloc(tmem, 512);
