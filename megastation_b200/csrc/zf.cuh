@@ -40,6 +40,11 @@ mb_status zf_mixed_run(float2 *csi, void *img_w, uint32_t groups, uint32_t M, ui
                        const mb_zf_opts *opts, int32_t *status, float *cond, cudaStream_t st,
                        bool write_w = true, float *wmax = nullptr, const ZfNetView *net = nullptr,
                        uint32_t path = 0);
+// the mixed-precision detector by a direct FP32 solve (zf_direct.cu), same
+// outputs; MB_UNSUPPORTED for K > 16 or when a group's CSI does not fit in
+// shared memory
+mb_status zf_direct_run(float2 *csi, void *img, uint32_t groups, uint32_t M, uint32_t K, float cond_thr,
+                        int32_t *status, float *cond, cudaStream_t st, bool write_w, float *wmax);
 // the same ZF fused with the tensor-core equalizer: each CTA keeps its
 // group's detector image in shared memory and equalizes the group's
 // columns of nb symbols of planar BF16 samples y_lp [nb][re|im][M][S_pad]

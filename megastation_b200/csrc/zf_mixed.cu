@@ -40,6 +40,7 @@
 #include "gj.cuh"
 #include "tc.cuh"
 #include "zf.cuh"
+#include "zf_fp64.cuh"
 
 namespace mb {
 
@@ -81,49 +82,6 @@ __host__ __device__ constexpr uint32_t zfm_gx_bytes(uint32_t K) {
 __host__ __device__ constexpr uint32_t zfm_x_bytes(uint32_t K) {
   const uint32_t two_tiles = 2 * 128 * kKT * 2;
   return zfm_gx_bytes(K) > two_tiles ? zfm_gx_bytes(K) : two_tiles;
-}
-
-__device__ __forceinline__ uint32_t img_off(uint32_t r, uint32_t kk, uint32_t MM) {
-  // canonical K-major, no swizzle: [k tile][row group][k chunk][row][8]
-  const uint32_t kt = kk / kKT, kin = kk % kKT;
-  return kt * (MM * kKT * 2) + (r / 8) * 1024 + (kin / 8) * 128 + (r % 8) * 16 + (kin % 8) * 2;
-}
-
-// In-place Cholesky of the K x K Hermitian matrix A (lower, leading dim lda)
-// by all threads; returns false when a pivot is not positive.
-template <typename C, typename R>
-__device__ bool chol_smem(C *A, uint32_t K, uint32_t lda, int *flag) {
-  const int tid = threadIdx.x, nt = blockDim.x;
-  if (tid == 0) *flag = 0;
-  __syncthreads();
-  for (uint32_t j = 0; j < K; j++) {
-    if (tid == 0) {
-      R d = A[j * lda + j].x;
-      if (!(d > (R)0)) {
-        *flag = 1;
-        d = (R)1;
-      }
-      A[j * lda + j].x = sqrt(d);
-      A[j * lda + j].y = 0;
-    }
-    __syncthreads();
-    const R inv = (R)1 / A[j * lda + j].x;
-    for (uint32_t i = j + 1 + tid; i < K; i += nt) {
-      A[i * lda + j].x *= inv;
-      A[i * lda + j].y *= inv;
-    }
-    __syncthreads();
-    const uint32_t rem = K - j - 1;
-    for (uint32_t q = tid; q < rem * rem; q += nt) {
-      const uint32_t i = j + 1 + q / rem, k = j + 1 + q % rem;
-      if (k > i) continue;
-      const C a = A[i * lda + j], b = A[k * lda + j];
-      A[i * lda + k].x -= a.x * b.x + a.y * b.y;
-      A[i * lda + k].y -= a.y * b.x - a.x * b.y;
-    }
-    __syncthreads();
-  }
-  return *flag == 0;
 }
 
 // C = A B for K x K complex matrices in shared memory (leading dims given);
@@ -1142,60 +1100,8 @@ __global__ void __launch_bounds__(kThreads, 2)
 
   // ------------------------------------------------- FP64 fallback groups
   if (!fail && st == 2) {
-    using D2 = double2;
-    D2 *Gd = reinterpret_cast<D2 *>(Gs);  // reuses Gs and Xs (2 K*ld float2)
-    const uint32_t ldd = K + 1;
-    for (uint32_t e = tid; e < K * K; e += kThreads) {
-      const uint32_t i = e / K, j = e % K;
-      if (j > i) continue;
-      double sr = 0, si = 0;
-      for (uint32_t b = 0; b < M; b++) {
-        const float2 a = cg[b * K + i], c = cg[b * K + j];
-        sr += (double)a.x * c.x + (double)a.y * c.y;
-        si += (double)a.y * c.x - (double)a.x * c.y;
-      }
-      Gd[i * ldd + j] = make_double2(sr, si);
-    }
-    __syncthreads();
-    const bool pd = chol_smem<D2, double>(Gd, K, ldd, &flag);
-    for (uint32_t c = tid; c < q.nkt * tile_bytes / 16; c += kThreads)
-      reinterpret_cast<uint4 *>(imgw)[c] = make_uint4(0, 0, 0, 0);
-    __syncthreads();
-    if (!pd) st = 1;
-    for (uint32_t b = tid; b < M; b += kThreads) {
-      D2 z[64];
-      for (uint32_t i = 0; i < K; i++) {
-        const float2 cv = cg[b * K + i];
-        D2 s = make_double2(cv.x, cv.y);
-        for (uint32_t k = 0; k < i && pd; k++) {
-          const D2 l = Gd[i * ldd + k];
-          s.x -= l.x * z[k].x - l.y * z[k].y;
-          s.y -= l.x * z[k].y + l.y * z[k].x;
-        }
-        const double d = pd ? Gd[i * ldd + i].x : 1.0;
-        z[i] = make_double2(s.x / d, s.y / d);
-      }
-      for (int i = (int)K - 1; i >= 0 && pd; i--) {
-        D2 s = z[i];
-        for (uint32_t k = i + 1; k < K; k++) {
-          const D2 l = Gd[k * ldd + i];
-          s.x -= l.x * z[k].x + l.y * z[k].y;
-          s.y -= l.x * z[k].y - l.y * z[k].x;
-        }
-        const double d = Gd[i * ldd + i].x;
-        z[i] = make_double2(s.x / d, s.y / d);
-      }
-      // every thread reads its own column b of C before overwriting it
-      for (uint32_t u = 0; u < K; u++) {
-        const float2 w = pd ? make_float2((float)z[u].x, (float)z[u].y) : make_float2(0.f, 0.f);
-        cg[b * K + u] = w;
-        wmx = fmaxf(wmx, sqrtf(w.x * w.x + w.y * w.y));
-        *reinterpret_cast<__nv_bfloat16 *>(imgw + img_off(2 * u, b, MM)) = __float2bfloat16_rn(w.x);
-        *reinterpret_cast<__nv_bfloat16 *>(imgw + img_off(2 * u, Mp + b, MM)) = __float2bfloat16_rn(-w.y);
-        *reinterpret_cast<__nv_bfloat16 *>(imgw + img_off(2 * u + 1, b, MM)) = __float2bfloat16_rn(w.y);
-        *reinterpret_cast<__nv_bfloat16 *>(imgw + img_off(2 * u + 1, Mp + b, MM)) = __float2bfloat16_rn(w.x);
-      }
-    }
+    // Gd reuses Gs and Xs (2 K*ld float2)
+    st = zf_fp64_group<64>(cg, imgw, reinterpret_cast<double2 *>(Gs), &flag, M, K, Mp, MM, q.nkt, wmx);
   }
 
   if (q.wmax) {
@@ -1356,6 +1262,12 @@ static mb_status zf_mixed_launch(float2 *csi, void *img_w, uint32_t groups, uint
   if (K == 0 || K > 64) return MB_UNSUPPORTED;
   const bool learned = opts && opts->init == 1;
   if (opts && opts->init > 1) return MB_BAD_ARG;
+  const float cond_thr = opts && opts->cond_threshold > 0 ? opts->cond_threshold : 1e4f;
+  if (!learned && !fe && path != 2) {
+    // K <= 16 and a group's CSI in shared memory: the direct solve
+    const mb_status r = zf_direct_run(csi, img_w, groups, M, K, cond_thr, status, cond, st, write_w, wmax);
+    if (r != MB_UNSUPPORTED) return r;
+  }
   if (learned && (!net || !net->w1 || net->width == 0 || net->width > kZfInitMaxWidth)) return MB_BAD_ARG;
   const TcShape s = tc_shape(M, K);
   const DeviceTables *tab = device_tables();
@@ -1375,7 +1287,7 @@ static mb_status zf_mixed_launch(float2 *csi, void *img_w, uint32_t groups, uint
   q.nkt = s.nkt;
   q.nh = s.Mp / kKT;
   q.ns_iters = opts ? opts->ns_iters : 2;
-  q.cond_thr = opts && opts->cond_threshold > 0 ? opts->cond_threshold : 1e4f;
+  q.cond_thr = cond_thr;
   // bulk copies want 16-byte aligned addresses and sizes: the network's six
   // arrays (width a multiple of 4), and CSI k tiles (K even)
   auto a16 = [](const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
