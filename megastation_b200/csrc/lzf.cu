@@ -210,9 +210,14 @@ __device__ __forceinline__ void interp_pos(uint32_t s, uint32_t u, uint32_t sg, 
 }
 
 // Rows of the CSI staged in shared memory are ldc(K) long: the next even
-// number (16-byte loads of two users) plus one 16-byte chunk, so that
-// neighbouring antennas sit in different banks; K < 8 keeps K.
-__host__ __device__ constexpr uint32_t ldc_of(uint32_t K) { return K < 8 ? K : (K + 1) / 2 * 2 + 2; }
+// number (16-byte loads of two users), plus one 16-byte chunk from K = 8 on, so
+// that neighbouring antennas sit in different banks; one user stays one.
+__host__ __device__ constexpr uint32_t ldc_of(uint32_t K) {
+  return K == 1 ? 1 : (K + 1) / 2 * 2 + (K < 8 ? 0 : 2);
+}
+// The K x K matrices are padded with zeros to KP x KP (KP the power of two from
+// 4 on that holds K), rows of ldm(KP): a 16-byte chunk more, for the same reason.
+__host__ __device__ constexpr uint32_t ldm_of(uint32_t KP) { return KP + 2; }
 
 // elements i and i + 1 (vec: i is even and a 16-byte load will do)
 __device__ __forceinline__ float4 pair_at(const float2 *p, bool vec) {
@@ -223,64 +228,84 @@ __device__ __forceinline__ float4 pair_at(const float2 *p, bool vec) {
 // c_s [M][ldc] of subcarrier s into shared memory; ig / iw: per (s, u) the
 // lower pilot group and the weight of the upper one (interp_pos, tabulated).
 // A thread keeps one user; the element past a row's users is 0 for K odd.
+template <int KP>
 __device__ __forceinline__ void interp_smem(const float2 *csi, const int *ig, const float *iw, float2 *c,
                                             uint32_t s, uint32_t M, uint32_t K, uint32_t G, uint32_t ldc) {
-  uint32_t kp = 1;
-  while (kp < K) kp *= 2;
-  const uint32_t u = threadIdx.x % kp, step = blockDim.x / kp;
+  constexpr uint32_t step = 256 / KP;
+  const uint32_t u = threadIdx.x % KP, b0 = threadIdx.x / KP;
   if (u >= K) {
     if (u == K && ldc > K)
-      for (uint32_t b = threadIdx.x / kp; b < M; b += step) c[b * ldc + u] = make_float2(0.f, 0.f);
+      for (uint32_t b = b0; b < M; b += step) c[b * ldc + u] = make_float2(0.f, 0.f);
     return;
   }
   const int g0 = ig[s * K + u];
   const float t = iw[s * K + u];
-  const float2 *lo = csi + (uint64_t)g0 * M * K + u, *hi = G > 1 ? lo + (uint64_t)M * K : lo;
+  const float2 *lo = csi + ((uint64_t)g0 * M + b0) * K + u, *hi = G > 1 ? lo + (uint64_t)M * K : lo;
+  float2 *d = c + b0 * ldc + u;
 #pragma unroll 8
-  for (uint32_t b = threadIdx.x / kp; b < M; b += step) {
-    const float2 a = __ldg(lo + (uint64_t)b * K), d = __ldg(hi + (uint64_t)b * K);
-    c[b * ldc + u] = make_float2((1.f - t) * a.x + t * d.x, (1.f - t) * a.y + t * d.y);
+  for (uint32_t b = b0; b < M; b += step) {
+    const float2 a = __ldg(lo), e = __ldg(hi);
+    *d = make_float2((1.f - t) * a.x + t * e.x, (1.f - t) * a.y + t * e.y);
+    lo += step * K;
+    hi += step * K;
+    d += step * ldc;
   }
 }
 
-// The Gram of the staged CSI into gm [K][K] (in shared memory): 2 x 2 outputs
+// The Gram of the staged CSI into gm (KP x KP, the padding zero): 2 x 2 outputs
 // a thread, the antennas split over up to four groups of threads whose sums
-// meet in gm, b1, b2, b3 ([K][K] scratch each).  All threads.
+// meet in gm, b1, b2, b3 (a matrix each).  All 256 threads.
+template <int KP>
 __device__ __forceinline__ void gram_smem(const float2 *c, float2 *gm, float2 *b1, float2 *b2, float2 *b3, uint32_t M,
                                           uint32_t K, uint32_t ldc) {
-  const uint32_t T2 = (K + 1) / 2, nt = T2 * T2, parts = min(4u, blockDim.x / nt), tid = threadIdx.x;
-  const uint32_t part = tid / nt, u = tid % nt / T2 * 2, v = tid % T2 * 2;
+  constexpr uint32_t T2 = KP / 2, nt = T2 * T2, parts = 256 / nt < 4 ? 256 / nt : 4, ldm = ldm_of(KP);
+  const uint32_t tid = threadIdx.x, part = tid / nt, u = tid % nt / T2 * 2, v = tid % T2 * 2;
   const bool vec = ldc % 2 == 0;
-  if (part < parts) {
-    float2 a[2][2] = {{cz<float2>(), cz<float2>()}, {cz<float2>(), cz<float2>()}};
+  float2 a[2][2] = {{cz<float2>(), cz<float2>()}, {cz<float2>(), cz<float2>()}};
+  if (part < parts && u < K && v < K) {
+    const float2 *pu = c + part * ldc + u, *pv = c + part * ldc + v;
 #pragma unroll 4
     for (uint32_t b = part; b < M; b += parts) {
-      const float4 cu = pair_at(c + b * ldc + u, vec), cv = pair_at(c + b * ldc + v, vec);
+      const float4 cu = pair_at(pu, vec), cv = pair_at(pv, vec);
       const float2 u0 = make_float2(cu.x, cu.y), u1 = make_float2(cu.z, cu.w);
       const float2 v0 = make_float2(cv.x, cv.y), v1 = make_float2(cv.z, cv.w);
       a[0][0] = cjfma(v0, u0, a[0][0]);
       a[0][1] = cjfma(v1, u0, a[0][1]);
       a[1][0] = cjfma(v0, u1, a[1][0]);
       a[1][1] = cjfma(v1, u1, a[1][1]);
+      pu += parts * ldc;
+      pv += parts * ldc;
     }
+  }
+  if (part < parts) {
     float2 *d = part == 0 ? gm : part == 1 ? b1 : part == 2 ? b2 : b3;
 #pragma unroll
     for (int i = 0; i < 2; i++)
 #pragma unroll
       for (int j = 0; j < 2; j++)
-        if (u + i < K && v + j < K) d[(u + i) * K + v + j] = a[i][j];
+        d[(u + i) * ldm + v + j] = u + i < K && v + j < K ? a[i][j] : make_float2(0.f, 0.f);
   }
   __syncthreads();
-  for (uint32_t e = tid; parts > 1 && e < K * K; e += blockDim.x) {
-    float2 s = gm[e];
-    for (uint32_t q = 1; q < parts; q++) {
-      const float2 w = (q == 1 ? b1 : q == 2 ? b2 : b3)[e];
-      s.x += w.x;
-      s.y += w.y;
+  if (parts > 1) {
+    for (uint32_t e = tid; e < KP * KP; e += 256) {
+      const uint32_t o = e / KP * ldm + e % KP;
+      float2 s = gm[o];
+      for (uint32_t q = 1; q < parts; q++) {
+        const float2 w = (q == 1 ? b1 : q == 2 ? b2 : b3)[o];
+        s.x += w.x;
+        s.y += w.y;
+      }
+      gm[o] = s;
     }
-    gm[e] = s;
+    __syncthreads();
   }
-  __syncthreads();
+}
+
+// gj_inverse for any KP here (its smallest grid is 16 x 16)
+template <int KP>
+__device__ __forceinline__ bool inverse_smem(const float2 *G, float2 *X, uint32_t K, float2 *prow, int *bad) {
+  constexpr uint32_t ldm = ldm_of(KP);
+  return KP <= 16 ? gj_inverse<16>(G, X, K, ldm, prow, bad) : gj_inverse<32>(G, X, K, ldm, prow, bad);
 }
 
 __global__ void interp_table_kernel(int *ig, float *iw, uint32_t K, uint32_t S, uint32_t sg, uint32_t G) {
@@ -294,22 +319,27 @@ __global__ void interp_table_kernel(int *ig, float *iw, uint32_t K, uint32_t S, 
 }
 
 // The Gram at each group's centre subcarrier and its inverse, a CTA per group
+template <int KP>
 __global__ void __launch_bounds__(256) centre_kernel(const float2 *csi, const int *ig, const float *iw,
                                                      const uint32_t *cidx, float2 *Gc, float2 *Xc, uint32_t M,
                                                      uint32_t K, uint32_t G, int *flag) {
   extern __shared__ __align__(16) unsigned char sgm[];
   __shared__ int bad;
+  constexpr uint32_t ldm = ldm_of(KP), mat = KP * ldm;
   const uint32_t g = blockIdx.x, KK = K * K, ldc = ldc_of(K);
-  float2 *gm = reinterpret_cast<float2 *>(sgm), *b1 = gm + KK, *b2 = b1 + KK, *b3 = b2 + KK, *c = b3 + KK;
-  if (threadIdx.x == 0) bad = 0;
-  interp_smem(csi, ig, iw, c, cidx[g], M, K, G, ldc);
-  __syncthreads();
-  gram_smem(c, gm, b1, b2, b3, M, K, ldc);
-  for (uint32_t e = threadIdx.x; e < KK; e += blockDim.x) Gc[(uint64_t)g * KK + e] = gm[e];
+  float2 *gm = reinterpret_cast<float2 *>(sgm), *b1 = gm + mat, *b2 = b1 + mat, *b3 = b2 + mat, *c = b3 + mat;
   float2 *prow = c + M * ldc + 2;
-  const bool ok = K <= 16 ? gj_inverse<16>(gm, b1, K, K, prow, &bad) : gj_inverse<32>(gm, b1, K, K, prow, &bad);
+  if (threadIdx.x == 0) bad = 0;
+  interp_smem<KP>(csi, ig, iw, c, cidx[g], M, K, G, ldc);
+  __syncthreads();
+  gram_smem<KP>(c, gm, b1, b2, b3, M, K, ldc);
+  const bool ok = inverse_smem<KP>(gm, b1, K, prow, &bad);
   if (threadIdx.x == 0 && flag) flag[g] = ok ? 0 : 1;
-  for (uint32_t e = threadIdx.x; e < KK; e += blockDim.x) Xc[(uint64_t)g * KK + e] = b1[e];
+  for (uint32_t e = threadIdx.x; e < KK; e += 256) {
+    const uint32_t o = e / K * ldm + e % K;
+    Gc[(uint64_t)g * KK + e] = gm[o];
+    Xc[(uint64_t)g * KK + e] = b1[o];
+  }
 }
 
 // per group g: ||Gc[g]||_F, and for j = -1, +1, +2 the relative distance
@@ -366,41 +396,54 @@ __global__ void features2_kernel(const float *st, float *F, uint32_t S, uint32_t
 // diagnostic), the initial iterate (coarse / learned blend / exact
 // Gauss-Jordan), Newton-Schulz steps, then the detector W_s = X C, all in
 // shared memory with the CSI staged once; X is also stored for the residual.
-// FP32 and shared-memory bound: the Gram and W take 2 x 2 and 2 x 4 outputs a
-// thread with 16-byte loads.  1200 subcarriers of 128 x 16, two steps: 24 us
-// for a Gram kernel and 43 us for the rest, an output a thread; 50 us for
-// both here.
-__global__ void __launch_bounds__(256) sub_detect_kernel(const float2 *csi, const int *ig, const float *iw,
+// Bound by instruction issue (FP32 products of small matrices), so the Gram and
+// W take 2 x 2 and 2 x 4 outputs a thread with 16-byte loads and the K x K
+// products run over the compile-time padding KP.  1200 subcarriers of 128 x 16,
+// two steps: 24 us for a Gram kernel and 43 us for the rest, an output a
+// thread; 50 us for both with run-time K, 37 us here.
+template <int KP>
+__global__ void __launch_bounds__(256, 4) sub_detect_kernel(const float2 *csi, const int *ig, const float *iw,
                                                          float2 *Gm, const float2 *Xc, const float *alpha, int mode,
                                                          uint32_t iters, float2 *Xout, float2 *W, uint32_t M,
                                                          uint32_t K, uint32_t sg, uint32_t G, int *flag) {
   extern __shared__ __align__(16) unsigned char dsm[];
   __shared__ int bad;
   __shared__ float e0sq;  // ||I - G X0||_F^2 of the initial iterate
+  constexpr uint32_t ldm = ldm_of(KP), mat = KP * ldm;
+  constexpr uint32_t NR = KP == 32 ? 4 : 1, rstep = 256 / KP;  // outputs a thread in a K x K product, rows apart
   const uint32_t KK = K * K, ldc = ldc_of(K), tid = threadIdx.x;
-  float2 *g = reinterpret_cast<float2 *>(dsm), *x = g + KK, *t = x + KK, *r4 = t + KK;
-  float2 *c = r4 + KK, *prow = c + M * ldc + 2;
+  float2 *g = reinterpret_cast<float2 *>(dsm), *x = g + mat, *t = x + mat, *r4 = t + mat;
+  float2 *c = r4 + mat, *prow = c + M * ldc + 2;
   const uint32_t s = blockIdx.x, grp = s / sg;
+  const uint32_t q = tid % KP, r0 = tid / KP;  // this thread's outputs (r0 + rstep i, q); r0 >= KP: none
   if (tid == 0) {
     bad = 0;
     e0sq = 0.f;
   }
-  interp_smem(csi, ig, iw, c, s, M, K, G, ldc);
+  interp_smem<KP>(csi, ig, iw, c, s, M, K, G, ldc);
   __syncthreads();
-  gram_smem(c, g, x, t, r4, M, K, ldc);
-  for (uint32_t e = tid; e < KK; e += blockDim.x) Gm[(uint64_t)s * KK + e] = g[e];
-  auto exact = [&]() {
-    return K <= 16 ? gj_inverse<16>(g, x, K, K, prow, &bad) : gj_inverse<32>(g, x, K, K, prow, &bad);
-  };
+  gram_smem<KP>(c, g, x, t, r4, M, K, ldc);
+#pragma unroll
+  for (uint32_t i = 0; i < NR; i++) {
+    const uint32_t r = r0 + i * rstep;
+    if (r < K && q < K) Gm[(uint64_t)s * KK + r * K + q] = g[r * ldm + q];
+  }
   if (mode == 2) {
-    const bool ok = exact();
+    const bool ok = inverse_smem<KP>(g, x, K, prow, &bad);
     if (tid == 0 && flag) flag[s] = ok ? 0 : 1;
-  } else {
-    for (uint32_t e = tid; e < KK; e += blockDim.x) {
-      float2 acc = make_float2(0.f, 0.f);
+  }
+  // the start (or, exact, X's padding)
+#pragma unroll
+  for (uint32_t i = 0; i < NR; i++) {
+    const uint32_t r = r0 + i * rstep, e = r * K + q;
+    if (r >= KP) break;
+    float2 acc = make_float2(0.f, 0.f);
+    if (r < K && q < K) {
+      if (mode == 2) continue;
       if (mode == 0) {
         acc = Xc[(uint64_t)grp * KK + e];
       } else {
+#pragma unroll
         for (int j = 0; j < kBlend; j++) {
           const int gj = min(max((int)grp + j - 1, 0), (int)G - 1);
           const float a = alpha[(uint64_t)s * kBlend + j];
@@ -409,21 +452,38 @@ __global__ void __launch_bounds__(256) sub_detect_kernel(const float2 *csi, cons
           acc.y += a * v.y;
         }
       }
-      x[e] = acc;
     }
-    if (tid == 0 && flag) flag[s] = 0;
+    x[r * ldm + q] = acc;
   }
+  if (mode != 2 && tid == 0 && flag) flag[s] = 0;
   __syncthreads();
+  // row r of A times column q of B, over the padding too
+  auto product = [&](const float2 *A, const float2 *B, float2 (&acc)[NR]) {
+#pragma unroll
+    for (uint32_t i = 0; i < NR; i++) acc[i] = make_float2(0.f, 0.f);
+    if (r0 >= KP) return;
+#pragma unroll
+    for (uint32_t k = 0; k < KP; k += 2) {
+      const float2 b0 = B[k * ldm + q], b1 = B[(k + 1) * ldm + q];
+#pragma unroll
+      for (uint32_t i = 0; i < NR; i++) {
+        const float4 a = *reinterpret_cast<const float4 *>(A + (r0 + i * rstep) * ldm + k);
+        acc[i] = cfma(make_float2(a.x, a.y), b0, acc[i]);
+        acc[i] = cfma(make_float2(a.z, a.w), b1, acc[i]);
+      }
+    }
+  };
   for (uint32_t it = 0; it < iters; it++) {
+    float2 acc[NR];
     float part = 0.f;
-    for (uint32_t e = tid; e < KK; e += blockDim.x) {
-      const uint32_t r = e / K, q = e % K;
-      float2 acc = make_float2(0.f, 0.f);
-#pragma unroll 8
-      for (uint32_t k = 0; k < K; k++) acc = cfma(g[r * K + k], x[k * K + q], acc);
-      t[e] = make_float2((r == q ? 2.f : 0.f) - acc.x, -acc.y);
-      const float ex = (r == q ? 1.f : 0.f) - acc.x;
-      part += ex * ex + acc.y * acc.y;
+    product(g, x, acc);
+#pragma unroll
+    for (uint32_t i = 0; i < NR; i++) {
+      const uint32_t r = r0 + i * rstep;
+      if (r >= KP) break;
+      t[r * ldm + q] = make_float2((r == q ? 2.f : 0.f) - acc[i].x, -acc[i].y);
+      const float ex = (r == q ? 1.f : 0.f) - acc[i].x;
+      if (r < K && q < K) part += ex * ex + acc[i].y * acc[i].y;
     }
     if (it == 0 && mode != 2) {
       for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
@@ -435,52 +495,45 @@ __global__ void __launch_bounds__(256) sub_detect_kernel(const float2 *csi, cons
       // off (the blend of neighbouring groups' inverses under a channel that
       // changes too fast across the band) takes the exact inverse instead,
       // flagged 2 (uniform: every thread read the same sum)
-      const bool ok = exact();
+      const bool ok = inverse_smem<KP>(g, x, K, prow, &bad);
       if (tid == 0 && flag) flag[s] = ok ? 2 : 1;
       break;
     }
-    float2 nx[4];
-    uint32_t n = 0;
-    for (uint32_t e = tid; e < KK; e += blockDim.x, n++) {
-      const uint32_t r = e / K, q = e % K;
-      float2 acc = make_float2(0.f, 0.f);
-#pragma unroll 8
-      for (uint32_t k = 0; k < K; k++) acc = cfma(x[r * K + k], t[k * K + q], acc);
-      nx[n] = acc;
-    }
+    product(x, t, acc);
     __syncthreads();
-    n = 0;
-    for (uint32_t e = tid; e < KK; e += blockDim.x, n++) x[e] = nx[n];
+#pragma unroll
+    for (uint32_t i = 0; i < NR; i++)
+      if (r0 + i * rstep < KP) x[(r0 + i * rstep) * ldm + q] = acc[i];
     __syncthreads();
   }
-  // X transposed into xt [v][u] (rows of an even length): a thread's two
-  // users are neighbours
-  const uint32_t ldx = (K + 1) / 2 * 2;
-  float2 *xt = t;  // with r4 behind it: room for K odd's rows of K + 1 (K = 1: two entries)
-  for (uint32_t e = tid; e < KK; e += blockDim.x) {
-    const float2 v = x[e];
-    Xout[(uint64_t)s * KK + e] = v;
-    xt[(e % K) * ldx + e / K] = v;
+  // X transposed into t (t[v][u]): a thread's two users are neighbours
+#pragma unroll
+  for (uint32_t i = 0; i < NR; i++) {
+    const uint32_t r = r0 + i * rstep;
+    if (r >= KP) break;
+    const float2 v = x[r * ldm + q];
+    if (r < K && q < K) Xout[(uint64_t)s * KK + r * K + q] = v;
+    t[q * ldm + r] = v;
   }
   __syncthreads();
-  const uint32_t T2 = (K + 1) / 2, nq = blockDim.x / T2, u = tid % T2 * 2, bq = tid / T2;
+  constexpr uint32_t T2 = KP / 2, nq = 256 / T2;
+  const uint32_t u = tid % T2 * 2, bq = tid / T2;
   const bool vc = ldc % 2 == 0, two = u + 1 < K, w16 = K % 2 == 0 && (reinterpret_cast<uintptr_t>(W) & 15) == 0;
-  if (bq >= nq) return;
+  if (u >= K) return;
   for (uint32_t b0 = bq; b0 < M; b0 += 4 * nq) {
     float2 a[4][2];
 #pragma unroll
     for (int i = 0; i < 4; i++) a[i][0] = a[i][1] = make_float2(0.f, 0.f);
-    auto step = [&](uint32_t v, const float2 (&cv)[4]) {
-      const float4 xv = pair_at(xt + v * ldx + u, true);
+    const float2 *xr = t + u, *cr[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) cr[i] = c + min(b0 + i * nq, M - 1) * ldc;
+    auto step = [&](const float4 &xv, const float2 (&cv)[4]) {
 #pragma unroll
       for (int i = 0; i < 4; i++) {
         a[i][0] = cfma(make_float2(xv.x, xv.y), cv[i], a[i][0]);
         a[i][1] = cfma(make_float2(xv.z, xv.w), cv[i], a[i][1]);
       }
     };
-    const float2 *cr[4];
-#pragma unroll
-    for (int i = 0; i < 4; i++) cr[i] = c + min(b0 + i * nq, M - 1) * ldc;
     uint32_t v = 0;
     if (vc)
 #pragma unroll 4
@@ -488,30 +541,30 @@ __global__ void __launch_bounds__(256) sub_detect_kernel(const float2 *csi, cons
         float2 c0[4], c1[4];
 #pragma unroll
         for (int i = 0; i < 4; i++) {
-          const float4 q = *reinterpret_cast<const float4 *>(cr[i] + v);
-          c0[i] = make_float2(q.x, q.y);
-          c1[i] = make_float2(q.z, q.w);
+          const float4 w = *reinterpret_cast<const float4 *>(cr[i] + v);
+          c0[i] = make_float2(w.x, w.y);
+          c1[i] = make_float2(w.z, w.w);
         }
-        step(v, c0);
-        step(v + 1, c1);
+        step(*reinterpret_cast<const float4 *>(xr + v * ldm), c0);
+        step(*reinterpret_cast<const float4 *>(xr + (v + 1) * ldm), c1);
       }
     for (; v < K; v++) {
       float2 c0[4];
 #pragma unroll
       for (int i = 0; i < 4; i++) c0[i] = cr[i][v];
-      step(v, c0);
+      step(*reinterpret_cast<const float4 *>(xr + v * ldm), c0);
     }
+    float2 *w = W + ((uint64_t)s * M + b0) * K + u;
 #pragma unroll
     for (int i = 0; i < 4; i++) {
-      const uint32_t b = b0 + i * nq;
-      if (b >= M) break;
-      float2 *w = W + ((uint64_t)s * M + b) * K + u;
+      if (b0 + i * nq >= M) break;
       if (w16) {
         *reinterpret_cast<float4 *>(w) = make_float4(a[i][0].x, a[i][0].y, a[i][1].x, a[i][1].y);
       } else {
         w[0] = a[i][0];
         if (two) w[1] = a[i][1];
       }
+      w += nq * K;
     }
   }
 }
@@ -595,16 +648,22 @@ extern "C" mb_status mb_lzf_create(uint32_t M, uint32_t K, uint32_t S, uint32_t 
 
 extern "C" uint32_t mb_lzf_num_features(uint32_t sg) { return sg + 6; }
 
-// four K x K matrices, the staged CSI and the pivot rows of the inverse
+static uint32_t kp_of(uint32_t K) { return K <= 4 ? 4 : K <= 8 ? 8 : K <= 16 ? 16 : 32; }
+// the kernel template for K users
+#define MB_LZF_OF(kernel, K) \
+  (kp_of(K) == 4 ? kernel<4> : kp_of(K) == 8 ? kernel<8> : kp_of(K) == 16 ? kernel<16> : kernel<32>)
+
+// four matrices, the staged CSI and the pivot rows of the inverse
 static size_t detect_smem(const mb_lzf *z) {
-  return sizeof(float2) * (4 * (size_t)z->K * z->K + (size_t)z->M * ldc_of(z->K) + 2 + 64);
+  const uint32_t KP = kp_of(z->K);
+  return sizeof(float2) * (4 * (size_t)KP * ldm_of(KP) + (size_t)z->M * ldc_of(z->K) + 2 + 64);
 }
 
 // centre Grams and their inverses, per-group feature statistics (FP32)
 static mb_status lzf_front(mb_lzf *z, const mb_c32 *csi, cudaStream_t st) {
   const uint32_t M = z->M, K = z->K;
-  centre_kernel<<<z->G, 256, detect_smem(z), st>>>(reinterpret_cast<const float2 *>(csi), z->ig, z->iw, z->cidx,
-                                                   z->Gc, z->Xc, M, K, z->G, z->flag);
+  MB_LZF_OF(centre_kernel, K)<<<z->G, 256, detect_smem(z), st>>>(
+      reinterpret_cast<const float2 *>(csi), z->ig, z->iw, z->cidx, z->Gc, z->Xc, M, K, z->G, z->flag);
   group_stats_kernel<<<z->G, 256, 0, st>>>(z->Gc, z->stats, K, z->G);
   MB_CUDA_TRY(cudaGetLastError());
   return MB_OK;
@@ -622,8 +681,11 @@ static mb_status lzf_configure(size_t *limit) {
   if (!(configured.load() & bit)) {
     MB_CUDA_TRY(cudaDeviceGetAttribute(&maxs, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     int l = maxs;
-    const void *ks[3] = {(const void *)centre_kernel, (const void *)sub_detect_kernel,
-                         (const void *)gram_kernel<double>};
+    const void *ks[] = {(const void *)centre_kernel<4>,      (const void *)centre_kernel<8>,
+                        (const void *)centre_kernel<16>,     (const void *)centre_kernel<32>,
+                        (const void *)sub_detect_kernel<4>,  (const void *)sub_detect_kernel<8>,
+                        (const void *)sub_detect_kernel<16>, (const void *)sub_detect_kernel<32>,
+                        (const void *)gram_kernel<double>};
     for (const void *k : ks) {
       cudaFuncAttributes fa;
       MB_CUDA_TRY(cudaFuncGetAttributes(&fa, k));
@@ -676,7 +738,7 @@ extern "C" mb_status mb_lzf_run(mb_lzf *z, const mb_c32 *csi, mb_mlp *mlp, int i
     if (r != MB_OK) return r;
   }
   const size_t smem = detect_smem(z);
-  sub_detect_kernel<<<S, 256, smem, st>>>(reinterpret_cast<const float2 *>(csi), z->ig, z->iw, z->Gs, z->Xc,
+  MB_LZF_OF(sub_detect_kernel, K)<<<S, 256, smem, st>>>(reinterpret_cast<const float2 *>(csi), z->ig, z->iw, z->Gs, z->Xc,
                                           init == MB_LZF_LEARNED ? z->alpha : nullptr, init, ns_iters, z->X,
                                           reinterpret_cast<float2 *>(W), M, K, z->sg, z->G, z->flag);
   MB_CUDA_TRY(cudaGetLastError());
