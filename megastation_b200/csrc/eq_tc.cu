@@ -29,6 +29,7 @@
 // timeout through the device error word.
 #include <algorithm>
 #include <atomic>
+#include <type_traits>
 
 #include "common.cuh"
 #include "eq_tc.cuh"
@@ -256,7 +257,7 @@ namespace mb {
 // The 256 threads hold the next 32 antennas of both operands in registers
 // (about 32 KB of loads in flight per CTA, three CTAs per SM) while the tensor
 // core multiplies the previous two tiles.  One call there: 130 us with
-// the three launches, 32 us with this one (kernel 30 us, 3.6 TB/s).
+// the three launches, 29 us with this one (kernel 26 us, 4.2 TB/s).
 // Layouts per tile (32 antennas, planes re and im one after the other):
 //   Y: MN-major, core matrices of 8 antennas x 8 columns, antenna groups 128 B
 //      apart, column chunks kTSbo apart;
@@ -298,7 +299,7 @@ __global__ void __launch_bounds__(kEqThreads, MM == 64 ? 3 : 2)
   const uint32_t c = 2 * v, l = c / p.sg, s = s_base + c - l * p.sg;
   const bool y0_on = c < ncols && s < p.S, y1_on = c < ncols && s + 1 < p.S;
   const float2 *yp = p.y + ((uint64_t)(l0 + l_off + l) * p.M + yb) * p.S + s;
-  const uint32_t y_dst = (v / 4) * kTSbo + (v % 4) * 4;
+  const uint32_t y_dst = (v / 4) * kTSbo + (v % 4) * 4 + yb * 16;  // antenna b of a chunk: 16 b bytes on
   // W: user u, the tile's antennas 8 kc .. 8 kc + 7
   const uint32_t u = tid % KP, kc = tid / KP;
   const bool w_on = kc < kTA / 8 && u < p.K;
@@ -307,25 +308,39 @@ __global__ void __launch_bounds__(kEqThreads, MM == 64 ? 3 : 2)
 
   float4 yr[kYUnits];
   float2 wr[8];
-  auto load = [&](uint32_t b0) {
+  // the next tile's operands (yp and wp move on with it): antennas left of M
+  // rows remain; a whole tile needs no look at the single rows
+  const uint64_t ys = (uint64_t)ystep * p.S;
+  const uint32_t nyu = kTA / ystep;  // column pairs per thread (uniform)
+  auto load_rows = [&](uint32_t left, auto whole) {
+    constexpr bool kWhole = decltype(whole)::value;
+    const float2 *q = yp;
 #pragma unroll
     for (int j = 0; j < kYUnits; j++) {
       yr[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-      const uint32_t b = yb + j * ystep;
-      if (b >= kTA || b0 + b >= p.M) continue;
-      const float2 *q = yp + (uint64_t)(b0 + j * ystep) * p.S;
-      if (vec && y1_on) {
-        yr[j] = __ldg(reinterpret_cast<const float4 *>(q));
-      } else {
-        if (y0_on) *reinterpret_cast<float2 *>(&yr[j].x) = __ldg(q);
-        if (y1_on) *reinterpret_cast<float2 *>(&yr[j].z) = __ldg(q + 1);
+      if (j < (int)nyu && (kWhole || yb + j * ystep < left)) {
+        if (vec && y1_on) {
+          yr[j] = __ldg(reinterpret_cast<const float4 *>(q));
+        } else {
+          if (y0_on) *reinterpret_cast<float2 *>(&yr[j].x) = __ldg(q);
+          if (y1_on) *reinterpret_cast<float2 *>(&yr[j].z) = __ldg(q + 1);
+        }
       }
+      q += ys;
     }
+    const float2 *w = wp;
 #pragma unroll
     for (int j = 0; j < 8; j++) {
       wr[j] = make_float2(0.f, 0.f);
-      if (w_on && b0 + 8 * kc + j < p.M) wr[j] = __ldg(wp + (uint64_t)(b0 + j) * p.K);
+      if (w_on && (kWhole || 8 * kc + j < left)) wr[j] = __ldg(w);
+      w += p.K;
     }
+    yp += (uint64_t)kTA * p.S;
+    wp += (uint64_t)kTA * p.K;
+  };
+  auto load = [&](uint32_t b0) {
+    if (b0 + kTA <= p.M) load_rows(kTA, std::true_type{});
+    else load_rows(p.M - b0, std::false_type{});
   };
   auto pack = [](float lo, float hi) {
     const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
@@ -335,9 +350,8 @@ __global__ void __launch_bounds__(kEqThreads, MM == 64 ? 3 : 2)
     if (c < ncols) {
 #pragma unroll
       for (int j = 0; j < kYUnits; j++) {
-        const uint32_t b = yb + j * ystep;
-        if (b >= kTA) break;
-        uint8_t *d = st + y_dst + (b / 8) * 128 + (b % 8) * 16;
+        if (j >= (int)nyu) break;
+        uint8_t *d = st + y_dst + j * ystep * 16;
         *reinterpret_cast<uint32_t *>(d) = pack(yr[j].x, yr[j].z);
         *reinterpret_cast<uint32_t *>(d + kTY) = pack(yr[j].y, yr[j].w);
       }
