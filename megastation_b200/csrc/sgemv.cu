@@ -276,12 +276,14 @@ __global__ void __launch_bounds__(256) precode_kernel(const PcParams p) {
     const uint32_t k0 = (p.S + e0 + p.start + p.N / 2) % p.N;
     uint32_t w = 1;  // lanes per row: a power of two up to 32
     while (w < n && w < 32) w *= 2;
-    for (uint32_t r = tid / w; r < nl * nb; r += blockDim.x / w) {
-      float2 *row = p.out + ((uint64_t)(l0 + r / nb) * p.M + b_base + r % nb) * p.N;
-      for (uint32_t e = tid % w; e < n; e += w) {
-        const uint32_t k = k0 + e;
-        row[k < p.N ? k : k - p.N] = make_float2(0.f, 0.f);
-      }
+    const uint32_t e1 = tid % w, rs = blockDim.x / w;
+    for (uint32_t l = 0; l < nl; l++) {
+      float2 *row = p.out + ((uint64_t)(l0 + l) * p.M + b_base + tid / w) * p.N;
+      for (uint32_t r = tid / w; r < nb; r += rs, row += (uint64_t)rs * p.N)
+        for (uint32_t e = e1; e < n; e += w) {
+          const uint32_t k = k0 + e;
+          row[k < p.N ? k : k - p.N] = make_float2(0.f, 0.f);
+        }
     }
   }
   const uint32_t s_begin = g * p.sg;
@@ -292,23 +294,24 @@ __global__ void __launch_bounds__(256) precode_kernel(const PcParams p) {
   for (int i = 0; i < TB; i++)
 #pragma unroll
     for (int j = 0; j < TC; j++) acc[i][j] = make_float2(0.f, 0.f);
-  const float2 *Pg = p.P + (uint64_t)g * p.K * p.M;
+  // this thread's loads: antenna pb and column sc, users pu / su and on
+  constexpr int NP = kPcUB * BT * TB / 256, NS = kPcUB * CT * TC / 256;
+  const uint32_t pb = tid % (BT * TB), pu = tid / (BT * TB);
+  const uint32_t sc = tid % (CT * TC), su = tid / (CT * TC);
+  const uint32_t sll = sc / p.sg, ssl = sc - sll * p.sg;
+  const bool p_on = b_base + pb < p.M, s_on = sc < ncols && ssl < ns;
+  const float2 *pp = p.P + ((uint64_t)g * p.K + pu) * p.M + b_base + pb;
+  const float2 *sp = p.s + ((uint64_t)(l0 + sll) * p.K + su) * p.S + s_begin + ssl;
+  constexpr uint32_t pstep = 256 / (BT * TB), sstep = 256 / (CT * TC);
   for (uint32_t u0 = 0; u0 < p.K; u0 += kPcUB) {
-    for (uint32_t e = tid; e < kPcUB * BT * TB; e += blockDim.x) {
-      uint32_t u = e / (BT * TB), b = e % (BT * TB);
-      float2 v = make_float2(0.f, 0.f);
-      if (u0 + u < p.K && b_base + b < p.M)
-        v = __ldg(Pg + (uint64_t)(u0 + u) * p.M + b_base + b);
-      Ps[u][b] = v;
-    }
-    for (uint32_t e = tid; e < kPcUB * CT * TC; e += blockDim.x) {
-      uint32_t u = e / (CT * TC), c = e % (CT * TC);
-      float2 v = make_float2(0.f, 0.f);
-      uint32_t ll = c / p.sg, sl = c % p.sg;
-      if (u0 + u < p.K && c < ncols && sl < ns)
-        v = __ldg(p.s + ((uint64_t)(l0 + ll) * p.K + u0 + u) * p.S + s_begin + sl);
-      Ss[u][c] = v;
-    }
+#pragma unroll
+    for (int j = 0; j < NP; j++)
+      Ps[pu + j * pstep][pb] = p_on && u0 + pu + j * pstep < p.K ? __ldg(pp + (uint64_t)(u0 + j * pstep) * p.M)
+                                                                 : make_float2(0.f, 0.f);
+#pragma unroll
+    for (int j = 0; j < NS; j++)
+      Ss[su + j * sstep][sc] = s_on && u0 + su + j * sstep < p.K ? __ldg(sp + (uint64_t)(u0 + j * sstep) * p.S)
+                                                                 : make_float2(0.f, 0.f);
     __syncthreads();
 #pragma unroll 4
     for (int u = 0; u < kPcUB; u++) {
@@ -325,16 +328,17 @@ __global__ void __launch_bounds__(256) precode_kernel(const PcParams p) {
     __syncthreads();
   }
 #pragma unroll
-  for (int i = 0; i < TB; i++)
+  for (int j = 0; j < TC; j++) {
+    const uint32_t c = tc + j * CT, ll = c / p.sg, sl = c - ll * p.sg;
+    if (c >= ncols || sl >= ns) continue;
+    const uint32_t k = (s_begin + sl + p.start + p.N / 2) % p.N;
+    float2 *o = p.out + ((uint64_t)(l0 + ll) * p.M + b_base + tb) * p.N + k;
 #pragma unroll
-    for (int j = 0; j < TC; j++) {
-      const uint32_t b = b_base + tb + i * BT, c = tc + j * CT;
-      if (b >= p.M || c >= ncols) continue;
-      const uint32_t ll = c / p.sg, sl = c % p.sg;
-      if (sl >= ns) continue;
-      const uint32_t k = (s_begin + sl + p.start + p.N / 2) % p.N;
-      p.out[((uint64_t)(l0 + ll) * p.M + b) * p.N + k] = acc[i][j];
+    for (int i = 0; i < TB; i++) {
+      if (b_base + tb + i * BT < p.M) *o = acc[i][j];
+      o += (uint64_t)BT * p.N;
     }
+  }
 }
 
 mb_status precode_fp32(const float2 *P, const float2 *s, float2 *out,
