@@ -204,7 +204,7 @@ __device__ __forceinline__ __half2 llr_clamp(__half2 v) {
 // has to tell them apart.  The interleaving puts both blocks' bits for entry e
 // at the same distance from bits 15 and 31, so one shift lines them up with
 // the FP16 sign bits.
-constexpr uint32_t kShortDeg = 10;
+constexpr uint32_t kShortDeg = 12;
 // bits 15 / 31 spread over their halves (byte permute with the selector's
 // sign-replicate bit: bytes 1 and 3's top bits)
 __device__ __forceinline__ uint32_t half_mask(uint32_t v) {
@@ -390,8 +390,12 @@ __global__ void __launch_bounds__(kMaxZ, 2) ldpc_decode_kernel(mb_ldpc h, const 
           ns = ldpc_node<4>(appb, ent + e0, deg, tid, Z4, st);
         else if (deg <= 6)
           ns = ldpc_node<6>(appb, ent + e0, deg, tid, Z4, st);
+        else if (deg <= 8)
+          ns = ldpc_node<8>(appb, ent + e0, deg, tid, Z4, st);
         else if (deg <= 10)
           ns = ldpc_node<10>(appb, ent + e0, deg, tid, Z4, st);
+        else if (deg <= 12)
+          ns = ldpc_node<12>(appb, ent + e0, deg, tid, Z4, st);
         else if (deg <= 20)
           ns = ldpc_node<20>(appb, ent + e0, deg, tid, Z4, st);
         else
