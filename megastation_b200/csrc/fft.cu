@@ -37,6 +37,7 @@ struct FftParams {
   uint64_t rows;         // n_sym * M
   uint32_t M, S, start, K, sg, ue_start;
   uint32_t S_pad;        // kUplinkLP row pitch (elements)
+  uint32_t sg_inv;       // kPilot: ceil(2^32 / sg), i / sg = high word of i sg_inv (i < 8192); 0: sg = 1
   uint32_t tail_rem;     // kPilot: S % sg when the short last group is filled (0: off)
   int in_dtype, out_dtype;
 };
@@ -171,21 +172,42 @@ struct Plan {
 __device__ __forceinline__ int pad(int i) { return i + (i >> 4); }
 
 // ---- loads and epilogues ------------------------------------------------
-__device__ __forceinline__ float2 load_iq(const FftParams &p, uint64_t e) {
-  switch (p.in_dtype) {
-    case MB_IQ_C32:
-      return __ldg(reinterpret_cast<const float2 *>(p.in) + e);
+// the 16 samples first, first + stride, ... of the input: all loads issued
+// before the first conversion, whatever the format
+__device__ __forceinline__ void load_iq16(const FftParams &p, uint64_t first, uint32_t stride, float2 (&v)[16]) {
+  switch (p.in_dtype) {  // uniform
+    case MB_IQ_C32: {
+      const float2 *q = reinterpret_cast<const float2 *>(p.in) + first;
+#pragma unroll
+      for (int i = 0; i < 16; i++) v[i] = __ldg(q + i * stride);
+      break;
+    }
     case MB_IQ_I16: {
-      short2 s = __ldg(reinterpret_cast<const short2 *>(p.in) + e);
-      return make_float2((float)s.x / 32768.f, (float)s.y / 32768.f);
+      const short2 *q = reinterpret_cast<const short2 *>(p.in) + first;
+      short2 r[16];
+#pragma unroll
+      for (int i = 0; i < 16; i++) r[i] = __ldg(q + i * stride);
+#pragma unroll
+      for (int i = 0; i < 16; i++) v[i] = make_float2((float)r[i].x / 32768.f, (float)r[i].y / 32768.f);
+      break;
     }
     case MB_IQ_I8: {
-      char2 s = reinterpret_cast<const char2 *>(p.in)[e];
-      return make_float2((float)s.x / 128.f, (float)s.y / 128.f);
+      const char2 *q = reinterpret_cast<const char2 *>(p.in) + first;
+      char2 r[16];
+#pragma unroll
+      for (int i = 0; i < 16; i++) r[i] = __ldg(q + i * stride);
+#pragma unroll
+      for (int i = 0; i < 16; i++) v[i] = make_float2((float)r[i].x / 128.f, (float)r[i].y / 128.f);
+      break;
     }
     default: {
-      __half2 h = reinterpret_cast<const __half2 *>(p.in)[e];
-      return __half22float2(h);
+      const __half2 *q = reinterpret_cast<const __half2 *>(p.in) + first;
+      __half2 r[16];
+#pragma unroll
+      for (int i = 0; i < 16; i++) r[i] = __ldg(q + i * stride);
+#pragma unroll
+      for (int i = 0; i < 16; i++) v[i] = __half22float2(r[i]);
+      break;
     }
   }
 }
@@ -234,7 +256,7 @@ __device__ __forceinline__ void epilogue(const FftParams &p, const RowCtx &c, ui
   } else if constexpr (MODE == kPilot) {
     const uint32_t i = (k - p.start - N / 2) & (N - 1);
     if (i < p.S) {
-      const uint32_t g = i / p.sg;
+      const uint32_t g = p.sg_inv ? __umulhi(i, p.sg_inv) : i;
       const uint32_t u = c.u0 + (i - g * p.sg);
       if (u < p.K) {
         const float2 ps = __ldg(p.pilot + i);
@@ -292,13 +314,9 @@ __global__ void __launch_bounds__(Plan<LOGN>::THREADS, Plan<LOGN>::MIN_BLOCKS)
     // ---- gather inputs
     if (pass == 0) {
       if (active) {
-        const uint64_t base = row * N;
-#pragma unroll
-        for (int bi = 0; bi < 16; bi++) {
-          // element j + r*N/R for butterfly j = t + (bi / R) * T, r = bi % R
-          const int j = t + (bi / R) * T, r = bi % R;
-          v[bi] = load_iq(p, base + j + r * (N / R));
-        }
+        // the first pass has radix 16: element t + r N / 16
+        static_assert(PL::P16 >= 1, "N >= 16");
+        load_iq16(p, row * N + t, N / 16, v);
       } else {
 #pragma unroll
         for (int bi = 0; bi < 16; bi++) v[bi] = make_float2(0.f, 0.f);
@@ -536,6 +554,7 @@ extern "C" mb_status mb_fft_pilot(mb_fft *f, const void *iq, int iq_dtype,
   p.start = f->d.ofdm_start;
   p.K = f->d.ue_num;
   p.sg = f->d.sc_group;
+  p.sg_inv = p.sg > 1 ? 0xFFFFFFFFu / p.sg + 1 : 0;
   p.ue_start = ue_start;
   p.in_dtype = iq_dtype;
   return launch_fft<kPilot>(f->logn, p, as_stream(stream));
@@ -587,6 +606,7 @@ mb_status mb::fft_pilot_fill(mb_fft *f, const void *iq, int iq_dtype, uint32_t n
   p.start = f->d.ofdm_start;
   p.K = f->d.ue_num;
   p.sg = f->d.sc_group;
+  p.sg_inv = p.sg > 1 ? 0xFFFFFFFFu / p.sg + 1 : 0;
   p.ue_start = 0;
   const uint32_t G = (p.S + p.sg - 1) / p.sg;
   p.tail_rem = G >= 2 ? p.S % p.sg : 0;
