@@ -43,8 +43,8 @@ mb_status zf_mixed_run(float2 *csi, void *img_w, uint32_t groups, uint32_t M, ui
 // the mixed-precision detector by a direct FP32 solve (zf_direct.cu), same
 // outputs; MB_UNSUPPORTED for K > 16 or when a group's CSI does not fit in
 // shared memory
-mb_status zf_direct_run(float2 *csi, void *img, uint32_t groups, uint32_t M, uint32_t K, float cond_thr,
-                        int32_t *status, float *cond, cudaStream_t st, bool write_w, float *wmax);
+mb_status zf_direct_run(float2 *csi, void *img, uint32_t groups, uint32_t M, uint32_t K, uint32_t ns_iters,
+                        float cond_thr, int32_t *status, float *cond, cudaStream_t st, bool write_w, float *wmax);
 // the same ZF fused with the tensor-core equalizer: each CTA keeps its
 // group's detector image in shared memory and equalizes the group's
 // columns of nb symbols of planar BF16 samples y_lp [nb][re|im][M][S_pad]

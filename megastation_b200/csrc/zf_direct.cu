@@ -5,15 +5,15 @@
 // round trips, pivots and refinement steps of a few hundred cycles each, two
 // CTAs per SM.  With up to 16 users the whole solve on the CUDA cores is
 // shorter than those round trips and small enough in registers and shared
-// memory for four CTAs per SM; its FP32 Gram and L D L^H need neither split
-// operands nor Newton-Schulz steps for an FP32 inverse X.  The rest is
+// memory for four CTAs per SM: FP32 Gram, its inverse X from L D L^H, and the
+// caller's Newton-Schulz steps on one entry a thread.  The rest is
 // zf_mixed.cu's: the 1-norm condition estimate, W = X C from BF16 X and C with
 // FP32 sums, the BF16 detector image, W (FP32) where asked for, and the FP64
 // solve of groups above the threshold or not positive definite in FP32.
 // 205 groups: 64 x 16 17 -> 12 us, 128 x 16 23 -> 18 us, 256 x 8 29 -> 16 us
 // (launch included); the same solve for 32 users loses (128 x 32: 34 -> 48 us),
 // its FP32 products outweigh the round trips.  32 uneven cells, 25 of them with
-// K <= 16: 677 -> 588 us a batched slot.
+// K <= 16: 675 -> 605 us a batched slot.
 #include <algorithm>
 #include <atomic>
 
@@ -31,7 +31,7 @@ struct ZfdParams {
   int32_t *status;
   float *cond, *wmax;
   uint32_t M, K, Mp, MM, nkt;
-  uint32_t write_w;
+  uint32_t write_w, ns_iters;
   float cond_thr;
 };
 
@@ -96,6 +96,7 @@ __global__ void __launch_bounds__(256, 4) zf_direct_kernel(const ZfdParams q) {
   double2 *Ad = reinterpret_cast<double2 *>(zd_smem + ((size_t)K * ldc * sizeof(C) + 15) / 16 * 16);
   C *A = reinterpret_cast<C *>(Ad);
   __shared__ __align__(16) float2 Xt[KP * KP];  // X transposed, rounded to BF16
+  __shared__ float2 Gm[KP * (KP + 1)], Xm[KP * (KP + 1)], Tm[KP * (KP + 1)];  // Newton-Schulz, zero padded
   __shared__ int not_pd;
   __shared__ float red[8];
   float2 *cg = q.csi + (uint64_t)g * M * K;
@@ -114,7 +115,8 @@ __global__ void __launch_bounds__(256, 4) zf_direct_kernel(const ZfdParams q) {
     for (uint32_t o = 1; o < TPR; o *= 2) rs += __shfl_xor_sync(0xffffffffu, rs, o);
     return block_max(rs, red);
   };
-  const float a1 = norm1(in ? make_float2(A[i * lda + j].x, A[i * lda + j].y) : make_float2(0.f, 0.f));
+  const float2 gij = in ? make_float2(A[i * lda + j].x, A[i * lda + j].y) : make_float2(0.f, 0.f);
+  const float a1 = norm1(gij);
   ldl_eliminate<float, KP>(A, lda, K, &not_pd);
   float cond = INFINITY;
   int st = 2;
@@ -128,6 +130,22 @@ __global__ void __launch_bounds__(256, 4) zf_direct_kernel(const ZfdParams q) {
         x.x = fmaf(li.x * lj.x + li.y * lj.y, d, x.x);
         x.y = fmaf(li.x * lj.y - li.y * lj.x, d, x.y);
       }
+    // X <- X (2I - G X)
+    const uint32_t o = i * (KP + 1) + j;
+    Gm[o] = gij;
+    for (uint32_t it = 0; it < q.ns_iters; it++) {
+      Xm[o] = x;
+      __syncthreads();
+      float2 s = make_float2(i == j ? -2.f : 0.f, 0.f);
+#pragma unroll
+      for (uint32_t k = 0; k < KP; k++) cfma(s, Gm[i * (KP + 1) + k], Xm[k * (KP + 1) + j]);
+      Tm[o] = make_float2(-s.x, -s.y);
+      __syncthreads();
+      x = make_float2(0.f, 0.f);
+#pragma unroll
+      for (uint32_t k = 0; k < KP; k++) cfma(x, Xm[i * (KP + 1) + k], Tm[k * (KP + 1) + j]);
+      __syncthreads();  // the next step overwrites X
+    }
     Xt[j * KP + i] = bf16_round(x);
     cond = a1 * norm1(x);  // its barriers also publish Xt
     if (cond <= q.cond_thr) st = 0;
@@ -202,11 +220,11 @@ size_t zfd_smem(uint32_t M, uint32_t K) {
 
 }  // namespace
 
-mb_status zf_direct_run(float2 *csi, void *img, uint32_t groups, uint32_t M, uint32_t K, float cond_thr,
-                        int32_t *status, float *cond, cudaStream_t st, bool write_w, float *wmax) {
+mb_status zf_direct_run(float2 *csi, void *img, uint32_t groups, uint32_t M, uint32_t K, uint32_t ns_iters,
+                        float cond_thr, int32_t *status, float *cond, cudaStream_t st, bool write_w, float *wmax) {
   const TcShape s = tc_shape(M, K);
   const ZfdParams p{csi, reinterpret_cast<uint8_t *>(img), status, cond, write_w ? wmax : nullptr, M, K, s.Mp, s.MM,
-                    s.nkt, write_w ? 1u : 0u, cond_thr};
+                    s.nkt, write_w ? 1u : 0u, ns_iters, cond_thr};
   const size_t smem = zfd_smem(M, K);
   static std::atomic<uint64_t> configured{0};
   static std::atomic<int> limit{0};

@@ -1262,10 +1262,12 @@ static mb_status zf_mixed_launch(float2 *csi, void *img_w, uint32_t groups, uint
   if (K == 0 || K > 64) return MB_UNSUPPORTED;
   const bool learned = opts && opts->init == 1;
   if (opts && opts->init > 1) return MB_BAD_ARG;
+  const uint32_t ns_iters = opts ? opts->ns_iters : 2;
   const float cond_thr = opts && opts->cond_threshold > 0 ? opts->cond_threshold : 1e4f;
   if (!learned && !fe && path != 2) {
     // K <= 16 and a group's CSI in shared memory: the direct solve
-    const mb_status r = zf_direct_run(csi, img_w, groups, M, K, cond_thr, status, cond, st, write_w, wmax);
+    const mb_status r = zf_direct_run(csi, img_w, groups, M, K, ns_iters, cond_thr, status, cond, st, write_w,
+                                      wmax);
     if (r != MB_UNSUPPORTED) return r;
   }
   if (learned && (!net || !net->w1 || net->width == 0 || net->width > kZfInitMaxWidth)) return MB_BAD_ARG;
@@ -1286,7 +1288,7 @@ static mb_status zf_mixed_launch(float2 *csi, void *img_w, uint32_t groups, uint
   q.Mp = s.Mp;
   q.nkt = s.nkt;
   q.nh = s.Mp / kKT;
-  q.ns_iters = opts ? opts->ns_iters : 2;
+  q.ns_iters = ns_iters;
   q.cond_thr = cond_thr;
   // bulk copies want 16-byte aligned addresses and sizes: the network's six
   // arrays (width a multiple of 4), and CSI k tiles (K even)

@@ -81,6 +81,11 @@ def test_direct_slot_matches_tensor_core_slot():
         llr, hard = cs(iq, stream=st)
         st.synchronize()
         out.append([(a.float().cpu(), h.cpu().numpy()) for a, h in zip(llr, hard)])
-    for (a, ha), (b, hb) in zip(*out):
-        assert float((a - b).norm() / b.norm()) <= 5e-3
+    for c, (a, ha), (b, hb) in zip(cfgs, *out):
+        # each path rounds X and C to BF16 (2^-9 an entry, differently scaled):
+        # W y is off by 2 * 2^-9 |X| |G| of the symbols, twice for the two paths
+        H = datagen.make_slot(c)["H"][:: c.sg]
+        G = np.conj(H.transpose(0, 2, 1)) @ H
+        amp = (np.abs(np.linalg.inv(G)) @ np.abs(G)).sum(2).max()
+        assert float((a - b).norm() / b.norm()) <= 2.0 ** -7 * amp
         assert np.mean(np.unpackbits(ha) != np.unpackbits(hb)) <= 1e-3
