@@ -153,6 +153,23 @@ def _load():
         "mb_ldpc_encode": (ST, [VP, VP, U64, VP, U64, U32, VP]),
         "mb_ldpc_decode": (ST, [VP, VP, U64, VP, U64, U32, U32, VP]),
         "mb_cells_set_zf_path": (ST, [VP, VP]),
+        "mb_mlp_create": (ST, [U32, U32, U32, U32, U64, ctypes.POINTER(VP)]),
+        "mb_mlp_destroy": (ST, [VP]),
+        "mb_mlp_num_params": (ST, [VP, ctypes.POINTER(U64)]),
+        "mb_mlp_get_params": (ST, [VP, VP]),
+        "mb_mlp_set_params": (ST, [VP, VP]),
+        "mb_mlp_get_grads": (ST, [VP, VP]),
+        "mb_mlp_forward": (ST, [VP, VP, U32, VP, VP]),
+        "mb_mlp_loss_grad": (ST, [VP, VP, VP, VP, VP, U32, VP, VP]),
+        "mb_mlp_adam_step": (ST, [VP, ctypes.c_float, VP]),
+        "mb_lzf_create": (ST, [U32, U32, U32, U32, ctypes.POINTER(VP)]),
+        "mb_lzf_destroy": (ST, [VP]),
+        "mb_lzf_num_features": (U32, [U32]),
+        "mb_lzf_features": (ST, [VP, VP, VP, VP]),
+        "mb_lzf_targets": (ST, [VP, VP, VP, VP, VP]),
+        "mb_lzf_run": (ST, [VP, VP, VP, I32, U32, VP, VP]),
+        "mb_lzf_flags": (ST, [VP, VP, VP]),
+        "mb_lzf_residual": (ST, [VP, VP, VP]),
         "mb_cells_set_tuning": (ST, [VP, ctypes.POINTER(U32), ctypes.POINTER(U32)]),
     }
     for name, (res, args) in sigs.items():

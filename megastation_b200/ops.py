@@ -9,6 +9,7 @@ tensor here.  All compute runs in libmegastation_b200.so; nothing here
 computes on the host.
 """
 import ctypes
+import functools
 
 import torch
 
@@ -23,12 +24,22 @@ _IQ_CODE = {
 }
 
 
+# Pointers and streams go to the library as plain integers (ctypes converts
+# them by the declared argument types), and the current stream is read as its
+# raw handle: a small operator's kernel takes about as long as the call's
+# Python (1024-point FFT of 32 rows: 9.6 -> 6.1 us a call).
+_get_device = torch._C._cuda_getDevice if hasattr(torch._C, "_cuda_getDevice") else None
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def _stream(stream):
     if stream is None:
-        return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+        if _raw_stream is None:
+            return torch.cuda.current_stream().cuda_stream
+        return _raw_stream(_get_device())
     if isinstance(stream, torch.cuda.Stream):
-        return ctypes.c_void_p(stream.cuda_stream)
-    return ctypes.c_void_p(int(stream))
+        return stream.cuda_stream
+    return int(stream)
 
 
 def _dev(t, name, dtype=None):
@@ -38,23 +49,20 @@ def _dev(t, name, dtype=None):
         raise ValueError(f"{name} must be contiguous")
     if dtype is not None and t.dtype != dtype:
         raise ValueError(f"{name} must be {dtype}, got {t.dtype}")
-    return ctypes.c_void_p(t.data_ptr())
+    return t.data_ptr()
 
 
 def _iq(t, name, M, N):
     """IQ tensor: [..., M, N] complex64 or [..., M, N, 2] int16/int8/float16."""
-    if t.dtype not in _IQ_CODE:
+    code = _IQ_CODE.get(t.dtype)
+    if code is None:
         raise ValueError(f"{name}: unsupported dtype {t.dtype}")
-    code = _IQ_CODE[t.dtype]
-    shape = tuple(t.shape) if code == _lib.MB_IQ_C32 else tuple(t.shape[:-1])
-    if code != _lib.MB_IQ_C32 and t.shape[-1] != 2:
+    shape, pair = t.shape, 0 if code == _lib.MB_IQ_C32 else 1
+    if pair and shape[-1] != 2:
         raise ValueError(f"{name}: integer IQ needs a trailing (I, Q) dimension")
-    if len(shape) < 2 or shape[-2:] != (M, N):
-        raise ValueError(f"{name}: expected [..., {M}, {N}] samples, got {tuple(t.shape)}")
-    n_sym = 1
-    for d in shape[:-2]:
-        n_sym *= d
-    return _dev(t, name), code, n_sym
+    if len(shape) < 2 + pair or shape[-1 - pair] != N or shape[-2 - pair] != M:
+        raise ValueError(f"{name}: expected [..., {M}, {N}] samples, got {tuple(shape)}")
+    return _dev(t, name), code, t.numel() // (M * N << pair)
 
 
 class _FFTBase:
@@ -317,6 +325,14 @@ class Equalize:
 
 
     @staticmethod
+    @functools.lru_cache(maxsize=64)
+    def _tc_scratch(K, M, S, sg, n_sym):
+        img, ylp = _lib.U64(), _lib.U64()
+        check(LIB.mb_equalize_tc_scratch(K, M, S, sg, n_sym, ctypes.byref(img), ctypes.byref(ylp)),
+              "mb_equalize_tc_scratch")
+        return img.value, ylp.value
+
+    @staticmethod
     def equalize_tc(csi, bsVec, ueVec, csi_skip, mod_order, cb_size, zeros, cb_blocks=1,
                     hard=None, scrambler=None, x=None, stream=None):
         """Mixed-precision variant on the tensor cores (BF16 W and y, FP32
@@ -324,11 +340,9 @@ class Equalize:
         M, K = csi.shape[-2], csi.shape[-1]
         S = bsVec.shape[-1]
         n_sym = bsVec.numel() // (M * S)
-        img, ylp = _lib.U64(), _lib.U64()
-        check(LIB.mb_equalize_tc_scratch(K, M, S, csi_skip, n_sym, ctypes.byref(img), ctypes.byref(ylp)),
-              "mb_equalize_tc_scratch")
-        s_img = torch.empty(img.value, dtype=torch.uint8, device=csi.device)
-        s_ylp = torch.empty(ylp.value, dtype=torch.uint8, device=csi.device)
+        img, ylp = Equalize._tc_scratch(K, M, S, csi_skip, n_sym)
+        s_img = torch.empty(img, dtype=torch.uint8, device=csi.device)
+        s_ylp = torch.empty(ylp, dtype=torch.uint8, device=csi.device)
         cb_stride = ueVec.shape[-1]
         if ueVec.numel() != n_sym * K * cb_blocks * cb_stride:
             raise ValueError("ueVec must be [n_sym, K*cb_blocks, cb_stride]")
