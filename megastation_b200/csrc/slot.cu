@@ -37,7 +37,8 @@ struct mb_slot {
   uint32_t S_pad;
   uint32_t sb_cap;    // uplink symbols the y / y_lp buffers hold (>= sym_batch)
   uint32_t eq_cols;   // tensor-core equalizer columns per CTA (0: 128)
-  uint32_t fft_ctas;  // CTAs of each tensor-core FFT launch (0: one per SM)
+  uint32_t fft_ctas;  // CTAs of each tensor-core FFT launch (0: fft_share)
+  uint32_t fft_share = 0;  // this cell's share of the SMs among batched cells (0: one CTA per SM)
   uint32_t zf_path;   // mixed ZF, K <= 32: 0 by K, 1 CUDA-core products, 2 tensor-core products
   mb_ldpc *ldpc = nullptr;  // decode stage's code (not owned), or null
   uint32_t ldpc_iters = 0;
@@ -270,11 +271,12 @@ static mb_status issue_uplink(mb_slot *s, const void *iq, uint16_t *llr,
   const char *iq_b = reinterpret_cast<const char *>(iq);
   mb_status r;
   const bool mixed = c.zf_precision == MB_ZF_MIXED;
+  const uint32_t fft_ctas = s->fft_ctas ? s->fft_ctas : s->fft_share;
   // uplink FFT of nb symbols from l0: FP32 rows for the SIMT equalizer, or
   // planar BF16 rows for the tensor-core equalizer
   auto fft_batch = [&](uint32_t l0, uint32_t nb, cudaStream_t fs) {
     const void *src = iq_b + (size_t)(c.P + l0) * sym_bytes;
-    return mixed ? fft_uplink_lp(s->fft, src, c.iq_dtype, nb, s->y_lp, s->S_pad, fs, s->fft_ctas)
+    return mixed ? fft_uplink_lp(s->fft, src, c.iq_dtype, nb, s->y_lp, s->S_pad, fs, fft_ctas)
                  : mb_fft_uplink(s->fft, src, c.iq_dtype, nb, reinterpret_cast<mb_c32 *>(s->y), fs);
   };
   // Mixed precision at N = 4096: the pilot symbols and the first uplink
@@ -310,7 +312,7 @@ static mb_status issue_uplink(mb_slot *s, const void *iq, uint16_t *llr,
   if (combined) {
     MARK(mk->fft_b[0]);
     r = fft_slot_tc(s->fft, iq, c.iq_dtype, c.P, nb0, reinterpret_cast<mb_c32 *>(s->csi), s->y_lp, s->S_pad, cs,
-                    s->fft_ctas);
+                    fft_ctas);
     if (r != MB_OK) return r;
     MARK(mk->fft_e[0]);
   }
@@ -653,6 +655,31 @@ extern "C" mb_status mb_cells_destroy(mb_cells *cs) {
   return MB_OK;
 }
 
+// The default CTAs of the cells' tensor-core FFT launches.  Such a CTA holds a
+// whole SM and spends about 14 us on its start (operands, tables, its code)
+// against about 2.5 us per two rows of complex float samples, so with several
+// such cells one CTA per SM and launch pays the start on every SM once per
+// cell, and nothing else runs there meanwhile.  Each cell gets SMs in
+// proportion to its rows instead: the launches fit beside one another and
+// every SM pays one start (32 cells, 12 of them of N = 4096: 605 -> 547 us a
+// batched slot).
+static mb_status cells_share_sms(mb_cells *cs) {
+  int dev = 0, sms = 0;
+  MB_CUDA_TRY(cudaGetDevice(&dev));
+  MB_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  auto rows = [](const mb_slot *s) -> uint64_t {
+    const mb_cell_desc &c = s->c;
+    return c.zf_precision == MB_ZF_MIXED && c.N == 4096 ? (uint64_t)(c.P + c.U) * c.M : 0;
+  };
+  uint64_t total = 0;
+  for (const auto *s : cs->slots) total += rows(s);
+  for (auto *s : cs->slots) {
+    const uint64_t r = rows(s);
+    s->fft_share = r ? (uint32_t)std::max<uint64_t>(1, (r * sms + total / 2) / total) : 0;
+  }
+  return MB_OK;
+}
+
 extern "C" mb_status mb_cells_create(const mb_cell_desc *cells, uint32_t n, mb_cells **out) {
   if (!cells || !out || n == 0) return MB_BAD_ARG;
   *out = nullptr;
@@ -678,6 +705,7 @@ extern "C" mb_status mb_cells_create(const mb_cell_desc *cells, uint32_t n, mb_c
     cudaError_t ce = cudaEventCreateWithFlags(&cs->fork, cudaEventDisableTiming);
     if (ce != cudaSuccess) st = record_error(ce);
   }
+  if (st == MB_OK) st = cells_share_sms(cs);
   if (st != MB_OK) {
     mb_cells_destroy(cs);
     return st;
