@@ -24,8 +24,8 @@
 // q_e = app - r_e (r_e the node's previous message to entry e, rebuilt from
 // its compressed state), min1, min2 and the parity of the sign bits of q,
 // then app = q_e + r'_e, r'_e = +-min(0.75 min, 256).  Rows
-// of up to 20 entries keep q in registers (ldpc_node, variants for 4, 6, 10
-// and 20 entries).  FP16 is the reference decoder's precision (cuPHY), and
+// of up to 20 entries keep q in registers (ldpc_node, a variant per two
+// degrees up to 12).  FP16 is the reference decoder's precision (cuPHY), and
 // the pairs halve the instructions per block; channel LLRs clamped to
 // +-1024 and messages to +-256 keep every value finite for up to 32 passes.
 // Within a layer the Z check nodes touch disjoint variables (a circulant is
@@ -272,12 +272,13 @@ __device__ __forceinline__ __half2 *app_slot(uint8_t *app, const uint2 &en, uint
   return reinterpret_cast<__half2 *>(app + (en.x + 4 * tid - (tid >= en.y ? Z4 : 0u)));
 }
 
-// One check node's update for the pair over a row of at most D entries, all
-// in registers: every app load issued before any store (a row holds one
+// One check node's update for the pair over a row of MIN to D entries, all in
+// registers: every app load issued before any store (a row holds one
 // circulant per column block, so the node's D slots are distinct), then
 // q_e = app - r_e (r_e from the node's previous state) with the min tracking,
-// then app = q_e + r'_e.  Returns the new state.
-template <int D>
+// then app = q_e + r'_e.  Returns the new state.  The entries up to MIN need no
+// look at the degree.
+template <int MIN, int D>
 __device__ __forceinline__ uint4 ldpc_node(uint8_t *app, const uint2 *ent, uint32_t deg, uint32_t tid, uint32_t Z4,
                                            const uint4 &st) {
   constexpr bool kShort = D <= (int)kShortDeg;
@@ -287,7 +288,7 @@ __device__ __forceinline__ uint4 ldpc_node(uint8_t *app, const uint2 *ent, uint3
   __half2 q[D];
 #pragma unroll
   for (int j = 0; j < D; j++) {
-    if (j < (int)deg) {
+    if (j < MIN || j < (int)deg) {
       __half2 *a = app_slot(app, ent[j], tid, Z4);
       if constexpr (kShort) slot[j] = a;
       q[j] = *a;
@@ -299,7 +300,7 @@ __device__ __forceinline__ uint4 ldpc_node(uint8_t *app, const uint2 *ent, uint3
   t.init();
 #pragma unroll
   for (int j = 0; j < D; j++) {
-    if (j < (int)deg) {
+    if (j < MIN || j < (int)deg) {
       q[j] = __hsub2(q[j], old_msg(st.x, st.y, j < 16 ? st.z : st.w, j < 16 ? y_lo : y_hi, j));
       t.add(q[j]);
     }
@@ -308,7 +309,7 @@ __device__ __forceinline__ uint4 ldpc_node(uint8_t *app, const uint2 *ent, uint3
   n.init(t, deg);
 #pragma unroll
   for (int j = 0; j < D; j++) {
-    if (j < (int)deg) {
+    if (j < MIN || j < (int)deg) {
       __half2 *a;
       if constexpr (kShort) a = slot[j];
       else a = app_slot(app, ent[j], tid, Z4);
@@ -352,7 +353,7 @@ __global__ void __launch_bounds__(kMaxZ, 2) ldpc_decode_kernel(mb_ldpc h, const 
   const uint32_t Z = h.Z, kb = h.kb, mb = h.mb, N = (kb + mb) * Z, tid = threadIdx.x, nt = blockDim.x;
   __half2 *app = reinterpret_cast<__half2 *>(dec_smem);
   uint2 *ent = reinterpret_cast<uint2 *>(dec_smem + (N + 1) / 2 * 2);  // [nnz]
-  uint32_t *r_ptr = reinterpret_cast<uint32_t *>(ent + h.nnz);         // [mb + 1]
+  uint32_t *row = reinterpret_cast<uint32_t *>(ent + h.nnz);           // [mb]
   const uint32_t cb = b0 + 2 * blockIdx.x;
   const bool two = 2 * blockIdx.x + 1 < nb;
   const __half *in0 = llr + (uint64_t)cb * llr_stride;
@@ -364,46 +365,59 @@ __global__ void __launch_bounds__(kMaxZ, 2) ldpc_decode_kernel(mb_ldpc h, const 
     ent[e] = make_uint2(4 * ((uint32_t)h.col[e] * Z + h.sh[e]), Z - h.sh[e]);
   uint8_t *appb = reinterpret_cast<uint8_t *>(app);
   const uint32_t Z4 = 4 * Z;
-  for (uint32_t i = tid; i <= mb; i += nt) r_ptr[i] = h.row_ptr[i];
+  // row i: first entry, degree in the upper half (27 entries of 8 bytes a row
+  // at most: the shared memory ends long before 2^16 of them)
+  for (uint32_t i = tid; i < mb; i += nt) row[i] = h.row_ptr[i] | (h.row_ptr[i + 1] - h.row_ptr[i]) << 16;
   __syncthreads();
   // Thread z only ever reads and writes check node z's state, so its loads
   // run two layers ahead of their use (a row's state is rewritten mb >= 4
   // layers before it is read again); the first pass starts from zero
   // messages without reading.
   uint4 *state = h.state + (uint64_t)blockIdx.x * mb * Z;
-  // the state of row r in pass it: none in the first pass nor past the last
-  auto load_state = [&](uint32_t it, uint32_t r) {
-    return (it == 0 || it >= max_iter || tid >= Z) ? make_uint4(0u, 0u, 0u, 0u) : state[r * Z + tid];
-  };
-  uint4 st_a = load_state(0, 0), st_b = load_state(0, 1);
-  for (uint32_t it = 0; it < max_iter; it++) {
-    for (uint32_t i = 0; i < mb; i++) {
-      const uint4 st = st_a;
-      st_a = st_b;
-      // row i + 2, in this pass or the next (mb >= 4)
-      st_b = i + 2 < mb ? load_state(it, i + 2) : load_state(it + 1, i + 2 - mb);
-      if (tid < Z) {
-        const uint32_t e0 = r_ptr[i], deg = r_ptr[i + 1] - e0;
-        // every thread of the layer takes the same branch
-        uint4 ns;
-        if (deg <= 4)
-          ns = ldpc_node<4>(appb, ent + e0, deg, tid, Z4, st);
-        else if (deg <= 6)
-          ns = ldpc_node<6>(appb, ent + e0, deg, tid, Z4, st);
-        else if (deg <= 8)
-          ns = ldpc_node<8>(appb, ent + e0, deg, tid, Z4, st);
-        else if (deg <= 10)
-          ns = ldpc_node<10>(appb, ent + e0, deg, tid, Z4, st);
-        else if (deg <= 12)
-          ns = ldpc_node<12>(appb, ent + e0, deg, tid, Z4, st);
-        else if (deg <= 20)
-          ns = ldpc_node<20>(appb, ent + e0, deg, tid, Z4, st);
+  const uint32_t layers = max_iter * mb;
+  uint4 st_a = make_uint4(0u, 0u, 0u, 0u), st_b = st_a;
+  uint32_t i = 0, i2 = 2, o = tid, o2 = 2 * Z + tid;  // this layer's row and the one two layers on, their state
+  for (uint32_t l = 0; l < layers; l++) {
+    const uint4 st = st_a;
+    st_a = st_b;
+    if (tid < Z) {
+      if (l + 2 >= mb && l + 2 < layers) st_b = state[o2];
+      const uint32_t rw = row[i], deg = rw >> 16;
+      const uint2 *en = ent + (rw & 0xFFFFu);
+      // every thread of the layer takes the same branch
+      uint4 ns;
+      if (deg <= 6) {
+        if (deg <= 2)
+          ns = ldpc_node<1, 2>(appb, en, deg, tid, Z4, st);
+        else if (deg <= 4)
+          ns = ldpc_node<3, 4>(appb, en, deg, tid, Z4, st);
         else
-          ns = ldpc_node_any(appb, ent + e0, deg, tid, Z4, st);
-        state[i * Z + tid] = ns;
+          ns = ldpc_node<5, 6>(appb, en, deg, tid, Z4, st);
+      } else if (deg <= 10) {
+        if (deg <= 8)
+          ns = ldpc_node<7, 8>(appb, en, deg, tid, Z4, st);
+        else
+          ns = ldpc_node<9, 10>(appb, en, deg, tid, Z4, st);
+      } else if (deg <= 12) {
+        ns = ldpc_node<11, 12>(appb, en, deg, tid, Z4, st);
+      } else if (deg <= 20) {
+        ns = ldpc_node<13, 20>(appb, en, deg, tid, Z4, st);
+      } else {
+        ns = ldpc_node_any(appb, en, deg, tid, Z4, st);
       }
-      __syncthreads();
+      state[o] = ns;
     }
+    o += Z;
+    o2 += Z;
+    if (++i == mb) {
+      i = 0;
+      o = tid;
+    }
+    if (++i2 == mb) {
+      i2 = 0;
+      o2 = tid;
+    }
+    __syncthreads();
   }
   // hard decisions of the information bits, MSB first, both blocks
   uint8_t *o0 = out + (uint64_t)cb * out_stride, *o1 = o0 + out_stride;
