@@ -659,12 +659,11 @@ static size_t detect_smem(const mb_lzf *z) {
   return sizeof(float2) * (4 * (size_t)KP * ldm_of(KP) + (size_t)z->M * ldc_of(z->K) + 2 + 64);
 }
 
-// centre Grams and their inverses, per-group feature statistics (FP32)
+// centre Grams and their inverses (FP32)
 static mb_status lzf_front(mb_lzf *z, const mb_c32 *csi, cudaStream_t st) {
   const uint32_t M = z->M, K = z->K;
   MB_LZF_OF(centre_kernel, K)<<<z->G, 256, detect_smem(z), st>>>(
       reinterpret_cast<const float2 *>(csi), z->ig, z->iw, z->cidx, z->Gc, z->Xc, M, K, z->G, z->flag);
-  group_stats_kernel<<<z->G, 256, 0, st>>>(z->Gc, z->stats, K, z->G);
   MB_CUDA_TRY(cudaGetLastError());
   return MB_OK;
 }
@@ -707,15 +706,21 @@ static mb_status lzf_shared_mem_ok(const mb_lzf *z) {
   return (size_t)z->M * z->K * sizeof(double2) <= limit && detect_smem(z) <= limit ? MB_OK : MB_UNSUPPORTED;
 }
 
+// the network's inputs from the centre Grams, as rows in memory
+static mb_status lzf_features_of(mb_lzf *z, float *features, cudaStream_t st) {
+  group_stats_kernel<<<z->G, 256, 0, st>>>(z->Gc, z->stats, z->K, z->G);
+  features2_kernel<<<grid_for((uint64_t)z->S * (z->sg + 6)), 256, 0, st>>>(z->stats, features, z->S, z->sg);
+  MB_CUDA_TRY(cudaGetLastError());
+  return MB_OK;
+}
+
 extern "C" mb_status mb_lzf_features(mb_lzf *z, const mb_c32 *csi, float *features, void *stream) {
   if (!z || !csi || !features) return MB_BAD_ARG;
   if (lzf_shared_mem_ok(z) != MB_OK) return MB_UNSUPPORTED;
   cudaStream_t st = as_stream(stream);
   mb_status r = lzf_front(z, csi, st);
   if (r != MB_OK) return r;
-  features2_kernel<<<grid_for((uint64_t)z->S * (z->sg + 6)), 256, 0, st>>>(z->stats, features, z->S, z->sg);
-  MB_CUDA_TRY(cudaGetLastError());
-  return MB_OK;
+  return lzf_features_of(z, features, st);
 }
 
 extern "C" mb_status mb_lzf_run(mb_lzf *z, const mb_c32 *csi, mb_mlp *mlp, int init,
@@ -728,12 +733,11 @@ extern "C" mb_status mb_lzf_run(mb_lzf *z, const mb_c32 *csi, mb_mlp *mlp, int i
   mb_status r = lzf_front(z, csi, st);
   if (r != MB_OK) return r;
   if (init == MB_LZF_LEARNED) {
-    // the features go straight into the network's input tiles where its shape allows
-    r = mlp_forward_stats(mlp, z->stats, z->sg, S, z->alpha, st);
+    // the network's kernel forms its inputs itself where its shape allows
+    r = mlp_forward_features(mlp, BlendFeatures{z->Gc, z->sg, K, z->G}, S, z->alpha, st);
     if (r == MB_UNSUPPORTED) {
-      features2_kernel<<<grid_for((uint64_t)S * (z->sg + 6)), 256, 0, st>>>(z->stats, z->feat, S, z->sg);
-      MB_CUDA_TRY(cudaGetLastError());
-      r = mb_mlp_forward(mlp, z->feat, S, z->alpha, st);
+      r = lzf_features_of(z, z->feat, st);
+      if (r == MB_OK) r = mb_mlp_forward(mlp, z->feat, S, z->alpha, st);
     }
     if (r != MB_OK) return r;
   }

@@ -634,7 +634,7 @@ extern "C" mb_status mb_mlp_forward(mb_mlp *n, const float *x, uint32_t batch, f
   if (!n || !x || !y) return MB_BAD_ARG;
   if (batch == 0) return MB_OK;
   if (n->img) {
-    MB_CUDA_TRY(mlp_fwd_tc(n->ss, n->img, n->p, x, nullptr, 0, batch, y,
+    MB_CUDA_TRY(mlp_fwd_tc(n->ss, n->img, n->p, x, {}, batch, y,
                            device_tables() ? device_tables()->err : nullptr, as_stream(stream)));
     return MB_OK;
   }
@@ -680,10 +680,9 @@ extern "C" mb_status mb_mlp_forward(mb_mlp *n, const float *x, uint32_t batch, f
   return MB_OK;
 }
 
-mb_status mb::mlp_forward_stats(mb_mlp *n, const float *stats, uint32_t sg, uint32_t B, float *y, cudaStream_t st) {
-  if (!n || !n->img || n->n_in != sg + 6) return MB_UNSUPPORTED;
-  MB_CUDA_TRY(mlp_fwd_tc(n->ss, n->img, n->p, nullptr, stats, sg, B, y,
-                         device_tables() ? device_tables()->err : nullptr, st));
+mb_status mb::mlp_forward_features(mb_mlp *n, const BlendFeatures &f, uint32_t B, float *y, cudaStream_t st) {
+  if (!n || !n->img || n->n_in != f.sg + 6) return MB_UNSUPPORTED;
+  MB_CUDA_TRY(mlp_fwd_tc(n->ss, n->img, n->p, nullptr, f, B, y, device_tables() ? device_tables()->err : nullptr, st));
   return MB_OK;
 }
 

@@ -40,9 +40,8 @@ struct StepParams {
   float *part;
   int *err;
   uint32_t B, tiles;
-  const float *stats;  // inference on features (see mlp_fwd_tc), or null
-  uint32_t sg;
-  float *y;            // inference: the outputs
+  BlendFeatures f;  // inference without x
+  float *y;         // inference: the outputs
 };
 
 // one operand: shared-memory address, leading and stride byte offsets, bytes
@@ -198,6 +197,43 @@ __global__ void __launch_bounds__(128 * MT, 1) mlp_step_kernel(const StepParams 
       tc::mbar_arrive_expect_tx(&wbar2, w2_bytes);
       tc::bulk_g2s(w2, q.img + s.img2(), w2_bytes, &wbar2);
     }
+    // inference on features: the six statistics of the tile's groups, a warp a
+    // group, in the (unused) dy region
+    float *fs = reinterpret_cast<float *>(dy);
+    const uint32_t fg0 = FWD && !q.x ? row0 / q.f.sg : 0;
+    if (FWD && !q.x) {
+      const uint32_t KK = q.f.K * q.f.K;
+      for (uint32_t g = fg0 + warp; g <= (row0 + nv - 1) / q.f.sg; g += nthr / 32) {
+        const float2 *c0 = q.f.gc + (uint64_t)g * KK;
+        float v[8] = {0, 0, 0, 0, 0, 0, 0, 0};  // ||C_g||^2, trace, then distances and traces of j = -1, 1, 2
+        for (uint32_t e = lane; e < KK; e += 32) {
+          const float2 a = __ldg(c0 + e);
+          const bool diag = e % (q.f.K + 1) == 0;
+          v[0] += a.x * a.x + a.y * a.y;
+          if (diag) v[1] += a.x;
+#pragma unroll
+          for (int k = 0; k < 3; k++) {
+            const int gj = (int)g + (k == 0 ? -1 : k);
+            if (gj < 0 || gj >= (int)q.f.G) continue;
+            const float2 b = __ldg(q.f.gc + (uint64_t)gj * KK + e);
+            v[2 + k] += (b.x - a.x) * (b.x - a.x) + (b.y - a.y) * (b.y - a.y);
+            if (diag) v[5 + k] += b.x;
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < 8; i++)
+          for (int o = 16; o > 0; o >>= 1) v[i] += __shfl_xor_sync(0xffffffffu, v[i], o);
+        if (lane < 3) {
+          const int gj = (int)g + (lane == 0 ? -1 : (int)lane);
+          const bool in = gj >= 0 && gj < (int)q.f.G;
+          const float n0 = sqrtf(v[0]), d = lane == 0 ? v[2] : lane == 1 ? v[3] : v[4],
+                      t = lane == 0 ? v[5] : lane == 1 ? v[6] : v[7];
+          fs[(g - fg0) * 6 + lane] = in && n0 > 0.f ? sqrtf(d) / n0 : 0.f;
+          fs[(g - fg0) * 6 + 3 + lane] = in && v[1] > 0.f ? t / v[1] - 1.f : 0.f;
+        }
+      }
+      __syncthreads();
+    }
     for (uint32_t e = tid; e < kT * (Ip / 8); e += nthr) {
       const uint32_t r = e / (Ip / 8), ch = e % (Ip / 8);
       float v[8];
@@ -206,8 +242,8 @@ __global__ void __launch_bounds__(128 * MT, 1) mlp_step_kernel(const StepParams 
         const uint32_t f = ch * 8 + j, row = row0 + r;
         v[j] = 0.f;
         if (r < nv && f < I) {
-          if (!FWD || !q.stats) v[j] = __ldg(q.x + (uint64_t)row * I + f);
-          else v[j] = f < q.sg ? (f == row % q.sg ? 1.f : 0.f) : __ldg(q.stats + row / q.sg * 6 + f - q.sg);
+          if (!FWD || q.x) v[j] = __ldg(q.x + (uint64_t)row * I + f);
+          else v[j] = f < q.f.sg ? (f == row % q.f.sg ? 1.f : 0.f) : fs[(row / q.f.sg - fg0) * 6 + f - q.f.sg];
         }
       }
       *reinterpret_cast<uint4 *>(xs + r / 8 * rsx + ch * 128 + r % 8 * 16) =
@@ -454,8 +490,8 @@ bool mlp_step_shape(uint32_t I, uint32_t W, uint32_t O, const uint64_t off[6], u
 }
 
 cudaError_t mlp_fwd_tc(const MlpStepShape &s, const __nv_bfloat16 *img, const float *params, const float *x,
-                       const float *stats, uint32_t sg, uint32_t B, float *y, int *err, cudaStream_t st) {
-  StepParams q{s, img, params, x, nullptr, nullptr, nullptr, nullptr, err, B, (B + kT - 1) / kT, stats, sg, y};
+                       const BlendFeatures &f, uint32_t B, float *y, int *err, cudaStream_t st) {
+  StepParams q{s, img, params, x, nullptr, nullptr, nullptr, nullptr, err, B, (B + kT - 1) / kT, f, y};
   const unsigned grid = std::min(q.tiles, kStepSlots);
   return s.Wp == 128 ? launch<1, true>(q, grid, st) : launch<2, true>(q, grid, st);
 }
@@ -463,7 +499,7 @@ cudaError_t mlp_fwd_tc(const MlpStepShape &s, const __nv_bfloat16 *img, const fl
 cudaError_t mlp_step(const MlpStepShape &s, const __nv_bfloat16 *img, const float *params, const float *x,
                      const float *A, const float *b, const float *c, uint32_t B, float *part, float *g, float *loss,
                      int *err, cudaStream_t st) {
-  StepParams q{s, img, params, x, A, b, c, part, err, B, (B + kT - 1) / kT, nullptr, 0, nullptr};
+  StepParams q{s, img, params, x, A, b, c, part, err, B, (B + kT - 1) / kT, {}, nullptr};
   const unsigned grid = std::min(q.tiles, kStepSlots);
   const cudaError_t e = s.Wp == 128 ? launch<1, false>(q, grid, st) : launch<2, false>(q, grid, st);
   if (e != cudaSuccess) return e;

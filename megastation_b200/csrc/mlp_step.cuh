@@ -43,13 +43,20 @@ __device__ __forceinline__ int mlp_step_img(const MlpStepShape &s, uint64_t i) {
   return (int)(base + (r / 8 * blocks + c / 8) * 64 + r % 8 * 8 + c % 8);
 }
 
-// y [B][O] = the network's outputs.  stats null: x [B][I]; else the input of
-// sample s is the per-subcarrier blend's features: one-hot s % sg, then the six
-// statistics stats[s / sg][6] (I = sg + 6)
+// The per-subcarrier blend's features of sample s from the groups' centre Grams
+// gc [G][K][K]: one-hot s % sg, then for the neighbours j = -1, 1, 2 of group
+// g = s / sg the relative distance ||C_{g+j} - C_g|| / ||C_g|| and the trace
+// ratio minus 1 (0 past the band's edges).
+struct BlendFeatures {
+  const float2 *gc;
+  uint32_t sg, K, G;
+};
+// y [B][O] = the network's outputs for x [B][I], or (x null) for the features
+// f (I = f.sg + 6)
 cudaError_t mlp_fwd_tc(const MlpStepShape &s, const __nv_bfloat16 *img, const float *params, const float *x,
-                       const float *stats, uint32_t sg, uint32_t B, float *y, int *err, cudaStream_t st);
+                       const BlendFeatures &f, uint32_t B, float *y, int *err, cudaStream_t st);
 // the same through a network's handle; MB_UNSUPPORTED when its shape does not allow it
-mb_status mlp_forward_stats(mb_mlp *n, const float *stats, uint32_t sg, uint32_t B, float *y, cudaStream_t st);
+mb_status mlp_forward_features(mb_mlp *n, const BlendFeatures &f, uint32_t B, float *y, cudaStream_t st);
 
 // gradients of the batch-mean quadratic loss into g (flat) and, if not null,
 // the loss; part: kStepSlots or ceil(B / kStepTile) slots, whichever is fewer
