@@ -40,7 +40,7 @@
 namespace mb {
 
 namespace {
-constexpr int kStages = 3;
+constexpr int kStages = 3;  // at most; two k tiles (up to 64 antennas) take two stages
 constexpr int kKT = 64;     // reduction elements per k tile (4 MMAs of K=16)
 constexpr int kCols = 128;  // MMA M: (symbol, subcarrier) columns per CTA
 constexpr int kEqThreads = 256;  // 8 warps: warps w and w + 4 read TMEM lane quadrant w
@@ -88,8 +88,7 @@ __global__ void __launch_bounds__(kEqThreads, 1)
   if (warp == 0 && lane == 0) {
     // ---- producer: y columns by tensor boxes, detector image by bulk copy
     const uint8_t *a_g = q.a_img + (uint64_t)g * q.nkt * a_tile;
-    for (uint32_t kt = 0; kt < q.nkt; kt++) {
-      const uint32_t s = kt % kStages, use = kt / kStages;
+    for (uint32_t kt = 0, s = 0, use = 0; kt < q.nkt; kt++) {
       if (use >= 1 && !tc::mbar_wait(&empty_bar[s], (use - 1) & 1)) {
         timed_out = 1;
         break;
@@ -106,14 +105,14 @@ __global__ void __launch_bounds__(kEqThreads, 1)
         const int32_t row = (int32_t)(((l_off + l) * 2 + plane) * p.M + b0);
         tc::tma_load_2d(sy + j * bw * 128, &ymap, (int32_t)(s_base + sl), row, &full_bar[s]);
       }
+      if (++s == q.stages) s = 0, use++;
     }
   } else if (warp == 1 && lane == 0) {
     // ---- MMA issuer.  Columns ncols..127 of the y stage are never loaded:
     // their D rows are garbage and no thread stores them.
     const uint32_t idesc = tc::idesc_bf16(kCols, q.N, true, false);
     bool ok = true;
-    for (uint32_t kt = 0; kt < q.nkt; kt++) {
-      const uint32_t s = kt % kStages, use = kt / kStages;
+    for (uint32_t kt = 0, s = 0, use = 0; kt < q.nkt; kt++) {
       if (!tc::mbar_wait(&full_bar[s], use & 1)) {
         ok = false;
         break;
@@ -133,6 +132,7 @@ __global__ void __launch_bounds__(kEqThreads, 1)
         tc::mma_f16(tmem, yd, ad, idesc, (kt | ks) != 0);
       }
       tc::mma_commit(&empty_bar[s]);
+      if (++s == q.stages) s = 0, use++;
     }
     if (ok) tc::mma_commit(&done_bar);
     else timed_out = 1;
@@ -223,7 +223,11 @@ mb_status equalize_tc(const EqParams &p, const void *a_img, const void *y_lp, ui
   q.err = err;
   q.tmem_cols = 32;
   while (q.tmem_cols < q.N) q.tmem_cols *= 2;
-  const size_t smem = (size_t)kStages * ((size_t)kCols * kKT * 2 + (size_t)s.MM * kKT * 2);
+  // two k tiles need no third stage: 48 instead of 72 KB (MM = 64), four
+  // CTAs per SM instead of three (32 uneven cells, most of up to 64 antennas:
+  // 547 -> 533 us a slot of each)
+  q.stages = std::min<uint32_t>(kStages, s.nkt);
+  const size_t smem = (size_t)q.stages * ((size_t)kCols * kKT * 2 + (size_t)s.MM * kKT * 2);
   const uint32_t G = (p.S + p.sg - 1) / p.sg;
   int dev = 0;
   MB_CUDA_TRY(cudaGetDevice(&dev));
