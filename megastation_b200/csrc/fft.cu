@@ -253,21 +253,6 @@ __device__ __forceinline__ void epilogue(const FftParams &p, const RowCtx &c, ui
       reinterpret_cast<__nv_bfloat16 *>(c.o0)[i] = __float2bfloat16_rn(v.x);
       reinterpret_cast<__nv_bfloat16 *>(c.o1)[i] = __float2bfloat16_rn(v.y);
     }
-  } else if constexpr (MODE == kPilot) {
-    const uint32_t i = (k - p.start - N / 2) & (N - 1);
-    if (i < p.S) {
-      const uint32_t g = p.sg_inv ? __umulhi(i, p.sg_inv) : i;
-      const uint32_t u = c.u0 + (i - g * p.sg);
-      if (u < p.K) {
-        const float2 ps = __ldg(p.pilot + i);
-        const float2 e = make_float2(v.x * ps.x + v.y * ps.y, v.x * ps.y - v.y * ps.x);
-        reinterpret_cast<float2 *>(p.out)[((uint64_t)g * p.M + c.b) * p.K + u] = e;
-        // a user with no pilot in the short last group takes its estimate
-        // from group G-2 (the slot's tail rule)
-        if (p.tail_rem && g + 2 == (p.S + p.sg - 1) / p.sg && i - g * p.sg >= p.tail_rem)
-          reinterpret_cast<float2 *>(p.out)[((uint64_t)(g + 1) * p.M + c.b) * p.K + u] = e;
-      }
-    }
   } else {
     if (p.out_dtype == MB_IQ_I16 || p.out_dtype == MB_IQ_I8) {
       const bool i16 = p.out_dtype == MB_IQ_I16;
@@ -288,6 +273,36 @@ __device__ __forceinline__ void epilogue(const FftParams &p, const RowCtx &c, ui
       const float sc = 1.f / (float)N;
       reinterpret_cast<float2 *>(c.o0)[k] = make_float2(v.x * sc, v.y * sc);
     }
+  }
+}
+
+// Pilot rows: the LS estimates of bins k[0..3].  The four pilot values are
+// loaded together, before any bin's bounds are looked at: behind the branches
+// each load waited for the previous bin's store (rows of 2048: 32 rows 6.8 ->
+// 5.4 us, 1664 rows 17.5 -> 14.7 us).
+template <int N>
+__device__ __forceinline__ void pilot_store4(const FftParams &p, const RowCtx &c, const uint32_t (&k)[4],
+                                             const float2 *v) {
+  uint32_t i[4];
+  float2 ps[4];
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    i[q] = (k[q] - p.start - N / 2) & (N - 1);
+    ps[q] = __ldg(p.pilot + min(i[q], p.S - 1));
+  }
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    if (i[q] >= p.S) continue;
+    const uint32_t g = p.sg_inv ? __umulhi(i[q], p.sg_inv) : i[q];
+    const uint32_t u = c.u0 + (i[q] - g * p.sg);
+    if (u >= p.K) continue;
+    const float2 x = v[q];
+    const float2 e = make_float2(x.x * ps[q].x + x.y * ps[q].y, x.x * ps[q].y - x.y * ps[q].x);
+    reinterpret_cast<float2 *>(p.out)[((uint64_t)g * p.M + c.b) * p.K + u] = e;
+    // a user with no pilot in the short last group takes its estimate
+    // from group G-2 (the slot's tail rule)
+    if (p.tail_rem && g + 2 == (p.S + p.sg - 1) / p.sg && i[q] - g * p.sg >= p.tail_rem)
+      reinterpret_cast<float2 *>(p.out)[((uint64_t)(g + 1) * p.M + c.b) * p.K + u] = e;
   }
 }
 
@@ -395,11 +410,17 @@ __global__ void __launch_bounds__(Plan<LOGN>::THREADS, Plan<LOGN>::MIN_BLOCKS)
       __syncthreads();
     } else if (active) {
       const RowCtx ctx = row_ctx<MODE, N>(p, row);
+      // last pass: Ns = N / R, so element bi is bin j + r Ns, j = t + (bi / R) T
+      auto bin = [&](int bi) { return (uint32_t)(t + (bi / R) * T + bi % R * Ns); };
+      if constexpr (MODE == kPilot) {
 #pragma unroll
-      for (int bi = 0; bi < 16; bi++) {
-        const int j = t + (bi / R) * T, r = bi % R;
-        // last pass: Ns = N / R, so idxD = j
-        epilogue<MODE, N>(p, ctx, (uint32_t)(j + r * Ns), v[bi]);
+        for (int bi = 0; bi < 16; bi += 4) {
+          const uint32_t k[4] = {bin(bi), bin(bi + 1), bin(bi + 2), bin(bi + 3)};
+          pilot_store4<N>(p, ctx, k, v + bi);
+        }
+      } else {
+#pragma unroll
+        for (int bi = 0; bi < 16; bi++) epilogue<MODE, N>(p, ctx, bin(bi), v[bi]);
       }
     }
     Ns *= R;
