@@ -18,17 +18,24 @@
 // component lies in [128, 256): then |Y| and |Z| stay below 2^15.5, inside
 // the FP16 range, and the scale is undone exactly before the BF16 store.
 //
-// One CTA per SM takes every gridDim-th unit of two rows, with 224 KB of
-// shared memory (F, one GEMM operand buffer, an output staging buffer and a
-// two-unit input ring) and 256 TMEM columns (the two GEMM accumulators).
-// Warp 8 is the control warp: one thread streams the units' rows into the
+// One CTA per SM takes every gridDim-th unit of two rows.  Samples of up to 4
+// bytes run through two pipelines of eight compute warps, complex floats
+// through one of sixteen.  A pipeline has a GEMM operand buffer, an output
+// staging buffer, an input ring and 256 TMEM columns (the two GEMM
+// accumulators); F is shared.  Its copy warp streams the units' rows into the
 // ring with 128-byte-swizzled TMA boxes (so the conversion reads are free of
-// bank conflicts), issues both GEMMs and writes the staged output rows back
-// with bulk copies.  Warps 0-7 convert the samples into the GEMM-1 operand,
-// twiddle the GEMM-1 result into the GEMM-2 operand (in the same buffer,
-// which GEMM 1 no longer needs) and stage the GEMM-2 result as BF16 rows.
-// Mbarriers hand each buffer between the roles, so a unit's loads, GEMMs,
-// conversion and stores overlap those of its neighbours.
+// bank conflicts) and writes the staged output rows back with bulk copies; its
+// GEMM warp issues both GEMMs.  The compute warps convert the samples into the
+// GEMM-1 operand, twiddle the GEMM-1 result into the GEMM-2 operand (in the
+// same buffer, which GEMM 1 no longer needs) and stage the GEMM-2 result as
+// BF16 rows.  Mbarriers hand each buffer between the roles, so a unit's loads,
+// GEMMs, conversion and stores overlap those of its neighbours.
+//
+// Bound by the chain of these phases, not by memory (3584 rows of int8: 29.4
+// us against 13 us for their bytes).  Two pipelines against one of sixteen
+// warps, 3584 rows: int8 30.9 -> 29.4 us, int16 37.7 -> 33.9, FP16 41.7 ->
+// 36.3, and complex floats, whose single pipeline loops over the same shorter
+// code, 45.0 -> 41.7.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -53,14 +60,12 @@ namespace {
 
 constexpr double kPi = 3.14159265358979323846;
 constexpr int kFtCompute = 512;                  // warps 0-15
-constexpr int kFtThreads = kFtCompute + 64;      // + the GEMM and copy warps
 constexpr uint32_t kFtN = 4096;
 constexpr uint32_t kMat = 32768;                 // one 128 x 128 FP16 operand
-constexpr uint32_t kStage = 65536;               // raw samples of one unit (c64)
 // staged output rows (r, plane) at (2 r + plane) * kStgPitch: 8192 B plus 64,
 // so the two planes of a row start on opposite halves of the 32 banks
 constexpr uint32_t kStgPitch = 8192 + 64;
-constexpr uint32_t kFtSmem = 2 * kMat + 2 * kStage + 4 * kStgPitch;  // F, AZ, ring, staging
+constexpr uint32_t kStgBytes = 4 * kStgPitch;
 
 // byte offset of element (row, kk) of a 128 x 128 K-major operand: 8-row
 // groups 2048 B apart, K core matrices (8 elements, 16 B) 128 B apart
@@ -107,6 +112,18 @@ struct Fmt {
   static constexpr uint32_t kBoxes = kBytes / 2;      // 128-byte boxes per 64-sample n1 row
   static constexpr uint32_t kPPC = kBytes / 2;        // 16-byte pieces per 8-sample chunk
   static constexpr uint32_t kUnitBytes = 2 * kFtN * kBytes;
+  // Independent pipelines per CTA.  One pipeline's 16 warps pass through the
+  // phases of a unit together and wait together for each GEMM and copy (issue
+  // slots half idle); two of eight warps each fill one another's waits.  The
+  // operand, ring and staging buffers of two fit beside F for samples of up
+  // to 4 bytes; complex floats, whose units take 64 KB and whose launch is
+  // near the copy rate as it is, keep one.
+  static constexpr uint32_t kNG = DT == MB_IQ_C32 ? 1 : 2;
+  static constexpr uint32_t kRing = DT == MB_IQ_C32 ? 131072 : 32768;  // a pipeline's ring
+  static constexpr uint32_t kSlots = kRing / kUnitBytes;               // units in it: two, or one of 4-byte samples
+  static constexpr uint32_t kGT = kFtCompute / kNG;                    // a pipeline's compute threads
+  static constexpr uint32_t kThreads = kFtCompute + 64 * kNG;          // + its GEMM and copy warps
+  static constexpr uint32_t kSmem = kMat + kNG * (kMat + kRing + kStgBytes);  // F, then operands, rings, staging
 };
 
 // integer samples have a known range: a fixed scale instead of the row maximum
@@ -178,8 +195,10 @@ __device__ __forceinline__ void row_scale(uint32_t mbits, float &scale, float &i
 __device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc::smem_u32(bar)) : "memory");
 }
-// named barrier among the compute warps
-__device__ __forceinline__ void compute_sync() { asm volatile("bar.sync 1, 512;" ::: "memory"); }
+// named barrier among a pipeline's n compute threads
+__device__ __forceinline__ void compute_sync(uint32_t grp, uint32_t n) {
+  asm volatile("bar.sync %0, %1;" ::"r"(grp + 1), "r"(n) : "memory");
+}
 
 // shared -> global bulk copy (16-byte aligned, size a multiple of 16)
 __device__ __forceinline__ void bulk_s2g(void *dst, const void *src, uint32_t bytes) {
@@ -208,65 +227,73 @@ __device__ __forceinline__ bool ft_wait(uint64_t *bar, uint32_t parity, volatile
 }
 
 template <int DT>
-__global__ void __launch_bounds__(kFtThreads, 1)
+__global__ void __launch_bounds__(Fmt<DT>::kThreads, 1)
     fft_tc_kernel(const __grid_constant__ CUtensorMap in_map, const FtParams p) {
   extern __shared__ __align__(1024) uint8_t ft_smem[];
-  // F, AZ and the ring start on 1024-byte boundaries (the swizzled TMA boxes
-  // need them); the staging rows follow
-  uint8_t *sF = ft_smem, *sAZ = ft_smem + kMat, *sRing = ft_smem + 2 * kMat;
-  uint8_t *sStg = sRing + 2 * kStage;
-  // GEMM operand buffers: integer samples fill at most half of a ring slot,
-  // so a second buffer (unit i uses buffer i & 1) sits behind ring slot 0's
-  // samples and the conversion of unit i + 1 need not wait for GEMM 2 of
-  // unit i to read the first; other sample types keep the one buffer.
-  // d2_full[u & 1] completes when GEMM 2 of unit u has finished.
-  constexpr bool kAZ2 = Fmt<DT>::kUnitBytes + kMat <= kStage;
-  uint8_t *const sAZ1 = kAZ2 ? sRing + Fmt<DT>::kUnitBytes : sAZ;
-  // Each barrier completes once per unit.  a_ready comes as a pair per ring
-  // slot, waited with parity (i >> 1) & 1: the copy warp may trail the
-  // compute warps by two units (while it drains a bulk store), and a plain
-  // parity wait would then alias a later phase.  full is per slot anyway;
-  // every other barrier's waiters are at most one phase behind.
-  __shared__ uint64_t bar_mats, full[2], a_ready[2], z_ready, st_ready, d1_full, d2_full[2], st_done;
-  __shared__ uint32_t tmem_slot;
-  __shared__ __align__(16) uint32_t s_rmax[16];
-  __shared__ volatile int s_fail;
   using F = Fmt<DT>;
+  constexpr uint32_t NG = F::kNG;
+  // Each barrier completes once per unit of its pipeline.  a_ready comes as a
+  // pair, waited with parity (i >> 1) & 1: the copy warp may trail the
+  // compute warps by two units (while it drains a bulk store), and a plain
+  // parity wait would then alias a later phase.  full is per ring slot;
+  // d2_full[u & 1] completes when GEMM 2 of unit u has finished; every other
+  // barrier's waiters are at most one phase behind.
+  struct Bars {
+    uint64_t full[2], a_ready[2], z_ready, st_ready, d1_full, d2_full[2], st_done;
+  };
+  __shared__ Bars bars[NG];
+  __shared__ uint64_t bar_mats;
+  __shared__ uint32_t tmem_slot;
+  __shared__ __align__(16) uint32_t s_rmax[NG][16];
+  __shared__ float s_inv[NG][2][2];  // [unit parity][row] inverse row scales
+  __shared__ volatile int s_fail;
 
   const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
+  // this thread's pipeline: compute warps in NG runs, then the GEMM warps, then the copy warps
+  constexpr uint32_t kGW = F::kGT / 32;
+  const uint32_t grp = warp < kFtCompute / 32 ? warp / kGW : (warp - kFtCompute / 32) % NG;
+  Bars &B = bars[grp];
+  // F, AZ and the rings start on 1024-byte boundaries (the swizzled TMA boxes
+  // need them); the staging rows follow
+  uint8_t *const sF = ft_smem, *const sAZ = ft_smem + kMat * (1 + grp),
+                *const sRing = ft_smem + kMat * (1 + NG) + grp * F::kRing,
+                *const sStg = ft_smem + kMat * (1 + NG) + NG * F::kRing + grp * kStgBytes;
   // this CTA's units: blockIdx.x, blockIdx.x + gridDim.x, ... (strided, so
   // the pilot rows at the front spread over all CTAs), taken in an order
   // rotated by the CTA index, so that the CTAs reach their pilot units (CSI
-  // stores, pilot loads) at different times rather than all at the start
+  // stores, pilot loads) at different times rather than all at the start;
+  // the pipelines take them in turn
   if (blockIdx.x >= p.units) return;
-  const uint32_t n_units = (p.units - blockIdx.x + gridDim.x - 1) / gridDim.x;
-  const uint32_t rot = blockIdx.x % n_units;
+  const uint32_t cta_units = (p.units - blockIdx.x + gridDim.x - 1) / gridDim.x;
+  const uint32_t rot = blockIdx.x % cta_units;
+  const uint32_t n_units = cta_units > grp ? (cta_units - grp + NG - 1) / NG : 0;
   auto unit_of = [&](uint32_t i) {
-    const uint32_t k = i + rot < n_units ? i + rot : i + rot - n_units;
+    const uint32_t j = i * NG + grp + rot, k = j < cta_units ? j : j - cta_units;
     return blockIdx.x + k * gridDim.x;
   };
 
   if (tid == kFtCompute) {
     tc::mbar_init(&bar_mats, 1);
-    tc::mbar_init(&full[0], 1);
-    tc::mbar_init(&full[1], 1);
-    tc::mbar_init(&a_ready[0], kFtCompute / 32);
-    tc::mbar_init(&a_ready[1], kFtCompute / 32);
-    tc::mbar_init(&z_ready, kFtCompute / 32);
-    tc::mbar_init(&st_ready, kFtCompute / 32);
-    tc::mbar_init(&d1_full, 1);
-    tc::mbar_init(&d2_full[0], 1);
-    tc::mbar_init(&d2_full[1], 1);
-    tc::mbar_init(&st_done, 1);
+    for (uint32_t g = 0; g < NG; g++) {
+      for (int k = 0; k < 2; k++) {
+        tc::mbar_init(&bars[g].full[k], 1);
+        tc::mbar_init(&bars[g].a_ready[k], kGW);
+        tc::mbar_init(&bars[g].d2_full[k], 1);
+      }
+      tc::mbar_init(&bars[g].z_ready, kGW);
+      tc::mbar_init(&bars[g].st_ready, kGW);
+      tc::mbar_init(&bars[g].d1_full, 1);
+      tc::mbar_init(&bars[g].st_done, 1);
+    }
     s_fail = 0;
     tc::fence_mbar_init();
     tc::prefetch_tmap(&in_map);
   }
-  if (warp == 0) tc::tmem_alloc(&tmem_slot, 256);
+  if (warp == 0) tc::tmem_alloc(&tmem_slot, 256 * NG);
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
-  const uint32_t tmem = tmem_slot;  // D1: columns 0..127, D2: 128..255
+  const uint32_t tmem = tmem_slot + 256 * grp;  // D1: columns 0..127, D2: 128..255
 
   // planar BF16 output row of uplink row lrow (rows counted after the
   // pilot rows), plane pl
@@ -276,7 +303,9 @@ __global__ void __launch_bounds__(kFtThreads, 1)
   };
   const uint32_t S8 = (p.S + 7) & ~7u;  // columns written by the bulk copies (<= S_pad)
 
-  if (warp == kFtCompute / 32) {
+  if (n_units == 0) {
+    // a pipeline without units
+  } else if (warp >= kFtCompute / 32 && warp < kFtCompute / 32 + (int)NG) {
     // ================================================== GEMM warp
     if (lane == 0) {
       const uint32_t fa = tc::smem_u32(sF);
@@ -284,8 +313,7 @@ __global__ void __launch_bounds__(kFtThreads, 1)
       // both GEMMs read the unit's operand buffer (MN-major) and F (K-major);
       // k step ks of the operand is 4096 bytes on, i.e. 256 in the
       // descriptor's address field (no carry: addresses stay below 256 KB)
-      const uint64_t da_0 = tc::smem_desc(tc::smem_u32(sAZ), 2048, 128);
-      const uint64_t da_1 = tc::smem_desc(tc::smem_u32(sAZ1), 2048, 128);
+      const uint64_t da = tc::smem_desc(tc::smem_u32(sAZ), 2048, 128);
       uint64_t db[8];
 #pragma unroll
       for (int ks = 0; ks < 8; ks++) db[ks] = tc::smem_desc(fa + ks * 256, 128, 2048);
@@ -293,44 +321,43 @@ __global__ void __launch_bounds__(kFtThreads, 1)
       bool ok = ft_wait(&bar_mats, 0, &s_fail);
       for (uint32_t i = 0; i < n_units && ok; i++) {
         // GEMM 1: D1 (128 (r, n2) x 128 (p', k1)) = A (samples) x F
-        if (!ft_wait(&a_ready[i & 1], (i >> 1) & 1, &s_fail)) break;
+        if (!ft_wait(&B.a_ready[i & 1], (i >> 1) & 1, &s_fail)) break;
         tc::fence_after_sync();
-        const uint64_t da = (i & 1) ? da_1 : da_0;
 #pragma unroll
         for (int ks = 0; ks < 8; ks++) tc::mma_f16(tmem, da + (uint64_t)(ks * 256), db[ks], idesc, ks > 0);
-        tc::mma_commit(&d1_full);
+        tc::mma_commit(&B.d1_full);
         n_d1++;
         // GEMM 2: D2 (128 (r, k1) x 128 (p', k2)) = Z x F
-        if (!ft_wait(&z_ready, i & 1, &s_fail)) break;
+        if (!ft_wait(&B.z_ready, i & 1, &s_fail)) break;
         tc::fence_after_sync();
 #pragma unroll
         for (int ks = 0; ks < 8; ks++) tc::mma_f16(tmem + 128, da + (uint64_t)(ks * 256), db[ks], idesc, ks > 0);
-        tc::mma_commit(&d2_full[i & 1]);
+        tc::mma_commit(&B.d2_full[i & 1]);
         n_d2++;
       }
       if (s_fail) {
         // a wait ran out: let the issued GEMMs drain (bounded)
-        if (n_d1) tc::mbar_wait(&d1_full, (n_d1 - 1) & 1, 100000000ull);
+        if (n_d1) tc::mbar_wait(&B.d1_full, (n_d1 - 1) & 1, 100000000ull);
         for (uint32_t u = n_d2 >= 2 ? n_d2 - 2 : 0; u < n_d2; u++)
-          tc::mbar_wait(&d2_full[u & 1], (u >> 1) & 1, 100000000ull);
+          tc::mbar_wait(&B.d2_full[u & 1], (u >> 1) & 1, 100000000ull);
       }
     }
-  } else if (warp == kFtCompute / 32 + 1) {
+  } else if (warp >= kFtCompute / 32 + (int)NG) {
     // ================================================== copy warp
     if (lane == 0) {
       uint32_t loads[2] = {0, 0};
       auto issue_load = [&](uint32_t i) {
         if (i >= n_units) return;
-        const uint32_t u = unit_of(i);
-        loads[i & 1]++;
-        uint8_t *slot = sRing + (i & 1) * kStage;
-        tc::mbar_arrive_expect_tx(&full[i & 1], F::kUnitBytes);
+        const uint32_t u = unit_of(i), sl = i % F::kSlots;
+        loads[sl]++;
+        uint8_t *slot = sRing + sl * F::kUnitBytes;
+        tc::mbar_arrive_expect_tx(&B.full[sl], F::kUnitBytes);
 #pragma unroll
         for (uint32_t r = 0; r < 2; r++)
 #pragma unroll
           for (uint32_t bx = 0; bx < F::kBoxes; bx++)
             tc::tma_load_2d(slot + (r * F::kBoxes + bx) * 8192, &in_map, (int32_t)(bx * 128),
-                            (int32_t)((2 * u + r) * 64), &full[i & 1]);
+                            (int32_t)((2 * u + r) * 64), &B.full[sl]);
       };
       // staged rows hold all 4096 bins in subcarrier order; the first
       // S rounded up to 8 go out by bulk copy (within the row pitch)
@@ -357,29 +384,30 @@ __global__ void __launch_bounds__(kFtThreads, 1)
         }
         bulk_commit();
       };
-      tc::mbar_arrive_expect_tx(&bar_mats, kMat);
-      tc::bulk_g2s(sF, p.mats, kMat, &bar_mats);
-      issue_load(0);
-      issue_load(1);
+      if (grp == 0) {  // (a CTA's first pipeline always has a unit)
+        tc::mbar_arrive_expect_tx(&bar_mats, kMat);
+        tc::bulk_g2s(sF, p.mats, kMat, &bar_mats);
+      }
+      for (uint32_t i = 0; i < F::kSlots; i++) issue_load(i);
       for (uint32_t i = 0; i < n_units; i++) {
-        // the ring slot of unit i takes unit i + 2 once unit i is converted
-        if (!ft_wait(&a_ready[i & 1], (i >> 1) & 1, &s_fail)) break;
-        issue_load(i + 2);
+        // the ring slot of unit i takes unit i + kSlots once unit i is converted
+        if (!ft_wait(&B.a_ready[i & 1], (i >> 1) & 1, &s_fail)) break;
+        issue_load(i + F::kSlots);
         if (i > 0) {
-          if (!ft_wait(&st_ready, (i - 1) & 1, &s_fail)) break;
+          if (!ft_wait(&B.st_ready, (i - 1) & 1, &s_fail)) break;
           issue_stores(i - 1);
           bulk_wait_read();
-          mbar_arrive(&st_done);
+          mbar_arrive(&B.st_done);
         }
       }
-      if (!s_fail && ft_wait(&st_ready, (n_units - 1) & 1, &s_fail)) issue_stores(n_units - 1);
+      if (!s_fail && ft_wait(&B.st_ready, (n_units - 1) & 1, &s_fail)) issue_stores(n_units - 1);
       bulk_wait_all();
       if (s_fail) {
         // a wait ran out: record it and let the loads in flight land (bounded)
         if (p.err) atomicOr(p.err, tc::kErrTimeout);
         for (int sl = 0; sl < 2; sl++)
-          if (loads[sl]) tc::mbar_wait(&full[sl], (loads[sl] - 1) & 1, 100000000ull);
-        tc::mbar_wait(&bar_mats, 0, 100000000ull);
+          if (loads[sl]) tc::mbar_wait(&B.full[sl], (loads[sl] - 1) & 1, 100000000ull);
+        if (grp == 0) tc::mbar_wait(&bar_mats, 0, 100000000ull);
       }
     }
   } else {
@@ -389,18 +417,18 @@ __global__ void __launch_bounds__(kFtThreads, 1)
       if (ok) ok = ft_wait(bar, parity, &s_fail);
       ok = __all_sync(0xffffffffu, ok);
     };
-    auto wait_d2 = [&](uint32_t u) { wait_ok(&d2_full[u & 1], (u >> 1) & 1); };
+    auto wait_d2 = [&](uint32_t u) { wait_ok(&B.d2_full[u & 1], (u >> 1) & 1); };
     auto arrive = [&](uint64_t *bar) {
       tc::fence_proxy_async_smem();
       tc::fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(bar);
     };
-    // Conversion: thread -> row rh of the unit, 2 chunks of 8 samples (n1,
-    // n2 .. n2 + 7); a warp covers 8 consecutive n1 x 4 chunks, so its
-    // 16-byte operand stores fill whole core matrices.  Offsets are the same
-    // for every unit.
-    const uint32_t rh = tid >> 8, wq = (tid >> 5) & 7;
+    // Conversion: thread -> row rh of the unit (both rows in turn where eight
+    // warps make a pipeline), 2 chunks of 8 samples (n1, n2 .. n2 + 7) of a
+    // row; a warp covers 8 consecutive n1 x 4 chunks, so its 16-byte operand
+    // stores fill whole core matrices.  Offsets are the same for every unit.
+    const uint32_t gwarp = warp - grp * kGW, rh = gwarp >> 3, wq = gwarp & 7;
     uint32_t r_off[2][F::kPPC], a_off[2];
 #pragma unroll
     for (int c2 = 0; c2 < 2; c2++) {
@@ -409,8 +437,9 @@ __global__ void __launch_bounds__(kFtThreads, 1)
       for (int w = 0; w < (int)F::kPPC; w++) r_off[c2][w] = ring_off<DT>(rh, n1, 8 * n2b + w * (16 / F::kBytes));
       a_off[c2] = mnmaj_off(64 * rh + 8 * n2b, n1);  // imaginary parts 8 K groups (16 KB) further
     }
-    // GEMM-1 epilogue: TMEM lane (r, n2), k1 in [16 part, 16 part + 16)
-    const uint32_t quad = warp & 3, part = warp >> 2;
+    // GEMM-1 epilogue: TMEM lane (r, n2), k1 in [16 part, 16 part + 16) for
+    // this warp's NG successive parts
+    const uint32_t quad = warp & 3, part0 = (gwarp >> 2) * NG;
     const uint32_t lane_row = quad * 32 + lane;
     const uint32_t tl = tmem + ((quad * 32) << 16);
     const uint32_t e_n2 = lane_row & 63, e_r = lane_row >> 6;
@@ -418,35 +447,40 @@ __global__ void __launch_bounds__(kFtThreads, 1)
     // the twiddle phase (15 FP32 complex products: about 2e-6 relative, far
     // below the FP16 rounding of the result); holding all 16 twiddles for the
     // whole kernel cost 32 registers and made the threads spill
-    float2 tw0 = __ldg(p.tw + ((e_n2 * 16 * part) & (kFtN - 1)));
-    if constexpr (kFixedScale<DT>) {
-      // integer samples: the FFT of q * 2^-8 (int16) or of q (int8) is the
-      // FFT of the normalised samples q / 2^15 or q / 2^7 times 2^7; the
-      // exact 1/128 rides in the twiddles (GEMM 2 is linear), so the
-      // epilogues need no multiply
-      tw0.x *= 1.0f / 128.0f;
-      tw0.y *= 1.0f / 128.0f;
+    float2 tw0[NG];
+#pragma unroll
+    for (uint32_t h = 0; h < NG; h++) {
+      tw0[h] = __ldg(p.tw + ((e_n2 * 16 * (part0 + h)) & (kFtN - 1)));
+      if constexpr (kFixedScale<DT>) {
+        // integer samples: the FFT of q * 2^-8 (int16) or of q (int8) is the
+        // FFT of the normalised samples q / 2^15 or q / 2^7 times 2^7; the
+        // exact 1/128 rides in the twiddles (GEMM 2 is linear), so the
+        // epilogues need no multiply
+        tw0[h].x *= 1.0f / 128.0f;
+        tw0[h].y *= 1.0f / 128.0f;
+      }
     }
     const float2 tws = __ldg(p.tw + e_n2);
-    const uint32_t z_off = mnmaj_off(64 * e_r + 16 * part, e_n2);
+    const uint32_t z_off = mnmaj_off(64 * e_r + 16 * part0, e_n2);
     // GEMM-2 epilogue: TMEM lane (r, k1), k2 in [16 part, 16 part + 16); bin
     // k1 + 64 k2 is subcarrier (k1 + 64 k2 - c) mod N.  With c even the even
     // lane's subcarrier is even: lane pairs swap one packed BF16 pair, then
     // the even lane writes the real pair (sc, sc + 1) and the odd lane the
     // imaginary pair (sc - 1, sc), two 64-byte runs in disjoint banks.
     const uint32_t s_r = lane_row >> 6, s_k1 = lane_row & 63;
-    const uint32_t s_base = (s_k1 + kFtN - p.c + 1024 * part) & (kFtN - 1);
+    const uint32_t s_base0 = s_k1 + kFtN - p.c + 1024 * part0;
     const bool odd = lane & 1, pairs = (p.c & 1) == 0;
     const uint32_t perm = odd ? 0x3276u : 0x5410u;
     uint8_t *stg_mine = sStg + (2 * s_r + (odd ? 1 : 0)) * kStgPitch;
     __nv_bfloat16 *stg_re = reinterpret_cast<__nv_bfloat16 *>(sStg + 2 * s_r * kStgPitch);
     __nv_bfloat16 *stg_im = reinterpret_cast<__nv_bfloat16 *>(sStg + (2 * s_r + 1) * kStgPitch);
-    __shared__ float s_inv[2][2];  // [unit parity][row] inverse row scales
 
-    auto store_unit = [&](uint32_t i) {
+    // part `part` of unit i
+    auto store_part = [&](uint32_t i, uint32_t part) {
+      const uint32_t s_base = (s_base0 + 1024 * (part - part0)) & (kFtN - 1);
       // row scale to undo (integer samples: none, the 1/128 is already in
       // the twiddles)
-      const float inv = kFixedScale<DT> ? 1.0f : s_inv[i & 1][s_r];
+      const float inv = kFixedScale<DT> ? 1.0f : s_inv[grp][i & 1][s_r];
       const uint32_t row = 2 * unit_of(i) + s_r;  // the same for the whole warp
       if (!kFixedScale<DT> && p.inverse) {
         // time sample n = k1 + 64 k2 of row s_r: conj of the forward bin,
@@ -477,7 +511,6 @@ __global__ void __launch_bounds__(kFtThreads, 1)
             }
           }
         }
-        arrive(&st_ready);
         return;
       }
       if (row < p.pilot_rows) {
@@ -508,7 +541,6 @@ __global__ void __launch_bounds__(kFtThreads, 1)
             }
           }
         }
-        arrive(&st_ready);
         return;
       }
       if (pairs) {
@@ -535,20 +567,57 @@ __global__ void __launch_bounds__(kFtThreads, 1)
           stg_im[sc] = __float2bfloat16_rn(vi[j] * inv);
         }
       }
-      arrive(&st_ready);
+    };
+    auto store_unit = [&](uint32_t i) {
+#pragma unroll 1
+      for (uint32_t h = 0; h < NG; h++) store_part(i, part0 + h);
+      arrive(&B.st_ready);
     };
 
     for (uint32_t i = 0; i < n_units; i++) {
-      const uint8_t *slot = sRing + (i & 1) * kStage;
+      const uint8_t *slot = sRing + (i % F::kSlots) * F::kUnitBytes;
       // (a) conversion: row maximum, power-of-two scale, FP16 operand A
-      wait_ok(&full[i & 1], (i >> 1) & 1);
-      uint4 re[2], im[2];
-      {
-        uint4 raw[2][F::kPPC];
+      wait_ok(&B.full[i % F::kSlots], (i / F::kSlots) & 1);
+      uint4 raw[2][F::kPPC];
+      auto load_raw = [&](uint32_t h) {
 #pragma unroll
         for (int c2 = 0; c2 < 2; c2++)
 #pragma unroll
-          for (int w = 0; w < (int)F::kPPC; w++) raw[c2][w] = *reinterpret_cast<const uint4 *>(slot + r_off[c2][w]);
+          for (int w = 0; w < (int)F::kPPC; w++)
+            raw[c2][w] = *reinterpret_cast<const uint4 *>(slot + h * F::kBoxes * 8192 + r_off[c2][w]);
+      };
+      float scale[NG];
+      if constexpr (!kFixedScale<DT>) {
+#pragma unroll
+        for (uint32_t h = 0; h < NG; h++) {
+          load_raw(h);
+          float m = 0.f;
+#pragma unroll
+          for (int c2 = 0; c2 < 2; c2++)
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+              const float2 v = chunk_sample<DT>(raw[c2], j);
+              m = fmaxf(m, fmaxf(fabsf(v.x), fabsf(v.y)));
+            }
+          const uint32_t mb = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
+          if (lane == 0) s_rmax[grp][(rh + h) * 8 + wq] = mb;
+        }
+        compute_sync(grp, F::kGT);
+#pragma unroll
+        for (uint32_t h = 0; h < NG; h++) {
+          const uint4 m0 = *reinterpret_cast<const uint4 *>(&s_rmax[grp][(rh + h) * 8]);
+          const uint4 m1 = *reinterpret_cast<const uint4 *>(&s_rmax[grp][(rh + h) * 8 + 4]);
+          const uint32_t rmax = max(max(max(m0.x, m0.y), max(m0.z, m0.w)), max(max(m1.x, m1.y), max(m1.z, m1.w)));
+          float inv;
+          row_scale(rmax, scale[h], inv);
+          if (wq == 0 && lane == 0) s_inv[grp][i & 1][rh + h] = inv;
+        }
+      }
+#pragma unroll 1
+      for (uint32_t h = 0; h < NG; h++) {
+        if (kFixedScale<DT> || NG > 1) load_raw(h);  // (one row per thread: still held)
+        const float sc = NG > 1 && h ? scale[NG - 1] : scale[0];
+        uint4 re[2], im[2];
         if constexpr (kFixedScale<DT>) {
           // integer samples: |q| <= 2^15 (int16) or 2^7 (int8) converts to
           // FP16 and a fixed power of two takes it below 2^7 (exact), so no
@@ -591,94 +660,80 @@ __global__ void __launch_bounds__(kFtThreads, 1)
             im[c2] = make_uint4(iw[0], iw[1], iw[2], iw[3]);
           }
         } else {
-          float m = 0.f;
-#pragma unroll
-          for (int c2 = 0; c2 < 2; c2++)
-#pragma unroll
-            for (int j = 0; j < 8; j++) {
-              const float2 v = chunk_sample<DT>(raw[c2], j);
-              m = fmaxf(m, fmaxf(fabsf(v.x), fabsf(v.y)));
-            }
-          const uint32_t mb = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
-          if (lane == 0) s_rmax[warp] = mb;
-          compute_sync();
-          const uint4 m0 = *reinterpret_cast<const uint4 *>(&s_rmax[rh * 8]);
-          const uint4 m1 = *reinterpret_cast<const uint4 *>(&s_rmax[rh * 8 + 4]);
-          const uint32_t rmax = max(max(max(m0.x, m0.y), max(m0.z, m0.w)), max(max(m1.x, m1.y), max(m1.z, m1.w)));
-          float scale, inv;
-          row_scale(rmax, scale, inv);
-          if ((tid & 255) == 0) s_inv[i & 1][rh] = inv;
-          const float iscale = p.inverse ? -scale : scale;  // conj(z) for the inverse
+          const float iscale = p.inverse ? -sc : sc;  // conj(z) for the inverse
 #pragma unroll
           for (int c2 = 0; c2 < 2; c2++) {
             float2 v[8];
 #pragma unroll
             for (int j = 0; j < 8; j++) v[j] = chunk_sample<DT>(raw[c2], j);
-            re[c2] = make_uint4(h2_bits(v[0].x * scale, v[1].x * scale), h2_bits(v[2].x * scale, v[3].x * scale),
-                                h2_bits(v[4].x * scale, v[5].x * scale), h2_bits(v[6].x * scale, v[7].x * scale));
+            re[c2] = make_uint4(h2_bits(v[0].x * sc, v[1].x * sc), h2_bits(v[2].x * sc, v[3].x * sc),
+                                h2_bits(v[4].x * sc, v[5].x * sc), h2_bits(v[6].x * sc, v[7].x * sc));
             im[c2] = make_uint4(h2_bits(v[0].y * iscale, v[1].y * iscale), h2_bits(v[2].y * iscale, v[3].y * iscale),
                                 h2_bits(v[4].y * iscale, v[5].y * iscale), h2_bits(v[6].y * iscale, v[7].y * iscale));
           }
         }
-      }
-      // the operand buffer holds Z of its previous unit (i - 2 with two
-      // buffers, i - 1 with one) until that unit's GEMM 2 has read it
-      uint8_t *az = (i & 1) ? sAZ1 : sAZ;
-      if (kAZ2 ? i > 1 : i > 0) wait_d2(kAZ2 ? i - 2 : i - 1);
-      tc::fence_after_sync();
-      if (ok) {
+        // the operand buffer holds Z of the previous unit until GEMM 2 has read it
+        if (h == 0) {
+          if (i > 0) wait_d2(i - 1);
+          tc::fence_after_sync();
+        }
+        if (ok) {
 #pragma unroll
-        for (int c2 = 0; c2 < 2; c2++) {
-          *reinterpret_cast<uint4 *>(az + a_off[c2]) = re[c2];
-          *reinterpret_cast<uint4 *>(az + a_off[c2] + 16384) = im[c2];
+          for (int c2 = 0; c2 < 2; c2++) {
+            *reinterpret_cast<uint4 *>(sAZ + h * 1024 + a_off[c2]) = re[c2];
+            *reinterpret_cast<uint4 *>(sAZ + h * 1024 + a_off[c2] + 16384) = im[c2];
+          }
         }
       }
-      arrive(&a_ready[i & 1]);
+      arrive(&B.a_ready[i & 1]);
       // (b) GEMM-2 epilogue of the previous unit into the staging rows,
       // once the bulk copies of the unit before it have read them
       if (i > 0) {
-        wait_d2(i - 1);  // D2 of unit i - 1 (already waited with one buffer)
-        tc::fence_after_sync();
-        if (i > 1) wait_ok(&st_done, (i - 2) & 1);
+        if (i > 1) wait_ok(&B.st_done, (i - 2) & 1);
         if (ok) store_unit(i - 1);
-        else arrive(&st_ready);
+        else arrive(&B.st_ready);
       }
       // (c) GEMM-1 epilogue: twiddle into the GEMM-2 operand Z
-      wait_ok(&d1_full, i & 1);
+      wait_ok(&B.d1_full, i & 1);
       tc::fence_after_sync();
       if (ok) {
-        float2 w = tw0;
-        // eight k1 at a time: half the accumulator registers live at once
+#pragma unroll 1
+        for (uint32_t h = 0; h < NG; h++) {
+          float2 w = NG > 1 && h ? tw0[NG - 1] : tw0[0];
+          // eight k1 at a time: half the accumulator registers live at once
 #pragma unroll
-        for (int g = 0; g < 2; g++) {
-          float yr[8], yi[8];
-          tc::tmem_ld8x2(tl + 16 * part + 8 * g, yr, tl + 64 + 16 * part + 8 * g, yi);
-          float zr[8], zi[8];
+          for (int g = 0; g < 2; g++) {
+            const uint32_t col = 16 * (part0 + h) + 8 * g;
+            float yr[8], yi[8];
+            tc::tmem_ld8x2(tl + col, yr, tl + 64 + col, yi);
+            float zr[8], zi[8];
 #pragma unroll
-          for (int b = 0; b < 8; b++) {
-            const float xr = yr[b], xi = yi[b];
-            zr[b] = xr * w.x - xi * w.y;
-            zi[b] = xr * w.y + xi * w.x;
-            w = make_float2(w.x * tws.x - w.y * tws.y, w.x * tws.y + w.y * tws.x);
+            for (int b = 0; b < 8; b++) {
+              const float xr = yr[b], xi = yi[b];
+              zr[b] = xr * w.x - xi * w.y;
+              zi[b] = xr * w.y + xi * w.x;
+              w = make_float2(w.x * tws.x - w.y * tws.y, w.x * tws.y + w.y * tws.x);
+            }
+            uint8_t *z = sAZ + z_off + h * 256 + g * 128;
+            *reinterpret_cast<uint4 *>(z) = make_uint4(h2_bits(zr[0], zr[1]), h2_bits(zr[2], zr[3]),
+                                                       h2_bits(zr[4], zr[5]), h2_bits(zr[6], zr[7]));
+            *reinterpret_cast<uint4 *>(z + 16384) = make_uint4(h2_bits(zi[0], zi[1]), h2_bits(zi[2], zi[3]),
+                                                               h2_bits(zi[4], zi[5]), h2_bits(zi[6], zi[7]));
           }
-          *reinterpret_cast<uint4 *>(az + z_off + g * 128) =
-              make_uint4(h2_bits(zr[0], zr[1]), h2_bits(zr[2], zr[3]), h2_bits(zr[4], zr[5]), h2_bits(zr[6], zr[7]));
-          *reinterpret_cast<uint4 *>(az + z_off + g * 128 + 16384) =
-              make_uint4(h2_bits(zi[0], zi[1]), h2_bits(zi[2], zi[3]), h2_bits(zi[4], zi[5]), h2_bits(zi[6], zi[7]));
         }
       }
-      arrive(&z_ready);
+      arrive(&B.z_ready);
     }
     // the last unit's inverse scales were written after the last barrier
-    if constexpr (!kFixedScale<DT>) compute_sync();
+    if constexpr (!kFixedScale<DT>) compute_sync(grp, F::kGT);
     wait_d2(n_units - 1);
     tc::fence_after_sync();
-    if (n_units > 1) wait_ok(&st_done, (n_units - 2) & 1);
+    if (n_units > 1) wait_ok(&B.st_done, (n_units - 2) & 1);
     if (ok) store_unit(n_units - 1);
   }
   tc::fence_before_sync();
   __syncthreads();
-  if (warp == 0) tc::tmem_dealloc(tmem, 256);
+  if (warp == 0) tc::tmem_dealloc(tmem_slot, 256 * NG);
 }
 
 using FtKernel = void (*)(const CUtensorMap, const FtParams);
@@ -691,6 +746,11 @@ FtKernel fft_tc_kernel_of(int dt) {
   }
 }
 
+uint32_t fft_tc_smem_of(int dt) {
+  return dt == MB_IQ_C32 ? Fmt<MB_IQ_C32>::kSmem : dt == MB_IQ_I16 ? Fmt<MB_IQ_I16>::kSmem
+         : dt == MB_IQ_I8 ? Fmt<MB_IQ_I8>::kSmem : Fmt<MB_IQ_F16>::kSmem;
+}
+
 // raises the dynamic shared memory limit of a sample type's kernel once per
 // device, and returns the device's SM count
 mb_status fft_tc_configure(int dt, int dev, int *sms) {
@@ -700,7 +760,7 @@ mb_status fft_tc_configure(int dt, int dev, int *sms) {
   const uint64_t bit = 1ull << (dev & 63);
   if (!(configured[which].load() & bit)) {
     MB_CUDA_TRY(cudaFuncSetAttribute(fft_tc_kernel_of(dt), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)kFtSmem));
+                                     (int)fft_tc_smem_of(dt)));
     int n = 0;
     MB_CUDA_TRY(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev));
     sm_count[dev & 63].store(n);
@@ -728,7 +788,8 @@ mb_status fft_tc_launch(const FftTcPlan *pl, const void *iq, int iq_dtype, FtPar
   p.units = (p.rows + 1) / 2;
   p.upc = upc ? upc : (p.units + (uint32_t)max(sms, 1) - 1) / (uint32_t)max(sms, 1);
   const uint32_t grid = (p.units + p.upc - 1) / p.upc;
-  fft_tc_kernel_of(iq_dtype)<<<grid, kFtThreads, kFtSmem, st>>>(map, p);
+  const uint32_t threads = iq_dtype == MB_IQ_C32 ? Fmt<MB_IQ_C32>::kThreads : Fmt<MB_IQ_I8>::kThreads;
+  fft_tc_kernel_of(iq_dtype)<<<grid, threads, fft_tc_smem_of(iq_dtype), st>>>(map, p);
   MB_LAUNCH_CHECK();
   return MB_OK;
 }
