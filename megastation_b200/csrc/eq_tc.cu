@@ -50,6 +50,7 @@ template <int MM, int QM>
 __global__ void __launch_bounds__(kEqThreads, 1)
     equalize_tc_kernel(const EqTcParams q, const __grid_constant__ CUtensorMap ymap) {
   extern __shared__ __align__(1024) uint8_t eq_smem[];
+  pdl_wait();
   __shared__ __align__(8) uint64_t full_bar[kStages];
   __shared__ __align__(8) uint64_t empty_bar[kStages];
   __shared__ __align__(8) uint64_t done_bar;
@@ -243,7 +244,8 @@ mb_status equalize_tc(const EqParams &p, const void *a_img, const void *y_lp, ui
                                    q.y16 != 0);
   if (tr != MB_OK) return tr;
   const dim3 grid(G, ny);
-  (s.MM == 64 ? eq_tc_kernel_of<64>(p.Qm) : eq_tc_kernel_of<128>(p.Qm))<<<grid, kEqThreads, smem, st>>>(q, ymap);
+  MB_CUDA_TRY(pdl_launch(s.MM == 64 ? eq_tc_kernel_of<64>(p.Qm) : eq_tc_kernel_of<128>(p.Qm), grid, kEqThreads, smem,
+                         st, q, ymap));
   MB_LAUNCH_CHECK();
   return MB_OK;
 }
@@ -280,6 +282,7 @@ __global__ void __launch_bounds__(kEqThreads, MM == 64 ? 3 : 2)
     equalize_tc_c32_kernel(const EqParams p, uint32_t l0, uint32_t nb, uint32_t spc, uint32_t N,
                            uint32_t tmem_cols, uint32_t vw_log2, uint32_t vec, int *err) {
   extern __shared__ __align__(128) uint8_t ec_smem[];
+  pdl_wait();
   __shared__ __align__(8) uint64_t bar[2];
   __shared__ uint32_t tmem_base_slot;
   constexpr uint32_t a_plane = MM / 8 * kTSbo, stage_bytes = 2 * kTY + 2 * a_plane;
@@ -442,8 +445,7 @@ static void eq_tc_c32_launch(const EqParams &p, uint32_t l0, uint32_t nb, int *e
   while ((2u << vw) < spc * p.sg) vw++;
   const uint32_t vec = p.S % 2 == 0 && (reinterpret_cast<uintptr_t>(p.y) & 15) == 0;
   const dim3 grid((p.S + p.sg - 1) / p.sg, ny);
-  k<<<grid, kEqThreads, smem, st>>>(p, l0, nb, spc, N, tmem_cols, vw, vec, err);
-  *e = cudaGetLastError();
+  *e = pdl_launch(k, grid, kEqThreads, smem, st, p, l0, nb, spc, N, tmem_cols, vw, vec, err);
 }
 
 mb_status equalize_tc_c32(const EqParams &p, int *err, cudaStream_t st) {

@@ -313,6 +313,7 @@ __global__ void __launch_bounds__(Plan<LOGN>::THREADS, Plan<LOGN>::MIN_BLOCKS)
   constexpr int N = PL::N, T = PL::T;
   constexpr bool INV = MODE == kIfft;
   extern __shared__ float2 smem_fft[];
+  pdl_wait();
 
   const int lrow = threadIdx.x / T;      // row within CTA
   const int t = threadIdx.x % T;         // thread within row
@@ -446,7 +447,7 @@ static mb_status launch_one(const FftParams &p, cudaStream_t st) {
   const uint64_t blocks = (p.rows + PL::ROWS - 1) / PL::ROWS;
   if (blocks == 0) return MB_OK;
   if (blocks > 0x7fffffffull) return MB_BAD_SHAPE;
-  fft_kernel<LOGN, MODE><<<(unsigned)blocks, PL::THREADS, smem, st>>>(p);
+  MB_CUDA_TRY(pdl_launch(fft_kernel<LOGN, MODE>, (unsigned)blocks, PL::THREADS, smem, st, p));
   MB_LAUNCH_CHECK();
   return MB_OK;
 }

@@ -230,6 +230,7 @@ template <int DT>
 __global__ void __launch_bounds__(Fmt<DT>::kThreads, 1)
     fft_tc_kernel(const __grid_constant__ CUtensorMap in_map, const FtParams p) {
   extern __shared__ __align__(1024) uint8_t ft_smem[];
+  pdl_wait();
   using F = Fmt<DT>;
   constexpr uint32_t NG = F::kNG;
   // Each barrier completes once per unit of its pipeline.  a_ready comes as a
@@ -789,7 +790,7 @@ mb_status fft_tc_launch(const FftTcPlan *pl, const void *iq, int iq_dtype, FtPar
   p.upc = upc ? upc : (p.units + (uint32_t)max(sms, 1) - 1) / (uint32_t)max(sms, 1);
   const uint32_t grid = (p.units + p.upc - 1) / p.upc;
   const uint32_t threads = iq_dtype == MB_IQ_C32 ? Fmt<MB_IQ_C32>::kThreads : Fmt<MB_IQ_I8>::kThreads;
-  fft_tc_kernel_of(iq_dtype)<<<grid, threads, fft_tc_smem_of(iq_dtype), st>>>(map, p);
+  MB_CUDA_TRY(pdl_launch(fft_tc_kernel_of(iq_dtype), grid, threads, fft_tc_smem_of(iq_dtype), st, map, p));
   MB_LAUNCH_CHECK();
   return MB_OK;
 }

@@ -101,6 +101,7 @@ __global__ void __launch_bounds__(kEncThreads) ldpc_encode_kernel(mb_ldpc h, con
                                                                   uint64_t info_stride, uint8_t *cw,
                                                                   uint64_t cw_stride) {
   extern __shared__ uint32_t enc_smem[];
+  pdl_wait();
   const uint32_t Z = h.Z, kb = h.kb, mb = h.mb, tid = threadIdx.x, nt = blockDim.x;
   const uint32_t nw = (Z + 31) / 32;                // words per block of Z bits
   const uint32_t nx = ((kb + mb) * Z + 31) / 32 + 2;
@@ -350,6 +351,7 @@ __global__ void __launch_bounds__(kMaxZ, 2) ldpc_decode_kernel(mb_ldpc h, const 
   // the pair's a-posteriori LLRs [(kb + mb) Z] (__half2), then the entries
   // {col * Z, shift} and the row pointers
   extern __shared__ uint32_t dec_smem[];
+  pdl_wait();
   const uint32_t Z = h.Z, kb = h.kb, mb = h.mb, N = (kb + mb) * Z, tid = threadIdx.x, nt = blockDim.x;
   __half2 *app = reinterpret_cast<__half2 *>(dec_smem);
   uint2 *ent = reinterpret_cast<uint2 *>(dec_smem + (N + 1) / 2 * 2);  // [nnz]
@@ -568,7 +570,8 @@ extern "C" mb_status mb_ldpc_encode(mb_ldpc *h, const uint8_t *info, uint64_t in
     return MB_BAD_SHAPE;
   if (batch == 0) return MB_OK;
   const size_t smem = 4 * (((size_t)(h->kb + h->mb) * h->Z + 31) / 32 + 2 + 4 * (size_t)((h->Z + 31) / 32) + 1);
-  ldpc_encode_kernel<<<batch, kEncThreads, smem, as_stream(stream)>>>(*h, info, info_stride, cw, cw_stride);
+  MB_CUDA_TRY(pdl_launch(ldpc_encode_kernel, batch, kEncThreads, smem, as_stream(stream), *h, info, info_stride, cw,
+                         cw_stride));
   MB_LAUNCH_CHECK();
   return MB_OK;
 }
@@ -591,8 +594,8 @@ extern "C" mb_status mb_ldpc_decode(mb_ldpc *h, const uint16_t *llr, uint64_t ll
   // check-node state
   for (uint32_t b0 = 0; b0 < batch; b0 += h->max_batch) {
     const uint32_t nb = std::min(h->max_batch, batch - b0);
-    ldpc_decode_kernel<<<(nb + 1) / 2, threads, smem, as_stream(stream)>>>(
-        *h, reinterpret_cast<const __half *>(llr), llr_stride, out, out_stride, max_iter, b0, nb);
+    MB_CUDA_TRY(pdl_launch(ldpc_decode_kernel, (nb + 1) / 2, threads, smem, as_stream(stream), *h,
+                           reinterpret_cast<const __half *>(llr), llr_stride, out, out_stride, max_iter, b0, nb));
     MB_LAUNCH_CHECK();
   }
   return MB_OK;

@@ -325,6 +325,7 @@ __global__ void __launch_bounds__(256) centre_kernel(const float2 *csi, const in
                                                      uint32_t K, uint32_t G, int *flag) {
   extern __shared__ __align__(16) unsigned char sgm[];
   __shared__ int bad;
+  pdl_wait();
   constexpr uint32_t ldm = ldm_of(KP), mat = KP * ldm;
   const uint32_t g = blockIdx.x, KK = K * K, ldc = ldc_of(K);
   float2 *gm = reinterpret_cast<float2 *>(sgm), *b1 = gm + mat, *b2 = b1 + mat, *b3 = b2 + mat, *c = b3 + mat;
@@ -407,6 +408,7 @@ __global__ void __launch_bounds__(256, 4) sub_detect_kernel(const float2 *csi, c
                                                          uint32_t iters, float2 *Xout, float2 *W, uint32_t M,
                                                          uint32_t K, uint32_t sg, uint32_t G, int *flag) {
   extern __shared__ __align__(16) unsigned char dsm[];
+  pdl_wait();
   __shared__ int bad;
   __shared__ float e0sq;  // ||I - G X0||_F^2 of the initial iterate
   constexpr uint32_t ldm = ldm_of(KP), mat = KP * ldm;
@@ -662,9 +664,8 @@ static size_t detect_smem(const mb_lzf *z) {
 // centre Grams and their inverses (FP32)
 static mb_status lzf_front(mb_lzf *z, const mb_c32 *csi, cudaStream_t st) {
   const uint32_t M = z->M, K = z->K;
-  MB_LZF_OF(centre_kernel, K)<<<z->G, 256, detect_smem(z), st>>>(
-      reinterpret_cast<const float2 *>(csi), z->ig, z->iw, z->cidx, z->Gc, z->Xc, M, K, z->G, z->flag);
-  MB_CUDA_TRY(cudaGetLastError());
+  MB_CUDA_TRY(pdl_launch(MB_LZF_OF(centre_kernel, K), z->G, 256, detect_smem(z), st,
+                         reinterpret_cast<const float2 *>(csi), z->ig, z->iw, z->cidx, z->Gc, z->Xc, M, K, z->G, z->flag));
   return MB_OK;
 }
 
@@ -742,10 +743,9 @@ extern "C" mb_status mb_lzf_run(mb_lzf *z, const mb_c32 *csi, mb_mlp *mlp, int i
     if (r != MB_OK) return r;
   }
   const size_t smem = detect_smem(z);
-  MB_LZF_OF(sub_detect_kernel, K)<<<S, 256, smem, st>>>(reinterpret_cast<const float2 *>(csi), z->ig, z->iw, z->Gs, z->Xc,
-                                          init == MB_LZF_LEARNED ? z->alpha : nullptr, init, ns_iters, z->X,
-                                          reinterpret_cast<float2 *>(W), M, K, z->sg, z->G, z->flag);
-  MB_CUDA_TRY(cudaGetLastError());
+  MB_CUDA_TRY(pdl_launch(MB_LZF_OF(sub_detect_kernel, K), S, 256, smem, st, reinterpret_cast<const float2 *>(csi), z->ig,
+                         z->iw, z->Gs, z->Xc, init == MB_LZF_LEARNED ? z->alpha : nullptr, init, ns_iters, z->X,
+                         reinterpret_cast<float2 *>(W), M, K, z->sg, z->G, z->flag));
   return MB_OK;
 }
 

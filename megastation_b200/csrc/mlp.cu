@@ -283,6 +283,7 @@ __device__ __forceinline__ void put_bf16(float v, uint64_t i, __nv_bfloat16 *wb,
 __global__ void adam_kernel(float *p, const float *g, float *m, float *v, uint64_t n, float lr,
                             float b1, float b2, float eps, float c1, float c2, __nv_bfloat16 *wb,
                             __nv_bfloat16 *img, const MlpStepShape s) {
+  pdl_wait();
   const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float gi = g[i];
@@ -731,9 +732,8 @@ extern "C" mb_status mb_mlp_adam_step(mb_mlp *n, float lr, void *stream) {
   const float b1 = 0.9f, b2 = 0.999f;
   const float c1 = 1.f - std::pow(b1, (float)n->step), c2 = 1.f - std::pow(b2, (float)n->step);
   const unsigned blocks = (unsigned)((n->n_params + 255) / 256);
-  adam_kernel<<<blocks, 256, 0, st>>>(n->p, n->g, n->m, n->v, n->n_params, lr, b1, b2, 1e-8f, c1, c2,
-                                      n->wb, n->img, n->ss);
-  MB_CUDA_TRY(cudaGetLastError());
+  MB_CUDA_TRY(pdl_launch(adam_kernel, blocks, 256, 0, st, n->p, n->g, n->m, n->v, n->n_params, lr, b1, b2, 1e-8f, c1, c2,
+                         n->wb, n->img, n->ss));
   return MB_OK;
 }
 

@@ -76,6 +76,7 @@ __device__ __forceinline__ void put16(uint8_t *m, uint32_t n, uint32_t c, const 
 template <int MT, bool FWD>
 __global__ void __launch_bounds__(128 * MT, 1) mlp_step_kernel(const StepParams q) {
   extern __shared__ __align__(1024) uint8_t st_smem[];
+  pdl_wait();
   __shared__ __align__(8) uint64_t bar, bar_g, wbar1, wbar2;
   __shared__ uint32_t tmem_slot;
   __shared__ float red[2][kStepMaxOut + 1];
@@ -430,6 +431,7 @@ __global__ void __launch_bounds__(128 * MT, 1) mlp_step_kernel(const StepParams 
 __global__ void __launch_bounds__(256) mlp_step_reduce_kernel(const float4 *part, uint32_t slots, uint64_t slot4,
                                                               uint64_t n_params, float *g, float *loss) {
   __shared__ float4 sums[4][64];
+  pdl_wait();
   const uint32_t f = threadIdx.x % 64, r = threadIdx.x / 64;
   const uint64_t e4 = (uint64_t)blockIdx.x * 64 + f;
   const uint32_t per = (slots + 3) / 4, k1 = min(slots, (r + 1) * per);
@@ -470,8 +472,7 @@ cudaError_t launch(const StepParams &q, unsigned grid, cudaStream_t st) {
     if (e != cudaSuccess) return e;
     configured.fetch_or(bit);
   }
-  mlp_step_kernel<MT, FWD><<<grid, 128 * MT, base + kT * q.s.Ip * 2, st>>>(q);
-  return cudaGetLastError();
+  return pdl_launch(mlp_step_kernel<MT, FWD>, grid, 128 * MT, base + kT * q.s.Ip * 2, st, q);
 }
 
 }  // namespace
@@ -504,9 +505,8 @@ cudaError_t mlp_step(const MlpStepShape &s, const __nv_bfloat16 *img, const floa
   const cudaError_t e = s.Wp == 128 ? launch<1, false>(q, grid, st) : launch<2, false>(q, grid, st);
   if (e != cudaSuccess) return e;
   const uint64_t slot4 = s.slot / 4;
-  mlp_step_reduce_kernel<<<(unsigned)((slot4 + 63) / 64), 256, 0, st>>>(reinterpret_cast<const float4 *>(part), grid,
-                                                                        slot4, s.n_params, g, loss);
-  return cudaGetLastError();
+  return pdl_launch(mlp_step_reduce_kernel, (unsigned)((slot4 + 63) / 64), 256, 0, st,
+                    reinterpret_cast<const float4 *>(part), grid, slot4, s.n_params, g, loss);
 }
 
 }  // namespace mb

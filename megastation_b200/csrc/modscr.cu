@@ -58,6 +58,7 @@ __global__ void modulate_kernel(const uint8_t *in, float2 *out,
                                 uint64_t in_bytes, uint64_t num_carriers,
                                 uint64_t num_ues, uint32_t Qm,
                                 uint32_t pilot_spacing, const float2 *pilots) {
+  pdl_wait();
   const uint64_t c = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
   const uint64_t u = blockIdx.y;
   if (c >= num_carriers || u >= num_ues) return;
@@ -112,9 +113,8 @@ extern "C" mb_status mb_modulate(const uint8_t *in, mb_c32 *out,
   if (num_carriers == 0 || num_ues == 0) return MB_OK;
   if (!device_tables()) return MB_CUDA_ERROR;  // the QAM maps are uploaded with the tables
   dim3 grid((unsigned)((num_carriers + 255) / 256), (unsigned)num_ues);
-  modulate_kernel<<<grid, 256, 0, as_stream(stream)>>>(
-      in, reinterpret_cast<float2 *>(out), in_bytes, num_carriers, num_ues, Qm,
-      pilot_spacing, reinterpret_cast<const float2 *>(pilot_table));
+  MB_CUDA_TRY(pdl_launch(modulate_kernel, grid, 256, 0, as_stream(stream), in, reinterpret_cast<float2 *>(out), in_bytes,
+                         num_carriers, num_ues, Qm, pilot_spacing, reinterpret_cast<const float2 *>(pilot_table)));
   MB_LAUNCH_CHECK();
   return MB_OK;
 }

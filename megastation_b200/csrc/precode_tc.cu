@@ -52,6 +52,7 @@ struct PcParams {
 
 __global__ void __launch_bounds__(kPcThreads, 1) precode_tc_kernel(const PcParams q) {
   extern __shared__ __align__(1024) uint8_t pc_smem[];
+  pdl_wait();
   __shared__ __align__(8) uint64_t img_bar, done_bar;
   __shared__ uint32_t tmem_slot;
   const uint32_t g = blockIdx.x, h = blockIdx.y;
@@ -161,6 +162,7 @@ __global__ void __launch_bounds__(kPcThreads, 1) precode_tc_kernel(const PcParam
 // 16-byte chunks of rows 2b (Re z) and 2b+1 (Im z) in planes 0 and 1.
 __global__ void precoder_image_kernel(const float2 *P, __nv_bfloat16 *img, uint32_t M, uint32_t K,
                                       uint32_t Kp, uint32_t H, uint32_t nkt) {
+  pdl_wait();
   const uint32_t g = blockIdx.x, h = blockIdx.y;
   uint8_t *out = reinterpret_cast<uint8_t *>(img) + ((uint64_t)g * H + h) * nkt * kBTile;
   const float2 *Pg = P + (uint64_t)g * K * M;
@@ -212,8 +214,8 @@ mb_status precoder_image(const float2 *P, void *img, uint32_t G, uint32_t M, uin
   if (!precode_tc_supported(K, 1)) return MB_UNSUPPORTED;
   if (G == 0) return MB_OK;
   const PcShape s = precode_tc_shape(M, K);
-  precoder_image_kernel<<<dim3(G, s.H), 256, 0, st>>>(P, reinterpret_cast<__nv_bfloat16 *>(img), M, K, s.Kp, s.H,
-                                                     s.nkt);
+  MB_CUDA_TRY(pdl_launch(precoder_image_kernel, dim3(G, s.H), 256, 0, st, P, reinterpret_cast<__nv_bfloat16 *>(img), M, K,
+                         s.Kp, s.H, s.nkt));
   MB_LAUNCH_CHECK();
   return MB_OK;
 }
@@ -255,7 +257,7 @@ mb_status precode_tc(const void *img, const float2 *sym, void *z, uint32_t M, ui
     configured.fetch_or(bit);
   }
   const uint32_t G = (S + sg - 1) / sg;
-  precode_tc_kernel<<<dim3(G, s.H, nz), kPcThreads, smem, st>>>(q);
+  MB_CUDA_TRY(pdl_launch(precode_tc_kernel, dim3(G, s.H, nz), kPcThreads, smem, st, q));
   MB_LAUNCH_CHECK();
   return MB_OK;
 }

@@ -138,6 +138,7 @@ constexpr int kEqKB = 16;  // antennas per shared-memory k tile
 template <int TU, int TC>
 __global__ void __launch_bounds__(256) equalize_fp32_kernel(const EqParams p) {
   constexpr int CT = 32, UT = 8;
+  pdl_wait();
   constexpr int NW = (kEqKB * UT * TU + 255) / 256, NY = kEqKB * CT * TC / 256;  // loads per thread and tile
   __shared__ float2 Ws[kEqKB][UT * TU];
   __shared__ float2 Ys[kEqKB][CT * TC];
@@ -220,7 +221,7 @@ template <int TU, int TC>
 static mb_status launch_eq(const EqParams &p, uint32_t G, cudaStream_t st) {
   dim3 grid(G, (p.n_sym + p.L - 1) / p.L);
   size_t smem = p.hard && p.sg % 8 ? sizeof(uint32_t) * p.L * p.K * p.hw_words : 0;
-  equalize_fp32_kernel<TU, TC><<<grid, 256, smem, st>>>(p);
+  MB_CUDA_TRY(pdl_launch(equalize_fp32_kernel<TU, TC>, grid, 256, smem, st, p));
   MB_LAUNCH_CHECK();
   return MB_OK;
 }
@@ -257,6 +258,7 @@ constexpr int kPcUB = 16;  // users per shared-memory k tile
 template <int TB, int TC>
 __global__ void __launch_bounds__(256) precode_kernel(const PcParams p) {
   constexpr int CT = 32, BT = 8;
+  pdl_wait();
   __shared__ float2 Ps[kPcUB][BT * TB];
   __shared__ float2 Ss[kPcUB][CT * TC];
   const uint32_t G = (p.S + p.sg - 1) / p.sg;
@@ -354,11 +356,11 @@ mb_status precode_fp32(const float2 *P, const float2 *s, float2 *out,
   constexpr int TB = 4;
   dim3 grid(G, (n_sym + L - 1) / L, (M + 8 * TB - 1) / (8 * TB));
   if (ncols <= 32)
-    precode_kernel<TB, 1><<<grid, 256, 0, st>>>(p);
+    MB_CUDA_TRY(pdl_launch(precode_kernel<TB, 1>, grid, 256, 0, st, p));
   else if (ncols <= 64)
-    precode_kernel<TB, 2><<<grid, 256, 0, st>>>(p);
+    MB_CUDA_TRY(pdl_launch(precode_kernel<TB, 2>, grid, 256, 0, st, p));
   else if (ncols <= 128)
-    precode_kernel<TB, 4><<<grid, 256, 0, st>>>(p);
+    MB_CUDA_TRY(pdl_launch(precode_kernel<TB, 4>, grid, 256, 0, st, p));
   else
     return MB_UNSUPPORTED;
   MB_LAUNCH_CHECK();

@@ -28,6 +28,7 @@ namespace mb {
 // cannot race with the read.
 __global__ void zf_fill_tail_kernel(float2 *csi, uint32_t G, uint32_t M,
                                     uint32_t K, uint32_t rem, uint32_t sg) {
+  pdl_wait();
   const uint64_t total = (uint64_t)M * K;
   for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < total;
        e += (uint64_t)gridDim.x * blockDim.x) {
@@ -49,6 +50,7 @@ template <typename T, int KP>
 __global__ void __launch_bounds__(256)
     zf_chol_kernel(float2 *csi, float2 *precoder, uint32_t M, uint32_t K,
                    int32_t *status, float *cond_out) {
+  pdl_wait();
   extern __shared__ __align__(16) unsigned char zf_smem_raw[];
   using C = Cplx<T>;
   const uint32_t g = blockIdx.x;
@@ -127,6 +129,7 @@ __global__ void __launch_bounds__(256)
     precoder_kernel(const float2 *W, float2 *P, uint32_t M, uint32_t K, uint32_t mb) {
   namespace cg = cooperative_groups;
   extern __shared__ float2 pc_tile[];  // [mb][ldt]
+  pdl_wait();
   __shared__ float red[8], cmax;
   const cg::cluster_group cl = cg::this_cluster();
   const uint32_t cn = cl.num_blocks(), rank = cl.block_rank(), g = blockIdx.x / cn;
@@ -216,6 +219,7 @@ __global__ void __launch_bounds__(256)
     precoder_scale_kernel(const float2 *W, float2 *P, const float *wmax, uint32_t M, uint32_t K,
                           uint32_t tiles_b) {
   __shared__ float2 tile[32][33];
+  pdl_wait();
   const uint32_t g = blockIdx.x;
   const uint32_t b0 = (blockIdx.y % tiles_b) * 32, u0 = (blockIdx.y / tiles_b) * 32;
   const uint32_t tx = threadIdx.x % 32, ty = threadIdx.x / 32;
@@ -249,7 +253,7 @@ mb_status zf_fill_tail(float2 *csi, uint32_t groups, uint32_t S, uint32_t sg,
   uint32_t rem = (uint32_t)(S - full);
   uint64_t total = (uint64_t)M * K;
   unsigned blocks = (unsigned)std::min<uint64_t>((total + 255) / 256, 1024);
-  zf_fill_tail_kernel<<<blocks, 256, 0, st>>>(csi, groups, M, K, rem, sg);
+  MB_CUDA_TRY(pdl_launch(zf_fill_tail_kernel, blocks, 256, 0, st, csi, groups, M, K, rem, sg));
   MB_LAUNCH_CHECK();
   return MB_OK;
 }
@@ -273,7 +277,7 @@ static mb_status zf_chol_launch(float2 *csi, float2 *precoder, uint32_t groups, 
   }
   if (smem + (size_t)static_smem.load() > (size_t)maxs) return MB_UNSUPPORTED;
   if (groups == 0) return MB_OK;
-  zf_chol_kernel<T, KP><<<groups, 256, smem, st>>>(csi, precoder, M, K, status, cond);
+  MB_CUDA_TRY(pdl_launch(zf_chol_kernel<T, KP>, groups, 256, smem, st, csi, precoder, M, K, status, cond));
   MB_LAUNCH_CHECK();
   return MB_OK;
 }
@@ -294,7 +298,7 @@ mb_status precoder_scale(const float2 *W, float2 *P, const float *wmax, uint32_t
                          uint32_t groups, cudaStream_t st) {
   if (groups == 0) return MB_OK;
   const uint32_t tb = (M + 31) / 32, tu = (K + 31) / 32;
-  precoder_scale_kernel<<<dim3(groups, tb * tu), 256, 0, st>>>(W, P, wmax, M, K, tb);
+  MB_CUDA_TRY(pdl_launch(precoder_scale_kernel, dim3(groups, tb * tu), 256, 0, st, W, P, wmax, M, K, tb));
   MB_LAUNCH_CHECK();
   return MB_OK;
 }
@@ -322,17 +326,19 @@ mb_status precoder_launch(const float2 *W, float2 *P, uint32_t M, uint32_t K,
     MB_CUDA_TRY(cudaFuncSetAttribute(precoder_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, maxs - 1024));
     configured.fetch_or(bit);
   }
-  cudaLaunchAttribute at{};
-  at.id = cudaLaunchAttributeClusterDimension;
-  at.val.clusterDim.x = cn;
-  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cudaLaunchAttribute at[2]{};
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = cn;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // as pdl_launch()
+  at[1].val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t lc{};
   lc.gridDim = dim3(groups * cn);
   lc.blockDim = dim3(256);
   lc.dynamicSmemBytes = smem;
   lc.stream = st;
-  lc.attrs = &at;
-  lc.numAttrs = 1;
+  lc.attrs = at;
+  lc.numAttrs = 2;
   MB_CUDA_TRY(cudaLaunchKernelEx(&lc, precoder_kernel, W, P, M, K, mb));
   MB_LAUNCH_CHECK();
   return MB_OK;

@@ -87,6 +87,7 @@ __device__ __forceinline__ void product_bf16(const float2 *Xt, Cplx<float> *Cs, 
 
 __global__ void __launch_bounds__(256, 4) zf_direct_kernel(const ZfdParams q) {
   extern __shared__ __align__(16) unsigned char zd_smem[];
+  pdl_wait();
   using C = Cplx<float>;
   constexpr int KP = 16;
   constexpr uint32_t TPR = 256 / KP;  // threads per row of A
@@ -242,7 +243,7 @@ mb_status zf_direct_run(float2 *csi, void *img, uint32_t groups, uint32_t M, uin
   }
   if (K > 16 || smem > (size_t)limit.load()) return MB_UNSUPPORTED;
   if (groups == 0) return MB_OK;
-  zf_direct_kernel<<<groups, 256, smem, st>>>(p);
+  MB_CUDA_TRY(pdl_launch(zf_direct_kernel, groups, 256, smem, st, p));
   MB_LAUNCH_CHECK();
   return MB_OK;
 }

@@ -423,6 +423,7 @@ __global__ void __launch_bounds__(kThreads, 2)
   // waves, the second with 57 of 148 SMs busy (184 us; 130 us with two)
   static_assert(QMF == 0 || MM == 64, "the fused equalize needs K <= 32");
   extern __shared__ __align__(1024) uint8_t zsm[];
+  pdl_wait();
   __shared__ __align__(8) uint64_t tile_bar[2];
   __shared__ __align__(8) uint64_t mma_bar;
   __shared__ __align__(8) uint64_t stage_bar[4];  // CSI tiles staged by bulk copies
@@ -1363,7 +1364,7 @@ static mb_status zf_mixed_launch(float2 *csi, void *img_w, uint32_t groups, uint
   }
   if (smem > avail) return MB_UNSUPPORTED;
   if (groups == 0) return MB_OK;
-  kern<<<groups, kThreads, smem, st>>>(q, ymap);
+  MB_CUDA_TRY(pdl_launch(kern, groups, kThreads, smem, st, q, ymap));
   MB_LAUNCH_CHECK();
   return MB_OK;
 }
