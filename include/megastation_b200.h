@@ -377,8 +377,7 @@ typedef struct {
   uint32_t c_init;
   int32_t out_dtype;            /* downlink IFFT output mb_iq_dtype */
   uint32_t sym_batch;           /* uplink symbols per FFT/equalize batch */
-  uint32_t use_graph;           /* replay the uplink slot as a CUDA graph (captured when a
-                                   pointer set comes a second time) */
+  uint32_t use_graph;           /* replay the uplink slot as a CUDA graph */
 } mb_cell_desc;
 
 typedef struct mb_slot mb_slot;
@@ -485,8 +484,7 @@ mb_status mb_slot_buffers(mb_slot *slot, mb_c32 **csi, mb_c32 **precoder);
  * BandProcess.  A set of cells of uneven shape (each an mb_cell_desc) runs
  * one uplink slot per call as ONE CUDA graph launch: the graph forks into a
  * branch per cell (that cell's slot) and joins, so the cells' kernels run
- * concurrently.  A (pointer set, stream) is issued directly the first time,
- * captured the second and replayed from then on.  Every
+ * concurrently.  Graphs are captured once per (pointer set, stream).  Every
  * argument array has one entry per cell, in creation order; llr, hard and
  * group_status arrays (and their entries) may be NULL as in
  * mb_slot_uplink.  stream must not be the legacy default stream. */

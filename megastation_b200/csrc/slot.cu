@@ -66,7 +66,7 @@ struct mb_slot {
     uint8_t *hard;
     int32_t *status;
     cudaStream_t stream;
-    cudaGraphExec_t exec;  // null: seen once, not captured
+    cudaGraphExec_t exec;
     uint64_t last_use;
   };
   std::vector<GraphEntry> graphs;
@@ -132,8 +132,7 @@ static size_t iq_elem_bytes(int dt) {
 
 extern "C" mb_status mb_slot_destroy(mb_slot *s) {
   if (!s) return MB_BAD_ARG;
-  for (auto &e : s->graphs)
-    if (e.exec) cudaGraphExecDestroy(e.exec);
+  for (auto &e : s->graphs) cudaGraphExecDestroy(e.exec);
   free_marks(s);
   if (s->fft) mb_fft_destroy(s->fft);
   if (s->scr) mb_scrambler_destroy(s->scr);
@@ -259,32 +258,6 @@ void mb::slot_io_bytes(const mb_slot *s, uint64_t *iq, uint64_t *llr, uint64_t *
 
 extern "C" mb_status mb_slot_create(const mb_cell_desc *cell, mb_slot **out) {
   return slot_create(cell, false, out);
-}
-
-// A pointer set is issued kernel by kernel the first time it is seen and
-// captured the second: capturing and instantiating the graph takes longer than
-// the slot, and a caller with new buffers each time would pay it for every one.
-// First, second and third call in us, waited for: one 256 x 32 cell 205, 100,
-// 97 with the capture first and 116, 215, 98 so; 32 cells 4031, 751, 728 and
-// 859, 3633, 595.  Not while the caller captures the stream, which stays the
-// error that it was.
-static bool issue_directly(cudaStream_t st) {
-  cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
-  return cudaStreamIsCapturing(st, &c) == cudaSuccess && c == cudaStreamCaptureStatusNone;
-}
-
-// the cache's next entry: a new one, or the least recently used of `most`
-template <typename E>
-static E &graph_entry(std::vector<E> &graphs, size_t most) {
-  if (graphs.size() < most) {
-    graphs.emplace_back();
-    return graphs.back();
-  }
-  auto lru = std::min_element(graphs.begin(), graphs.end(),
-                              [](const E &a, const E &b) { return a.last_use < b.last_use; });
-  if (lru->exec) cudaGraphExecDestroy(lru->exec);
-  *lru = E{};
-  return *lru;
 }
 
 static mb_status issue_uplink(mb_slot *s, const void *iq, uint16_t *llr,
@@ -459,12 +432,12 @@ extern "C" mb_status mb_slot_uplink(mb_slot *s, const void *iq, uint16_t *llr,
   mb_slot::GraphEntry *hit = nullptr;
   for (auto &e : s->graphs)
     if (e.iq == iq && e.llr == llr && e.hard == hard && e.status == status && e.stream == st) hit = &e;
-  if (!hit && issue_directly(st)) {
-    const mb_status r = issue_uplink(s, iq, llr, hard, status, st, nullptr);
-    if (r == MB_OK) graph_entry(s->graphs, kGraphCache) = {iq, llr, hard, status, st, nullptr, ++s->graph_clock};
-    return r;
-  }
-  if (!hit || !hit->exec) {
+  // The first call of a pointer set captures it, so one call ahead of time
+  // prepares it and every later one is a replay.  First and later calls, waited
+  // for: one 256 x 32 cell 205 and 97 us, 32 cells 4,031 and 728.  Issuing the
+  // first call directly and capturing the second (116 and 215 us, 859 and 3,633)
+  // put the capture into the first slot after a warm-up.
+  if (!hit) {
     MB_CUDA_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
     mb_status r = issue_uplink(s, iq, llr, hard, status, st, nullptr);
     cudaGraph_t g = nullptr;
@@ -479,8 +452,15 @@ extern "C" mb_status mb_slot_uplink(mb_slot *s, const void *iq, uint16_t *llr,
     e = cudaGraphInstantiate(&exec, g, cudaGraphInstantiateFlagUseNodePriority);
     cudaGraphDestroy(g);
     if (e != cudaSuccess) return record_error(e);
-    if (!hit) hit = &graph_entry(s->graphs, kGraphCache);
-    *hit = {iq, llr, hard, status, st, exec, 0};
+    if (s->graphs.size() >= kGraphCache) {
+      auto lru = s->graphs.begin();
+      for (auto it = s->graphs.begin(); it != s->graphs.end(); ++it)
+        if (it->last_use < lru->last_use) lru = it;
+      cudaGraphExecDestroy(lru->exec);
+      s->graphs.erase(lru);
+    }
+    s->graphs.push_back({iq, llr, hard, status, st, exec, 0});
+    hit = &s->graphs.back();
   }
   hit->last_use = ++s->graph_clock;
   MB_CUDA_TRY(cudaGraphLaunch(hit->exec, st));
@@ -637,8 +617,7 @@ extern "C" mb_status mb_slot_set_zf_init(mb_slot *s, const mb_mlp *net) {
   }
   if (net == s->zf_net) return MB_OK;
   // captured slots hold the previous choice in their kernel parameters
-  for (auto &e : s->graphs)
-    if (e.exec) cudaGraphExecDestroy(e.exec);
+  for (auto &e : s->graphs) cudaGraphExecDestroy(e.exec);
   s->graphs.clear();
   s->zf_net = net;
   return MB_OK;
@@ -658,7 +637,7 @@ struct mb_cells {
   cudaEvent_t fork = nullptr;
   struct Entry {
     std::vector<const void *> key;
-    cudaGraphExec_t exec;  // null: seen once, not captured
+    cudaGraphExec_t exec;
     uint64_t last_use;
   };
   std::vector<Entry> graphs;
@@ -666,8 +645,7 @@ struct mb_cells {
 };
 
 static void cells_drop_graphs(mb_cells *cs) {
-  for (auto &e : cs->graphs)
-    if (e.exec) cudaGraphExecDestroy(e.exec);
+  for (auto &e : cs->graphs) cudaGraphExecDestroy(e.exec);
   cs->graphs.clear();
 }
 
@@ -758,31 +736,19 @@ static mb_status cells_launch(mb_cells *cs, const void *const *iq, uint16_t *con
   mb_cells::Entry *hit = nullptr;
   for (auto &e : cs->graphs)
     if (e.key == key) hit = &e;
-  // every cell on its branch stream, forked from st and joined to it
-  mb_status r = MB_OK;
-  cudaError_t ce = cudaSuccess;
-  auto issue = [&] {
-    ce = cudaEventRecord(cs->fork, st);
+  if (!hit) {
+    MB_CUDA_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
+    mb_status r = MB_OK;
+    cudaError_t ce = cudaEventRecord(cs->fork, st);
     for (uint32_t c = 0; c < n && r == MB_OK && ce == cudaSuccess; c++) {
       ce = cudaStreamWaitEvent(cs->branch[c], cs->fork, 0);
       if (ce != cudaSuccess) break;
       r = issue_uplink(cs->slots[c], iq[c], llr ? llr[c] : nullptr, hard ? hard[c] : nullptr,
                        status ? status[c] : nullptr, cs->branch[c], nullptr);
+      if (r != MB_OK) break;
       ce = cudaEventRecord(cs->join[c], cs->branch[c]);
       if (ce == cudaSuccess) ce = cudaStreamWaitEvent(st, cs->join[c], 0);
     }
-  };
-  constexpr size_t kGraphCache = 8;
-  if (!hit && issue_directly(st)) {
-    issue();
-    if (r != MB_OK) return r;
-    MB_CUDA_TRY(ce);
-    graph_entry(cs->graphs, kGraphCache) = {key, nullptr, ++cs->clock};
-    return MB_OK;
-  }
-  if (!hit || !hit->exec) {
-    MB_CUDA_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-    issue();
     cudaGraph_t g = nullptr;
     cudaError_t ee = cudaStreamEndCapture(st, &g);
     if (r != MB_OK || ce != cudaSuccess || ee != cudaSuccess) {
@@ -794,8 +760,16 @@ static mb_status cells_launch(mb_cells *cs, const void *const *iq, uint16_t *con
     ce = cudaGraphInstantiate(&exec, g, cudaGraphInstantiateFlagUseNodePriority);
     cudaGraphDestroy(g);
     if (ce != cudaSuccess) return record_error(ce);
-    if (!hit) hit = &graph_entry(cs->graphs, kGraphCache);
-    *hit = {key, exec, 0};
+    constexpr size_t kGraphCache = 8;
+    if (cs->graphs.size() >= kGraphCache) {
+      auto lru = cs->graphs.begin();
+      for (auto it = cs->graphs.begin(); it != cs->graphs.end(); ++it)
+        if (it->last_use < lru->last_use) lru = it;
+      cudaGraphExecDestroy(lru->exec);
+      cs->graphs.erase(lru);
+    }
+    cs->graphs.push_back({key, exec, 0});
+    hit = &cs->graphs.back();
   }
   hit->last_use = ++cs->clock;
   MB_CUDA_TRY(cudaGraphLaunch(hit->exec, st));

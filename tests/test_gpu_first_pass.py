@@ -1,6 +1,9 @@
-"""A slot's pointer set is issued kernel by kernel the first time, captured the
-second and replayed from then on: all three, with more sets than the cache
-keeps (16 for a slot, 8 for batched cells), give the same bits."""
+"""A slot's pointer set is captured on its first call and replayed from then
+on: every call, with more sets than the cache keeps (16 for a slot, 8 for
+batched cells), gives the same bits, and one call ahead of time prepares a
+set, the second already being a replay."""
+import time
+
 import pytest
 import torch
 
@@ -62,3 +65,41 @@ def test_cells_passes(mb):
             ref = [t.clone() for t in llr + hard]
         assert all(torch.equal(a, b) for a, b in zip(llr + hard, ref, strict=True))
     assert mb.ops.device_error() == 0
+
+
+def host_us(call, sets):
+    """Host time of the second call of each set (the least over the sets: noise
+    only adds), and of later ones (the median)."""
+    second, later = [], []
+    for x in sets:
+        times = []
+        for _ in range(6):
+            torch.cuda.synchronize()
+            t = time.perf_counter()
+            call(x)
+            times.append((time.perf_counter() - t) * 1e6)
+        second.append(times[1])
+        later += times[2:]
+    torch.cuda.synchronize()
+    return min(second), sorted(later)[len(later) // 2]
+
+
+def test_second_slot_is_a_replay(mb):
+    from megastation_b200 import datagen, slot
+    cfg = config(U=13)
+    iq = torch.from_numpy(datagen.make_slot(cfg)["iq"]).cuda()
+    run = slot.UplinkSlot(cfg, precision="fp32", sym_batch=1, use_graph=True)  # 28 launches
+    st = torch.cuda.Stream()
+    second, later = host_us(lambda x: run(x, stream=st), [iq.clone() for _ in range(6)])
+    # a replay is one launch; capturing 28 and instantiating them costs several times that
+    assert second < 3 * later, (second, later)
+
+
+def test_second_call_of_cells_is_a_replay(mb):
+    from megastation_b200 import cells, datagen
+    cfgs = [config(seed=i, U=3) for i in range(8)]
+    sets = [[torch.from_numpy(datagen.make_slot(c)["iq"]).cuda() for c in cfgs] for _ in range(5)]
+    run = cells.Cells(cfgs)
+    st = torch.cuda.Stream()
+    second, later = host_us(lambda x: run(x, stream=st), sets)
+    assert second < 3 * later, (second, later)
