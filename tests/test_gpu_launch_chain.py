@@ -1,7 +1,9 @@
 """Kernels of a chain are set up while the one ahead drains and wait for its
 completion on the device.  Chains over buffers that are written again each time, run
 back to back and with a synchronisation after every call, must agree bit for
-bit: a read before the wait, or of a line cached before it, would show."""
+bit: a read before the wait, or of a line cached before it, would show.  So must
+the same chains in a caller's graph, where the edges between kernels are
+programmatic and those to copies are not."""
 import numpy as np
 import pytest
 import torch
@@ -106,3 +108,84 @@ def test_training(mb, width, batch):
         return [torch.from_numpy(np.ascontiguousarray(v)) for v in (net.params(), net.grads())]
 
     twice(chain)
+
+
+@pytest.mark.parametrize("copies", [False, True])
+@pytest.mark.parametrize("mixed,M,K,N,S", [(False, 64, 16, 2048, 1200), (True, 64, 32, 4096, 3276),
+                                           (True, 96, 48, 4096, 1204)])
+def test_uplink_in_a_callers_graph(mb, copies, mixed, M, K, N, S):
+    """Three rounds of pilots, detector, precoder and equalizer in one graph,
+    with a copy node between every two launches or with none."""
+    sg, n_sym, Qm, n = 16, 3, 4, 3
+    G, P, start = -(-S // sg), -(-K // sg), (N - S) // 2
+    g = torch.Generator(device="cuda").manual_seed(K + 1)
+    src = [torch.randn(n, P, M, N, 2, generator=g, device="cuda").mul(2000).short() for _ in range(3)]
+    y = [torch.randn(n_sym, M, S, dtype=torch.complex64, generator=g, device="cuda") for _ in range(n)]
+    pilot, scr = mb.PilotFFT(start, N, S, M, K, sg), mb.Scrambler(num_bits=S * Qm)
+    zf = mb.Beamform(M, K, G, precision=mb._lib.MB_ZF_MIXED if mixed else mb._lib.MB_ZF_FP32)
+    iq, stage = torch.empty_like(src[0]), src[0].clone()
+    csi = torch.zeros(G, M, K, dtype=torch.complex64, device="cuda")
+    W = torch.zeros_like(csi)
+    pre = torch.zeros(n, G, K, M, dtype=torch.complex64, device="cuda")
+    llr = torch.zeros(n, n_sym, K, S * Qm, dtype=torch.float16, device="cuda")
+    eq = mb.Equalize.equalize_tc if mixed else mb.Equalize.equalize
+
+    def chain():
+        iq.copy_(stage)
+        for i in range(n):
+            (pilot.mixed if mixed else pilot)(iq[i], csi)
+            if copies:
+                W.copy_(csi)
+            w = W if copies else csi
+            zf.beamform_uplink(w, S, sg)
+            if copies:
+                csi.copy_(W)
+            mb.Beamform.beamform_downlink(csi, pre[i])
+            if copies:
+                W.copy_(csi)
+            eq(w, y[i], llr[i], sg, Qm, S * Qm, 0, scrambler=scr)
+
+    ref = []
+    for s in src:
+        stage.copy_(s)
+        chain()
+        torch.cuda.synchronize()
+        ref.append((pre.clone(), llr.clone()))
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        chain()
+    for i in (0, 1, 2, 1, 0):
+        stage.copy_(src[i])
+        pre.zero_(), llr.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(pre, ref[i][0]) and torch.equal(llr, ref[i][1])
+    assert mb.ops.device_error() == 0
+
+
+def test_training_in_a_callers_graph(mb):
+    from megastation_b200 import learned
+    g = torch.Generator(device="cuda").manual_seed(7)
+    x, A = torch.rand(500, 22, generator=g, device="cuda"), torch.eye(4, device="cuda").expand(500, 4, 4).contiguous()
+    b, loss = torch.randn(500, 4, generator=g, device="cuda"), torch.zeros(1, device="cuda")
+    y = torch.zeros(500, 4, device="cuda")
+    net = learned.MLP(22, 128, 4, max_batch=500)
+    p0 = (0.05 * np.random.default_rng(0).standard_normal(net.params().size)).astype(np.float32)
+
+    def chain():  # (the optimiser's step count is the handle's, so it stays outside)
+        for _ in range(3):
+            net.loss_grad(x, A, b, loss=loss)
+            net.forward(x, out=y)
+
+    net.set_params(p0)
+    chain()
+    torch.cuda.synchronize()
+    ref = [loss.clone(), y.clone(), torch.from_numpy(net.grads())]
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        chain()
+    loss.zero_(), y.zero_()
+    graph.replay()
+    torch.cuda.synchronize()
+    for a, c in zip([loss, y, torch.from_numpy(net.grads())], ref, strict=True):
+        assert torch.equal(a, c)
