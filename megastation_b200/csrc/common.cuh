@@ -51,7 +51,12 @@ __device__ __forceinline__ void cfma(float2 &acc, float2 a, float2 b) {
 // that one has completed and its writes are visible.  So pdl_wait() is the
 // first statement of every thread, before any access to global memory and
 // before any return: a CTA that left without it would let the next kernel of
-// the chain start with the last but one still running.  It saves 1 to 3 us a
+// the chain start with the last but one still running.  Whatever an earlier
+// kernel may have written (a caller's buffers too: the writer is the caller's
+// last kernel) is read with ordinary loads behind it: __ldg says that the data
+// does not change while the kernel is resident, which holds only for tables
+// written when their handle was created (twiddles, pilot signs, descrambling
+// bytes, the code's B^-1).  It saves 1 to 3 us a
 // launch in a chain (pilots to detector of 64 x 16 in FP32, two launches: 16.4
 // -> 13.5 us; modulate, precode and inverse FFT of 128 x 16: 26.0 -> 20.4; a
 // training step of three: 56 -> 50).  No kernel lets the next one start

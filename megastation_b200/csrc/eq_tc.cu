@@ -327,10 +327,10 @@ __global__ void __launch_bounds__(kEqThreads, MM == 64 ? 3 : 2)
       yr[j] = make_float4(0.f, 0.f, 0.f, 0.f);
       if (j < (int)nyu && (kWhole || yb + j * ystep < left)) {
         if (vec && y1_on) {
-          yr[j] = __ldg(reinterpret_cast<const float4 *>(q));
+          yr[j] = *reinterpret_cast<const float4 *>(q);
         } else {
-          if (y0_on) *reinterpret_cast<float2 *>(&yr[j].x) = __ldg(q);
-          if (y1_on) *reinterpret_cast<float2 *>(&yr[j].z) = __ldg(q + 1);
+          if (y0_on) *reinterpret_cast<float2 *>(&yr[j].x) = *q;
+          if (y1_on) *reinterpret_cast<float2 *>(&yr[j].z) = q[1];
         }
       }
       q += ys;
@@ -339,7 +339,7 @@ __global__ void __launch_bounds__(kEqThreads, MM == 64 ? 3 : 2)
 #pragma unroll
     for (int j = 0; j < 8; j++) {
       wr[j] = make_float2(0.f, 0.f);
-      if (w_on && (kWhole || 8 * kc + j < left)) wr[j] = __ldg(w);
+      if (w_on && (kWhole || 8 * kc + j < left)) wr[j] = *w;
       w += p.K;
     }
     yp += (uint64_t)kTA * p.S;

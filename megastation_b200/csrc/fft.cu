@@ -179,14 +179,14 @@ __device__ __forceinline__ void load_iq16(const FftParams &p, uint64_t first, ui
     case MB_IQ_C32: {
       const float2 *q = reinterpret_cast<const float2 *>(p.in) + first;
 #pragma unroll
-      for (int i = 0; i < 16; i++) v[i] = __ldg(q + i * stride);
+      for (int i = 0; i < 16; i++) v[i] = q[i * stride];
       break;
     }
     case MB_IQ_I16: {
       const short2 *q = reinterpret_cast<const short2 *>(p.in) + first;
       short2 r[16];
 #pragma unroll
-      for (int i = 0; i < 16; i++) r[i] = __ldg(q + i * stride);
+      for (int i = 0; i < 16; i++) r[i] = q[i * stride];
 #pragma unroll
       for (int i = 0; i < 16; i++) v[i] = make_float2((float)r[i].x / 32768.f, (float)r[i].y / 32768.f);
       break;
@@ -195,7 +195,7 @@ __device__ __forceinline__ void load_iq16(const FftParams &p, uint64_t first, ui
       const char2 *q = reinterpret_cast<const char2 *>(p.in) + first;
       char2 r[16];
 #pragma unroll
-      for (int i = 0; i < 16; i++) r[i] = __ldg(q + i * stride);
+      for (int i = 0; i < 16; i++) r[i] = q[i * stride];
 #pragma unroll
       for (int i = 0; i < 16; i++) v[i] = make_float2((float)r[i].x / 128.f, (float)r[i].y / 128.f);
       break;
@@ -204,7 +204,7 @@ __device__ __forceinline__ void load_iq16(const FftParams &p, uint64_t first, ui
       const __half2 *q = reinterpret_cast<const __half2 *>(p.in) + first;
       __half2 r[16];
 #pragma unroll
-      for (int i = 0; i < 16; i++) r[i] = __ldg(q + i * stride);
+      for (int i = 0; i < 16; i++) r[i] = q[i * stride];
 #pragma unroll
       for (int i = 0; i < 16; i++) v[i] = __half22float2(r[i]);
       break;

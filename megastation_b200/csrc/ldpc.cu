@@ -113,9 +113,9 @@ __global__ void __launch_bounds__(kEncThreads) ldpc_encode_kernel(mb_ldpc h, con
   for (uint32_t w = tid; w < nx; w += nt) {
     uint32_t v = 0;
     if (in_al && 4 * w + 4 <= in_bytes) {
-      v = __byte_perm(__ldg(reinterpret_cast<const uint32_t *>(in) + w), 0, 0x0123);
+      v = __byte_perm(reinterpret_cast<const uint32_t *>(in)[w], 0, 0x0123);
     } else {
-      for (uint32_t b = 4 * w; b < 4 * w + 4; b++) v = (v << 8) | (b < in_bytes ? __ldg(in + b) : 0u);
+      for (uint32_t b = 4 * w; b < 4 * w + 4; b++) v = (v << 8) | (b < in_bytes ? in[b] : 0u);
     }
     x[w] = 32 * w < in_bits ? first_bits(v, in_bits - 32 * w) : 0u;
   }

@@ -244,7 +244,7 @@ __device__ __forceinline__ void interp_smem(const float2 *csi, const int *ig, co
   float2 *d = c + b0 * ldc + u;
 #pragma unroll 8
   for (uint32_t b = b0; b < M; b += step) {
-    const float2 a = __ldg(lo), e = __ldg(hi);
+    const float2 a = *lo, e = *hi;
     *d = make_float2((1.f - t) * a.x + t * e.x, (1.f - t) * a.y + t * e.y);
     lo += step * K;
     hi += step * K;

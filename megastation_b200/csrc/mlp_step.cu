@@ -208,7 +208,7 @@ __global__ void __launch_bounds__(128 * MT, 1) mlp_step_kernel(const StepParams 
         const float2 *c0 = q.f.gc + (uint64_t)g * KK;
         float v[8] = {0, 0, 0, 0, 0, 0, 0, 0};  // ||C_g||^2, trace, then distances and traces of j = -1, 1, 2
         for (uint32_t e = lane; e < KK; e += 32) {
-          const float2 a = __ldg(c0 + e);
+          const float2 a = c0[e];
           const bool diag = e % (q.f.K + 1) == 0;
           v[0] += a.x * a.x + a.y * a.y;
           if (diag) v[1] += a.x;
@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(128 * MT, 1) mlp_step_kernel(const StepParams 
           for (int k = 0; k < 3; k++) {
             const int gj = (int)g + (k == 0 ? -1 : k);
             if (gj < 0 || gj >= (int)q.f.G) continue;
-            const float2 b = __ldg(q.f.gc + (uint64_t)gj * KK + e);
+            const float2 b = q.f.gc[(uint64_t)gj * KK + e];
             v[2 + k] += (b.x - a.x) * (b.x - a.x) + (b.y - a.y) * (b.y - a.y);
             if (diag) v[5 + k] += b.x;
           }
@@ -243,7 +243,7 @@ __global__ void __launch_bounds__(128 * MT, 1) mlp_step_kernel(const StepParams 
         const uint32_t f = ch * 8 + j, row = row0 + r;
         v[j] = 0.f;
         if (r < nv && f < I) {
-          if (!FWD || q.x) v[j] = __ldg(q.x + (uint64_t)row * I + f);
+          if (!FWD || q.x) v[j] = q.x[(uint64_t)row * I + f];
           else v[j] = f < q.f.sg ? (f == row % q.f.sg ? 1.f : 0.f) : fs[(row / q.f.sg - fg0) * 6 + f - q.f.sg];
         }
       }
@@ -251,9 +251,9 @@ __global__ void __launch_bounds__(128 * MT, 1) mlp_step_kernel(const StepParams 
           make_uint4(pack2(v[0], v[1]), pack2(v[2], v[3]), pack2(v[4], v[5]), pack2(v[6], v[7]));
     }
     if (!FWD && stage_abc) {
-      for (uint32_t e = tid; e < nv * O * O; e += nthr) abc[e] = __ldg(q.A + (uint64_t)row0 * O * O + e);
-      for (uint32_t e = tid; e < nv * O; e += nthr) abc[kT * 16 + e] = __ldg(q.b + (uint64_t)row0 * O + e);
-      for (uint32_t e = tid; e < nv; e += nthr) abc[kT * 20 + e] = q.c ? __ldg(q.c + row0 + e) : 0.f;
+      for (uint32_t e = tid; e < nv * O * O; e += nthr) abc[e] = q.A[(uint64_t)row0 * O * O + e];
+      for (uint32_t e = tid; e < nv * O; e += nthr) abc[kT * 16 + e] = q.b[(uint64_t)row0 * O + e];
+      for (uint32_t e = tid; e < nv; e += nthr) abc[kT * 20 + e] = q.c ? q.c[row0 + e] : 0.f;
     }
     if (!tc::mbar_wait(&wbar1, pass & 1)) ok = false;
     publish();
@@ -298,7 +298,7 @@ __global__ void __launch_bounds__(128 * MT, 1) mlp_step_kernel(const StepParams 
         if (tid < nv) {
 #pragma unroll
           for (uint32_t r = 0; r < 16; r++)
-            if (r < O) d[r] = y[r] + __ldg(b3 + r);
+            if (r < O) d[r] = y[r] + b3[r];
         }
       }
       continue;
@@ -312,7 +312,7 @@ __global__ void __launch_bounds__(128 * MT, 1) mlp_step_kernel(const StepParams 
       const float *bi = stage_abc ? abc + kT * 16 + tid * O : q.b + (uint64_t)(row0 + (in ? tid : 0)) * O;
 #pragma unroll
       for (uint32_t r = 0; r < 16; r++) {
-        y[r] = r < O ? y[r] + __ldg(q.params + s.off[5] + r) : 0.f;
+        y[r] = r < O ? y[r] + q.params[s.off[5] + r] : 0.f;
         g[r] = 0.f;
       }
       float quad_y = 0.f, lin = 0.f;
@@ -337,7 +337,7 @@ __global__ void __launch_bounds__(128 * MT, 1) mlp_step_kernel(const StepParams 
       *reinterpret_cast<uint4 *>(d) = make_uint4(pack2(g[0], g[1]), pack2(g[2], g[3]), pack2(g[4], g[5]), pack2(g[6], g[7]));
       *reinterpret_cast<uint4 *>(d + 128) =
           make_uint4(pack2(g[8], g[9]), pack2(g[10], g[11]), pack2(g[12], g[13]), pack2(g[14], g[15]));
-      const float ci = stage_abc ? abc[kT * 20 + tid] : (q.c && in ? __ldg(q.c + row0 + tid) : 0.f);
+      const float ci = stage_abc ? abc[kT * 20 + tid] : (q.c && in ? q.c[row0 + tid] : 0.f);
       float li = in ? (quad_y - 2.f * lin + ci) / (float)q.B : 0.f;
       for (uint32_t r = 0; r <= O; r++) {
         float v = li;

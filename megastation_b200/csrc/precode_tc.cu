@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(kPcThreads, 1) precode_tc_kernel(const PcParam
       float2 v[8];
 #pragma unroll
       for (int j = 0; j < 8; j++)
-        v[j] = col_ok && u0 + j < q.K ? __ldg(src + (uint64_t)(u0 + j) * q.S) : make_float2(0.f, 0.f);
+        v[j] = col_ok && u0 + j < q.K ? src[(uint64_t)(u0 + j) * q.S] : make_float2(0.f, 0.f);
       uint32_t re[4], im[4];
 #pragma unroll
       for (int j = 0; j < 4; j++) {
@@ -172,7 +172,7 @@ __global__ void precoder_image_kernel(const float2 *P, __nv_bfloat16 *img, uint3
     float2 p[8];
 #pragma unroll
     for (int j = 0; j < 8; j++)
-      p[j] = b < M && u0 + j < K ? __ldg(Pg + (uint64_t)(u0 + j) * M + b) : make_float2(0.f, 0.f);
+      p[j] = b < M && u0 + j < K ? Pg[(uint64_t)(u0 + j) * M + b] : make_float2(0.f, 0.f);
     // Re z = Re P Re s - Im P Im s; Im z = Im P Re s + Re P Im s
     uint32_t w[4][4];  // [ri * 2 + plane][pair]
 #pragma unroll

@@ -173,12 +173,12 @@ __global__ void __launch_bounds__(256) equalize_fp32_kernel(const EqParams p) {
 #pragma unroll
     for (int j = 0; j < NW; j++) {
       const uint32_t b = b0 + wb + j * wstep;
-      wr[j] = w_on && b < p.M ? __ldg(wp + (uint64_t)(b0 + j * wstep) * p.K) : make_float2(0.f, 0.f);
+      wr[j] = w_on && b < p.M ? wp[(uint64_t)(b0 + j * wstep) * p.K] : make_float2(0.f, 0.f);
     }
 #pragma unroll
     for (int j = 0; j < NY; j++) {
       const uint32_t b = b0 + yb + j * ystep;
-      yr[j] = y_on && b < p.M ? __ldg(yp + (uint64_t)(b0 + j * ystep) * p.S) : make_float2(0.f, 0.f);
+      yr[j] = y_on && b < p.M ? yp[(uint64_t)(b0 + j * ystep) * p.S] : make_float2(0.f, 0.f);
     }
   };
   load(0);
@@ -308,11 +308,11 @@ __global__ void __launch_bounds__(256) precode_kernel(const PcParams p) {
   for (uint32_t u0 = 0; u0 < p.K; u0 += kPcUB) {
 #pragma unroll
     for (int j = 0; j < NP; j++)
-      Ps[pu + j * pstep][pb] = p_on && u0 + pu + j * pstep < p.K ? __ldg(pp + (uint64_t)(u0 + j * pstep) * p.M)
+      Ps[pu + j * pstep][pb] = p_on && u0 + pu + j * pstep < p.K ? pp[(uint64_t)(u0 + j * pstep) * p.M]
                                                                  : make_float2(0.f, 0.f);
 #pragma unroll
     for (int j = 0; j < NS; j++)
-      Ss[su + j * sstep][sc] = s_on && u0 + su + j * sstep < p.K ? __ldg(sp + (uint64_t)(u0 + j * sstep) * p.S)
+      Ss[su + j * sstep][sc] = s_on && u0 + su + j * sstep < p.K ? sp[(uint64_t)(u0 + j * sstep) * p.S]
                                                                  : make_float2(0.f, 0.f);
     __syncthreads();
 #pragma unroll 4

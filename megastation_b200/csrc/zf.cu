@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(256)
   const uint32_t db = 256 / K, du = 256 % K;
 #pragma unroll 8
   for (uint32_t e = threadIdx.x; e < nb * K; e += 256) {
-    const float2 v = __ldg(wg + e);
+    const float2 v = wg[e];
     mx = fmaxf(mx, sqrtf(v.x * v.x + v.y * v.y));
     pc_tile[b * ldt + u] = v;
     b += db;
