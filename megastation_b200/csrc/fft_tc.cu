@@ -87,7 +87,7 @@ struct FtParams {
   float2 *csi;          // pilot: [G][M][K]
   const float2 *pilot;  // pilot: sign of each subcarrier
   uint32_t K, sg, ue_start, tail_rem, G;
-  uint32_t sg_magic;    // floor(i / sg) = umulhi(i, sg_magic) for i < 2^13
+  uint32_t sg_magic;    // ceil(2^32 / sg): floor(i / sg) = umulhi(i, sg_magic) for i < 2^13; 0: sg = 1
   const uint8_t *mats;
   const float2 *tw;
   uint32_t c;
@@ -532,7 +532,7 @@ __global__ void __launch_bounds__(Fmt<DT>::kThreads, 1)
 #pragma unroll
           for (int j = 0; j < 8; j++) {
             const uint32_t sc = (s_base + 64 * (jb + j)) & (kFtN - 1);
-            const uint32_t g = __umulhi(sc, p.sg_magic), sl = sc - g * p.sg, uu = u0 + sl;
+            const uint32_t g = p.sg_magic ? __umulhi(sc, p.sg_magic) : sc, sl = sc - g * p.sg, uu = u0 + sl;
             const float x = vr[j] * inv, y = vi[j] * inv;
             const float2 e = make_float2(x * ps[j].x + y * ps[j].y, x * ps[j].y - y * ps[j].x);
             if (sc < p.S && uu < p.K) {
@@ -905,7 +905,7 @@ mb_status fft_tc_pilot(const FftTcPlan *pl, const void *iq, int iq_dtype, uint32
   p.ue_start = ue_start;
   p.tail_rem = tail_rem;
   p.G = (S + sg - 1) / sg;
-  p.sg_magic = (uint32_t)((0x100000000ull + sg - 1) / sg);
+  p.sg_magic = sg > 1 ? 0xFFFFFFFFu / sg + 1 : 0;
   p.err = err;
   p.pilot_rows = p.rows;
   return fft_tc_launch(pl, iq, iq_dtype, p, st, upc);
@@ -932,7 +932,7 @@ mb_status fft_tc_slot(const FftTcPlan *pl, const void *iq, int iq_dtype, uint32_
   p.ue_start = 0;
   p.tail_rem = tail_rem;
   p.G = (S + sg - 1) / sg;
-  p.sg_magic = (uint32_t)((0x100000000ull + sg - 1) / sg);
+  p.sg_magic = sg > 1 ? 0xFFFFFFFFu / sg + 1 : 0;
   p.err = err;
   return fft_tc_launch(pl, iq, iq_dtype, p, st, upc);
 }

@@ -160,3 +160,30 @@ def test_pilot_fft_mixed_many_units(mb):
     scale = np.sqrt(np.mean(np.abs(r) ** 2, axis=(0, 3), keepdims=True))
     ratio = np.abs(got - r) / (2e-3 * scale)
     assert ratio.max() <= 1.0, (ratio.max(), np.unravel_index(ratio.argmax(), ratio.shape))
+
+
+# group sizes around the division's edges: one subcarrier a group (no reciprocal
+# in 32 bits), a power of two, odd ones, the largest
+@pytest.mark.parametrize("sg,K,n_sym,ue_start", [(1, 3, 3, 0), (1, 4, 2, 1), (2, 4, 2, 0), (3, 7, 3, 0),
+                                                 (31, 40, 2, 0), (4095, 2, 1, 0)])
+@pytest.mark.parametrize("dtype", [torch.int8, torch.complex64])
+def test_pilot_group_sizes(mb, sg, K, n_sym, ue_start, dtype):
+    """The tensor-core LS estimates against the FP32 operator's: 2e-3 of the
+    row's RMS (FP16 operands; the pilots have unit modulus), and what neither
+    writes stays as it was."""
+    N, S, M = 4096, 3277, 5
+    g = torch.Generator(device="cuda").manual_seed(sg + K)
+    if dtype == torch.int8:
+        iq = torch.randint(-128, 128, (n_sym, M, N, 2), generator=g, device="cuda").to(dtype)
+    else:
+        iq = torch.randn(n_sym, M, N, dtype=dtype, generator=g, device="cuda")
+    op = mb.PilotFFT((N - S) // 2, N, S, M, K, sg)
+    ref, got = (torch.full((-(-S // sg), M, K), 1e6, dtype=torch.complex64, device="cuda") for _ in range(2))
+    op(iq, ref, ue_start=ue_start)
+    op.mixed(iq, got, ue_start=ue_start)
+    torch.cuda.synchronize()
+    assert mb.ops.device_error() == 0
+    kept = ref == 1e6
+    assert torch.equal(got[kept], ref[kept])
+    rms = ref[~kept].abs().square().mean().sqrt()  # of all rows together: one row's is within 10%
+    assert float(rms) < 1e4 and float((got - ref)[~kept].abs().max()) <= 2e-3 * float(rms) * 1.1
