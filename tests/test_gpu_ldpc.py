@@ -266,3 +266,18 @@ def test_encoder_odd_lifting_sizes_and_strides(Z, stride_pad):
     assert (got[:, n:] == 0xA5).all()
     want = np.stack([np.packbits(ldpc.encode(g, info[k])[2 * Z:]) for k in range(3)])
     np.testing.assert_array_equal(got[:, :n], want)
+
+
+@pytest.mark.parametrize("Z", [3, 4, 5, 9, 11, 15, 16, 17, 30, 32, 33])
+def test_encoder_short_columns(Z):
+    """Columns around a word's length and its halves, whose rotation repeats
+    within a word, against the restated encoder."""
+    mb = _mb()
+    entries = _big_graph(Z, seed=5)
+    kb = ldpc.KB[1]
+    g = ldpc.Graph(entries, kb, Z, 9)
+    info = np.random.default_rng(Z).integers(0, 2, (3, kb * Z), dtype=np.uint8)
+    out = mb.Ldpc(entries, kb, Z, 9).encode(_pack(info))
+    torch.cuda.synchronize()
+    want = np.stack([np.packbits(ldpc.encode(g, info[k])[2 * Z:]) for k in range(3)])
+    np.testing.assert_array_equal(out.cpu().numpy(), want)
