@@ -46,7 +46,10 @@ __global__ void zf_fill_tail_kernel(float2 *csi, uint32_t G, uint32_t M,
 // dependent steps and the factor itself three barriers a column.  Latency
 // bound for small cells (75 groups of 64 x 16: 20.4 us
 // before, 9.0 us).
-template <typename T, int KP>
+// KP: users the elimination has registers for, KG: the Gram's blocks of 16
+// (three instead of four from 33 to 48 users, in FP32: 205 groups of 256 x 33
+// 102.5 -> 85 us, of 256 x 48 174 -> 153; the Cholesky form 96 and 266).
+template <typename T, int KP, int KG>
 __global__ void __launch_bounds__(256)
     zf_chol_kernel(float2 *csi, float2 *precoder, uint32_t M, uint32_t K,
                    int32_t *status, float *cond_out) {
@@ -67,7 +70,7 @@ __global__ void __launch_bounds__(256)
   const uint32_t db = nt / K, du = nt % K;
   zf_load_c<T>(cg, Cs, M, K, ldc);
   __syncthreads();
-  zf_gram<T, KP>(Cs, A, M, K, ldc, lda);
+  zf_gram<T, KG>(Cs, A, M, K, ldc, lda);
   __syncthreads();
   ldl_eliminate<T, KP>(A, lda, K, &not_pd);
   const bool bad = not_pd != 0;
@@ -258,7 +261,7 @@ mb_status zf_fill_tail(float2 *csi, uint32_t groups, uint32_t S, uint32_t sg,
   return MB_OK;
 }
 
-template <typename T, int KP>
+template <typename T, int KP, int KG = KP>
 static mb_status zf_chol_launch(float2 *csi, float2 *precoder, uint32_t groups, uint32_t M, uint32_t K, size_t smem,
                                 int32_t *status, float *cond, cudaStream_t st) {
   static std::atomic<uint64_t> configured{0};
@@ -269,15 +272,15 @@ static mb_status zf_chol_launch(float2 *csi, float2 *precoder, uint32_t groups, 
   const uint64_t bit = 1ull << (dev & 63);
   if (!(configured.load() & bit)) {
     cudaFuncAttributes fa;
-    MB_CUDA_TRY(cudaFuncGetAttributes(&fa, zf_chol_kernel<T, KP>));
-    MB_CUDA_TRY(cudaFuncSetAttribute(zf_chol_kernel<T, KP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    MB_CUDA_TRY(cudaFuncGetAttributes(&fa, zf_chol_kernel<T, KP, KG>));
+    MB_CUDA_TRY(cudaFuncSetAttribute(zf_chol_kernel<T, KP, KG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      maxs - (int)fa.sharedSizeBytes));
     static_smem = (int)fa.sharedSizeBytes;
     configured.fetch_or(bit);
   }
   if (smem + (size_t)static_smem.load() > (size_t)maxs) return MB_UNSUPPORTED;
   if (groups == 0) return MB_OK;
-  MB_CUDA_TRY(pdl_launch(zf_chol_kernel<T, KP>, groups, 256, smem, st, csi, precoder, M, K, status, cond));
+  MB_CUDA_TRY(pdl_launch(zf_chol_kernel<T, KP, KG>, groups, 256, smem, st, csi, precoder, M, K, status, cond));
   MB_LAUNCH_CHECK();
   return MB_OK;
 }
@@ -287,10 +290,16 @@ mb_status zf_chol(float2 *csi, float2 *precoder, uint32_t groups, uint32_t M,
                   cudaStream_t st) {
   const size_t smem = zf_chol_smem(M, K, dbl);
   if (dbl) {
-    auto f = K <= 16 ? zf_chol_launch<double, 16> : K <= 32 ? zf_chol_launch<double, 32> : zf_chol_launch<double, 64>;
+    auto f = K <= 16   ? zf_chol_launch<double, 16>
+             : K <= 32 ? zf_chol_launch<double, 32>
+             : K <= 48 ? zf_chol_launch<double, 64, 48>
+                       : zf_chol_launch<double, 64>;
     return f(csi, precoder, groups, M, K, smem, status, cond, st);
   }
-  auto f = K <= 16 ? zf_chol_launch<float, 16> : K <= 32 ? zf_chol_launch<float, 32> : zf_chol_launch<float, 64>;
+  auto f = K <= 16   ? zf_chol_launch<float, 16>
+           : K <= 32 ? zf_chol_launch<float, 32>
+           : K <= 48 ? zf_chol_launch<float, 64, 48>
+                     : zf_chol_launch<float, 64>;
   return f(csi, precoder, groups, M, K, smem, status, cond, st);
 }
 

@@ -15,7 +15,7 @@ def _csi(G, M, K, seed):
 
 @pytest.mark.parametrize("prec", ["fp32", "fp64"])
 @pytest.mark.parametrize("M,K", [(1, 1), (3, 2), (8, 5), (33, 16), (40, 17), (64, 32), (65, 33), (100, 50), (256, 64),
-                                 (300, 7), (513, 16), (64, 63)])
+                                 (300, 7), (513, 16), (64, 63), (96, 47), (96, 48), (96, 49)])
 def test_zf_edges(prec, M, K):
     if not torch.cuda.is_available():
         pytest.skip("no CUDA device")
