@@ -277,9 +277,9 @@ mb_status mb_equalize(const mb_c32 *W, const mb_c32 *y, uint32_t K,
  * same contract and outputs as mb_equalize): BF16 W and y, FP32
  * accumulation (tcgen05.mma), the same FP16 demapper and layouts.  The
  * caller provides two device scratch buffers whose sizes
- * mb_equalize_tc_scratch returns (neither may be NULL; this build rounds W
- * and y to BF16 on their way into shared memory and leaves the buffers as
- * they are).  Requires sg % 8 == 0 and K <= 64. */
+ * mb_equalize_tc_scratch returns.  Neither may be NULL; since W and y are
+ * rounded to BF16 on their way into shared memory the sizes are 16 bytes and
+ * the buffers stay as they are (larger ones do as well).  Requires sg % 8 == 0 and K <= 64. */
 mb_status mb_equalize_tc_scratch(uint32_t K, uint32_t M, uint32_t S,
                                  uint32_t sg, uint32_t n_sym,
                                  uint64_t *img_bytes, uint64_t *ylp_bytes);

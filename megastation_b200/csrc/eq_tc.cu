@@ -474,17 +474,15 @@ mb_status equalize_tc_c32(const EqParams &p, int *err, cudaStream_t st) {
 
 using namespace mb;
 
-static uint32_t s_pad_of(uint32_t S) { return (S + 7) / 8 * 8; }
-
 extern "C" mb_status mb_equalize_tc_scratch(uint32_t K, uint32_t M, uint32_t S, uint32_t sg,
                                             uint32_t n_sym, uint64_t *img_bytes,
                                             uint64_t *ylp_bytes) {
   if (!img_bytes || !ylp_bytes) return MB_BAD_ARG;
   if (K == 0 || K > 64 || M == 0 || S == 0 || sg == 0) return MB_BAD_SHAPE;
-  const TcShape s = tc_shape(M, K);
-  const uint32_t G = (S + sg - 1) / sg;
-  *img_bytes = (uint64_t)G * s.img_group_bytes;
-  *ylp_bytes = (uint64_t)n_sym * 2 * M * s_pad_of(S) * 2;
+  // W and y are rounded on their way into shared memory: what is left of the
+  // images and planar rows that stood here is that the pointers are not NULL
+  *img_bytes = 16;
+  *ylp_bytes = n_sym ? 16 : 0;
   return MB_OK;
 }
 

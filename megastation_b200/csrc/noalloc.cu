@@ -16,7 +16,9 @@
 namespace {
 
 // The entry point's limit: the BF16 operands of one symbol (detector images
-// of all groups and one symbol's rows) fit in 32 MiB.
+// of all groups and one symbol's rows) fit in 32 MiB.  No buffer of that size
+// stands behind it any more; it stays because hosts choose between this entry
+// point and mb_equalize_tc by its MB_TOO_LARGE.
 constexpr uint64_t kNoAllocScratchBytes = 32ull << 20;
 // The error word of this entry point's kernels (bit 1: a bounded mbarrier
 // wait gave up), fixed because the library's own error word is allocated on

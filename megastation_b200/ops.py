@@ -10,6 +10,7 @@ computes on the host.
 """
 import ctypes
 import functools
+import operator
 
 import torch
 
@@ -324,6 +325,8 @@ class Equalize:
                               hp, sp, xp, _stream(stream)), "Equalize.equalize")
 
 
+    # (kept by the numbers alone: an array or tensor would be kept by what it was, or
+    # not be taken at all)
     @staticmethod
     @functools.lru_cache(maxsize=64)
     def _tc_scratch(K, M, S, sg, n_sym):
@@ -340,7 +343,7 @@ class Equalize:
         M, K = csi.shape[-2], csi.shape[-1]
         S = bsVec.shape[-1]
         n_sym = bsVec.numel() // (M * S)
-        img, ylp = Equalize._tc_scratch(K, M, S, csi_skip, n_sym)
+        img, ylp = Equalize._tc_scratch(K, M, S, operator.index(csi_skip), n_sym)
         s_img = torch.empty(img, dtype=torch.uint8, device=csi.device)
         s_ylp = torch.empty(ylp, dtype=torch.uint8, device=csi.device)
         cb_stride = ueVec.shape[-1]
