@@ -37,8 +37,17 @@ def test_zf_edges(prec, M, K):
     kappa = float(torch.linalg.cond(A).max())
     eps = 2.0 ** -24 if prec == "fp32" else 2.0 ** -24  # FP64 results are stored in FP32
     bound = (K + M) * eps * (kappa if prec == "fp32" else 1.0)
-    err = (d.cpu().to(torch.complex128) - ref).norm() / ref.norm()
+    got = d.cpu().to(torch.complex128)
+    err = (got - ref).norm() / ref.norm()
     assert float(err) <= max(bound, 4 * eps)
+    if prec == "fp32":
+        # The forward bound says little once kappa is large ((64, 63): 1e4, 9%); the residual of A W = C does not
+        # grow with it: the Gram's M roundings, the elimination's K and the two products' 2 K, of eps each and of
+        # either sign (so their root), relative to |A| |W|.  Seen: 1e-7 at (64, 63), 3.2e-7 at (513, 16).
+        X = got.transpose(1, 2)
+        res = (A @ X - Ch).flatten(1).norm(dim=1)
+        size = torch.linalg.matrix_norm(A, 2) * X.flatten(1).norm(dim=1)
+        assert (res <= (M + 3 * K) ** 0.5 * eps * size).all()
     assert (status.cpu() == 0).all()
     # (max / min pivot) of L D L^H is below the condition number
     assert (cond.cpu() <= 1.01 * kappa + 1e-3).all() and (cond.cpu() >= 0.99).all()
