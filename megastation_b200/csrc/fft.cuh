@@ -36,7 +36,7 @@ mb_status fft_tc_uplink_lp(const FftTcPlan *plan, const void *iq, int iq_dtype, 
                            uint32_t upc = 0);
 // pilot FFT of n_sym comb-pilot symbols into csi [G][M][K] as mb_fft_pilot,
 // with the short-last-group fill when tail_rem != 0 (fft_pilot_fill)
-bool fft_tc_pilot_supported(const FftTcPlan *plan, const void *iq);
+bool fft_tc_pilot_supported(const FftTcPlan *plan, const void *iq, uint32_t sg);
 mb_status fft_tc_pilot(const FftTcPlan *plan, const void *iq, int iq_dtype, uint32_t n_sym, uint32_t M, uint32_t S,
                        uint32_t K, uint32_t sg, uint32_t ue_start, uint32_t tail_rem, const float2 *pilot,
                        float2 *csi, int *err, cudaStream_t st, uint32_t upc = 0);

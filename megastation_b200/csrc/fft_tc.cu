@@ -87,7 +87,7 @@ struct FtParams {
   float2 *csi;          // pilot: [G][M][K]
   const float2 *pilot;  // pilot: sign of each subcarrier
   uint32_t K, sg, ue_start, tail_rem, G;
-  uint32_t sg_magic;    // ceil(2^32 / sg): floor(i / sg) = umulhi(i, sg_magic) for i < 2^13; 0: sg = 1
+  uint32_t sg_magic;    // ceil(2^32 / sg), sg > 1: floor(i / sg) = umulhi(i, sg_magic) for i < 2^13
   const uint8_t *mats;
   const float2 *tw;
   uint32_t c;
@@ -532,7 +532,7 @@ __global__ void __launch_bounds__(Fmt<DT>::kThreads, 1)
 #pragma unroll
           for (int j = 0; j < 8; j++) {
             const uint32_t sc = (s_base + 64 * (jb + j)) & (kFtN - 1);
-            const uint32_t g = p.sg_magic ? __umulhi(sc, p.sg_magic) : sc, sl = sc - g * p.sg, uu = u0 + sl;
+            const uint32_t g = __umulhi(sc, p.sg_magic), sl = sc - g * p.sg, uu = u0 + sl;
             const float x = vr[j] * inv, y = vi[j] * inv;
             const float2 e = make_float2(x * ps[j].x + y * ps[j].y, x * ps[j].y - y * ps[j].x);
             if (sc < p.S && uu < p.K) {
@@ -885,14 +885,16 @@ mb_status fft_tc_inverse(const FftTcPlan *pl, const void *in, int in_dtype, uint
   return fft_tc_launch(pl, in, in_dtype, p, st, 0);
 }
 
-bool fft_tc_pilot_supported(const FftTcPlan *pl, const void *iq) {
-  return pl && (reinterpret_cast<uintptr_t>(iq) & 15) == 0;
+// sg = 1 goes to the FP32 kernel: its reciprocal does not fit 32 bits, and a
+// select in the epilogue cost every other group size 2% (1024 rows of int16)
+bool fft_tc_pilot_supported(const FftTcPlan *pl, const void *iq, uint32_t sg) {
+  return pl && (reinterpret_cast<uintptr_t>(iq) & 15) == 0 && sg != 1;
 }
 
 mb_status fft_tc_pilot(const FftTcPlan *pl, const void *iq, int iq_dtype, uint32_t n_sym, uint32_t M, uint32_t S,
                        uint32_t K, uint32_t sg, uint32_t ue_start, uint32_t tail_rem, const float2 *pilot,
                        float2 *csi, int *err, cudaStream_t st, uint32_t upc) {
-  if (!fft_tc_pilot_supported(pl, iq) || S > kFtN || sg == 0 || sg >= kFtN || !pilot || !csi) return MB_BAD_ARG;
+  if (!fft_tc_pilot_supported(pl, iq, sg) || S > kFtN || sg == 0 || sg >= kFtN || !pilot || !csi) return MB_BAD_ARG;
   if (n_sym == 0 || M == 0) return MB_OK;
   FtParams p{};
   p.rows = n_sym * M;
@@ -905,7 +907,7 @@ mb_status fft_tc_pilot(const FftTcPlan *pl, const void *iq, int iq_dtype, uint32
   p.ue_start = ue_start;
   p.tail_rem = tail_rem;
   p.G = (S + sg - 1) / sg;
-  p.sg_magic = sg > 1 ? 0xFFFFFFFFu / sg + 1 : 0;
+  p.sg_magic = 0xFFFFFFFFu / sg + 1;
   p.err = err;
   p.pilot_rows = p.rows;
   return fft_tc_launch(pl, iq, iq_dtype, p, st, upc);
@@ -914,7 +916,7 @@ mb_status fft_tc_pilot(const FftTcPlan *pl, const void *iq, int iq_dtype, uint32
 mb_status fft_tc_slot(const FftTcPlan *pl, const void *iq, int iq_dtype, uint32_t P, uint32_t U, uint32_t M,
                       uint32_t S, uint32_t K, uint32_t sg, uint32_t tail_rem, const float2 *pilot, float2 *csi,
                       void *y_lp, uint32_t S_pad, int *err, cudaStream_t st, uint32_t upc) {
-  if (!fft_tc_lp_supported(pl, iq, S_pad, y_lp) || S > kFtN || S > S_pad || sg == 0 || sg >= kFtN || !pilot ||
+  if (!fft_tc_lp_supported(pl, iq, S_pad, y_lp) || S > kFtN || S > S_pad || sg <= 1 || sg >= kFtN || !pilot ||
       !csi)
     return MB_BAD_ARG;
   FtParams p{};
@@ -932,7 +934,7 @@ mb_status fft_tc_slot(const FftTcPlan *pl, const void *iq, int iq_dtype, uint32_
   p.ue_start = 0;
   p.tail_rem = tail_rem;
   p.G = (S + sg - 1) / sg;
-  p.sg_magic = sg > 1 ? 0xFFFFFFFFu / sg + 1 : 0;
+  p.sg_magic = 0xFFFFFFFFu / sg + 1;
   p.err = err;
   return fft_tc_launch(pl, iq, iq_dtype, p, st, upc);
 }
