@@ -19,8 +19,9 @@
 // the FP16 range, and the scale is undone exactly before the BF16 store.
 //
 // One CTA per SM takes every gridDim-th unit of two rows.  Samples of up to 4
-// bytes run through two pipelines of eight compute warps, complex floats
-// through one of sixteen.  A pipeline has a GEMM operand buffer, an output
+// bytes run through two pipelines of eight compute warps where a CTA has units
+// for both, complex floats and short launches through one of sixteen (the rule
+// is at fft_tc_launch).  A pipeline has a GEMM operand buffer, an output
 // staging buffer, an input ring and 256 TMEM columns (the two GEMM
 // accumulators); F is shared.  Its copy warp streams the units' rows into the
 // ring with 128-byte-swizzled TMA boxes (so the conversion reads are free of
@@ -112,18 +113,23 @@ struct Fmt {
   static constexpr uint32_t kBoxes = kBytes / 2;      // 128-byte boxes per 64-sample n1 row
   static constexpr uint32_t kPPC = kBytes / 2;        // 16-byte pieces per 8-sample chunk
   static constexpr uint32_t kUnitBytes = 2 * kFtN * kBytes;
-  // Independent pipelines per CTA.  One pipeline's 16 warps pass through the
-  // phases of a unit together and wait together for each GEMM and copy (issue
-  // slots half idle); two of eight warps each fill one another's waits.  The
-  // operand, ring and staging buffers of two fit beside F for samples of up
-  // to 4 bytes; complex floats, whose units take 64 KB and whose launch is
-  // near the copy rate as it is, keep one.
-  static constexpr uint32_t kNG = DT == MB_IQ_C32 ? 1 : 2;
-  static constexpr uint32_t kRing = DT == MB_IQ_C32 ? 131072 : 32768;  // a pipeline's ring
-  static constexpr uint32_t kSlots = kRing / kUnitBytes;               // units in it: two, or one of 4-byte samples
-  static constexpr uint32_t kGT = kFtCompute / kNG;                    // a pipeline's compute threads
-  static constexpr uint32_t kThreads = kFtCompute + 64 * kNG;          // + its GEMM and copy warps
-  static constexpr uint32_t kSmem = kMat + kNG * (kMat + kRing + kStgBytes);  // F, then operands, rings, staging
+};
+
+// NG independent pipelines per CTA.  One pipeline's 16 warps pass through the
+// phases of a unit together and wait together for each GEMM and copy (issue
+// slots half idle); two of eight warps each fill one another's waits.  The
+// operand, ring and staging buffers of two fit beside F for samples of up
+// to 4 bytes; complex floats, whose units take 64 KB and whose launch is
+// near the copy rate as it is, have one only.
+template <int DT, int NG>
+struct Pipes : Fmt<DT> {
+  static_assert(NG == 1 || DT != MB_IQ_C32, "two rings of complex floats do not fit");
+  static constexpr uint32_t kNG = NG;
+  static constexpr uint32_t kRing = NG == 1 ? 2 * Fmt<DT>::kUnitBytes : 32768;  // a pipeline's ring
+  static constexpr uint32_t kSlots = kRing / Fmt<DT>::kUnitBytes;  // units in it: two, or one of 4-byte samples
+  static constexpr uint32_t kGT = kFtCompute / NG;                 // a pipeline's compute threads
+  static constexpr uint32_t kThreads = kFtCompute + 64 * NG;       // + its GEMM and copy warps
+  static constexpr uint32_t kSmem = kMat + NG * (kMat + kRing + kStgBytes);  // F, then operands, rings, staging
 };
 
 // integer samples have a known range: a fixed scale instead of the row maximum
@@ -226,12 +232,12 @@ __device__ __forceinline__ bool ft_wait(uint64_t *bar, uint32_t parity, volatile
   return true;
 }
 
-template <int DT>
-__global__ void __launch_bounds__(Fmt<DT>::kThreads, 1)
+template <int DT, int NG_>
+__global__ void __launch_bounds__(Pipes<DT, NG_>::kThreads, 1)
     fft_tc_kernel(const __grid_constant__ CUtensorMap in_map, const FtParams p) {
   extern __shared__ __align__(1024) uint8_t ft_smem[];
   pdl_wait();
-  using F = Fmt<DT>;
+  using F = Pipes<DT, NG_>;
   constexpr uint32_t NG = F::kNG;
   // Each barrier completes once per unit of its pipeline.  a_ready comes as a
   // pair, waited with parity (i >> 1) & 1: the copy warp may trail the
@@ -738,21 +744,24 @@ __global__ void __launch_bounds__(Fmt<DT>::kThreads, 1)
 }
 
 using FtKernel = void (*)(const CUtensorMap, const FtParams);
-FtKernel fft_tc_kernel_of(int dt) {
+struct FtVariant {
+  FtKernel kernel;
+  uint32_t threads, smem;
+};
+template <int DT, int NG>
+FtVariant fft_tc_variant() {
+  return {fft_tc_kernel<DT, NG>, Pipes<DT, NG>::kThreads, Pipes<DT, NG>::kSmem};
+}
+FtVariant fft_tc_variant_of(int dt, bool two) {
   switch (dt) {
-    case MB_IQ_C32: return fft_tc_kernel<MB_IQ_C32>;
-    case MB_IQ_I16: return fft_tc_kernel<MB_IQ_I16>;
-    case MB_IQ_I8: return fft_tc_kernel<MB_IQ_I8>;
-    default: return fft_tc_kernel<MB_IQ_F16>;
+    case MB_IQ_C32: return fft_tc_variant<MB_IQ_C32, 1>();
+    case MB_IQ_I16: return two ? fft_tc_variant<MB_IQ_I16, 2>() : fft_tc_variant<MB_IQ_I16, 1>();
+    case MB_IQ_I8: return two ? fft_tc_variant<MB_IQ_I8, 2>() : fft_tc_variant<MB_IQ_I8, 1>();
+    default: return two ? fft_tc_variant<MB_IQ_F16, 2>() : fft_tc_variant<MB_IQ_F16, 1>();
   }
 }
 
-uint32_t fft_tc_smem_of(int dt) {
-  return dt == MB_IQ_C32 ? Fmt<MB_IQ_C32>::kSmem : dt == MB_IQ_I16 ? Fmt<MB_IQ_I16>::kSmem
-         : dt == MB_IQ_I8 ? Fmt<MB_IQ_I8>::kSmem : Fmt<MB_IQ_F16>::kSmem;
-}
-
-// raises the dynamic shared memory limit of a sample type's kernel once per
+// raises the dynamic shared memory limit of a sample type's kernels once per
 // device, and returns the device's SM count
 mb_status fft_tc_configure(int dt, int dev, int *sms) {
   static std::atomic<uint64_t> configured[4] = {};
@@ -760,8 +769,10 @@ mb_status fft_tc_configure(int dt, int dev, int *sms) {
   const int which = dt == MB_IQ_C32 ? 0 : dt == MB_IQ_I16 ? 1 : dt == MB_IQ_I8 ? 2 : 3;
   const uint64_t bit = 1ull << (dev & 63);
   if (!(configured[which].load() & bit)) {
-    MB_CUDA_TRY(cudaFuncSetAttribute(fft_tc_kernel_of(dt), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)fft_tc_smem_of(dt)));
+    for (int two = 0; two < 2; two++) {
+      const FtVariant v = fft_tc_variant_of(dt, two);
+      MB_CUDA_TRY(cudaFuncSetAttribute(v.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)v.smem));
+    }
     int n = 0;
     MB_CUDA_TRY(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev));
     sm_count[dev & 63].store(n);
@@ -789,8 +800,16 @@ mb_status fft_tc_launch(const FftTcPlan *pl, const void *iq, int iq_dtype, FtPar
   p.units = (p.rows + 1) / 2;
   p.upc = upc ? upc : (p.units + (uint32_t)max(sms, 1) - 1) / (uint32_t)max(sms, 1);
   const uint32_t grid = (p.units + p.upc - 1) / p.upc;
-  const uint32_t threads = iq_dtype == MB_IQ_C32 ? Fmt<MB_IQ_C32>::kThreads : Fmt<MB_IQ_I8>::kThreads;
-  MB_CUDA_TRY(pdl_launch(fft_tc_kernel_of(iq_dtype), grid, threads, fft_tc_smem_of(iq_dtype), st, map, p));
+  // Two pipelines need units for both: a CTA's only unit is through sooner with
+  // all 16 warps (up to 296 rows, two / one: pilots int8 8.0 / 7.35 us, int16 8.5 /
+  // 7.75; inverse from FP16 8.7 / 7.2), and so are three units of 4-byte samples,
+  // of which one pipeline would take two, but for BF16 rows (600 rows: pilots
+  // int16 16.0 / 15.5, inverse 14.9 / 13.8, uplink int16 11.4 / 11.6; int8 pilots
+  // 14.65 / 14.75).
+  const bool lp_rows = !p.inverse && p.pilot_rows < p.rows;
+  const bool two = p.upc > 1 && !(p.upc == 3 && bytes == 4 && !lp_rows);
+  const FtVariant v = fft_tc_variant_of(iq_dtype, two);
+  MB_CUDA_TRY(pdl_launch(v.kernel, grid, v.threads, v.smem, st, map, p));
   MB_LAUNCH_CHECK();
   return MB_OK;
 }

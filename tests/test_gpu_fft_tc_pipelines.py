@@ -57,3 +57,23 @@ def test_inverse_rows(mb, M, D):
     got = torch.view_as_complex(out.double())
     rms = ref.abs().square().mean(-1, keepdim=True).sqrt()
     assert ((got - ref).abs() <= 2.0 ** -10 * ref.abs() + 2e-3 * rms).all()
+
+
+# one unit a CTA and three of 4-byte samples take one pipeline, the others two
+@pytest.mark.parametrize("M,P", [(5, 1), (37, 8), (33, 9), (199, 3), (211, 5)])
+@pytest.mark.parametrize("dtype", [torch.int8, torch.int16, torch.float16])
+def test_pilot_rows(mb, dtype, M, P):
+    """The LS estimates against the FP32 operator's: 2e-3 of the rows' RMS
+    (FP16 operands; the pilots have unit modulus, the rows one power)."""
+    sg, g = 16, torch.Generator(device="cuda").manual_seed(M + P)
+    full = {torch.int8: 128, torch.int16: 32768}.get(dtype)
+    iq = torch.randint(-full, full, (P, M, N, 2), generator=g, device="cuda").to(dtype) if full else \
+        torch.randn(P, M, N, 2, generator=g, device="cuda").to(dtype)
+    op = mb.PilotFFT((N - S) // 2, N, S, M, sg * P, sg)
+    ref, got = (torch.zeros(-(-S // sg), M, sg * P, dtype=torch.complex64, device="cuda") for _ in range(2))
+    op(iq, ref)
+    op.mixed(iq, got)
+    torch.cuda.synchronize()
+    assert mb.ops.device_error() == 0
+    rms = ref.abs().square().mean().sqrt()  # within 10% of each row's
+    assert float(rms) > 0 and float((got - ref).abs().max()) <= 2e-3 * float(rms) * 1.1
