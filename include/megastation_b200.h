@@ -519,8 +519,10 @@ mb_status mb_cells_set_fft_ctas(mb_cells *cells, const uint32_t *fft_ctas);
  * its matrix products when K <= 32 -- 0 by K (the tensor cores for
  * 16 < K, the CUDA cores below; the default), 1 the CUDA cores, 2 the
  * tensor cores (tcgen05, split-BF16 operands, FP32 accumulation; its
- * round trips cost more than a small group's products).  mb_cells_autotune
- * tries the choice the rule did not make per class, last. */
+ * round trips cost more than a small group's products).  With 0 and 1 a cell
+ * of K <= 16 without a learned start runs the direct FP32 solve in place of
+ * the tensor-core kernel, as long as a group's CSI fits in shared memory.
+ * mb_cells_autotune tries the choice the rule did not make per class, last. */
 mb_status mb_cells_get_zf_path(const mb_cells *cells, uint32_t *zf_path);
 mb_status mb_cells_set_zf_path(mb_cells *cells, const uint32_t *zf_path);
 mb_status mb_cells_set_tuning(mb_cells *cells, const uint32_t *sym_batch,

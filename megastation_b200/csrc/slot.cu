@@ -39,7 +39,7 @@ struct mb_slot {
   uint32_t eq_cols;   // tensor-core equalizer columns per CTA (0: 128)
   uint32_t fft_ctas;  // CTAs of each tensor-core FFT launch (0: fft_share)
   uint32_t fft_share = 0;  // this cell's share of the SMs among batched cells (0: one CTA per SM)
-  uint32_t zf_path;   // mixed ZF, K <= 32: 0 by K, 1 CUDA-core products, 2 tensor-core products
+  uint32_t zf_path;   // mixed ZF, K <= 32: 0 by K, 1 CUDA cores (K <= 16: the direct solve), 2 tensor-core products
   mb_ldpc *ldpc = nullptr;  // decode stage's code (not owned), or null
   uint32_t ldpc_iters = 0;
   // downlink from information bits: the scrambled bits [D][K][info bytes]

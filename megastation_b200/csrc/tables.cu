@@ -237,7 +237,7 @@ extern "C" mb_status mb_device_error(int *out, int clear) {
   MB_CUDA_TRY(cudaDeviceSynchronize());
   MB_CUDA_TRY(cudaMemcpy(out, t->err, sizeof(int), cudaMemcpyDeviceToHost));
   if (clear) MB_CUDA_TRY(cudaMemset(t->err, 0, sizeof(int)));
-  int na = 0;  // the fixed-scratch equalizer keeps its own word
+  int na = 0;  // mb_equalize_tc_noalloc keeps its own word
   const mb_status s = noalloc_error_word(&na, clear != 0);
   if (s != MB_OK) return s;
   *out |= na;
