@@ -67,30 +67,20 @@ __device__ __forceinline__ void cfma(float2 &acc, float2 a, float2 b) {
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // launch of a kernel that calls pdl_wait(); what precedes it in the stream may
-// be anything.  carveout: the share of an SM's memory asked for as shared
-// memory, in percent, the rest being L1 (negative: the driver's choice, as much
-// as the most resident CTAs take)
+// be anything
 template <typename... P, typename... A>
-inline cudaError_t pdl_launch_carveout(int carveout, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
-                                       cudaStream_t st, A &&...args) {
-  cudaLaunchAttribute at[2]{};
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  at[1].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
-  at[1].val.sharedMemCarveout = (unsigned)carveout;
+inline cudaError_t pdl_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A &&...args) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t c{};
   c.gridDim = grid;
   c.blockDim = block;
   c.dynamicSmemBytes = smem;
   c.stream = st;
-  c.attrs = at;
-  c.numAttrs = carveout < 0 ? 1 : 2;
+  c.attrs = &at;
+  c.numAttrs = 1;
   return cudaLaunchKernelEx(&c, kernel, std::forward<A>(args)...);
-}
-
-template <typename... P, typename... A>
-inline cudaError_t pdl_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A &&...args) {
-  return pdl_launch_carveout(-1, kernel, grid, block, smem, st, std::forward<A>(args)...);
 }
 
 inline cudaStream_t as_stream(void *s) { return reinterpret_cast<cudaStream_t>(s); }

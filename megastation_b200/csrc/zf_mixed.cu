@@ -1339,7 +1339,6 @@ static mb_status zf_mixed_launch(float2 *csi, void *img_w, uint32_t groups, uint
   MB_CUDA_TRY(cudaDeviceGetAttribute(&maxs, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
   static std::atomic<uint64_t> configured[6] = {};
   static std::atomic<int> static_smem[6] = {};
-  static std::atomic<int> sm_count[64] = {}, sm_smem[64] = {};
   int which = 0;
   const ZfmKernel kern = zfm_kernel_of(s.MM, qmf, &which);
   const uint64_t bit = 1ull << (dev & 63);
@@ -1349,11 +1348,6 @@ static mb_status zf_mixed_launch(float2 *csi, void *img_w, uint32_t groups, uint
     MB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      maxs - (int)fa.sharedSizeBytes));
     static_smem[which] = (int)fa.sharedSizeBytes;
-    int sms = 0, per_sm = 0;
-    MB_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    MB_CUDA_TRY(cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
-    sm_count[dev & 63] = sms;
-    sm_smem[dev & 63] = per_sm;
     configured[which].fetch_or(bit);
   }
   const size_t avail = (size_t)maxs - (size_t)static_smem[which].load();
@@ -1370,16 +1364,7 @@ static mb_status zf_mixed_launch(float2 *csi, void *img_w, uint32_t groups, uint
   }
   if (smem > avail) return MB_UNSUPPORTED;
   if (groups == 0) return MB_OK;
-  // 32 < K <= 64, no more groups than SMs: shared memory for one CTA and the
-  // rest as L1, where the FP64 solve's columns (1 KB a thread) then stay; with
-  // room for a second CTA, which never comes, they went to L2 (75 groups of 64 x
-  // 64, all in FP64: 425 us against 294, of 128 x 64 480 against 373)
-  int carveout = -1;
-  if (s.MM == 128 && groups <= (uint32_t)sm_count[dev & 63].load()) {
-    const size_t need = smem + (size_t)static_smem[which].load() + 1024, all = (size_t)sm_smem[dev & 63].load();
-    carveout = (int)std::min<size_t>(100, (need * 100 + all - 1) / all);
-  }
-  MB_CUDA_TRY(pdl_launch_carveout(carveout, kern, groups, kThreads, smem, st, q, ymap));
+  MB_CUDA_TRY(pdl_launch(kern, groups, kThreads, smem, st, q, ymap));
   MB_LAUNCH_CHECK();
   return MB_OK;
 }
