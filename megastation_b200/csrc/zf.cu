@@ -72,7 +72,7 @@ __global__ void __launch_bounds__(256)
   __syncthreads();
   zf_gram<T, KG>(Cs, A, M, K, ldc, lda);
   __syncthreads();
-  ldl_eliminate<T, KP>(A, lda, K, &not_pd);
+  ldl_eliminate<T, KP>(A, lda, K, &not_pd, A);
   const bool bad = not_pd != 0;
   ldl_products<T>(A, Cs, M, K, ldc, lda);
 

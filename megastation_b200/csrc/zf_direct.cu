@@ -35,6 +35,12 @@ struct ZfdParams {
   float cond_thr;
 };
 
+// bytes of C, or of the FP64 solve's tile (at least its two pivot buffers)
+__host__ __device__ __forceinline__ uint32_t zfd_c_bytes(uint32_t M, uint32_t K) {
+  const uint32_t c = (K * (M + 1) * (uint32_t)sizeof(float2) + 15) / 16 * 16, t = zf_fp64_tile_bytes(K);
+  return c > t ? c : t > 512 ? t : 512;
+}
+
 // the largest of a block's values; red: 8 floats
 __device__ __forceinline__ float block_max(float v, float *red) {
   for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
@@ -85,6 +91,14 @@ __device__ __forceinline__ void product_bf16(const float2 *Xt, Cplx<float> *Cs, 
   }
 }
 
+// a call: in line it would take the kernel's 64 registers a thread with it (spills
+// of 340 bytes a thread instead of 72)
+__device__ __noinline__ Fp64Group fp64_group_call(float2 *cg, uint8_t *img, double2 *Gd, double2 *Ct, uint32_t T,
+                                                  int *flag, uint32_t M, uint32_t K, uint32_t Mp, uint32_t MM,
+                                                  uint32_t nkt) {
+  return zf_fp64_group<16>(cg, img, Gd, Ct, T, flag, M, K, Mp, MM, nkt);
+}
+
 __global__ void __launch_bounds__(256, 4) zf_direct_kernel(const ZfdParams q) {
   extern __shared__ __align__(16) unsigned char zd_smem[];
   pdl_wait();
@@ -92,9 +106,10 @@ __global__ void __launch_bounds__(256, 4) zf_direct_kernel(const ZfdParams q) {
   constexpr int KP = 16;
   constexpr uint32_t TPR = 256 / KP;  // threads per row of A
   const uint32_t g = blockIdx.x, M = q.M, K = q.K, ldc = M + 1, lda = K + 1, tid = threadIdx.x;
-  // C [K][M+1], then room for A [K][K+1] in FP64 (FP32 uses half of it)
+  // C [K][M+1] (or the FP64 solve's tile of it), then room for A [K][K+1] in
+  // FP64 (FP32 uses half of it)
   C *Cs = reinterpret_cast<C *>(zd_smem);
-  double2 *Ad = reinterpret_cast<double2 *>(zd_smem + ((size_t)K * ldc * sizeof(C) + 15) / 16 * 16);
+  double2 *Ad = reinterpret_cast<double2 *>(zd_smem + zfd_c_bytes(M, K));
   C *A = reinterpret_cast<C *>(Ad);
   __shared__ __align__(16) float2 Xt[KP * KP];  // X transposed, rounded to BF16
   __shared__ float2 Gm[KP * (KP + 1)], Xm[KP * (KP + 1)], Tm[KP * (KP + 1)];  // Newton-Schulz, zero padded
@@ -118,7 +133,7 @@ __global__ void __launch_bounds__(256, 4) zf_direct_kernel(const ZfdParams q) {
   };
   const float2 gij = in ? make_float2(A[i * lda + j].x, A[i * lda + j].y) : make_float2(0.f, 0.f);
   const float a1 = norm1(gij);
-  ldl_eliminate<float, KP>(A, lda, K, &not_pd);
+  ldl_eliminate<float, KP>(A, lda, K, &not_pd, A);
   float cond = INFINITY;
   int st = 2;
   if (!not_pd) {  // uniform
@@ -201,7 +216,11 @@ __global__ void __launch_bounds__(256, 4) zf_direct_kernel(const ZfdParams q) {
       }
     }
   } else {
-    st = zf_fp64_group<KP>(cg, img, Ad, &not_pd, M, K, q.Mp, q.MM, q.nkt, mx);
+    // half as many antennas in FP64 as C has in FP32, an odd number
+    const uint32_t T = max(kFp64Tile, ((M + 1) / 2 - 1) | 1u);
+    const Fp64Group r = fp64_group_call(cg, img, Ad, reinterpret_cast<double2 *>(Cs), T, &not_pd, M, K, q.Mp, q.MM, q.nkt);
+    st = r.status;
+    mx = r.wmax;
   }
   if (q.wmax) {
     mx = block_max(mx, red);
@@ -215,8 +234,7 @@ __global__ void __launch_bounds__(256, 4) zf_direct_kernel(const ZfdParams q) {
 
 size_t zfd_smem(uint32_t M, uint32_t K) {
   // the pivot buffers of a small A reach past it (two of 16 entries)
-  const size_t c = ((size_t)K * (M + 1) * sizeof(float2) + 15) / 16 * 16;
-  return c + std::max<size_t>((size_t)K * (K + 1) * sizeof(double2), 2 * 16 * sizeof(float2));
+  return zfd_c_bytes(M, K) + std::max<size_t>((size_t)K * (K + 1) * sizeof(double2), 2 * 16 * sizeof(float2));
 }
 
 }  // namespace

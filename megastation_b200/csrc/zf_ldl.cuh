@@ -93,11 +93,11 @@ __device__ __forceinline__ void zf_gram(const Cplx<T> *Cs, Cplx<T> *A, uint32_t 
 // L^{-1} strictly below it (what lies above is scratch).  The row of thread t is t / TPR, its
 // columns t % TPR + TPR m in registers, rotated by one slot every TPR pivots
 // so that the pivot column always sits in slot 0; the pivot row goes through
-// shared memory, two buffers of KP at the head of A (free while the rows are
-// in registers; a small A's buffers run on into the 1 KB behind it): one
-// barrier a pivot.
+// shared memory, two buffers of KP at prow (A itself will do, free while the
+// rows are in registers; a small A's buffers run on into the 1 KB behind it):
+// one barrier a pivot.  *not_pd = 1 when a pivot is not positive.
 template <typename T, int KP>
-__device__ __forceinline__ void ldl_eliminate(Cplx<T> *A, uint32_t lda, uint32_t K, int *not_pd) {
+__device__ __forceinline__ void ldl_eliminate(Cplx<T> *A, uint32_t lda, uint32_t K, int *not_pd, Cplx<T> *prow) {
   constexpr int TPR = 256 / KP, NC = KP / TPR > 0 ? KP / TPR : 1;
   const uint32_t i = threadIdx.x / TPR, sub = threadIdx.x % TPR;
   Cplx<T> v[NC];
@@ -116,7 +116,7 @@ __device__ __forceinline__ void ldl_eliminate(Cplx<T> *A, uint32_t lda, uint32_t
         Cplx<T> f;  // this row's entry in column k
         f.x = __shfl_sync(0xffffffffu, v[0].x, s, TPR);
         f.y = __shfl_sync(0xffffffffu, v[0].y, s, TPR);
-        Cplx<T> *pr = A + (k & 1) * KP;
+        Cplx<T> *pr = prow + (k & 1) * KP;
         if (i == k) {
           T d = f.x;
           if (!(d > (T)0)) {

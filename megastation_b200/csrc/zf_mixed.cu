@@ -1101,8 +1101,14 @@ __global__ void __launch_bounds__(kThreads, 2)
 
   // ------------------------------------------------- FP64 fallback groups
   if (!fail && st == 2) {
-    // Gd reuses Gs and Xs (2 K*ld float2)
-    st = zf_fp64_group<64>(cg, imgw, reinterpret_cast<double2 *>(Gs), &flag, M, K, Mp, MM, q.nkt, wmx);
+    // Gd reuses Gs and Xs (2 K*ld float2), the tile of C the iterate's images
+    // (MM == 64: 16 KB) or the lo tiles (MM == 128: 32 KB)
+    const Fp64Group r =
+        zf_fp64_group<MM / 2>(cg, imgw, reinterpret_cast<double2 *>(Gs),
+                              reinterpret_cast<double2 *>(MM == 64 ? y_img : lo_base), kFp64Tile, &flag, M, K, Mp, MM, q.nkt);
+    st = r.status;
+    wmx = r.wmax;
+    static_assert(zf_fp64_tile_bytes(32) <= 2 * kSqImg && zf_fp64_tile_bytes(64) <= 2 * 128 * kKT * 2, "");
   }
 
   if (q.wmax) {

@@ -46,6 +46,6 @@ def test_dependent_kernels_wait_before_anything_else():
             assert re.match(r"(extern\s+)?__shared__|constexpr|using|static_assert|namespace", line), f"{k}: {line!r}"
     launched = set()
     for _, text in texts:
-        for m in re.finditer(r"pdl_launch(?:_carveout)?\(", text):
+        for m in re.finditer(r"pdl_launch\(", text):
             launched |= {w for w in re.findall(r"\b(\w+_kernel)\b", text[m.end():m.end() + 160])}
     assert len(launched) > 10 and launched <= waiting, launched - waiting

@@ -1,6 +1,6 @@
-"""Mixed-precision zero forcing of 33 to 64 users: the FP64 solve and the
-learned start, in launches of fewer and of more groups than SMs (which differ in
-how an SM's memory is split), against FP64 and against one another."""
+"""Mixed-precision zero forcing: the FP64 solve at the edges of its tiles of
+antennas and of its paddings of users, and the learned start of 33 to 64 users, in
+launches of fewer and of more groups than SMs, against FP64 and one another."""
 import numpy as np
 import pytest
 import torch
@@ -44,7 +44,9 @@ def _twice(mb, C, **kw):
     return a.to(torch.complex128), sa
 
 
-@pytest.mark.parametrize("M,K", [(64, 33), (64, 48), (64, 64), (70, 50), (130, 64)])
+# tiles of 31 antennas (up to 16 users: half as many as the CSI's, an odd number)
+@pytest.mark.parametrize("M,K", [(2, 2), (31, 5), (62, 16), (63, 7), (257, 16), (31, 17), (93, 32), (94, 31), (64, 33),
+                                 (64, 48), (64, 64), (70, 50), (130, 64)])
 def test_fp64_groups(mb, M, K):
     C = _csi(5, M, K)
     C[3, :, K - 1] = 0  # no channel: W = 0
