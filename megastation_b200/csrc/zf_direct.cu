@@ -91,14 +91,6 @@ __device__ __forceinline__ void product_bf16(const float2 *Xt, Cplx<float> *Cs, 
   }
 }
 
-// a call: in line it would take the kernel's 64 registers a thread with it (spills
-// of 340 bytes a thread instead of 72)
-__device__ __noinline__ Fp64Group fp64_group_call(float2 *cg, uint8_t *img, double2 *Gd, double2 *Ct, uint32_t T,
-                                                  int *flag, uint32_t M, uint32_t K, uint32_t Mp, uint32_t MM,
-                                                  uint32_t nkt) {
-  return zf_fp64_group<16>(cg, img, Gd, Ct, T, flag, M, K, Mp, MM, nkt);
-}
-
 __global__ void __launch_bounds__(256, 4) zf_direct_kernel(const ZfdParams q) {
   extern __shared__ __align__(16) unsigned char zd_smem[];
   pdl_wait();
@@ -218,7 +210,7 @@ __global__ void __launch_bounds__(256, 4) zf_direct_kernel(const ZfdParams q) {
   } else {
     // half as many antennas in FP64 as C has in FP32, an odd number
     const uint32_t T = max(kFp64Tile, ((M + 1) / 2 - 1) | 1u);
-    const Fp64Group r = fp64_group_call(cg, img, Ad, reinterpret_cast<double2 *>(Cs), T, &not_pd, M, K, q.Mp, q.MM, q.nkt);
+    const Fp64Group r = zf_fp64_group_call<KP, 64>(cg, img, Ad, reinterpret_cast<double2 *>(Cs), T, &not_pd, M, K);
     st = r.status;
     mx = r.wmax;
   }

@@ -35,8 +35,8 @@ struct Fp64Group {
 // share them.  A thread per antenna with its column in local memory walked K^2
 // dependent steps, from L2 where two CTAs left an SM little L1 (and shared memory
 // cut to one CTA, 294 us, kept other launches off the SM: six cells of 33 to 64
-// users 234 -> 295 us).  75 groups, all in FP64, before / now: 64 x 64 425 / 185
-// us, 128 x 64 480 / 221, 128 x 32 131 / 76, 256 x 16 66 / 53.
+// users 234 -> 295 us).  75 groups, all in FP64, before / now: 64 x 64 425 / 189
+// us, 128 x 64 480 / 226, 128 x 32 133 / 80, 256 x 16 66 / 53.
 template <int KP>
 __device__ __forceinline__ Fp64Group zf_fp64_group(float2 *cg, uint8_t *imgw, double2 *Gd, double2 *Ct, uint32_t T,
                                                    int *flag, uint32_t M, uint32_t K, uint32_t Mp, uint32_t MM,
@@ -114,7 +114,7 @@ __device__ __forceinline__ Fp64Group zf_fp64_group(float2 *cg, uint8_t *imgw, do
     const uint32_t n = min(T, M - b0);
     if (pd) {
       load(b0, n);
-      ldl_products<double>(A, Cs, n, K, T, lda);
+      ldl_products<double, KP <= 32 ? 1 : 4>(A, Cs, n, K, T, lda);  // (unrolled, the callers of the call spill)
     }
     each(n, [&](uint32_t e, uint32_t tb, uint32_t u) {
       const uint32_t b = b0 + tb;
@@ -130,6 +130,18 @@ __device__ __forceinline__ Fp64Group zf_fp64_group(float2 *cg, uint8_t *imgw, do
     __syncthreads();
   }
   return {pd ? 2 : 1, wmx};
+}
+
+// The same as a call, which leaves the caller's registers alone: in line
+// zf_direct.cu's kernel spills 340 bytes a thread instead of 72 and zf_mixed.cu's
+// for up to 32 users 44 instead of none. With more users that kernel has it in
+// line (205 groups of 256 x 64: 166.7 us a pass of pilots, detector and precoder, 168.7
+// as a call).
+template <int KP, uint32_t MM>
+__device__ __noinline__ Fp64Group zf_fp64_group_call(float2 *cg, uint8_t *imgw, double2 *Gd, double2 *Ct, uint32_t T,
+                                                     int *flag, uint32_t M, uint32_t K) {
+  const uint32_t Mp = (M + kZfTile - 1) / kZfTile * kZfTile;  // as tc_shape()
+  return zf_fp64_group<KP>(cg, imgw, Gd, Ct, T, flag, M, K, Mp, MM, 2 * Mp / kZfTile);
 }
 
 }  // namespace mb

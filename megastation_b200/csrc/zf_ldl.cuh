@@ -167,8 +167,9 @@ __device__ __forceinline__ void ldl_eliminate(Cplx<T> *A, uint32_t lda, uint32_t
 // (part, column b), `cols` columns and `parts` blocks side by side.
 // Z = L^{-1} C from the last rows up (a row reads the rows above it), then
 // L^{-H} D^{-1} Z from the first rows down; the barriers keep the blocks of one
-// round, whose rows read one another's old values, apart.
-template <typename T>
+// round, whose rows read one another's old values, apart.  U steps of a row are
+// unrolled.
+template <typename T, int U = 4>
 __device__ __forceinline__ void ldl_products(const Cplx<T> *A, Cplx<T> *Cs, uint32_t M, uint32_t K, uint32_t ldc,
                                              uint32_t lda) {
   using C = Cplx<T>;
@@ -190,7 +191,7 @@ __device__ __forceinline__ void ldl_products(const Cplx<T> *A, Cplx<T> *Cs, uint
         const C *l[4];
 #pragma unroll
         for (int q = 0; q < 4; q++) l[q] = A + min(i0 + q, K - 1) * lda;
-#pragma unroll 4
+#pragma unroll U
         for (uint32_t k = 0; k < i0; k++) {
           const C c = Cs[k * ldc + b];
 #pragma unroll
@@ -244,7 +245,7 @@ __device__ __forceinline__ void ldl_products(const Cplx<T> *A, Cplx<T> *Cs, uint
             z[q].y += w.x * c.y - w.y * c.x;
           }
         }
-#pragma unroll 4
+#pragma unroll U
         for (uint32_t k = i0 + 4; k < K; k++) {
           const C c = Cs[k * ldc + b];
 #pragma unroll

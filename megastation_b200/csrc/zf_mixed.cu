@@ -28,8 +28,8 @@
 //     tensor-core equalizer consumes (eq_tc.cu); the plane-1 half is P D0.
 //     The epilogue stores that image (BF16) and W in the CSI layout (FP32).
 //  4. Groups whose Gram is not positive definite in FP32, or whose condition
-//     estimate exceeds cond_threshold, are redone in FP64 (Gram, Cholesky,
-//     solve) and reported with status 2 (1 if even FP64 fails).
+//     estimate exceeds cond_threshold, are redone in FP64 (Gram, L D L^H,
+//     products) and reported with status 2 (1 if even FP64 fails).
 #include <algorithm>
 #include <atomic>
 #include <cstring>
@@ -1103,9 +1103,10 @@ __global__ void __launch_bounds__(kThreads, 2)
   if (!fail && st == 2) {
     // Gd reuses Gs and Xs (2 K*ld float2), the tile of C the iterate's images
     // (MM == 64: 16 KB) or the lo tiles (MM == 128: 32 KB)
-    const Fp64Group r =
-        zf_fp64_group<MM / 2>(cg, imgw, reinterpret_cast<double2 *>(Gs),
-                              reinterpret_cast<double2 *>(MM == 64 ? y_img : lo_base), kFp64Tile, &flag, M, K, Mp, MM, q.nkt);
+    double2 *Gd = reinterpret_cast<double2 *>(Gs), *Ct = reinterpret_cast<double2 *>(MM == 64 ? y_img : lo_base);
+    Fp64Group r;
+    if constexpr (MM == 64) r = zf_fp64_group_call<32, 64>(cg, imgw, Gd, Ct, kFp64Tile, &flag, M, K);
+    else r = zf_fp64_group<64>(cg, imgw, Gd, Ct, kFp64Tile, &flag, M, K, Mp, MM, q.nkt);
     st = r.status;
     wmx = r.wmax;
     static_assert(zf_fp64_tile_bytes(32) <= 2 * kSqImg && zf_fp64_tile_bytes(64) <= 2 * 128 * kKT * 2, "");
