@@ -175,13 +175,14 @@ mb_status mb_ifft_downlink_mixed(mb_fft *fft, const void *in, int in_dtype, uint
 /* ------------------------------------------------------- zero forcing --- */
 /* Replaces Beamform (beamform/beamform.h:27-84). */
 typedef enum {
-  /* FP32 Gram + FP32 Cholesky + triangular solves: the reference's math
-   * (cuBLAS Cgemm + cuSOLVER potrf/potrs, beamform.cu:74-122) */
+  /* FP32 Gram + FP32 L D L^H (Cholesky without the square roots) and the
+   * products with L^{-1}, for the reference's cuBLAS Cgemm + cuSOLVER
+   * potrf/potrs (beamform.cu:74-122) */
   MB_ZF_FP32 = 0,
   /* BF16 Gram on tensor cores (FP32 accumulate), FP32 inverse refined by
-   * Newton-Schulz, FP64 Cholesky for groups above cond_threshold */
+   * Newton-Schulz, FP64 L D L^H for groups above cond_threshold */
   MB_ZF_MIXED = 1,
-  /* FP64 Cholesky for every group */
+  /* FP64 L D L^H for every group */
   MB_ZF_FP64 = 2
 } mb_zf_precision;
 

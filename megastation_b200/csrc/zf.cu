@@ -4,11 +4,11 @@
 // CgemmStridedBatched for the Gram C C^H, cusolverDnCpotrfBatched and
 // cusolverDnCpotrsBatched with G*M single right-hand sides) with ONE CTA per
 // subcarrier group that keeps C in shared memory for the whole solve: Gram,
-// Cholesky, the M triangular solves and the write-back of W = (C C^H)^{-1} C
-// in the CSI layout.  The downlink precoder P = W^T / max|W|
+// L D L^H (Cholesky without the square roots) with L^{-1}, the products of
+// W = (C C^H)^{-1} C with it and the write-back in the CSI layout.  The downlink precoder P = W^T / max|W|
 // (beam_utils.cuh:40-80) can be emitted from the same CTA.
 //
-// FP32 (MB_ZF_FP32) follows the reference's arithmetic; FP64 (MB_ZF_FP64)
+// FP32 (MB_ZF_FP32) has the reference's precision; FP64 (MB_ZF_FP64)
 // runs the same schedule in double.  Unlike the reference, which ignores
 // cuSOLVER's info array, a non positive definite Gram is reported per group
 // (status 1) and its W is zeroed.
@@ -96,7 +96,7 @@ __global__ void __launch_bounds__(256)
   }
   if (status && tid == 0) status[g] = bad ? 1 : 0;
   if (cond_out && tid == 0) {
-    // cheap estimate from the Cholesky diagonal: (max l_ii / min l_ii)^2
+    // cheap estimate from the pivots: max d_ii / min d_ii
     T lo = A[0].x, hi = A[0].x;
     for (uint32_t i = 1; i < K; i++) {
       T d = A[i * lda + i].x;

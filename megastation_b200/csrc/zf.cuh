@@ -10,7 +10,7 @@ namespace mb {
 // copies users without a pilot in a short last group from group G-2
 mb_status zf_fill_tail(float2 *csi, uint32_t groups, uint32_t S, uint32_t sg,
                        uint32_t M, uint32_t K, cudaStream_t st);
-// Cholesky ZF in FP32 or FP64, W in place; optional fused precoder
+// L D L^H ZF in FP32 or FP64, W in place; optional fused precoder
 mb_status zf_chol(float2 *csi, float2 *precoder, uint32_t groups, uint32_t M,
                   uint32_t K, bool dbl, int32_t *status, float *cond,
                   cudaStream_t st);
